@@ -110,14 +110,6 @@ __global__ void init_layout_kernel(uint64_t *keys, uint8_t *vals) {
     }
 }
 
-__global__ void guard_keys_kernel(uint64_t *keys, uint8_t *vals, uint32_t row_num) {
-    // init_gpma_insertions (gpma.cuh:70-78): (r << 32) | 0xFFFFFFFF, value 1
-    for (uint32_t r = blockIdx.x * blockDim.x + threadIdx.x; r < row_num; r += gridDim.x * blockDim.x) {
-        keys[r] = ((uint64_t)r << 32) + COL_NONE;
-        vals[r] = 1;
-    }
-}
-
 __global__ void mask_values_kernel(const uint64_t *keys, const uint8_t *vals, uint8_t *out, uint32_t size) {
     for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < size; t += gridDim.x * blockDim.x)
         out[t] = keys[t] == KEY_NONE ? 0 : vals[t];
@@ -342,25 +334,21 @@ gpma_status gpma_create(uint32_t row_num, void *stream, gpma_graph **out) {
         GPMA_CUDA(cudaGetDevice(&g->device));
         GPMA_CUDA(cudaDeviceGetAttribute(&g->sms, cudaDevAttrMultiProcessorCount, g->device));
         g->row_num = row_num;
+        GPMA_TRY(dev_alloc(&g->row_offset, (uint64_t)row_num + 1));
+        if (row_num > 0)
+            return create_array(g, s);
         g->cap = 4;
         GPMA_TRY(dev_alloc(&g->keys, 4));
         GPMA_TRY(dev_alloc(&g->values, 4));
-        GPMA_TRY(dev_alloc(&g->row_offset, (uint64_t)row_num + 1));
         GPMA_TRY(ensure_scratch(g, 4));
-        GPMA_CUDA(cudaMemsetAsync(g->row_offset, 0, sizeof(uint32_t) * ((uint64_t)row_num + 1), s));
+        GPMA_CUDA(cudaMemsetAsync(g->row_offset, 0, sizeof(uint32_t), s));
         init_layout_kernel<<<1, 32, 0, s>>>(g->keys, g->values);
         GPMA_CUDA(cudaGetLastError());
         g->geo.size = 4;
         g->geo.seg = 2;
         g->geo.height = 1;
         recalculate_density(g->geo);
-        GPMA_TRY(refresh_heads(g, s));
-        if (row_num == 0)
-            return GPMA_OK;
-        GPMA_TRY(ensure_buffers(g->buf, row_num, 1));
-        guard_keys_kernel<<<small_grid(row_num, g->sms), BLOCK, 0, s>>>(g->buf.bkeys[0], g->buf.bvals[0], row_num);
-        GPMA_CUDA(cudaGetLastError());
-        return update_device(g, row_num, s, /*check_keys=*/false);  // the guards use the reserved column
+        return refresh_heads(g, s);
     }();
     if (st != GPMA_OK) {
         release(g);
@@ -399,13 +387,13 @@ gpma_status gpma_update(gpma_graph *g, const uint64_t *keys, const uint8_t *valu
     cudaStream_t s = (cudaStream_t)stream;
     GPMA_TRY(ensure_buffers(g->buf, n, 1));
     if (is_device_pointer(keys) && is_device_pointer(values))
-        return update_device(g, n, s, true, keys, values);  // the kernel reads the caller's batch in place
+        return update_device(g, n, s, keys, values);  // the kernel reads the caller's batch in place
     {
         // page-locked host batches: the kernel reads them over the host link
         // itself (the keys twice: ranks, then the scatter), no staging copy
         const void *dk = mapped_host_pointer(keys), *dv = mapped_host_pointer(values);
         if (dk && dv)
-            return update_device(g, n, s, true, static_cast<const uint64_t *>(dk), static_cast<const uint8_t *>(dv));
+            return update_device(g, n, s, static_cast<const uint64_t *>(dk), static_cast<const uint8_t *>(dv));
     }
     GPMA_TRY(copy_in(g, g->buf.bkeys[0], keys, n * sizeof(uint64_t), s));
     GPMA_TRY(copy_in(g, g->buf.bvals[0], values, n, s));
@@ -591,7 +579,7 @@ gpma_status gpma_batch_update(gpma_batch *b, gpma_graph *const *graphs, const ui
         GPMA_TRY(copy_in(graphs[i], b->buf.bkeys[0] + off[j], keys[i], counts[i] * sizeof(uint64_t), s));
         GPMA_TRY(copy_in(graphs[i], b->buf.bvals[0] + off[j], values[i], counts[i], s));
     }
-    return update_graphs(gs.data(), off.data(), (uint32_t)gs.size(), b->buf, b->sms, s, true, b->profiling, b->ev,
+    return update_graphs(gs.data(), off.data(), (uint32_t)gs.size(), b->buf, b->sms, s, b->profiling, b->ev,
                          &b->prof);
 }
 
@@ -638,7 +626,7 @@ gpma_status gpma_batch_update_packed(gpma_batch *b, gpma_graph *const *graphs, c
     GPMA_TRY(packed_stage(b, P, keys, values, offsets, s));
     GPMA_CUDA(P.gather.launch(s));
     b->prof.kernel_launches += 1;
-    return update_graphs(P.gs.data(), P.off.data(), P.m, b->buf, b->sms, s, true, b->profiling, b->ev, &b->prof);
+    return update_graphs(P.gs.data(), P.off.data(), P.m, b->buf, b->sms, s, b->profiling, b->ev, &b->prof);
 }
 
 gpma_status gpma_batch_bfs_multi(gpma_batch *b, gpma_graph *const *graphs, const uint32_t *const *srcs,

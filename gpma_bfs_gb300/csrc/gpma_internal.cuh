@@ -398,16 +398,19 @@ gpma_status ensure_scratch(gpma_graph *g, uint32_t slots);
 // Recomputes heads[s] = keys[s * seg] over the whole array (after the array
 // was written outside the level loop: creation, root rebuild, load).
 gpma_status refresh_heads(gpma_graph *g, cudaStream_t s);
+// The first array (row guards and initial entries) of a graph whose row_num,
+// row_offset and sms are set.
+gpma_status create_array(gpma_graph *g, cudaStream_t s);
 // Segments whose heads entry differs from the array (0 when consistent).
 gpma_status count_bad_heads(gpma_graph *g, cudaStream_t s, uint64_t *bad);
 // One launch updating graphs[0..k) with the batches already staged in
 // buf.bkeys[0]/bvals[0] at offsets off[0..k]. Graphs must be ordered by
-// segment length. check_keys=false only for the internal guard insertion.
+// segment length.
 // in_k / in_v: the batch in device memory elsewhere (read in place) instead.
 gpma_status update_graphs(gpma_graph *const *graphs, const uint64_t *off, uint32_t k, BatchBuffers &buf, int sms,
-                          cudaStream_t s, bool check_keys, bool profiling, cudaEvent_t *ev, gpma_profile *prof,
+                          cudaStream_t s, bool profiling, cudaEvent_t *ev, gpma_profile *prof,
                           const uint64_t *in_k = nullptr, const uint8_t *in_v = nullptr);
-gpma_status update_device(gpma_graph *g, uint64_t n, cudaStream_t s, bool check_keys = true,
+gpma_status update_device(gpma_graph *g, uint64_t n, cudaStream_t s,
                           const uint64_t *in_k = nullptr, const uint8_t *in_v = nullptr);
 // The three host parts of update_graphs, for callers that enqueue the launch
 // themselves (a CUDA graph step). update_plan sizes the buffers, fills the
@@ -423,7 +426,7 @@ gpma_status update_device(gpma_graph *g, uint64_t n, cudaStream_t s, bool check_
 // in_k / in_v (device, optional): the batch is read from there instead of
 // buf.bkeys[0] / buf.bvals[0] (which the sort then only writes).
 gpma_status update_plan(gpma_graph *const *graphs, const uint64_t *off, uint32_t k, BatchBuffers &buf, int sms,
-                        bool check_keys, size_t *tab_bytes, KernelLaunch *L, const uint32_t *abort = nullptr,
+                        size_t *tab_bytes, KernelLaunch *L, const uint32_t *abort = nullptr,
                         const uint64_t *in_k = nullptr, const uint8_t *in_v = nullptr);
 gpma_status update_clear(BatchBuffers &buf, cudaStream_t s);
 size_t update_status_bytes(uint32_t k);

@@ -44,10 +44,10 @@ constexpr uint32_t SORT_VALUE_MASK = (1u << 30) - 1;
 
 // Histograms of all 8 digits into hist[g][8][256] for each graph g < G and
 // the totals into hist[G][8][256] (zeroed by the caller); sets
-// st->invalid_keys when check_keys and a reserved column occurs. Each CTA
+// st->invalid_keys when a reserved column occurs. Each CTA
 // walks a contiguous key range graph by graph.
 __device__ __forceinline__ void sort_histogram(const uint64_t *__restrict__ keys, const uint32_t *boff, uint32_t G,
-                                               uint32_t *hist, DeviceStatus *st, bool check_keys, uint32_t *sh) {
+                                               uint32_t *hist, DeviceStatus *st, uint32_t *sh) {
     const uint32_t n = boff[G];
     const uint32_t per = (n + gridDim.x - 1) / gridDim.x;
     const uint32_t lo = min(n, blockIdx.x * per), hi = min(n, lo + per);
@@ -77,7 +77,7 @@ __device__ __forceinline__ void sort_histogram(const uint64_t *__restrict__ keys
         }
         pos = end;
     }
-    if (__syncthreads_or(bad) && check_keys && threadIdx.x == 0)
+    if (__syncthreads_or(bad) && threadIdx.x == 0)
         atomicOr(&st->invalid_keys, 1u);
 }
 
@@ -326,7 +326,7 @@ __device__ __forceinline__ uint32_t graph_at(const uint32_t *boff, uint32_t G, u
 
 // Q1: ranks and buckets (and the reserved-column check of the digit histogram).
 __device__ void bsort_rank(const uint64_t *keys, const uint32_t *boff, uint32_t G, const GraphDesc *gd,
-                           const BucketSort &Q, DeviceStatus *st, bool check_keys) {
+                           const BucketSort &Q, DeviceStatus *st) {
     uint32_t lo, hi;
     bsort_range(boff[G], lo, hi);
     uint32_t bad = 0, g = 0xFFFFFFFFu;
@@ -361,7 +361,7 @@ __device__ void bsort_rank(const uint64_t *keys, const uint32_t *boff, uint32_t 
             }
         }
     }
-    if (__syncthreads_or(bad) && check_keys && threadIdx.x == 0)
+    if (__syncthreads_or(bad) && threadIdx.x == 0)
         atomicOr(&st->invalid_keys, 1u);
 }
 

@@ -260,7 +260,7 @@ gpma_status step_run(gpma_step *st, const uint64_t *keys, const uint8_t *values,
         gpma_graph *gl[1] = {g};
         size_t tab_bytes = 0;
         KernelLaunch upd;
-        GPMA_TRY(update_plan(gl, off, 1, g->buf, g->sms, true, &tab_bytes, &upd));
+        GPMA_TRY(update_plan(gl, off, 1, g->buf, g->sms, &tab_bytes, &upd));
         BfsPlan bp;
         const bool profiling = g->profiling;
         g->profiling = false;  // no per-level stamps inside a recorded step
@@ -490,7 +490,7 @@ gpma_status batch_step_run(gpma_batch_step *st, const uint64_t *keys, const uint
     GPMA_TRY(packed_stage(b, pp, keys, values, offsets, s, /*with_table=*/false));
     size_t tab_bytes = 0;
     KernelLaunch upd;
-    GPMA_TRY(update_plan(pp.gs.data(), pp.off.data(), pp.m, b->buf, b->sms, true, &tab_bytes, &upd));
+    GPMA_TRY(update_plan(pp.gs.data(), pp.off.data(), pp.m, b->buf, b->sms, &tab_bytes, &upd));
     BatchBfsPlan bp;
     GPMA_TRY(batch_bfs_plan(b, graphs, srcs, nsrc, k, nullptr, &bp));
     if (!st->exec || bake_batch(b, pp, tab_bytes, upd, bp) != st->baked) {
@@ -583,7 +583,7 @@ gpma_status batch_step_run_many(gpma_batch_step *st, uint32_t S, const uint64_t 
         b->buf.parity = p0;
         for (uint32_t t = 0; t < S; ++t) {
             GPMA_TRY(packed_plan(b, graphs, keys[t], values[t], off_of(t), k, &pp[t], M.d_abort));
-            GPMA_TRY(update_plan(pp[t].gs.data(), pp[t].off.data(), pp[t].m, b->buf, b->sms, true, &tabb[t], &upd[t],
+            GPMA_TRY(update_plan(pp[t].gs.data(), pp[t].off.data(), pp[t].m, b->buf, b->sms, &tabb[t], &upd[t],
                                  M.d_abort));
             parity[t] = b->buf.parity;
             b->buf.parity ^= 1;

@@ -87,7 +87,6 @@ struct UpdateArgs {
     uint32_t *sort_tiles;   // 8 tile counters (zeroed per update)
     uint32_t *sort_status;  // look-back words, 8 x tiles x 256 (zeroed per update)
     BucketSort q;           // bucket sort state (q.nq == 0: digit passes only)
-    bool check_keys;
     uint32_t *leaf;
     uint64_t *ikeys[2];
     uint8_t *ivals[2];
@@ -1008,7 +1007,7 @@ __global__ void __launch_bounds__(BLOCK, MINB) update_kernel(UpdateArgs A) {
     const uint8_t *bv = A.bv[1];
     bool digits = A.q.nq == 0;
     if (!digits) {
-        bsort_rank(A.in_k, A.boff, A.G, A.gd, A.q, st, A.check_keys);
+        bsort_rank(A.in_k, A.boff, A.G, A.gd, A.q, st);
         if (!grid_barrier(&st->bar, &st->err, A.stall, A.stall_limit_ns))
             return;
         if (ld_volatile(&st->invalid_keys) != 0)
@@ -1030,7 +1029,7 @@ __global__ void __launch_bounds__(BLOCK, MINB) update_kernel(UpdateArgs A) {
         }
     }
     if (digits) {
-        sort_histogram(A.in_k, A.boff, A.G, A.sort_hist, st, A.check_keys, reinterpret_cast<uint32_t *>(smem));
+        sort_histogram(A.in_k, A.boff, A.G, A.sort_hist, st, reinterpret_cast<uint32_t *>(smem));
         if (!grid_barrier(&st->bar, &st->err, A.q.nq == 0 ? A.stall : 0u, A.stall_limit_ns))
             return;
         if (ld_volatile(&st->invalid_keys) != 0)
@@ -2209,6 +2208,43 @@ __global__ void compacted_layout_kernel(uint64_t *keys, uint8_t *vals, uint64_t 
     }
 }
 
+// The array of a new graph: the row guards and the two KEY_MAX entries of the
+// initial 4-slot array, redispatched (M = row_num + 2 elements, gap_key in the
+// gaps) or, where that many do not fit the root's density (dropped), the two
+// KEY_MAX entries alone at the front. The guards are in key order as they are
+// numbered, so every slot is written from its index: one pass of coalesced
+// 16-byte stores. Before, the guards went through the batch update, whose sort
+// finds them all in one bucket (1.6M atomics on one word, 7.1 ms for 1,632,803
+// rows); creating that graph and loading 15.3M edges went from 16.2 to 7.2 ms.
+__global__ void guard_layout_kernel(uint64_t *keys, uint8_t *vals, uint64_t *heads, uint32_t *row_offset,
+                                    uint32_t row_num, uint32_t size, uint32_t log2seg, uint32_t log2F,
+                                    uint64_t gap_key, bool dropped) {
+    const uint64_t M = (uint64_t)row_num + 2;
+    const uint32_t seg_mask = (1u << log2seg) - 1;
+    if (blockIdx.x == 0 && threadIdx.x == 0)
+        row_offset[0] = 0;
+    // a thread writes slots 2 p and 2 p + 1: one segment (segments hold 2 slots or more)
+    for (uint32_t p = blockIdx.x * blockDim.x + threadIdx.x; p < size >> 1; p += gridDim.x * blockDim.x) {
+        const uint32_t slot = 2 * p, s = slot >> log2seg, ln = slot & seg_mask;
+        uint64_t f0 = seg_first(s, M, log2F), f1 = seg_first(s + 1, M, log2F);
+        uint64_t k[2];
+        uint32_t v[2];
+#pragma unroll
+        for (uint32_t j = 0; j < 2; ++j) {
+            const uint64_t i = dropped ? row_num + (uint64_t)(slot + j) : f0 + ln + j;
+            const bool have = dropped ? slot + j < 2 : ln + j < f1 - f0;
+            k[j] = !have ? gap_key : i < row_num ? (i << 32) | COL_NONE : KEY_MAX;
+            v[j] = have ? 1u : 0u;
+            if (have && i < row_num)
+                row_offset[i + 1] = slot + j;
+        }
+        *reinterpret_cast<ulonglong2 *>(keys + slot) = make_ulonglong2(k[0], k[1]);
+        *reinterpret_cast<uint16_t *>(vals + slot) = (uint16_t)(v[0] | (v[1] << 8));
+        if (ln == 0)
+            heads[s] = k[0];
+    }
+}
+
 __global__ void heads_kernel(const uint64_t *keys, uint64_t *heads, uint32_t segs, uint32_t log2seg) {
     for (uint32_t s = blockIdx.x * blockDim.x + threadIdx.x; s < segs; s += gridDim.x * blockDim.x)
         heads[s] = keys[(size_t)s << log2seg];
@@ -2226,6 +2262,22 @@ __global__ void heads_check_kernel(const uint64_t *keys, const uint64_t *heads, 
 int grid_for(uint64_t work, int sms, int per_sm) {
     uint64_t g = (work + BLOCK - 1) / BLOCK;
     return (int)std::max<uint64_t>(1, std::min<uint64_t>(g, (uint64_t)sms * per_sm));
+}
+
+// The geometry of an array resized to hold `elements` (gpma.cuh:917-930);
+// false when it would need more than MAX_SLOTS slots.
+bool geometry_for(uint64_t elements, Geometry *geo) {
+    uint64_t tree_size = 4;
+    while (std::floor(UPPER_ROOT * (double)tree_size) < (double)elements) {
+        tree_size *= 2;
+        if (tree_size > MAX_SLOTS)
+            return false;
+    }
+    geo->size = (uint32_t)tree_size;
+    geo->seg = 1u << (fls32(fls32(geo->size)) - 1);
+    geo->height = fls32(geo->size / geo->seg) - 1;
+    recalculate_density(*geo);
+    return true;
 }
 
 // resize_gpma + (root rebalance | significant_insert) of one graph.
@@ -2266,21 +2318,13 @@ gpma_status root_rebuild(gpma_graph *g, bool significant, const uint64_t *pend_k
         return device_error("the compaction of the root rebuild", (uint32_t)h_cst[1]);
     const uint32_t live = (uint32_t)h_cst[0];
     // 2. new geometry (gpma.cuh:917-930)
-    uint64_t merge = (uint64_t)live + pend_n;
-    uint64_t tree_size = 4;
-    while (std::floor(UPPER_ROOT * (double)tree_size) < (double)merge) {
-        tree_size *= 2;
-        if (tree_size > MAX_SLOTS) {
-            set_error("GPMA would need more than 2^31 slots (%llu live + %u insertions)", (unsigned long long)live,
-                      pend_n);
-            return GPMA_ERR_CAPACITY;
-        }
-    }
+    const uint64_t merge = (uint64_t)live + pend_n;
     Geometry geo;
-    geo.size = (uint32_t)tree_size;
-    geo.seg = 1u << (fls32(fls32(geo.size)) - 1);
-    geo.height = fls32(geo.size / geo.seg) - 1;
-    recalculate_density(geo);
+    if (!geometry_for(merge, &geo)) {
+        set_error("GPMA would need more than 2^31 slots (%llu live + %u insertions)", (unsigned long long)live,
+                  pend_n);
+        return GPMA_ERR_CAPACITY;
+    }
     // 3. storage
     if (geo.size > g->cap) {
         uint64_t *nk = nullptr;
@@ -2427,6 +2471,37 @@ const void *update_kernel_ptr(int variant) {
 }
 
 }  // namespace
+
+// The first array of a new graph with row_num >= 1 rows (init_gpma_insertions,
+// gpma.cuh:70-82): what an update of the 4-slot array by all guards leaves.
+// Leaf and root of that array (upper bounds 1 and 2) reject any insertion, so
+// that update always ends in the root rebalance, or, from SIGNIFICANT_INSERTS
+// guards on, in the bulk rebuild; the layout of either is written directly.
+gpma_status create_array(gpma_graph *g, cudaStream_t s) {
+    const uint64_t elements = (uint64_t)g->row_num + 2;
+    if (!geometry_for(elements, &g->geo)) {
+        set_error("GPMA would need more than 2^31 slots (2 live + %u insertions)", g->row_num);
+        return GPMA_ERR_CAPACITY;
+    }
+    const Geometry &geo = g->geo;
+    const uint32_t log2seg = fls32(geo.seg) - 1;
+    GPMA_TRY(dev_alloc(&g->keys, geo.size));
+    GPMA_TRY(dev_alloc(&g->values, geo.size));
+    g->cap = geo.size;
+    GPMA_TRY(dev_alloc(&g->heads, geo.size >> log2seg));
+    g->heads_cap = geo.size >> log2seg;
+    GPMA_TRY(ensure_scratch(g, geo.size));
+    const bool significant = g->row_num >= SIGNIFICANT_INSERTS;
+    const bool dropped = !significant && !(geo.lower[geo.height] <= elements && elements <= geo.upper[geo.height]);
+    if (dropped)
+        GPMA_CUDA(cudaMemsetAsync(g->row_offset, 0, sizeof(uint32_t) * ((uint64_t)g->row_num + 1), s));
+    guard_layout_kernel<<<grid_for(geo.size >> 1, g->sms, 8), BLOCK, 0, s>>>(
+        g->keys, g->values, g->heads, g->row_offset, g->row_num, geo.size, log2seg, fls32(geo.size) - 1 - log2seg,
+        significant ? 0ull : KEY_NONE, dropped);
+    GPMA_CUDA(cudaGetLastError());
+    GPMA_CUDA(cudaStreamSynchronize(s));
+    return GPMA_OK;
+}
 
 gpma_status refresh_heads(gpma_graph *g, cudaStream_t s) {
     const uint32_t log2seg = fls32(g->geo.seg) - 1;
@@ -2653,7 +2728,7 @@ gpma_status ensure_buffers(BatchBuffers &b, uint64_t n, uint32_t graphs) {
 }
 
 gpma_status update_plan(gpma_graph *const *graphs, const uint64_t *off, uint32_t k, BatchBuffers &buf, int sms,
-                        bool check_keys, size_t *tab_bytes, KernelLaunch *L, const uint32_t *abort,
+                        size_t *tab_bytes, KernelLaunch *L, const uint32_t *abort,
                         const uint64_t *in_k, const uint8_t *in_v) {
     static_assert(sizeof(UpdateArgs) <= KernelLaunch::ARG_BYTES, "update arguments exceed the launch record");
     const uint64_t n = off[k];
@@ -2798,7 +2873,6 @@ gpma_status update_plan(gpma_graph *const *graphs, const uint64_t *off, uint32_t
         A.q.rec = reinterpret_cast<uint4 *>(buf.qrec);
         A.q.bound = buf.qbound;
     }
-    A.check_keys = check_keys;
     A.leaf = buf.leaf;
     A.rkeys = buf.rkeys;
     A.rvals = buf.rvals;
@@ -2899,13 +2973,13 @@ bool update_needs_host(const unsigned char *stat, uint32_t k) {
 }
 
 gpma_status update_graphs(gpma_graph *const *graphs, const uint64_t *off, uint32_t k, BatchBuffers &buf, int sms,
-                          cudaStream_t s, bool check_keys, bool profiling, cudaEvent_t *ev, gpma_profile *prof,
+                          cudaStream_t s, bool profiling, cudaEvent_t *ev, gpma_profile *prof,
                           const uint64_t *in_k, const uint8_t *in_v) {
     if (off[k] == 0)
         return GPMA_OK;
     size_t tab_bytes = 0;
     KernelLaunch L;
-    GPMA_TRY(update_plan(graphs, off, k, buf, sms, check_keys, &tab_bytes, &L, nullptr, in_k, in_v));
+    GPMA_TRY(update_plan(graphs, off, k, buf, sms, &tab_bytes, &L, nullptr, in_k, in_v));
     // the tables (descriptors, batch and bucket offsets) are the same from
     // one slide step to the next: an identical table is not uploaded again
     if (!buf.tab_shadow_valid || buf.tab_shadow.size() != tab_bytes ||
@@ -2926,11 +3000,11 @@ gpma_status update_graphs(gpma_graph *const *graphs, const uint64_t *off, uint32
 }
 
 // Single-graph update of the n-key batch staged in g->buf.bkeys[0]/bvals[0].
-gpma_status update_device(gpma_graph *g, uint64_t n, cudaStream_t s, bool check_keys, const uint64_t *in_k,
+gpma_status update_device(gpma_graph *g, uint64_t n, cudaStream_t s, const uint64_t *in_k,
                           const uint8_t *in_v) {
     const uint64_t off[2] = {0, n};
     gpma_graph *gs[1] = {g};
-    return update_graphs(gs, off, 1, g->buf, g->sms, s, check_keys, g->profiling, g->ev, &g->prof, in_k, in_v);
+    return update_graphs(gs, off, 1, g->buf, g->sms, s, g->profiling, g->ev, &g->prof, in_k, in_v);
 }
 
 }  // namespace gpma
