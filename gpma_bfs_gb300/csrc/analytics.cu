@@ -13,12 +13,14 @@
 //   acc[v]    += contrib[u] for every edge (float atomics),
 //   rank'[v]   = (1 - d) / n + d * (acc[v] + dangling / n);
 // it stops after `iterations` or when sum |rank' - rank| < tol.
-// Weakly connected components: parents start as the node ids; every edge
-// hooks the larger of its endpoints' parents under the smaller (atomicMin),
-// then pointer jumping shortens every chain; repeated until no edge hooks.
-// Parents only decrease and stay inside their component, so each node ends
-// labelled with the smallest node id of its component, whatever the order of
-// the atomics.
+// Weakly connected components: parents start as the node ids; an edge links
+// its endpoints' trees by hooking the larger root under the smaller (a
+// compare-and-swap retried from the parents it found), so one sweep over the
+// edges finishes the components. A first pass links the edges in the first few
+// slots of every row and flattens the trees; the sweep then finds most
+// endpoints with equal parents and only reads. Parents only decrease and stay
+// inside their component, so each node ends labelled with the smallest node id
+// of its component, whatever the order of the atomics.
 #include "gpma_internal.cuh"
 
 namespace gpma {
@@ -27,7 +29,7 @@ namespace {
 enum : uint32_t {
     AN_ERR = 0,
     AN_ITERS = 1,
-    AN_CHANGED = 2,  // 3 rotating flags (components)
+    AN_ROOTS = 2,    // components counted
     AN_BAR = 6,      // GridBarrier (2 words)
     AN_DBL = 8,      // doubles from word 8: dangling[3], delta[3]
     AN_WORDS = 8 + 12,
@@ -36,6 +38,7 @@ enum : uint32_t {
 struct AnArgs {
     const uint64_t *keys;
     const uint8_t *vals;
+    const uint32_t *ro;  // row offsets (components)
     uint32_t n, size;
     uint32_t *deg;     // out-degree (PageRank)
     float *rank, *acc, *contrib;
@@ -201,67 +204,132 @@ __global__ void __launch_bounds__(BLOCK) pagerank_kernel(AnArgs A) {
         A.ctl[AN_ITERS] = it;
 }
 
+// Joins the trees of nodes p1 and p2 (any nodes of them): the larger of the
+// two is hooked under the smaller if it is a root, else its parent goes on
+// instead. Parents are read through L1: every walk ends at the same few nodes
+// near the root, and reading those from L2 (240 us against 81 for the second
+// sampled pass), or trying a swap on each node of a walk (7.8 ms for the whole
+// call), serialises there. An old parent is still a node of the tree, and the
+// swap's result is never old. The larger node decreases in every step, so the
+// loop ends.
+__device__ __forceinline__ void cc_link(uint32_t *parent, uint32_t p1, uint32_t p2) {
+    while (p1 != p2) {
+        const uint32_t hi = max(p1, p2), lo = min(p1, p2);
+        uint32_t up = parent[hi];
+        if (up == hi) {
+            up = atomicCAS(&parent[hi], hi, lo);
+            if (up == hi)
+                return;
+        }
+        p1 = up;
+        p2 = parent[lo];
+    }
+}
+
+// Every node of the grid's stride to the root of its (decreasing) chain;
+// returns the roots among them.
+__device__ __forceinline__ uint32_t cc_flatten(uint32_t *parent, uint32_t n, uint32_t gtid, uint32_t nthreads) {
+    uint32_t roots = 0;
+    for (uint32_t v = gtid; v < n; v += nthreads) {
+        const uint32_t first = parent[v];
+        uint32_t p = first;
+        for (uint32_t q = parent[p]; q != p; q = parent[p])
+            p = q;
+        if (p != first)
+            parent[v] = p;
+        roots += p == v;
+    }
+    return roots;
+}
+
+// Slots at the start of every row that the sampled passes look at: the guard
+// of the row before and, at the array's density, the row's first edges.
+constexpr uint32_t CC_SAMPLE = 4;
+
+// Links edge number `which` among the first CC_SAMPLE slots of rows 0, step,
+// 2 * step, ...
+__device__ __forceinline__ void cc_sample(const AnArgs &A, uint32_t which, uint32_t step, uint32_t gtid,
+                                          uint32_t nthreads) {
+    for (uint64_t t = (uint64_t)gtid * step; t < A.n; t += (uint64_t)nthreads * step) {
+        const uint32_t u = (uint32_t)t;
+        const uint32_t r1 = A.ro[u + 1], b = A.ro[u];
+        uint32_t e = min(r1, A.size);
+        if (!in_bounds(A.ctl + AN_ERR, b <= r1 && r1 <= A.size, BS_ROW))
+            e = b;  // an inconsistent row_offset: the row is skipped
+        uint64_t k[CC_SAMPLE];
+        uint32_t val[CC_SAMPLE];
+#pragma unroll
+        for (uint32_t j = 0; j < CC_SAMPLE; ++j) {
+            k[j] = b + j < e ? A.keys[b + j] : KEY_NONE;
+            val[j] = b + j < e ? A.vals[b + j] : 0u;
+        }
+        uint32_t v = u, seen = 0;
+#pragma unroll
+        for (uint32_t j = 0; j < CC_SAMPLE; ++j) {
+            const uint32_t w = (uint32_t)k[j];
+            const bool edge = val[j] != 0 && w < A.n;  // guards and empty slots: w is 0xFFFFFFFF
+            if (edge && seen == which)
+                v = w;
+            seen += edge;
+        }
+        if (v != u)
+            cc_link(A.parent, A.parent[u], A.parent[v]);
+    }
+}
+
+// Bound by the 4-byte parent gathers of the edges' targets (L2) beside one
+// read of the array. Hooking parents found once per round took three sweeps
+// with an atomicMin per edge in the first: 2.11 ms on 15.3M edges, 1.6M nodes
+// (33.5M slots); linking to completion takes one sweep, and few of its edges
+// link anything after the sampled passes, whose trees are flattened after each
+// so that the next pass finds roots with one read: 0.22 ms.
 __global__ void __launch_bounds__(BLOCK) components_kernel(AnArgs A) {
     GridBarrier *bar = reinterpret_cast<GridBarrier *>(A.ctl + AN_BAR);
     uint32_t *err = A.ctl + AN_ERR;
+    __shared__ uint32_t tmp[BLOCK / 32 + 1];
     const uint32_t gtid = blockIdx.x * BLOCK + threadIdx.x, nthreads = gridDim.x * BLOCK;
     const uint32_t groups = A.size >> 3;
     for (uint32_t v = gtid; v < A.n; v += nthreads)
         A.parent[v] = v;
     if (!grid_barrier(bar, err))
         return;
-    uint32_t it = 0;
-    for (;; ++it) {
-        if (blockIdx.x == 0 && threadIdx.x == 0)
-            A.ctl[AN_CHANGED + (it + 1) % 3] = 0;
-        uint32_t changed = 0;
-        // hook: every edge joins its endpoints' parents, the larger under the smaller
-        for (uint32_t o = gtid; o < groups || (A.size < 8 && o == 0); o += nthreads) {
-            uint32_t u[8], v[8];
-            bool e[8];
-            if (A.size < 8)
-                load_small(A, u, v, e);
-            else
-                load8(A, o, u, v, e);
-            uint32_t pu[8], pv[8];
-#pragma unroll
-            for (int j = 0; j < 8; ++j) {
-                pu[j] = e[j] ? A.parent[u[j]] : 0u;
-                pv[j] = e[j] ? A.parent[v[j]] : 0u;
-            }
-#pragma unroll
-            for (int j = 0; j < 8; ++j) {
-                if (e[j] && pu[j] != pv[j]) {
-                    const uint32_t hi = max(pu[j], pv[j]), lo = min(pu[j], pv[j]);
-                    if (atomicMin(&A.parent[hi], lo) > lo)
-                        changed = 1;
-                }
-            }
-            if (A.size < 8)
-                break;
-        }
+    // the first edge of every row, then the second of every 8th row (the large
+    // component forms, with an eighth of the walks that would meet in it; 81 us
+    // without this pass, 64 with it), then of all rows
+    for (uint32_t pass = 0; pass < 3; ++pass) {
+        cc_sample(A, pass > 0, pass == 1 ? 8 : 1, gtid, nthreads);
         if (!grid_barrier(bar, err))
             return;
-        // pointer jumping: every node to the end of its (decreasing) chain
-        for (uint32_t v = gtid; v < A.n; v += nthreads) {
-            uint32_t p = A.parent[v];
-            uint32_t q = A.parent[p];
-            while (q != p) {
-                p = q;
-                q = A.parent[p];
-            }
-            if (A.parent[v] != p)
-                A.parent[v] = p;
-        }
-        if (__syncthreads_or(changed) && threadIdx.x == 0)
-            atomicAdd(A.ctl + AN_CHANGED + it % 3, 1u);
+        cc_flatten(A.parent, A.n, gtid, nthreads);
         if (!grid_barrier(bar, err))
             return;
-        if (cta_broadcast_read(A.ctl + AN_CHANGED + it % 3) == 0)
-            break;
     }
+    for (uint32_t o = gtid; o < groups || (A.size < 8 && o == 0); o += nthreads) {
+        uint32_t u[8], v[8];
+        bool e[8];
+        if (A.size < 8)
+            load_small(A, u, v, e);
+        else
+            load8(A, o, u, v, e);
+        // parents read once (an older parent is still a node of the tree)
+        uint32_t pu[8], pv[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            pu[j] = e[j] ? A.parent[u[j]] : 0u;
+            pv[j] = e[j] ? A.parent[v[j]] : 0u;
+        }
+#pragma unroll
+        for (int j = 0; j < 8; ++j)
+            if (pu[j] != pv[j])
+                cc_link(A.parent, pu[j], pv[j]);
+    }
+    if (!grid_barrier(bar, err))
+        return;
+    const uint32_t roots = block_sum(cc_flatten(A.parent, A.n, gtid, nthreads), tmp);
+    if (threadIdx.x == 0 && roots)
+        atomicAdd(A.ctl + AN_ROOTS, roots);
     if (gtid == 0)
-        A.ctl[AN_ITERS] = it + 1;
+        A.ctl[AN_ITERS] = 1;
 }
 
 int an_fit[64] = {};
@@ -382,22 +450,16 @@ gpma_status gpma_components(gpma_graph *g, uint32_t *labels, uint64_t *component
         AnArgs A{};
         A.keys = g->keys;
         A.vals = g->values;
+        A.ro = g->row_offset;
         A.n = n;
         A.size = g->geo.size;
         A.parent = parent;
         A.ctl = ctl;
         GPMA_TRY(launch((const void *)components_kernel, A, g->sms, s, h_ctl));
-        std::vector<uint32_t> host(n);
-        GPMA_CUDA(cudaMemcpyAsync(host.data(), parent, sizeof(uint32_t) * n, cudaMemcpyDeviceToHost, s));
+        GPMA_TRY(copy_any(labels, parent, sizeof(uint32_t) * n, s));
         GPMA_CUDA(cudaStreamSynchronize(s));
-        GPMA_TRY(copy_any(labels, host.data(), sizeof(uint32_t) * n, s));
-        GPMA_CUDA(cudaStreamSynchronize(s));
-        if (components) {
-            uint64_t c = 0;
-            for (uint32_t v = 0; v < n; ++v)
-                c += host[v] == v;
-            *components = c;
-        }
+        if (components)
+            *components = h_ctl[AN_ROOTS];
         if (rounds)
             *rounds = h_ctl[AN_ITERS];
         g->prof.kernel_launches += 1;

@@ -165,7 +165,7 @@ GPMA_API gpma_status gpma_pagerank(gpma_graph *g, float damping, uint32_t iterat
 /* Weakly connected components: labels (host or device, row_num entries)
  * receives, for every node, the smallest node id of its component (exact and
  * deterministic); components (optional) the number of components, isolated
- * nodes included; rounds (optional) the hook-and-jump rounds run. */
+ * nodes included; rounds (optional) the sweeps over all edges that were run. */
 GPMA_API gpma_status gpma_components(gpma_graph *g, uint32_t *labels, uint64_t *components, uint32_t *rounds,
                                      void *stream);
 

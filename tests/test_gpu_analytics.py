@@ -79,3 +79,49 @@ def test_analytics_on_device_outputs_and_empty_edges(built_lib):
     G.pagerank(g, 0.85, 5, out=r)
     np.testing.assert_allclose(r.cpu().numpy(), np.full(100, 0.01), rtol=1e-5)
     g.close()
+
+
+def _labels(n, s, d):
+    """Smallest node id of each node's component, by label propagation with pointer jumping."""
+    lab = np.arange(n)
+    while True:
+        new = lab.copy()
+        np.minimum.at(new, s, lab[d])
+        np.minimum.at(new, d, lab[s])
+        new = new[new]
+        if np.array_equal(new, lab):
+            return lab
+        lab = new
+
+
+@pytest.mark.parametrize("shape", ["one", "pair", "path_up", "path_down", "star", "late_edges", "sparse"])
+def test_components_link_shapes(built_lib, shape):
+    """Tree shapes at the edges of the linking: arrays of 4 slots, long chains in
+    both id orders, one hub, rows whose only joining edges lie behind the sampled
+    slots, many small components; deleted edges link nothing."""
+    import gpma_bfs_gb300 as G
+
+    rng = np.random.default_rng(5)
+    n = {"one": 1, "pair": 2, "star": 3001, "sparse": 5000}.get(shape, 4097)
+    i = np.arange(n - 1)
+    s, d = {
+        "one": (i, i),
+        "pair": (np.array([1]), np.array([0])),
+        "path_up": (i, i + 1),
+        "path_down": (i + 1, i),
+        "star": (np.full(n - 1, n - 1), i),
+        "late_edges": (i // 40 * 40, i + 1),
+        "sparse": (rng.integers(0, n, n // 3), rng.integers(0, n, n // 3)),
+    }[shape]
+    g = G.GPMA(n)
+    if len(s):
+        keys = np.unique(G.edges_to_keys(s.astype(np.uint32), d.astype(np.uint32)))
+        gone = rng.random(len(keys)) < (0.02 if n > 2 else 0)
+        G.update_gpma(g, keys, np.ones(len(keys), np.uint8))
+        G.update_gpma(g, keys[gone], np.zeros(int(gone.sum()), np.uint8))
+        keys = keys[~gone]
+        s, d = (keys >> np.uint64(32)).astype(np.int64), (keys & np.uint64(0xFFFFFFFF)).astype(np.int64)
+    want = _labels(n, s, d)
+    got, count, _ = G.components(g)
+    assert np.array_equal(got, want) and count == len(np.unique(want))
+    g.close()
