@@ -125,3 +125,38 @@ def test_components_link_shapes(built_lib, shape):
     got, count, _ = G.components(g)
     assert np.array_equal(got, want) and count == len(np.unique(want))
     g.close()
+
+
+@pytest.mark.parametrize("iterations,tol", [(3, 0.0), (4, 0.0), (25, 0.0), (400, 1e-4)])
+def test_pagerank_row_lengths(built_lib, iterations, tol):
+    """In-edge rows at the edges of the gathered layout (none, one step, the
+    longest short row, one chunk, one more than a chunk, several chunks), on both sides of the iteration count that lays the in-edges out.
+    float32 sums of up to 9,000 positive terms in partial sums, 25 iterations:
+    well under the 2e-4 of the test above."""
+    import gpma_bfs_gb300 as G
+
+    n = 12000
+    lens = {0: 0, 1: 1, 2: 15, 3: 16, 4: 17, 5: 63, 6: 64, 7: 65, 8: 4095, 9: 4096, 10: 4097, 11: 9000, n - 1: 300}
+    rng = np.random.default_rng(3)
+    s = np.concatenate([rng.choice(np.arange(20, n - 20), k, replace=False) for k in lens.values()])
+    d = np.concatenate([np.full(k, v) for v, k in lens.items()])
+    keys = G.edges_to_keys(s.astype(np.uint32), d.astype(np.uint32))
+    gone = np.sort(rng.choice(len(keys), 50, replace=False))
+    g = G.GPMA(n)
+    G.update_gpma(g, np.concatenate([keys, G.edges_to_keys(np.uint32([30]), np.uint32([31]))]),
+                  np.ones(len(keys) + 1, np.uint8))
+    G.update_gpma(g, keys[gone], np.zeros(50, np.uint8))
+    # lengths stay exact: the deleted edges come back, one other edge goes
+    G.update_gpma(g, np.concatenate([keys[gone], G.edges_to_keys(np.uint32([30]), np.uint32([31]))]),
+                  np.concatenate([np.ones(50, np.uint8), np.zeros(1, np.uint8)]))
+    got, its = G.pagerank(g, 0.85, iterations, tol=tol)
+    if tol:  # the first iteration whose change is below tol, give or take the rounding of the sum
+        r = [_pagerank_f64(n, s, d, 0.85, t) for t in range(80)]
+        change = [np.abs(b - a).sum() for a, b in zip(r, r[1:])]
+        assert change[its - 1] < 2 * tol and (its < 2 or change[its - 2] > tol / 2)
+    else:
+        assert its == iterations
+    np.testing.assert_allclose(got, _pagerank_f64(n, s, d, 0.85, its), rtol=2e-4, atol=1e-9)
+    again, _ = G.pagerank(g, 0.85, iterations, tol=tol)
+    np.testing.assert_allclose(again, got, rtol=2e-4)
+    g.close()
