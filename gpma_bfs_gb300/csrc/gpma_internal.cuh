@@ -467,7 +467,7 @@ gpma_status batch_bfs_run(gpma_batch *b, gpma_graph *const *graphs, const uint32
 // to stage[i] when stage is non-null); batch_bfs_enqueue_readback copies the
 // control words and counts back; batch_bfs_finish checks and reports them.
 struct BatchBfsPlan {
-    static constexpr int CLEARS = 5;
+    static constexpr int CLEARS = 2;
     size_t tab_bytes;
     void *clear_ptr[CLEARS];
     size_t clear_bytes[CLEARS];

@@ -7,16 +7,20 @@
 //
 // The nodes of all graphs form one index space (graph g owns
 // [voff[g], voff[g+1])). Each node carries three 64-bit masks, one bit lane
-// per source: visited, frontier, next. One persistent cooperative kernel runs
-// every level, separated by bounded grid barriers:
+// per source: visited (reached before this level), frontier and seen (visited
+// and what this level has reached so far). One persistent cooperative kernel
+// runs every level, separated by bounded grid barriers:
 //   expand (phase 1): a warp takes 32 consecutive nodes; the rows of those in
 //     the frontier are walked as one concatenated slot range (warp-level load
-//     balancing) and every edge ORs the source's frontier mask, minus the
-//     target's visited lanes, into next[target]; rows longer than 64 slots
-//     are queued as 128-slot chunks instead;
+//     balancing, MS_LANE_SLOTS slots per lane per step) and every edge ORs the
+//     source's frontier mask, minus the lanes already there, into
+//     seen[target]; rows longer than 64 slots are queued as 128-slot chunks;
 //   expand (phase 2): every warp takes chunks;
-//   commit: next minus visited becomes the new frontier, joins visited, and
-//     gives each newly reached (node, lane) its level.
+//   commit: seen minus visited becomes the new frontier, visited becomes seen,
+//     and each newly reached (node, lane) gets its level: a warp's 32 nodes
+//     lane by lane of the mask, so that a lane's levels leave together.
+// A final pass counts the reached nodes per lane with warp votes and writes
+// level 0 where a lane never came.
 // The traversed-edge count (edges scanned from reached nodes, per source) is
 // summed on the fly for GTEPS.
 #include "gpma_internal.cuh"
@@ -38,7 +42,7 @@ enum : uint32_t {
 };
 
 constexpr uint32_t MS_BIG_ROW = 64;
-constexpr uint32_t MS_CHUNK_SLOTS = 128;
+constexpr uint32_t MS_CHUNK_SLOTS = 128;  // one step of a warp
 // Chunk list entries for `slots` slots over all graphs: rows over MS_BIG_ROW
 // slots yield at most len/128 + 1 chunks each, at most slots/65 such rows, so
 // a level queues fewer than slots/128 + slots/65 < slots/32 chunks.
@@ -60,7 +64,7 @@ struct MsArgs {
     const uint64_t *soff;  // slot offsets of the concatenated arrays, G + 1 (multiples of 4)
     uint64_t *visited;
     uint64_t *frontier;
-    uint64_t *next;
+    uint64_t *seen;
     uint4 *chunks;         // {slot begin, slot end, graph, node}
     uint32_t chunk_cap;
     uint32_t *ctl;
@@ -74,23 +78,47 @@ __device__ __forceinline__ uint32_t graph_of_node(const MsArgs &A, uint32_t u) {
     return A.G == 1 ? 0u : segment_of(A.voff, A.G, u);
 }
 
-// One slot of graph g scanned with frontier mask fm; returns 1 if it is an edge.
-__device__ __forceinline__ uint32_t ms_visit(const MsArgs &A, const MsGraph &Gr, uint32_t g, uint32_t s, uint64_t fm) {
-    const uint64_t key = Gr.keys[s];
-    const uint32_t w = (uint32_t)key;
-    if (w == 0xFFFFFFFFu || Gr.vals[s] == 0 || w >= Gr.n)
-        return 0;
-    const uint32_t gw = A.voff[g] + w;
-    const uint64_t nb = fm & ~A.visited[gw];
-    if (nb && (A.next[gw] & nb) != nb)
-        atomicOr((unsigned long long *)&A.next[gw], (unsigned long long)nb);
-    return 1;
+// Slots a lane takes per step of a row walk or a chunk, all loaded before any
+// of them is used.
+constexpr uint32_t MS_LANE_SLOTS = 4;
+
+// N edge slots of one lane: slot sl[j] (SIZE_NONE: none) of a graph with nodes
+// from vo on, scanned with frontier mask fm[j]. The targets' seen masks are all
+// read before the first update; a mask read too early costs an atomic that
+// changes nothing. Returns the lanes that traverse the edges.
+template <uint32_t N>
+__device__ __forceinline__ uint32_t ms_visit(const MsArgs &A, const MsGraph *const (&gr)[N], const uint32_t (&vo)[N],
+                                             const uint32_t (&sl)[N], const uint64_t (&fm)[N]) {
+    uint32_t w[N];
+    uint64_t nb[N];
+#pragma unroll
+    for (uint32_t j = 0; j < N; ++j) {
+        uint64_t k = KEY_NONE;
+        uint8_t v = 0;
+        if (sl[j] != SIZE_NONE) {
+            k = gr[j]->keys[sl[j]];
+            v = gr[j]->vals[sl[j]];
+        }
+        w[j] = v != 0 && (uint32_t)k < gr[j]->n ? (uint32_t)k : 0xFFFFFFFFu;  // the reserved column is no node
+    }
+#pragma unroll
+    for (uint32_t j = 0; j < N; ++j)
+        nb[j] = w[j] != 0xFFFFFFFFu ? fm[j] & ~A.seen[vo[j] + w[j]] : 0ull;
+    uint32_t lanes = 0;
+#pragma unroll
+    for (uint32_t j = 0; j < N; ++j) {
+        if (w[j] != 0xFFFFFFFFu)
+            lanes += __popcll(fm[j]);
+        if (nb[j])
+            atomicOr((unsigned long long *)&A.seen[vo[j] + w[j]], (unsigned long long)nb[j]);
+    }
+    return lanes;
 }
 
 // Dense levels: 4 consecutive slots of the sweep over every graph's array
 // (node offset vo, n nodes). The key's high word is its source row. The
-// frontier masks of all 4, then the visited and next masks of their targets,
-// are loaded before any update. Returns the lanes that traverse the 4 slots.
+// frontier masks of all 4, then the seen masks of their targets, are loaded
+// before any update. Returns the lanes that traverse the 4 slots.
 __device__ __forceinline__ uint32_t ms_dense_visit4(const MsArgs &A, uint32_t vo, uint32_t n,
                                                     const uint64_t (&k)[4], uint32_t v4) {
     uint32_t dst[4];
@@ -104,13 +132,13 @@ __device__ __forceinline__ uint32_t ms_dense_visit4(const MsArgs &A, uint32_t vo
     }
 #pragma unroll
     for (int j = 0; j < 4; ++j)
-        nb[j] = fm[j] ? fm[j] & ~A.visited[vo + dst[j]] : 0ull;
+        nb[j] = fm[j] ? fm[j] & ~A.seen[vo + dst[j]] : 0ull;
     uint32_t lanes = 0;
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
         lanes += __popcll(fm[j]);
-        if (nb[j] && (A.next[vo + dst[j]] & nb[j]) != nb[j])
-            atomicOr((unsigned long long *)&A.next[vo + dst[j]], (unsigned long long)nb[j]);
+        if (nb[j])
+            atomicOr((unsigned long long *)&A.seen[vo + dst[j]], (unsigned long long)nb[j]);
     }
     return lanes;
 }
@@ -149,7 +177,14 @@ __global__ void __launch_bounds__(BLOCK) msbfs_kernel(MsArgs A) {
     const uint32_t nthreads = gridDim.x * BLOCK;
     const uint32_t N = A.voff[A.G];
     unsigned long long traversed = 0;
-    // seed the sources (masks cleared by the host)
+    for (uint32_t w = gtid; w < N; w += nthreads) {
+        A.visited[w] = 0;
+        A.frontier[w] = 0;
+        A.seen[w] = 0;
+    }
+    if (!grid_barrier_gen(bar, err))
+        return;
+    // seed the sources
     for (uint32_t t = gtid; t < A.G * 64; t += nthreads) {
         const uint32_t g = t >> 6, j = t & 63;
         const MsGraph &Gr = A.gr[g];
@@ -158,6 +193,7 @@ __global__ void __launch_bounds__(BLOCK) msbfs_kernel(MsArgs A) {
         const uint32_t s = A.src[t];
         atomicOr((unsigned long long *)&A.visited[A.voff[g] + s], 1ull << j);
         atomicOr((unsigned long long *)&A.frontier[A.voff[g] + s], 1ull << j);
+        atomicOr((unsigned long long *)&A.seen[A.voff[g] + s], 1ull << j);
         atomicAdd(fslots(A, 1), (unsigned long long)ms_row_slots(Gr, s));
         if (Gr.levels)
             Gr.levels[(size_t)j * Gr.n + s] = 1;
@@ -178,8 +214,7 @@ __global__ void __launch_bounds__(BLOCK) msbfs_kernel(MsArgs A) {
             s_fs = *reinterpret_cast<volatile unsigned long long *>(fslots(A, level));
         __syncthreads();
         const bool dense = A.dense_div && s_fs * A.dense_div >= A.soff[A.G];
-        // expand, dense: every slot of every graph, 4 per thread per step; the
-        // frontier masks stay in place until the commit clears them
+        // expand, dense: every slot of every graph, 4 per thread per step
         const uint64_t quads = dense ? A.soff[A.G] >> 2 : 0;
         for (uint64_t q = gtid; q < quads; q += nthreads) {
             const uint64_t t = q << 2;
@@ -200,7 +235,6 @@ __global__ void __launch_bounds__(BLOCK) msbfs_kernel(MsArgs A) {
                 continue;
             uint32_t g = 0, b = 0, e = 0, len = 0;
             if (f) {
-                A.frontier[u] = 0;  // consumed; the commit phase writes the next frontier
                 g = graph_of_node(A, u);
                 const MsGraph &Gr = A.gr[g];
                 const uint32_t lu = u - A.voff[g];
@@ -223,11 +257,8 @@ __global__ void __launch_bounds__(BLOCK) msbfs_kernel(MsArgs A) {
                     const uint32_t pos = cb + ch_incl - nch;
                     for (uint32_t c = 0; c < nch; ++c)
                         A.chunks[pos + c] = make_uint4(b + c * MS_CHUNK_SLOTS, min(e, b + (c + 1) * MS_CHUNK_SLOTS), g, u);
-                    if (nch) {
-                        // the chunk reads the mask from frontier[u]: keep it until commit
-                        A.frontier[u] = f;
+                    if (nch)
                         len = 0;
-                    }
                 } else {
                     for (uint32_t c = cb + lane; c < min(cb + ch_total, A.chunk_cap); c += 32)
                         A.chunks[c] = make_uint4(0, 0, 0, 0);
@@ -236,22 +267,30 @@ __global__ void __launch_bounds__(BLOCK) msbfs_kernel(MsArgs A) {
             const uint32_t incl = warp_incl_scan(len);
             const uint32_t excl = incl - len;
             const uint32_t total = __shfl_sync(0xFFFFFFFFu, incl, 31);
-            for (uint32_t p0 = 0; p0 < total; p0 += 32) {
-                const uint32_t p = p0 + lane;
-                uint32_t r = 0;
+            const uint32_t vo = f ? A.voff[g] : 0u;
+            for (uint32_t p0 = 0; p0 < total; p0 += 32 * MS_LANE_SLOTS) {
+                uint32_t sl[MS_LANE_SLOTS], rvo[MS_LANE_SLOTS];
+                const MsGraph *gr[MS_LANE_SLOTS];
+                uint64_t fm[MS_LANE_SLOTS];
 #pragma unroll
-                for (uint32_t step = 16; step >= 1; step >>= 1) {
-                    const uint32_t cand = r + step;
-                    const uint32_t ex_c = __shfl_sync(0xFFFFFFFFu, excl, cand & 31);
-                    if (cand < 32 && ex_c <= p)
-                        r = cand;
+                for (uint32_t j = 0; j < MS_LANE_SLOTS; ++j) {
+                    const uint32_t p = p0 + 32 * j + lane;
+                    uint32_t r = 0;
+#pragma unroll
+                    for (uint32_t step = 16; step >= 1; step >>= 1) {
+                        const uint32_t cand = r + step;
+                        const uint32_t ex_c = __shfl_sync(0xFFFFFFFFu, excl, cand & 31);
+                        if (cand < 32 && ex_c <= p)
+                            r = cand;
+                    }
+                    const uint32_t rb = __shfl_sync(0xFFFFFFFFu, b, r);
+                    const uint32_t rex = __shfl_sync(0xFFFFFFFFu, excl, r);
+                    gr[j] = A.gr + __shfl_sync(0xFFFFFFFFu, g, r);
+                    rvo[j] = __shfl_sync(0xFFFFFFFFu, vo, r);
+                    fm[j] = __shfl_sync(0xFFFFFFFFu, f, r);
+                    sl[j] = p < total ? rb + (p - rex) : SIZE_NONE;
                 }
-                const uint32_t rb = __shfl_sync(0xFFFFFFFFu, b, r);
-                const uint32_t rex = __shfl_sync(0xFFFFFFFFu, excl, r);
-                const uint32_t rg = __shfl_sync(0xFFFFFFFFu, g, r);
-                const uint64_t rf = __shfl_sync(0xFFFFFFFFu, f, r);
-                if (p < total)
-                    traversed += ms_visit(A, A.gr[rg], rg, rb + (p - rex), rf) * (unsigned long long)__popcll(rf);
+                traversed += ms_visit<MS_LANE_SLOTS>(A, gr, rvo, sl, fm);
             }
         }
         if (!dense && !grid_barrier_gen(bar, err))
@@ -264,37 +303,58 @@ __global__ void __launch_bounds__(BLOCK) msbfs_kernel(MsArgs A) {
                 continue;
             const uint64_t fm = A.frontier[ch.w];
             const MsGraph &Gr = A.gr[ch.z];
-            for (uint32_t s = ch.x + lane; s < ch.y; s += 32)
-                traversed += ms_visit(A, Gr, ch.z, s, fm) * (unsigned long long)__popcll(fm);
+            const uint32_t vo = A.voff[ch.z];
+            uint32_t sl[MS_LANE_SLOTS], cvo[MS_LANE_SLOTS];
+            const MsGraph *gr[MS_LANE_SLOTS];
+            uint64_t fms[MS_LANE_SLOTS];
+#pragma unroll
+            for (uint32_t j = 0; j < MS_LANE_SLOTS; ++j) {
+                const uint32_t sj = ch.x + 32 * j + lane;  // a chunk is one step
+                sl[j] = sj < ch.y ? sj : SIZE_NONE;
+                cvo[j] = vo;
+                gr[j] = &Gr;
+                fms[j] = fm;
+            }
+            traversed += ms_visit<MS_LANE_SLOTS>(A, gr, cvo, sl, fms);
         }
         if (!grid_barrier_gen(bar, err))
             return;
         // commit
         uint32_t changed = 0;
         unsigned long long fnext = 0;
-        for (uint32_t w = gtid; w < N; w += nthreads) {
-            const uint64_t nxt = A.next[w];
-            const uint64_t vis = A.visited[w];
-            const uint64_t nx = nxt & ~vis;
-            if (A.frontier[w])
-                A.frontier[w] = 0;  // chunked rows kept their mask until now
-            if (nxt)
-                A.next[w] = 0;
-            if (nx) {
+        for (uint32_t w0 = gwarp * 32; w0 < N; w0 += nwarps * 32) {
+            const uint32_t w = w0 + lane;
+            const uint64_t seen = w < N ? A.seen[w] : 0ull;
+            const uint64_t nx = w < N ? seen & ~A.visited[w] : 0ull;
+            if (w < N)
                 A.frontier[w] = nx;
-                A.visited[w] = vis | nx;
+            if (!__any_sync(0xFFFFFFFFu, nx != 0ull))
+                continue;
+            uint32_t g = 0;
+            if (nx) {
+                A.visited[w] = seen;
                 changed = 1;
-                const uint32_t g = graph_of_node(A, w);
-                const MsGraph &Gr = A.gr[g];
-                fnext += ms_row_slots(Gr, w - A.voff[g]);
-                if (Gr.levels) {
-                    const uint32_t lw = w - A.voff[g];
-                    uint64_t m = nx;
-                    while (m) {
-                        const int bit = __ffsll((long long)m) - 1;
-                        m &= m - 1;
-                        Gr.levels[(size_t)bit * Gr.n + lw] = level + 1;
-                    }
+                g = graph_of_node(A, w);
+                fnext += ms_row_slots(A.gr[g], w - A.voff[g]);
+            }
+            // the levels of one mask lane at a time; nodes of several graphs
+            // in the warp (nx != 0 for some of each) graph by graph
+            uint32_t todo = __ballot_sync(0xFFFFFFFFu, nx != 0ull);
+            while (todo) {
+                const uint32_t g0 = __shfl_sync(0xFFFFFFFFu, g, __ffs(todo) - 1);
+                const bool mine = nx && g == g0;
+                todo &= ~__ballot_sync(0xFFFFFFFFu, mine);
+                const MsGraph &Gr = A.gr[g0];
+                if (!Gr.levels)
+                    continue;
+                uint32_t *lv = Gr.levels + (w - A.voff[g0]);
+                uint64_t any = ((uint64_t)__reduce_or_sync(0xFFFFFFFFu, mine ? (uint32_t)(nx >> 32) : 0u) << 32) |
+                               __reduce_or_sync(0xFFFFFFFFu, mine ? (uint32_t)nx : 0u);
+                while (any) {
+                    const int bit = __ffsll((long long)any) - 1;
+                    any &= any - 1;
+                    if (mine && ((nx >> bit) & 1))
+                        lv[(size_t)bit * Gr.n] = level + 1;
                 }
             }
         }
@@ -310,8 +370,10 @@ __global__ void __launch_bounds__(BLOCK) msbfs_kernel(MsArgs A) {
         if (cta_broadcast_read(A.ctl + MS_CHANGE + level % 3) == 0)
             break;
     }
-    // reached (graph, lane) counts: each CTA walks a contiguous node range
-    // graph by graph with shared-memory lane counters
+    // reached (graph, lane) counts, and level 0 where a lane never came: each
+    // CTA walks a contiguous node range graph by graph, a warp 32 nodes at a
+    // time, mask lane by mask lane (one vote per lane of the mask counts 32
+    // nodes; lane l of the warp keeps mask lanes l and l + 32)
     __shared__ unsigned int cnt[64];
     const uint32_t per = (N + gridDim.x - 1) / gridDim.x;
     const uint32_t lo = min(N, blockIdx.x * per), hi = min(N, lo + per);
@@ -319,17 +381,27 @@ __global__ void __launch_bounds__(BLOCK) msbfs_kernel(MsArgs A) {
     while (__syncthreads_or(pos < hi)) {
         const uint32_t g = graph_of_node(A, pos);
         const uint32_t end = min(hi, A.voff[g + 1]);
+        const MsGraph &Gr = A.gr[g];
         if (threadIdx.x < 64)
             cnt[threadIdx.x] = 0;
         __syncthreads();
-        for (uint32_t w = pos + threadIdx.x; w < end; w += BLOCK) {
-            uint64_t m = A.visited[w];
-            while (m) {
-                const int bit = __ffsll((long long)m) - 1;
-                m &= m - 1;
-                atomicAdd(&cnt[bit], 1u);
+        uint32_t c0 = 0, c1 = 0;
+        for (uint32_t w0 = pos + (threadIdx.x & ~31u); w0 < end; w0 += BLOCK) {
+            const uint32_t w = w0 + lane;
+            const uint64_t m = w < end ? A.visited[w] : 0ull;
+            for (uint32_t j = 0; j < Gr.nsrc; ++j) {
+                const bool in = (m >> j) & 1;
+                const uint32_t c = __popc(__ballot_sync(0xFFFFFFFFu, in));
+                c0 += j == lane ? c : 0u;
+                c1 += j == lane + 32 ? c : 0u;
+                if (Gr.levels && !in && w < end)
+                    Gr.levels[(size_t)j * Gr.n + (w - A.voff[g])] = 0;
             }
         }
+        if (c0)
+            atomicAdd(&cnt[lane], c0);
+        if (c1)
+            atomicAdd(&cnt[lane + 32], c1);
         __syncthreads();
         if (threadIdx.x < 64 && cnt[threadIdx.x])
             atomicAdd(&A.reached[(size_t)g * 64 + threadIdx.x], (unsigned long long)cnt[threadIdx.x]);
@@ -475,8 +547,8 @@ gpma_status batch_bfs_plan(gpma_batch *b, gpma_graph *const *graphs, const uint3
             src[64ull * i + j] = srcs[i][j];
     }
     P->tab_bytes = lay.bytes;
-    void *ptr[BatchBfsPlan::CLEARS] = {b->ms_mask[0], b->ms_mask[1], b->ms_mask[2], b->ms_ctl, b->ms_reached};
-    const size_t bytes[BatchBfsPlan::CLEARS] = {8 * N, 8 * N, 8 * N, sizeof(uint32_t) * MS_CTL_WORDS,
+    void *ptr[BatchBfsPlan::CLEARS] = {b->ms_ctl, b->ms_reached};  // the kernel clears the masks
+    const size_t bytes[BatchBfsPlan::CLEARS] = {sizeof(uint32_t) * MS_CTL_WORDS,
                                                 sizeof(unsigned long long) * (64ull * k + 1)};
     for (int i = 0; i < BatchBfsPlan::CLEARS; ++i) {
         P->clear_ptr[i] = ptr[i];
@@ -492,7 +564,7 @@ gpma_status batch_bfs_plan(gpma_batch *b, gpma_graph *const *graphs, const uint3
     A.dense_div = g_tuning.ms_dense_div;
     A.visited = b->ms_mask[0];
     A.frontier = b->ms_mask[1];
-    A.next = b->ms_mask[2];
+    A.seen = b->ms_mask[2];
     A.chunks = reinterpret_cast<uint4 *>(b->ms_chunks);
     A.chunk_cap = (uint32_t)std::min<uint64_t>(b->ms_chunk_cap, 0xFFFFFFFFull);
     A.ctl = b->ms_ctl;
@@ -529,14 +601,16 @@ gpma_status batch_bfs_finish(gpma_batch *b, const uint32_t *nsrc, uint32_t k, ui
 }
 
 // Multi-source BFS of graphs[0..k) with nsrc[i] sources each. Levels (when
-// levels != NULL) are written through device staging and copied to the
-// caller's pointers; reached receives sum(nsrc) counts.
+// levels != NULL) go to the caller's pointers, through device staging where
+// those are host memory; reached receives sum(nsrc) counts.
 gpma_status batch_bfs_run(gpma_batch *b, gpma_graph *const *graphs, const uint32_t *const *srcs, const uint32_t *nsrc,
                           uint32_t k, uint32_t *const *levels, uint64_t *reached, cudaStream_t s) {
-    // per-graph level staging, only when levels are requested
-    std::vector<uint32_t *> stage(k, nullptr);
+    // where the kernel writes each graph's levels: the caller's own device
+    // array, or staging memory copied out afterwards (every entry is written,
+    // so neither needs clearing)
+    std::vector<uint32_t *> stage(k, nullptr), staged(k, nullptr);
     auto cleanup = [&]() {
-        for (auto *p : stage)
+        for (auto *p : staged)
             if (p)
                 cudaFree(p);
     };
@@ -545,8 +619,12 @@ gpma_status batch_bfs_run(gpma_batch *b, gpma_graph *const *graphs, const uint32
             for (uint32_t i = 0; i < k; ++i) {
                 if (!levels[i])
                     continue;
-                GPMA_TRY(dev_alloc(&stage[i], (uint64_t)nsrc[i] * graphs[i]->row_num));
-                GPMA_CUDA(cudaMemsetAsync(stage[i], 0, sizeof(uint32_t) * nsrc[i] * (uint64_t)graphs[i]->row_num, s));
+                if (is_device_pointer(levels[i]) && reinterpret_cast<uintptr_t>(levels[i]) % sizeof(uint32_t) == 0) {
+                    stage[i] = levels[i];
+                    continue;
+                }
+                GPMA_TRY(dev_alloc(&staged[i], (uint64_t)nsrc[i] * graphs[i]->row_num));
+                stage[i] = staged[i];
             }
         }
         BatchBfsPlan P;
@@ -559,8 +637,8 @@ gpma_status batch_bfs_run(gpma_batch *b, gpma_graph *const *graphs, const uint32
         prof_mark(b->profiling, b->ev, 1, s);
         GPMA_TRY(batch_bfs_enqueue_readback(b, P, s));
         for (uint32_t i = 0; i < k; ++i)
-            if (stage[i])
-                GPMA_TRY(copy_any(levels[i], stage[i], sizeof(uint32_t) * nsrc[i] * (uint64_t)graphs[i]->row_num, s));
+            if (staged[i])
+                GPMA_TRY(copy_any(levels[i], staged[i], sizeof(uint32_t) * nsrc[i] * (uint64_t)graphs[i]->row_num, s));
         GPMA_CUDA(cudaStreamSynchronize(s));
         b->prof.bfs_ms += prof_elapsed(b->profiling, b->ev, 0, 1);
         return batch_bfs_finish(b, nsrc, k, reached);

@@ -311,7 +311,7 @@ gpma_status step_run(gpma_step *st, const uint64_t *keys, const uint8_t *values,
 // gather of the batches into segment-length order, then the persistent
 // update kernel) and one multi-source BFS over all of them, as one graph:
 //   gather table upload -> gather kernel -> update table upload -> update
-//   kernel (cooperative) -> BFS table upload -> 5 BFS clears -> multi-source
+//   kernel (cooperative) -> BFS table upload -> 2 BFS clears -> multi-source
 //   BFS kernel (cooperative) -> status, control and count read-back.
 // A step whose batch holds an empty or a bulk-sized (>= 5M keys) part, or
 // whose update needs host work, runs or finishes through the eager calls,
