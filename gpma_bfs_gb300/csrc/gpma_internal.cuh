@@ -258,6 +258,8 @@ struct gpma_batch {
     // multi-source BFS state over all graphs of a call
     uint64_t ms_cap = 0;               // nodes
     uint64_t *ms_mask[3] = {nullptr, nullptr, nullptr};
+    unsigned char *ms_planes = nullptr;  // bit planes of the levels, calls with levels only
+    uint64_t ms_planes_cap = 0;          // its bytes
     // per-call graph table (node and slot offsets, sources, descriptors), one
     // upload from its pinned mirror
     unsigned char *ms_tab = nullptr;

@@ -6,8 +6,8 @@
 // level L gets L+1, slots with column 0xFFFFFFFF or value 0 are not edges).
 //
 // The nodes of all graphs form one index space (graph g owns
-// [voff[g], voff[g+1])). Each node carries three 64-bit masks, one bit lane
-// per source: visited (reached before this level), frontier and seen (visited
+// [voff[g], voff[g+1])). Each node carries three masks of 32 or 64 bits, one bit
+// lane per source: visited (reached before this level), frontier and seen (visited
 // and what this level has reached so far). One persistent cooperative kernel
 // runs every level, separated by bounded grid barriers:
 //   expand (phase 1): a warp takes 32 consecutive nodes; the rows of those in
@@ -17,10 +17,8 @@
 //     seen[target]; rows longer than 64 slots are queued as 128-slot chunks;
 //   expand (phase 2): every warp takes chunks;
 //   commit: seen minus visited becomes the new frontier, visited becomes seen,
-//     and each newly reached (node, lane) gets its level: a warp's 32 nodes
-//     lane by lane of the mask, so that a lane's levels leave together.
-// A final pass counts the reached nodes per lane with warp votes and writes
-// level 0 where a lane never came.
+//     and the level of each newly reached (node, lane) goes into bit planes.
+// A final pass counts the reached nodes per lane and writes the levels.
 // The traversed-edge count (edges scanned from reached nodes, per source) is
 // summed on the fly for GTEPS.
 #include "gpma_internal.cuh"
@@ -47,6 +45,10 @@ constexpr uint32_t MS_CHUNK_SLOTS = 128;  // one step of a warp
 // slots yield at most len/128 + 1 chunks each, at most slots/65 such rows, so
 // a level queues fewer than slots/128 + slots/65 < slots/32 chunks.
 inline uint64_t ms_chunk_need(uint64_t slots) { return slots / 32 + 1024; }
+// Chunks a CTA collects in shared memory and adds to the grid's list under one
+// atomic; a warp that finds no room adds its own. (An atomic per warp and 32
+// nodes, all on one word, serialised at 4.4 ns apiece.)
+constexpr uint32_t MS_CTA_CHUNKS = 512;
 
 struct MsGraph {
     const uint64_t *keys;
@@ -62,9 +64,9 @@ struct MsArgs {
     const uint32_t *voff;  // G + 1
     const uint32_t *src;   // G * 64
     const uint64_t *soff;  // slot offsets of the concatenated arrays, G + 1 (multiples of 4)
-    uint64_t *visited;
-    uint64_t *frontier;
-    uint64_t *seen;
+    // masks of every node, 32 or 64 bits each (MsMask of the kernel)
+    void *visited, *frontier, *seen;
+    void *planes;          // MS_PLANES bit planes of the level of every (node, lane), or null without levels
     uint4 *chunks;         // {slot begin, slot end, graph, node}
     uint32_t chunk_cap;
     uint32_t *ctl;
@@ -74,6 +76,20 @@ struct MsArgs {
     const uint32_t *abort;  // non-zero: return at once (a recorded step after one needing host work)
 };
 
+// Levels below 2^MS_PLANES are kept as bit planes and written once, at the
+// end, whole rows of 32 nodes at a time; written when they are found, 16 lanes
+// of the social graph cost 18-54 us in each of the middle levels (partly filled
+// sectors of 104 MB). The few (node, lane) pairs of a deeper search go straight
+// to the level arrays.
+constexpr uint32_t MS_PLANES = 6;
+
+__device__ __forceinline__ uint32_t mask_count(uint32_t m) { return __popc(m); }
+__device__ __forceinline__ uint32_t mask_count(uint64_t m) { return __popcll(m); }
+__device__ __forceinline__ void mask_or(uint32_t *p, uint32_t m) { atomicOr(p, m); }
+__device__ __forceinline__ void mask_or(uint64_t *p, uint64_t m) {
+    atomicOr((unsigned long long *)p, (unsigned long long)m);
+}
+
 __device__ __forceinline__ uint32_t graph_of_node(const MsArgs &A, uint32_t u) {
     return A.G == 1 ? 0u : segment_of(A.voff, A.G, u);
 }
@@ -81,16 +97,22 @@ __device__ __forceinline__ uint32_t graph_of_node(const MsArgs &A, uint32_t u) {
 // Slots a lane takes per step of a row walk or a chunk, all loaded before any
 // of them is used.
 constexpr uint32_t MS_LANE_SLOTS = 4;
+// Nodes per thread per step of a commit: as many as leave the kernel at 64
+// registers, four CTAs per SM (social graph, 16 sources: 30 us per middle level
+// with 1, 12 with 4; 128 graphs, 64 sources: 39 with 1, 37 with 2, and with 4
+// the whole kernel half as fast again, at 108 registers).
+template <typename M>
+constexpr uint32_t ms_commit_nodes() { return sizeof(M) == 8 ? 2 : 4; }
 
 // N edge slots of one lane: slot sl[j] (SIZE_NONE: none) of a graph with nodes
 // from vo on, scanned with frontier mask fm[j]. The targets' seen masks are all
 // read before the first update; a mask read too early costs an atomic that
 // changes nothing. Returns the lanes that traverse the edges.
-template <uint32_t N>
-__device__ __forceinline__ uint32_t ms_visit(const MsArgs &A, const MsGraph *const (&gr)[N], const uint32_t (&vo)[N],
-                                             const uint32_t (&sl)[N], const uint64_t (&fm)[N]) {
+template <typename M, uint32_t N>
+__device__ __forceinline__ uint32_t ms_visit(M *seen, const MsGraph *const (&gr)[N], const uint32_t (&vo)[N],
+                                             const uint32_t (&sl)[N], const M (&fm)[N]) {
     uint32_t w[N];
-    uint64_t nb[N];
+    M nb[N];
 #pragma unroll
     for (uint32_t j = 0; j < N; ++j) {
         uint64_t k = KEY_NONE;
@@ -99,18 +121,19 @@ __device__ __forceinline__ uint32_t ms_visit(const MsArgs &A, const MsGraph *con
             k = gr[j]->keys[sl[j]];
             v = gr[j]->vals[sl[j]];
         }
-        w[j] = v != 0 && (uint32_t)k < gr[j]->n ? (uint32_t)k : 0xFFFFFFFFu;  // the reserved column is no node
+        // the reserved column is no node
+        w[j] = sl[j] != SIZE_NONE && v != 0 && (uint32_t)k < gr[j]->n ? (uint32_t)k : 0xFFFFFFFFu;
     }
 #pragma unroll
     for (uint32_t j = 0; j < N; ++j)
-        nb[j] = w[j] != 0xFFFFFFFFu ? fm[j] & ~A.seen[vo[j] + w[j]] : 0ull;
+        nb[j] = w[j] != 0xFFFFFFFFu ? fm[j] & ~seen[vo[j] + w[j]] : M(0);
     uint32_t lanes = 0;
 #pragma unroll
     for (uint32_t j = 0; j < N; ++j) {
         if (w[j] != 0xFFFFFFFFu)
-            lanes += __popcll(fm[j]);
+            lanes += mask_count(fm[j]);
         if (nb[j])
-            atomicOr((unsigned long long *)&A.seen[vo[j] + w[j]], (unsigned long long)nb[j]);
+            mask_or(&seen[vo[j] + w[j]], nb[j]);
     }
     return lanes;
 }
@@ -119,26 +142,27 @@ __device__ __forceinline__ uint32_t ms_visit(const MsArgs &A, const MsGraph *con
 // (node offset vo, n nodes). The key's high word is its source row. The
 // frontier masks of all 4, then the seen masks of their targets, are loaded
 // before any update. Returns the lanes that traverse the 4 slots.
-__device__ __forceinline__ uint32_t ms_dense_visit4(const MsArgs &A, uint32_t vo, uint32_t n,
-                                                    const uint64_t (&k)[4], uint32_t v4) {
+template <typename M>
+__device__ __forceinline__ uint32_t ms_dense_visit4(const M *frontier, M *seen, uint32_t n, const uint64_t (&k)[4],
+                                                    uint32_t v4) {
     uint32_t dst[4];
-    uint64_t fm[4], nb[4];
+    M fm[4], nb[4];
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
         const uint32_t src = (uint32_t)(k[j] >> 32);
         dst[j] = (uint32_t)k[j];
         const bool ok = dst[j] != 0xFFFFFFFFu && ((v4 >> (8 * j)) & 0xFFu) != 0 && src < n && dst[j] < n;
-        fm[j] = ok ? A.frontier[vo + src] : 0ull;
+        fm[j] = ok ? frontier[src] : M(0);
     }
 #pragma unroll
     for (int j = 0; j < 4; ++j)
-        nb[j] = fm[j] ? fm[j] & ~A.seen[vo + dst[j]] : 0ull;
+        nb[j] = fm[j] ? fm[j] & ~seen[dst[j]] : M(0);
     uint32_t lanes = 0;
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
-        lanes += __popcll(fm[j]);
+        lanes += mask_count(fm[j]);
         if (nb[j])
-            atomicOr((unsigned long long *)&A.seen[vo + dst[j]], (unsigned long long)nb[j]);
+            mask_or(&seen[dst[j]], nb[j]);
     }
     return lanes;
 }
@@ -156,15 +180,159 @@ __device__ __forceinline__ uint32_t graph_of_slot(const MsArgs &A, uint64_t t) {
     return lo;
 }
 
+// With several graphs the sweep goes round the CTAs in tiles of MS_TILE steps
+// of 4 slots per thread, so that a thread looks for the graph of its slots once
+// per tile, not once per step (128 graphs: 145-246 us per dense level before,
+// 118-185 after). One graph needs no search and goes step by step, which
+// spreads its busy rows more evenly (8 % less per level).
+constexpr uint32_t MS_TILE = 8;
+
+// One thread's 4 slots of step i of its CTA's sweep.
+struct MsQuad {
+    ulonglong2 k01, k23;
+    uint32_t v4, vo, n;  // the 4 values; node offset and nodes of the graph
+    uint32_t g = 0;
+    uint64_t base = 0, end = 0;  // the graph's concatenated slots (end 0: none looked up)
+    bool ok;
+    __device__ __forceinline__ void load(const MsArgs &A, uint32_t i) {
+        const uint32_t steps = A.G == 1 ? 1u : MS_TILE;
+        const uint64_t tile = blockIdx.x + (uint64_t)(i / steps) * gridDim.x;
+        const uint64_t t = (tile * (steps * BLOCK) + (i % steps) * BLOCK + threadIdx.x) << 2;
+        ok = t < A.soff[A.G];
+        if (!ok)
+            return;
+        if (t >= end) {
+            g = A.G == 1 ? 0u : graph_of_slot(A, t);
+            base = A.soff[g];
+            end = A.soff[g + 1];
+            vo = A.voff[g];
+            n = A.gr[g].n;
+        }
+        const uint32_t s = (uint32_t)(t - base);
+        const MsGraph &Gr = A.gr[g];
+        k01 = *reinterpret_cast<const ulonglong2 *>(Gr.keys + s);
+        k23 = *reinterpret_cast<const ulonglong2 *>(Gr.keys + s + 2);
+        v4 = *reinterpret_cast<const uint32_t *>(Gr.vals + s);
+    }
+};
+
 __device__ __forceinline__ unsigned long long *fslots(const MsArgs &A, uint32_t level) {
     return reinterpret_cast<unsigned long long *>(A.ctl + MS_FSLOTS) + level % 3;
 }
 
-__device__ __forceinline__ uint32_t ms_row_slots(const MsGraph &Gr, uint32_t v) {
-    const uint32_t b = Gr.ro[v], e = min(Gr.ro[v + 1], Gr.size);
-    return e > b ? e - b : 0u;
+// Bit matrix transpose over a warp: bit i of lane l's result is bit l of lane
+// i's word.
+__device__ __forceinline__ uint32_t warp_transpose(uint32_t x, uint32_t lane) {
+    uint32_t m = 0x0000FFFFu;  // the bits whose index has bit `j` clear
+#pragma unroll
+    for (uint32_t j = 16; j >= 1; j >>= 1) {
+        const uint32_t y = __shfl_xor_sync(0xFFFFFFFFu, x, j);
+        x = (lane & j) ? (x & ~m) | ((y >> j) & m) : (x & m) | ((y & m) << j);
+        m ^= m << (j >> 1);
+    }
+    return x;
 }
 
+// The end of level lv - 1 (lv = 1: the seeds): what seen holds beyond visited
+// is the frontier of level lv and gets that level; visited becomes seen. The
+// first commit and the first use of a plane write every entry, so only seen is
+// cleared beforehand. Counts the next frontier's row slots and flags a change.
+template <typename M>
+__device__ __forceinline__ void ms_commit(const MsArgs &A, uint32_t lv, uint32_t N, uint32_t gwarp, uint32_t nwarps,
+                                          uint32_t lane) {
+    constexpr uint32_t MS_COMMIT = ms_commit_nodes<M>();
+    M *visited = (M *)A.visited, *frontier = (M *)A.frontier, *planes = (M *)A.planes;
+    const M *seen = (const M *)A.seen;
+    uint32_t changed = 0;
+    unsigned long long fnext = 0;
+    const bool in_planes = lv < (1u << MS_PLANES), new_plane = in_planes && planes && (lv & (lv - 1)) == 0;
+    const uint32_t top = 31 - __clz(lv);
+    // every load of a kind is issued before its use: the passes over the masks
+    // are short, so their chains of loads decide
+    for (uint64_t w0 = (uint64_t)gwarp * 32 * MS_COMMIT; w0 < N; w0 += (uint64_t)nwarps * 32 * MS_COMMIT) {
+        M now[MS_COMMIT], nx[MS_COMMIT];
+#pragma unroll
+        for (uint32_t u = 0; u < MS_COMMIT; ++u) {
+            const uint64_t w = w0 + 32 * u + lane;
+            now[u] = w < N ? seen[w] : M(0);
+            nx[u] = w < N && lv > 1 ? visited[w] : M(0);
+        }
+        uint32_t g[MS_COMMIT], r0[MS_COMMIT], r1[MS_COMMIT];
+#pragma unroll
+        for (uint32_t u = 0; u < MS_COMMIT; ++u) {
+            const uint32_t w = (uint32_t)(w0 + 32 * u + lane);
+            nx[u] = now[u] & ~nx[u];
+            g[u] = r0[u] = r1[u] = 0;
+            if (nx[u]) {
+                g[u] = graph_of_node(A, w);
+                const uint32_t *ro = A.gr[g[u]].ro + (w - A.voff[g[u]]);
+                r0[u] = ro[0];
+                r1[u] = ro[1];
+            }
+        }
+#pragma unroll
+        for (uint32_t u = 0; u < MS_COMMIT; ++u) {
+            const uint64_t w = w0 + 32 * u + lane;
+            if (w >= N)
+                continue;
+            frontier[w] = nx[u];
+            if (nx[u] || lv == 1)
+                visited[w] = now[u];
+            if (new_plane)
+                planes[(size_t)top * N + w] = nx[u];
+        }
+        if (in_planes && planes) {
+            for (uint32_t b = 0; b < MS_PLANES; ++b) {
+                if (!((lv >> b) & 1) || (new_plane && b == top))
+                    continue;
+                M old[MS_COMMIT];
+#pragma unroll
+                for (uint32_t u = 0; u < MS_COMMIT; ++u)
+                    old[u] = nx[u] ? planes[(size_t)b * N + w0 + 32 * u + lane] : M(0);
+#pragma unroll
+                for (uint32_t u = 0; u < MS_COMMIT; ++u)
+                    if (nx[u])
+                        planes[(size_t)b * N + w0 + 32 * u + lane] = old[u] | nx[u];
+            }
+        }
+#pragma unroll
+        for (uint32_t u = 0; u < MS_COMMIT; ++u) {
+            if (!nx[u])
+                continue;
+            changed = 1;
+            const MsGraph &Gr = A.gr[g[u]];
+            const uint32_t e = min(r1[u], Gr.size);
+            fnext += e > r0[u] ? e - r0[u] : 0u;
+            if (in_planes || !Gr.levels)
+                continue;
+            const uint32_t lw = (uint32_t)(w0 + 32 * u + lane) - A.voff[g[u]];
+            for (M m = nx[u]; m; m &= m - 1) {
+                const uint32_t bit = sizeof(M) == 8 ? __ffsll((long long)m) - 1 : __ffs((int)m) - 1;
+                Gr.levels[(size_t)bit * Gr.n + lw] = lv;
+            }
+        }
+    }
+    // one atomic per CTA and word (a plain store of a flag here, to the line
+    // that the barrier polls, made every commit 35 us longer)
+    if (__syncthreads_or(changed) && threadIdx.x == 0)
+        atomicAdd(A.ctl + MS_CHANGE + (lv - 1) % 3, 1u);
+#pragma unroll
+    for (int d = 16; d >= 1; d >>= 1)
+        fnext += __shfl_xor_sync(0xFFFFFFFFu, fnext, d);
+    __shared__ unsigned long long s_fnext[BLOCK / 32];
+    if (lane == 0)
+        s_fnext[threadIdx.x >> 5] = fnext;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int i = 1; i < BLOCK / 32; ++i)
+            fnext += s_fnext[i];
+        if (fnext)
+            atomicAdd(fslots(A, lv), fnext);
+    }
+}
+
+// M: uint32_t for up to 32 sources in every graph, uint64_t for up to 64.
+template <typename M>
 __global__ void __launch_bounds__(BLOCK) msbfs_kernel(MsArgs A) {
     if (A.abort && *(const volatile uint32_t *)A.abort)
         return;
@@ -176,28 +344,21 @@ __global__ void __launch_bounds__(BLOCK) msbfs_kernel(MsArgs A) {
     const uint32_t gtid = blockIdx.x * BLOCK + threadIdx.x;
     const uint32_t nthreads = gridDim.x * BLOCK;
     const uint32_t N = A.voff[A.G];
+    M *seen = (M *)A.seen;
+    const M *frontier = (const M *)A.frontier;
     unsigned long long traversed = 0;
-    for (uint32_t w = gtid; w < N; w += nthreads) {
-        A.visited[w] = 0;
-        A.frontier[w] = 0;
-        A.seen[w] = 0;
+    for (uint32_t w = gtid; w < N; w += nthreads)
+        seen[w] = 0;
+    if (!grid_barrier_gen(bar, err))
+        return;
+    for (uint32_t t = gtid; t < A.G * 64; t += nthreads) {
+        const uint32_t g = t >> 6, j = t & 63;
+        if (j < A.gr[g].nsrc)
+            mask_or(&seen[A.voff[g] + A.src[t]], M(1) << j);
     }
     if (!grid_barrier_gen(bar, err))
         return;
-    // seed the sources
-    for (uint32_t t = gtid; t < A.G * 64; t += nthreads) {
-        const uint32_t g = t >> 6, j = t & 63;
-        const MsGraph &Gr = A.gr[g];
-        if (j >= Gr.nsrc)
-            continue;
-        const uint32_t s = A.src[t];
-        atomicOr((unsigned long long *)&A.visited[A.voff[g] + s], 1ull << j);
-        atomicOr((unsigned long long *)&A.frontier[A.voff[g] + s], 1ull << j);
-        atomicOr((unsigned long long *)&A.seen[A.voff[g] + s], 1ull << j);
-        atomicAdd(fslots(A, 1), (unsigned long long)ms_row_slots(Gr, s));
-        if (Gr.levels)
-            Gr.levels[(size_t)j * Gr.n + s] = 1;
-    }
+    ms_commit<M>(A, 1, N, gwarp, nwarps, lane);
     if (!grid_barrier_gen(bar, err))
         return;
     uint32_t level = 1;
@@ -209,35 +370,43 @@ __global__ void __launch_bounds__(BLOCK) msbfs_kernel(MsArgs A) {
         }
         uint32_t *chunk_cnt = A.ctl + MS_CHUNKS + level % 3;
         __shared__ unsigned long long s_fs;
+        __shared__ uint4 s_chunks[MS_CTA_CHUNKS];
+        __shared__ uint32_t s_nch, s_end;  // entries claimed, entries filled
         __syncthreads();
-        if (threadIdx.x == 0)
+        if (threadIdx.x == 0) {
+            s_nch = 0;
+            s_end = MS_CTA_CHUNKS;
             s_fs = *reinterpret_cast<volatile unsigned long long *>(fslots(A, level));
+        }
         __syncthreads();
         const bool dense = A.dense_div && s_fs * A.dense_div >= A.soff[A.G];
-        // expand, dense: every slot of every graph, 4 per thread per step
-        const uint64_t quads = dense ? A.soff[A.G] >> 2 : 0;
-        for (uint64_t q = gtid; q < quads; q += nthreads) {
-            const uint64_t t = q << 2;
-            const uint32_t g = A.G == 1 ? 0u : graph_of_slot(A, t);
-            const MsGraph &Gr = A.gr[g];
-            const uint32_t s = (uint32_t)(t - A.soff[g]);
-            const ulonglong2 k01 = *reinterpret_cast<const ulonglong2 *>(Gr.keys + s);
-            const ulonglong2 k23 = *reinterpret_cast<const ulonglong2 *>(Gr.keys + s + 2);
-            const uint32_t v4 = *reinterpret_cast<const uint32_t *>(Gr.vals + s);
-            const uint64_t k[4] = {k01.x, k01.y, k23.x, k23.y};
-            traversed += ms_dense_visit4(A, A.voff[g], Gr.n, k, v4);
+        if (dense) {
+            // expand, dense: every slot of every graph, 4 per thread per step,
+            // the next step's slots read while this one's masks are gathered
+            MsQuad nq;
+            nq.load(A, 0);
+            for (uint32_t i = 1; nq.ok; ++i) {
+                const uint64_t k[4] = {nq.k01.x, nq.k01.y, nq.k23.x, nq.k23.y};
+                const uint32_t v4 = nq.v4, vo = nq.vo, n = nq.n;
+                nq.load(A, i);
+                traversed += ms_dense_visit4<M>(frontier + vo, seen + vo, n, k, v4);
+            }
         }
-        // expand, phase 1 (sparse levels)
+        // expand, phase 1 (sparse levels); the next 32 masks are read ahead
+        M nf = !dense && gwarp * 32 + lane < N ? frontier[gwarp * 32 + lane] : M(0);
         for (uint32_t base = gwarp * 32; !dense && base < N; base += nwarps * 32) {
             const uint32_t u = base + lane;
-            const uint64_t f = u < N ? A.frontier[u] : 0ull;
-            if (__ballot_sync(0xFFFFFFFFu, f != 0ull) == 0)
+            const M f = nf;
+            const uint64_t un = (uint64_t)u + nwarps * 32;
+            nf = un < N ? frontier[un] : M(0);
+            if (__ballot_sync(0xFFFFFFFFu, f != 0) == 0)
                 continue;
-            uint32_t g = 0, b = 0, e = 0, len = 0;
+            uint32_t g = 0, vo = 0, b = 0, e = 0, len = 0;
             if (f) {
                 g = graph_of_node(A, u);
+                vo = A.voff[g];
                 const MsGraph &Gr = A.gr[g];
-                const uint32_t lu = u - A.voff[g];
+                const uint32_t lu = u - vo;
                 const uint32_t r1 = Gr.ro[lu + 1];
                 b = Gr.ro[lu];
                 e = min(r1, Gr.size);
@@ -249,29 +418,40 @@ __global__ void __launch_bounds__(BLOCK) msbfs_kernel(MsArgs A) {
             const uint32_t ch_incl = warp_incl_scan(nch);
             const uint32_t ch_total = __shfl_sync(0xFFFFFFFFu, ch_incl, 31);
             if (ch_total) {
+                // into the CTA's list, or, once that is full, the grid's
                 uint32_t cb = 0;
                 if (lane == 0)
-                    cb = atomicAdd(chunk_cnt, ch_total);
+                    cb = atomicAdd(&s_nch, ch_total);
                 cb = __shfl_sync(0xFFFFFFFFu, cb, 0);
-                if (cb + ch_total <= A.chunk_cap) {
+                uint4 *list = s_chunks;
+                uint32_t cap = MS_CTA_CHUNKS;
+                if (cb + ch_total > cap) {
+                    if (lane == 0) {
+                        atomicMin(&s_end, cb);  // every later warp finds no room either
+                        cb = atomicAdd(chunk_cnt, ch_total);
+                    }
+                    cb = __shfl_sync(0xFFFFFFFFu, cb, 0);
+                    list = A.chunks;
+                    cap = A.chunk_cap;
+                }
+                if (cb + ch_total <= cap) {
                     const uint32_t pos = cb + ch_incl - nch;
                     for (uint32_t c = 0; c < nch; ++c)
-                        A.chunks[pos + c] = make_uint4(b + c * MS_CHUNK_SLOTS, min(e, b + (c + 1) * MS_CHUNK_SLOTS), g, u);
+                        list[pos + c] = make_uint4(b + c * MS_CHUNK_SLOTS, min(e, b + (c + 1) * MS_CHUNK_SLOTS), g, u);
                     if (nch)
                         len = 0;
                 } else {
-                    for (uint32_t c = cb + lane; c < min(cb + ch_total, A.chunk_cap); c += 32)
-                        A.chunks[c] = make_uint4(0, 0, 0, 0);
+                    for (uint32_t c = cb + lane; c < min(cb + ch_total, cap); c += 32)
+                        list[c] = make_uint4(0, 0, 0, 0);
                 }
             }
             const uint32_t incl = warp_incl_scan(len);
             const uint32_t excl = incl - len;
             const uint32_t total = __shfl_sync(0xFFFFFFFFu, incl, 31);
-            const uint32_t vo = f ? A.voff[g] : 0u;
             for (uint32_t p0 = 0; p0 < total; p0 += 32 * MS_LANE_SLOTS) {
                 uint32_t sl[MS_LANE_SLOTS], rvo[MS_LANE_SLOTS];
                 const MsGraph *gr[MS_LANE_SLOTS];
-                uint64_t fm[MS_LANE_SLOTS];
+                M fm[MS_LANE_SLOTS];
 #pragma unroll
                 for (uint32_t j = 0; j < MS_LANE_SLOTS; ++j) {
                     const uint32_t p = p0 + 32 * j + lane;
@@ -290,112 +470,93 @@ __global__ void __launch_bounds__(BLOCK) msbfs_kernel(MsArgs A) {
                     fm[j] = __shfl_sync(0xFFFFFFFFu, f, r);
                     sl[j] = p < total ? rb + (p - rex) : SIZE_NONE;
                 }
-                traversed += ms_visit<MS_LANE_SLOTS>(A, gr, rvo, sl, fm);
+                traversed += ms_visit<M, MS_LANE_SLOTS>(seen, gr, rvo, sl, fm);
             }
         }
-        if (!dense && !grid_barrier_gen(bar, err))
-            return;
+        if (!dense) {
+            // the CTA's chunks join the grid's list under one atomic
+            __syncthreads();
+            const uint32_t mine = min(s_nch, s_end);
+            __syncthreads();
+            if (threadIdx.x == 0 && mine)
+                s_nch = atomicAdd(chunk_cnt, mine);
+            __syncthreads();
+            for (uint32_t c = threadIdx.x; c < mine; c += BLOCK)
+                if (in_bounds(err, s_nch + c < A.chunk_cap, BS_ROW))  // the list holds every level's chunks
+                    A.chunks[s_nch + c] = s_chunks[c];
+            if (!grid_barrier_gen(bar, err))
+                return;
+        }
         // expand, phase 2: long-row chunks
         const uint32_t nch_all = dense ? 0u : min(cta_broadcast_read(chunk_cnt), A.chunk_cap);
         for (uint32_t c = gwarp; c < nch_all; c += nwarps) {
             const uint4 ch = A.chunks[c];
             if (ch.x >= ch.y)
                 continue;
-            const uint64_t fm = A.frontier[ch.w];
-            const MsGraph &Gr = A.gr[ch.z];
+            const M f = frontier[ch.w];
             const uint32_t vo = A.voff[ch.z];
             uint32_t sl[MS_LANE_SLOTS], cvo[MS_LANE_SLOTS];
             const MsGraph *gr[MS_LANE_SLOTS];
-            uint64_t fms[MS_LANE_SLOTS];
+            M fm[MS_LANE_SLOTS];
 #pragma unroll
             for (uint32_t j = 0; j < MS_LANE_SLOTS; ++j) {
                 const uint32_t sj = ch.x + 32 * j + lane;  // a chunk is one step
                 sl[j] = sj < ch.y ? sj : SIZE_NONE;
                 cvo[j] = vo;
-                gr[j] = &Gr;
-                fms[j] = fm;
+                gr[j] = A.gr + ch.z;
+                fm[j] = f;
             }
-            traversed += ms_visit<MS_LANE_SLOTS>(A, gr, cvo, sl, fms);
+            traversed += ms_visit<M, MS_LANE_SLOTS>(seen, gr, cvo, sl, fm);
         }
         if (!grid_barrier_gen(bar, err))
             return;
-        // commit
-        uint32_t changed = 0;
-        unsigned long long fnext = 0;
-        for (uint32_t w0 = gwarp * 32; w0 < N; w0 += nwarps * 32) {
-            const uint32_t w = w0 + lane;
-            const uint64_t seen = w < N ? A.seen[w] : 0ull;
-            const uint64_t nx = w < N ? seen & ~A.visited[w] : 0ull;
-            if (w < N)
-                A.frontier[w] = nx;
-            if (!__any_sync(0xFFFFFFFFu, nx != 0ull))
-                continue;
-            uint32_t g = 0;
-            if (nx) {
-                A.visited[w] = seen;
-                changed = 1;
-                g = graph_of_node(A, w);
-                fnext += ms_row_slots(A.gr[g], w - A.voff[g]);
-            }
-            // the levels of one mask lane at a time; nodes of several graphs
-            // in the warp (nx != 0 for some of each) graph by graph
-            uint32_t todo = __ballot_sync(0xFFFFFFFFu, nx != 0ull);
-            while (todo) {
-                const uint32_t g0 = __shfl_sync(0xFFFFFFFFu, g, __ffs(todo) - 1);
-                const bool mine = nx && g == g0;
-                todo &= ~__ballot_sync(0xFFFFFFFFu, mine);
-                const MsGraph &Gr = A.gr[g0];
-                if (!Gr.levels)
-                    continue;
-                uint32_t *lv = Gr.levels + (w - A.voff[g0]);
-                uint64_t any = ((uint64_t)__reduce_or_sync(0xFFFFFFFFu, mine ? (uint32_t)(nx >> 32) : 0u) << 32) |
-                               __reduce_or_sync(0xFFFFFFFFu, mine ? (uint32_t)nx : 0u);
-                while (any) {
-                    const int bit = __ffsll((long long)any) - 1;
-                    any &= any - 1;
-                    if (mine && ((nx >> bit) & 1))
-                        lv[(size_t)bit * Gr.n] = level + 1;
-                }
-            }
-        }
-        if (__syncthreads_or(changed) && threadIdx.x == 0)
-            atomicAdd(A.ctl + MS_CHANGE + level % 3, 1u);
-#pragma unroll
-        for (int d = 16; d >= 1; d >>= 1)
-            fnext += __shfl_xor_sync(0xFFFFFFFFu, fnext, d);
-        if (lane == 0 && fnext)
-            atomicAdd(fslots(A, level + 1), fnext);
+        ms_commit<M>(A, level + 1, N, gwarp, nwarps, lane);
         if (!grid_barrier_gen(bar, err))
             return;
         if (cta_broadcast_read(A.ctl + MS_CHANGE + level % 3) == 0)
             break;
     }
-    // reached (graph, lane) counts, and level 0 where a lane never came: each
-    // CTA walks a contiguous node range graph by graph, a warp 32 nodes at a
-    // time, mask lane by mask lane (one vote per lane of the mask counts 32
-    // nodes; lane l of the warp keeps mask lanes l and l + 32)
+    // reached (graph, lane) counts, and the levels from their planes (0 where a
+    // lane never came): each CTA walks a contiguous node range graph by graph,
+    // a warp 32 nodes at a time. Transposed over the warp, lane l's word holds
+    // mask lane l of the 32 nodes, so one population count serves 32 of them
+    // (a vote per mask lane took 109 us on 3M nodes and 64 lanes).
     __shared__ unsigned int cnt[64];
     const uint32_t per = (N + gridDim.x - 1) / gridDim.x;
     const uint32_t lo = min(N, blockIdx.x * per), hi = min(N, lo + per);
+    const M *visited = (const M *)A.visited, *planes = (const M *)A.planes;
+    // planes in use: every level is at most level + 1 (the last commit found nothing)
+    const uint32_t np = min(MS_PLANES, 32u - __clz(level + 1));
     uint32_t pos = lo;
     while (__syncthreads_or(pos < hi)) {
         const uint32_t g = graph_of_node(A, pos);
         const uint32_t end = min(hi, A.voff[g + 1]);
-        const MsGraph &Gr = A.gr[g];
+        const uint32_t nsrc = A.gr[g].nsrc, n = A.gr[g].n;
+        uint32_t *levels = A.gr[g].levels;
+        const uint32_t v0 = A.voff[g];
         if (threadIdx.x < 64)
             cnt[threadIdx.x] = 0;
         __syncthreads();
         uint32_t c0 = 0, c1 = 0;
         for (uint32_t w0 = pos + (threadIdx.x & ~31u); w0 < end; w0 += BLOCK) {
             const uint32_t w = w0 + lane;
-            const uint64_t m = w < end ? A.visited[w] : 0ull;
-            for (uint32_t j = 0; j < Gr.nsrc; ++j) {
-                const bool in = (m >> j) & 1;
-                const uint32_t c = __popc(__ballot_sync(0xFFFFFFFFu, in));
-                c0 += j == lane ? c : 0u;
-                c1 += j == lane + 32 ? c : 0u;
-                if (Gr.levels && !in && w < end)
-                    Gr.levels[(size_t)j * Gr.n + (w - A.voff[g])] = 0;
+            const M m = w < end ? visited[w] : M(0);
+            c0 += __popc(warp_transpose((uint32_t)m, lane));
+            if (sizeof(M) == 8)
+                c1 += __popc(warp_transpose((uint32_t)((uint64_t)m >> 32), lane));
+            if (!levels || w >= end)
+                continue;
+            M pl[MS_PLANES];
+#pragma unroll
+            for (uint32_t b = 0; b < MS_PLANES; ++b)
+                pl[b] = b < np ? planes[(size_t)b * N + w] : M(0);
+            for (uint32_t j = 0; j < nsrc; ++j) {
+                uint32_t lv = 0;
+#pragma unroll
+                for (uint32_t b = 0; b < MS_PLANES; ++b)
+                    lv |= (uint32_t)((pl[b] >> j) & 1) << b;
+                if (lv != 0 || !((m >> j) & 1))  // else a deep level, already written
+                    levels[(size_t)j * n + (w - v0)] = lv;
             }
         }
         if (c0)
@@ -416,20 +577,25 @@ __global__ void __launch_bounds__(BLOCK) msbfs_kernel(MsArgs A) {
         A.ctl[MS_LEVELS] = level;
 }
 
-int g_ms_fit[64] = {};  // resident CTAs per SM, per device
+const void *ms_kernel_ptr(bool wide) {
+    return wide ? (const void *)msbfs_kernel<uint64_t> : (const void *)msbfs_kernel<uint32_t>;
+}
 
-int ms_grid_size(int sms) {
+int g_ms_fit[64][2] = {};  // resident CTAs per SM of the two mask widths, per device
+
+int ms_grid_size(int sms, bool wide) {
     int dev = 0;
     cudaGetDevice(&dev);
     if (dev < 0 || dev >= 64)
         dev = 0;
-    if (g_ms_fit[dev] == 0) {
+    int &fit = g_ms_fit[dev][wide];
+    if (fit == 0) {
         int per_sm = 0;
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, msbfs_kernel, BLOCK, 0) != cudaSuccess)
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, ms_kernel_ptr(wide), BLOCK, 0) != cudaSuccess)
             return 0;
-        g_ms_fit[dev] = std::min(per_sm, MAX_BLOCKS_PER_SM);
+        fit = std::min(per_sm, MAX_BLOCKS_PER_SM);
     }
-    return sms * blocks_per_sm(g_ms_fit[dev], g_tuning.ms_blocks_per_sm);
+    return sms * blocks_per_sm(fit, g_tuning.ms_blocks_per_sm);
 }
 
 }  // namespace
@@ -437,6 +603,8 @@ int ms_grid_size(int sms) {
 void free_batch_bfs(gpma_batch *b) {
     for (int i = 0; i < 3; ++i)
         dev_free(b->ms_mask[i]);
+    dev_free(b->ms_planes);
+    b->ms_planes_cap = 0;
     dev_free(b->ms_tab);
     if (b->h_ms_tab)
         cudaFreeHost(b->h_ms_tab);
@@ -478,7 +646,12 @@ gpma_status batch_bfs_plan(gpma_batch *b, gpma_graph *const *graphs, const uint3
                            const uint32_t *nsrc, uint32_t k, uint32_t *const *stage, BatchBfsPlan *P,
                            const uint32_t *abort) {
     static_assert(sizeof(MsArgs) <= KernelLaunch::ARG_BYTES, "multi-source BFS arguments exceed the launch record");
-    const int grid = ms_grid_size(b->sms);
+    // masks of 32 bits where no graph has more than 32 sources: half the mask
+    // bytes of every commit, gather and plane
+    bool wide = false;
+    for (uint32_t i = 0; i < k; ++i)
+        wide = wide || nsrc[i] > 32;
+    const int grid = ms_grid_size(b->sms, wide);
     if (grid == 0) {
         set_error("multi-source BFS kernel cannot be resident");
         return GPMA_ERR_CUDA;
@@ -495,6 +668,16 @@ gpma_status batch_bfs_plan(gpma_batch *b, gpma_graph *const *graphs, const uint3
         for (int i = 0; i < 3; ++i)
             GPMA_TRY(dev_alloc(&b->ms_mask[i], std::max<uint64_t>(N, 1)));
         b->ms_cap = std::max<uint64_t>(N, 1);
+    }
+    bool any_levels = false;
+    for (uint32_t i = 0; stage && i < k; ++i)
+        any_levels = any_levels || stage[i];
+    const uint64_t plane_bytes = any_levels ? (wide ? 8 : 4) * MS_PLANES * N : 0;
+    if (plane_bytes > b->ms_planes_cap) {
+        dev_free(b->ms_planes);
+        b->ms_planes_cap = 0;
+        GPMA_TRY(dev_alloc(&b->ms_planes, plane_bytes));
+        b->ms_planes_cap = plane_bytes;
     }
     const MsTabLayout lay(k);
     if (k > b->ms_gcap || !b->ms_tab) {
@@ -565,13 +748,14 @@ gpma_status batch_bfs_plan(gpma_batch *b, gpma_graph *const *graphs, const uint3
     A.visited = b->ms_mask[0];
     A.frontier = b->ms_mask[1];
     A.seen = b->ms_mask[2];
+    A.planes = any_levels ? b->ms_planes : nullptr;
     A.chunks = reinterpret_cast<uint4 *>(b->ms_chunks);
     A.chunk_cap = (uint32_t)std::min<uint64_t>(b->ms_chunk_cap, 0xFFFFFFFFull);
     A.ctl = b->ms_ctl;
     A.reached = reinterpret_cast<unsigned long long *>(b->ms_reached);
     A.traversed = reinterpret_cast<unsigned long long *>(b->ms_reached) + 64ull * k;
     A.abort = abort;
-    P->main.set((const void *)msbfs_kernel, grid, 0, &A, sizeof(A));
+    P->main.set(ms_kernel_ptr(wide), grid, 0, &A, sizeof(A));
     P->ctl_bytes = sizeof(uint32_t) * MS_CTL_WORDS;
     P->reached_bytes = sizeof(unsigned long long) * (64ull * k + 1);
     return GPMA_OK;

@@ -62,3 +62,20 @@ def test_levels_and_counts_equal_oracle(built_lib, k, dense_div):
         G.set_tuning(**old)
     for g, _, _ in gs:
         g.close()
+
+
+@pytest.mark.parametrize("k", [5, 40])
+@pytest.mark.parametrize("n", [62, 63, 64, 65, 300])
+def test_levels_of_long_paths(built_lib, k, n):
+    """Depths around the number of levels the bit planes hold (63) and far past it."""
+    import gpma_bfs_gb300 as G
+
+    i = np.arange(n - 1, dtype=np.uint32)
+    keys = np.concatenate([G.edges_to_keys(i, i + 1), G.edges_to_keys(np.uint32([n - 1]), np.uint32([0]))])
+    g = G.GPMA(n)
+    G.update_gpma(g, keys, np.ones(len(keys), np.uint8))
+    src = (np.arange(k) * 7 % n).astype(np.uint32)
+    levels, reached = G.gpma_bfs_multi(g, src)
+    want = (np.arange(n)[None, :] - src[:, None].astype(np.int64)) % n + 1
+    assert np.array_equal(levels, want) and all(int(r) == n for r in reached)
+    g.close()
