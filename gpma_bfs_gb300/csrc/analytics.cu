@@ -34,9 +34,10 @@ enum : uint32_t {
     AN_ROOTS = 2,    // components counted
     AN_CHUNKS = 3,   // PageRank by gathering: chunks of long in-edge rows
     AN_MULTI = 4,    // ... and rows of more than one chunk
-    AN_BAR = 6,      // GridBarrier (2 words)
     AN_DBL = 8,      // doubles from word 8: dangling[3], delta[3]
-    AN_WORDS = 8 + 12,
+    AN_WORDS = 8 + 12,        // what the host reads
+    AN_BAR = BAR_ALIGN_WORDS, // GridBarrier
+    AN_ALL = AN_BAR + BAR_WORDS,
 };
 
 constexpr int AN_MAX_FIT = 8;  // CTAs per SM
@@ -661,12 +662,12 @@ gpma_status an_buffers(gpma_graph *g, uint32_t **base, uint32_t **ctl) {
     if (!g->an_buf || g->an_cap < n) {
         dev_free(g->an_buf);
         g->an_cap = 0;
-        GPMA_TRY(dev_alloc(&g->an_buf, 5ull * n + an_cta_words(g) + AN_WORDS + 2));
+        GPMA_TRY(dev_alloc(&g->an_buf, 5ull * n + an_cta_words(g) + AN_ALL + BAR_ALIGN_WORDS));
         g->an_cap = n;
     }
     *base = g->an_buf;
-    // 8-byte aligned: the control words hold doubles
-    *ctl = g->an_buf + ((5ull * n + an_cta_words(g) + 1) & ~1ull);
+    // on a line of their own, as the barrier among them wants
+    *ctl = g->an_buf + ((5ull * n + an_cta_words(g) + BAR_ALIGN_WORDS - 1) & ~uint64_t(BAR_ALIGN_WORDS - 1));
     return GPMA_OK;
 }
 
@@ -699,7 +700,7 @@ gpma_status gpma_pagerank(gpma_graph *g, float damping, uint32_t iterations, dou
     gpma_status st = [&]() -> gpma_status {
         uint32_t *base = nullptr, *ctl = nullptr;
         GPMA_TRY(an_buffers(g, &base, &ctl));
-        GPMA_CUDA(cudaMemsetAsync(ctl, 0, sizeof(uint32_t) * AN_WORDS, s));
+        GPMA_CUDA(cudaMemsetAsync(ctl, 0, sizeof(uint32_t) * AN_ALL, s));
         AnArgs A{};
         A.keys = g->keys;
         A.vals = g->values;
@@ -759,7 +760,7 @@ gpma_status gpma_components(gpma_graph *g, uint32_t *labels, uint64_t *component
         uint32_t *base = nullptr, *ctl = nullptr;
         GPMA_TRY(an_buffers(g, &base, &ctl));
         uint32_t *parent = base;
-        GPMA_CUDA(cudaMemsetAsync(ctl, 0, sizeof(uint32_t) * AN_WORDS, s));
+        GPMA_CUDA(cudaMemsetAsync(ctl, 0, sizeof(uint32_t) * AN_ALL, s));
         AnArgs A{};
         A.keys = g->keys;
         A.vals = g->values;

@@ -41,10 +41,11 @@ enum : uint32_t {
     CTL_LEVELS = 7,
     CTL_REACHED = 8,
     CTL_OVERFLOW = 9, // times a warp found the chunk list full and walked its long rows in place
-    CTL_BAR = 10,     // GridBarrier (2 words)
     CTL_SLOTS = 12,   // 3 rotating counters: slots of the current frontier's rows (measured levels)
-    CTL_WORDS = 16,
-    // profiling record after the control words: u64 start stamp of each level
+    CTL_WORDS = 16,   // what the host reads
+    CTL_BAR = BAR_ALIGN_WORDS,  // GridBarrier
+    CTL_ALL = CTL_BAR + BAR_WORDS,
+    // profiling record after those: u64 start stamp of each level
     // (and of the final check), then u32 per level: frontier size | dense << 31
     CTL_PROFILE_LEVELS = 64,
     CTL_PROFILE_WORDS = 3 * CTL_PROFILE_LEVELS,
@@ -474,9 +475,9 @@ gpma_status ensure_bfs(gpma_graph *g) {
     GPMA_TRY(dev_alloc(&g->bfs_visited, n / 32 + 2));
     GPMA_TRY(dev_alloc(&g->bfs_front[0], n / 32 + 2));
     GPMA_TRY(dev_alloc(&g->bfs_front[1], n / 32 + 2));
-    GPMA_TRY(dev_alloc(&g->bfs_ctl, CTL_WORDS + CTL_PROFILE_WORDS));
+    GPMA_TRY(dev_alloc(&g->bfs_ctl, CTL_ALL + CTL_PROFILE_WORDS));
     if (!g->h_bfs_ctl) {
-        cudaError_t e = cudaMallocHost((void **)&g->h_bfs_ctl, sizeof(uint32_t) * (CTL_WORDS + CTL_PROFILE_WORDS));
+        cudaError_t e = cudaMallocHost((void **)&g->h_bfs_ctl, sizeof(uint32_t) * (CTL_ALL + CTL_PROFILE_WORDS));
         if (e != cudaSuccess)
             return cuda_fail(e, "cudaMallocHost(bfs ctl)");
     }
@@ -518,7 +519,7 @@ gpma_status bfs_plan(gpma_graph *g, uint32_t src, BfsPlan *P) {
     const uint32_t n = g->row_num;
     const size_t bitmap = sizeof(uint32_t) * (n / 32 + 2);
     void *ptr[BfsPlan::CLEARS] = {g->bfs_levels, g->bfs_visited, g->bfs_ctl, g->bfs_front[0], g->bfs_front[1]};
-    const size_t bytes[BfsPlan::CLEARS] = {sizeof(uint32_t) * n, bitmap, sizeof(uint32_t) * CTL_WORDS, bitmap, bitmap};
+    const size_t bytes[BfsPlan::CLEARS] = {sizeof(uint32_t) * n, bitmap, sizeof(uint32_t) * CTL_ALL, bitmap, bitmap};
     for (int i = 0; i < BfsPlan::CLEARS; ++i) {
         P->clear_ptr[i] = ptr[i];
         P->clear_bytes[i] = bytes[i];
@@ -544,12 +545,12 @@ gpma_status bfs_plan(gpma_graph *g, uint32_t src, BfsPlan *P) {
     A.chunk_cap = g->bfs_chunk_cap;
     A.ctl = g->bfs_ctl;
     A.dense_div = g_tuning.bfs_dense_div;
-    A.stamps = g->profiling ? reinterpret_cast<unsigned long long *>(g->bfs_ctl + CTL_WORDS) : nullptr;
+    A.stamps = g->profiling ? reinterpret_cast<unsigned long long *>(g->bfs_ctl + CTL_ALL) : nullptr;
     A.stall = g_test_hooks.bfs_stall;
     A.stall_limit_ns = g_test_hooks.bfs_stall ? g_test_hooks.wait_limit_ns : WAIT_LIMIT_NS;
     P->main.set((const void *)bfs_kernel, g->sms * blocks_per_sm(g->bfs_grid, g_tuning.bfs_blocks_per_sm), 0, &A,
                 sizeof(A));
-    P->ctl_bytes = sizeof(uint32_t) * (CTL_WORDS + (g->profiling ? CTL_PROFILE_WORDS : 0));
+    P->ctl_bytes = sizeof(uint32_t) * (g->profiling ? CTL_ALL + CTL_PROFILE_WORDS : CTL_WORDS);
     return GPMA_OK;
 }
 
@@ -594,7 +595,7 @@ namespace {
 constexpr uint32_t NOALLOC_MAX_ROWS = 1u << 21;  // 2,097,152 nodes
 constexpr uint32_t NOALLOC_BITMAP_WORDS = NOALLOC_MAX_ROWS / 32 + 2;
 constexpr uint32_t NOALLOC_CHUNK_CAP = 1u << 16;  // more big-row chunks are walked in place
-constexpr size_t NOALLOC_WORDS = CTL_WORDS + 3ull * NOALLOC_BITMAP_WORDS + 2ull * NOALLOC_CHUNK_CAP;
+constexpr size_t NOALLOC_WORDS = CTL_ALL + 3ull * NOALLOC_BITMAP_WORDS + 2ull * NOALLOC_CHUNK_CAP;
 constexpr int NOALLOC_MAX_DEVICES = 64;
 
 static __device__ __align__(256) uint32_t g_noalloc_scratch[NOALLOC_WORDS];
@@ -647,7 +648,7 @@ gpma_status bfs_noalloc_run(gpma_graph *g, uint32_t src, uint32_t *levels, uint6
     int grid = 0;
     GPMA_TRY(noalloc_scratch(&scratch, &grid, g->sms));
     uint32_t *ctl = scratch;
-    uint32_t *visited = scratch + CTL_WORDS;
+    uint32_t *visited = scratch + CTL_ALL;
     uint32_t *front0 = visited + NOALLOC_BITMAP_WORDS;
     uint32_t *front1 = front0 + NOALLOC_BITMAP_WORDS;
     uint2 *chunks = reinterpret_cast<uint2 *>(front1 + NOALLOC_BITMAP_WORDS);
@@ -656,7 +657,7 @@ gpma_status bfs_noalloc_run(gpma_graph *g, uint32_t src, uint32_t *levels, uint6
     GPMA_CUDA(cudaMemsetAsync(visited, 0, sizeof(uint32_t) * (n / 32 + 2), s));
     GPMA_CUDA(cudaMemsetAsync(front0, 0, sizeof(uint32_t) * (n / 32 + 2), s));
     GPMA_CUDA(cudaMemsetAsync(front1, 0, sizeof(uint32_t) * (n / 32 + 2), s));
-    GPMA_CUDA(cudaMemsetAsync(ctl, 0, sizeof(uint32_t) * CTL_WORDS, s));
+    GPMA_CUDA(cudaMemsetAsync(ctl, 0, sizeof(uint32_t) * CTL_ALL, s));
     bfs_init_kernel<<<1, 1, 0, s>>>(levels, visited, front0, ctl, src);
     BfsArgs A;
     memset(&A, 0, sizeof(A));
@@ -703,7 +704,7 @@ extern "C" gpma_status gpma_bfs_level_profile(const gpma_graph *g, double *ms, u
     if (!g->profiling || !g->h_bfs_ctl)
         return GPMA_OK;
     const uint32_t L = std::min<uint32_t>(g->h_bfs_ctl[CTL_LEVELS], CTL_PROFILE_LEVELS - 1);
-    const uint64_t *st = reinterpret_cast<const uint64_t *>(g->h_bfs_ctl + CTL_WORDS);
+    const uint64_t *st = reinterpret_cast<const uint64_t *>(g->h_bfs_ctl + CTL_ALL);
     const uint32_t *info = reinterpret_cast<const uint32_t *>(st + CTL_PROFILE_LEVELS);
     *levels = L;
     for (uint32_t i = 0; i < std::min(L, capacity); ++i) {

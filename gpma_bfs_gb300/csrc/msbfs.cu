@@ -34,9 +34,10 @@ enum : uint32_t {
     MS_CHUNKS = 3,  // 3 rotating chunk counters
     MS_ERR = 6,
     MS_LEVELS = 7,
-    MS_BAR = 10,    // GridBarrier (2 words)
     MS_FSLOTS = 16, // 3 rotating u64 counters (words 16..21): slots of the rows in the next union frontier
-    MS_CTL_WORDS = 24,
+    MS_CTL_WORDS = 24,          // what the host reads
+    MS_BAR = BAR_ALIGN_WORDS,   // GridBarrier
+    MS_ALL = MS_BAR + BAR_WORDS,
 };
 
 constexpr uint32_t MS_BIG_ROW = 64;
@@ -349,17 +350,17 @@ __global__ void __launch_bounds__(BLOCK) msbfs_kernel(MsArgs A) {
     unsigned long long traversed = 0;
     for (uint32_t w = gtid; w < N; w += nthreads)
         seen[w] = 0;
-    if (!grid_barrier_gen(bar, err))
+    if (!grid_barrier(bar, err))
         return;
     for (uint32_t t = gtid; t < A.G * 64; t += nthreads) {
         const uint32_t g = t >> 6, j = t & 63;
         if (j < A.gr[g].nsrc)
             mask_or(&seen[A.voff[g] + A.src[t]], M(1) << j);
     }
-    if (!grid_barrier_gen(bar, err))
+    if (!grid_barrier(bar, err))
         return;
     ms_commit<M>(A, 1, N, gwarp, nwarps, lane);
-    if (!grid_barrier_gen(bar, err))
+    if (!grid_barrier(bar, err))
         return;
     uint32_t level = 1;
     for (;; ++level) {
@@ -484,7 +485,7 @@ __global__ void __launch_bounds__(BLOCK) msbfs_kernel(MsArgs A) {
             for (uint32_t c = threadIdx.x; c < mine; c += BLOCK)
                 if (in_bounds(err, s_nch + c < A.chunk_cap, BS_ROW))  // the list holds every level's chunks
                     A.chunks[s_nch + c] = s_chunks[c];
-            if (!grid_barrier_gen(bar, err))
+            if (!grid_barrier(bar, err))
                 return;
         }
         // expand, phase 2: long-row chunks
@@ -508,10 +509,10 @@ __global__ void __launch_bounds__(BLOCK) msbfs_kernel(MsArgs A) {
             }
             traversed += ms_visit<M, MS_LANE_SLOTS>(seen, gr, cvo, sl, fm);
         }
-        if (!grid_barrier_gen(bar, err))
+        if (!grid_barrier(bar, err))
             return;
         ms_commit<M>(A, level + 1, N, gwarp, nwarps, lane);
-        if (!grid_barrier_gen(bar, err))
+        if (!grid_barrier(bar, err))
             return;
         if (cta_broadcast_read(A.ctl + MS_CHANGE + level % 3) == 0)
             break;
@@ -703,7 +704,7 @@ gpma_status batch_bfs_plan(gpma_batch *b, gpma_graph *const *graphs, const uint3
         b->ms_chunk_cap = ms_chunk_need(slots);
     }
     if (!b->ms_ctl) {
-        GPMA_TRY(dev_alloc(&b->ms_ctl, MS_CTL_WORDS));
+        GPMA_TRY(dev_alloc(&b->ms_ctl, MS_ALL));
         GPMA_CUDA(cudaMallocHost((void **)&b->h_ms_ctl, sizeof(uint32_t) * MS_CTL_WORDS));
     }
     // the table, in the pinned mirror (the previous call's upload has finished)
@@ -731,7 +732,7 @@ gpma_status batch_bfs_plan(gpma_batch *b, gpma_graph *const *graphs, const uint3
     }
     P->tab_bytes = lay.bytes;
     void *ptr[BatchBfsPlan::CLEARS] = {b->ms_ctl, b->ms_reached};  // the kernel clears the masks
-    const size_t bytes[BatchBfsPlan::CLEARS] = {sizeof(uint32_t) * MS_CTL_WORDS,
+    const size_t bytes[BatchBfsPlan::CLEARS] = {sizeof(uint32_t) * MS_ALL,
                                                 sizeof(unsigned long long) * (64ull * k + 1)};
     for (int i = 0; i < BatchBfsPlan::CLEARS; ++i) {
         P->clear_ptr[i] = ptr[i];

@@ -103,6 +103,7 @@ struct UpdateArgs {
     uint32_t *chunk_cnt;
     uint32_t *cta_cnt;
     DeviceStatus *st;
+    GridBarrier *bar;
     // clean-up for the next launch: the other status slot (as words) and the
     // sort state this launch used
     uint32_t *next_slot;
@@ -764,7 +765,7 @@ __device__ bool grid_windows(const UpdateArgs &A, Windows L, uint32_t r0, uint32
         if (threadIdx.x == 0)
             A.chunk_cnt[c] = t;
     }
-    if (!grid_barrier(&A.st->bar, &A.st->err))
+    if (!grid_barrier(A.bar, &A.st->err))
         return false;
     // B2: per window, chunk offsets, live total and the density decision
     for (uint32_t w = r0 + blockIdx.x; w < r1; w += gridDim.x) {
@@ -791,7 +792,7 @@ __device__ bool grid_windows(const UpdateArgs &A, Windows L, uint32_t r0, uint32
                 ++acc;
         }
     }
-    if (!grid_barrier(&A.st->bar, &A.st->err))
+    if (!grid_barrier(A.bar, &A.st->err))
         return false;
     // B3: stable compaction of accepted windows into the graph's scratch arrays
     for (uint32_t c = blockIdx.x; c < total; c += gridDim.x) {
@@ -821,7 +822,7 @@ __device__ bool grid_windows(const UpdateArgs &A, Windows L, uint32_t r0, uint32
             }
         }
     }
-    if (!grid_barrier(&A.st->bar, &A.st->err))
+    if (!grid_barrier(A.bar, &A.st->err))
         return false;
     // B4: merge with the window's insertions and redispatch chunk by chunk
     uint64_t *mk = reinterpret_cast<uint64_t *>(smem);
@@ -1008,12 +1009,12 @@ __global__ void __launch_bounds__(BLOCK, MINB) update_kernel(UpdateArgs A) {
     bool digits = A.q.nq == 0;
     if (!digits) {
         bsort_rank(A.in_k, A.boff, A.G, A.gd, A.q, st);
-        if (!grid_barrier(&st->bar, &st->err, A.stall, A.stall_limit_ns))
+        if (!grid_barrier(A.bar, &st->err, A.stall, A.stall_limit_ns))
             return;
         if (ld_volatile(&st->invalid_keys) != 0)
             return;  // reserved-column keys: reject the batch before any change
         bsort_scan(A.q, A.cta_cnt, st, tmp);
-        if (!grid_barrier(&st->bar, &st->err))
+        if (!grid_barrier(A.bar, &st->err))
             return;
         digits = cta_broadcast_read(&st->sort_fallback) != 0;
         if (!digits) {
@@ -1021,16 +1022,16 @@ __global__ void __launch_bounds__(BLOCK, MINB) update_kernel(UpdateArgs A) {
             uint32_t *cpre = reinterpret_cast<uint32_t *>(smem + BSORT_SMEM_ITEM);
             bsort_chunk_prefix(A.cta_cnt, cpre, tmp);
             bsort_scatter(A.in_k, A.in_v, A.boff, A.G, A.q, cpre);
-            if (!grid_barrier(&st->bar, &st->err))
+            if (!grid_barrier(A.bar, &st->err))
                 return;
             bsort_items(A.bk[0], A.bv[1], A.boff, A.G, A.q, cpre, smem);
-            if (!grid_barrier(&st->bar, &st->err))
+            if (!grid_barrier(A.bar, &st->err))
                 return;
         }
     }
     if (digits) {
         sort_histogram(A.in_k, A.boff, A.G, A.sort_hist, st, reinterpret_cast<uint32_t *>(smem));
-        if (!grid_barrier(&st->bar, &st->err, A.q.nq == 0 ? A.stall : 0u, A.stall_limit_ns))
+        if (!grid_barrier(A.bar, &st->err, A.q.nq == 0 ? A.stall : 0u, A.stall_limit_ns))
             return;
         if (ld_volatile(&st->invalid_keys) != 0)
             return;  // reserved-column keys: reject the batch before any change
@@ -1054,7 +1055,7 @@ __global__ void __launch_bounds__(BLOCK, MINB) update_kernel(UpdateArgs A) {
                     sort_tile(p, tile, ink, inv, outk, outv, A.boff, A.toff, A.G, A.sort_hist, A.sort_status, st, smem,
                               tmp);
                 sel ^= 1u;
-                if (!grid_barrier(&st->bar, &st->err))
+                if (!grid_barrier(A.bar, &st->err))
                     return;
             }
         }
@@ -1148,7 +1149,7 @@ __global__ void __launch_bounds__(BLOCK, MINB) update_kernel(UpdateArgs A) {
             }
         }
     }
-    if (!grid_barrier(&st->bar, &st->err))
+    if (!grid_barrier(A.bar, &st->err))
         return;
     {
         // every CTA is past the sort (trivial-digit mask, passes): zero its
@@ -1180,7 +1181,7 @@ __global__ void __launch_bounds__(BLOCK, MINB) update_kernel(UpdateArgs A) {
         const uint32_t t = block_sum(cl, tmp);
         if (threadIdx.x == 0)
             CNT(scan_id)[blockIdx.x] = t;
-        if (!grid_barrier(&st->bar, &st->err))
+        if (!grid_barrier(A.bar, &st->err))
             return;
     }
     uint32_t base, m, unused_b, unused_t;
@@ -1220,7 +1221,7 @@ __global__ void __launch_bounds__(BLOCK, MINB) update_kernel(UpdateArgs A) {
         if (threadIdx.x == 0)
             CNT(scan_id ^ 1)[blockIdx.x] = t;
     }
-    if (!grid_barrier(&st->bar, &st->err))
+    if (!grid_barrier(A.bar, &st->err))
         return;
     if (A.G == 1 && m >= SIGNIFICANT_INSERTS) {
         if (stamper) {
@@ -1333,7 +1334,7 @@ __global__ void __launch_bounds__(BLOCK, MINB) update_kernel(UpdateArgs A) {
         base += tot;
     }
     scan_id ^= 1;
-    if (!grid_barrier(&st->bar, &st->err))
+    if (!grid_barrier(A.bar, &st->err))
         return;
     if (stamper)
         st->stamp[3] = globaltimer_ns();
@@ -1417,7 +1418,7 @@ __global__ void __launch_bounds__(BLOCK, MINB) update_kernel(UpdateArgs A) {
         }
         if (fused)  // the CTA's own range was dispatched (and flagged) by its own warps
             count_rejected(A, L, level, lo, hi, true, CNT(scan_id), CNTI(scan_id));
-        if (!grid_barrier(&st->bar, &st->err))
+        if (!grid_barrier(A.bar, &st->err))
             return;
         // Next level. Rejected windows keep their insertions, which are
         // compacted into the other buffer (new offsets from one scan over the
@@ -1435,7 +1436,7 @@ __global__ void __launch_bounds__(BLOCK, MINB) update_kernel(UpdateArgs A) {
         uint8_t *nv = nxt ? A.ivals[1] : A.ivals[0];
         if (!fused) {
             count_rejected(A, L, level, lo, hi, false, CNT(scan_id), CNTI(scan_id));
-            if (!grid_barrier(&st->bar, &st->err))
+            if (!grid_barrier(A.bar, &st->err))
                 return;
         }
         uint32_t nw_next, base_i, total_i;
@@ -1602,7 +1603,7 @@ __global__ void __launch_bounds__(BLOCK, MINB) update_kernel(UpdateArgs A) {
                 SLICES((level + 1) & 1)[2 * blockIdx.x] = olo;
                 SLICES((level + 1) & 1)[2 * blockIdx.x + 1] = ohi;
             }
-        } else if (!grid_barrier(&st->bar, &st->err)) {
+        } else if (!grid_barrier(A.bar, &st->err)) {
             return;
         }
         nw = nw_next;
@@ -2705,7 +2706,8 @@ gpma_status ensure_buffers(BatchBuffers &b, uint64_t n, uint32_t graphs) {
         b.boff = b.toff = b.qoff = b.qtoff = nullptr;
         b.gcap = 0;
         const size_t tab = sizeof(GraphDesc) * gc + 4 * sizeof(uint32_t) * (gc + 1);
-        const size_t slot = (STAT_GS_OFFSET + sizeof(GraphStatus) * gc + 255) & ~size_t(255);
+        const size_t bar = (STAT_GS_OFFSET + sizeof(GraphStatus) * gc + 127) & ~size_t(127);
+        const size_t slot = (bar + sizeof(GridBarrier) + 255) & ~size_t(255);
         GPMA_TRY(dev_alloc(&b.d_tab, tab));
         GPMA_TRY(dev_alloc(&b.d_stat, 2 * slot));
         cudaError_t e = cudaMallocHost((void **)&b.h_tab, tab);
@@ -2720,6 +2722,7 @@ gpma_status ensure_buffers(BatchBuffers &b, uint64_t n, uint32_t graphs) {
         b.qoff = b.toff + gc + 1;
         b.qtoff = b.qoff + gc + 1;
         b.stat_slot = slot;
+        b.stat_bar = bar;
         b.parity = 0;
         b.dirty = true;
         b.gcap = gc;
@@ -2884,6 +2887,7 @@ gpma_status update_plan(gpma_graph *const *graphs, const uint64_t *off, uint32_t
     A.chunk_cnt = buf.chunk_cnt;
     A.cta_cnt = buf.cta_cnt;
     A.st = reinterpret_cast<DeviceStatus *>(slot);
+    A.bar = reinterpret_cast<GridBarrier *>(slot + buf.stat_bar);
     A.next_slot = reinterpret_cast<uint32_t *>(next);
     A.next_slot_words = (uint32_t)(buf.stat_slot / sizeof(uint32_t));
     A.hist_words = hist_rows * 2048;
