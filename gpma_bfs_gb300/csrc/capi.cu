@@ -411,10 +411,7 @@ gpma_status gpma_bfs(gpma_graph *g, uint32_t src, uint32_t *levels, uint64_t *re
         return GPMA_ERR_INVALID;
     }
     cudaStream_t s = (cudaStream_t)stream;
-    GPMA_TRY(bfs_run(g, src, s, reached));
-    GPMA_TRY(copy_any(levels, g->bfs_levels, sizeof(uint32_t) * g->row_num, s));
-    GPMA_CUDA(cudaStreamSynchronize(s));
-    return GPMA_OK;
+    return bfs_run(g, src, levels, s, reached);
 }
 
 gpma_status gpma_validate(gpma_graph *g, uint64_t *bad, void *stream) {

@@ -209,6 +209,7 @@ struct BatchBuffers {
     // persistent-kernel scratch
     uint32_t *cta_cnt = nullptr;       // 8 * grid: four count arrays, two window-range arrays
 };
+constexpr uint32_t BFS_MAPS = 4;  // node bitmaps of a single-source BFS
 constexpr size_t STAT_GS_OFFSET = 128;
 static_assert(sizeof(DeviceStatus) <= STAT_GS_OFFSET, "status slot layout");
 
@@ -234,13 +235,14 @@ struct gpma_graph {
     gpma::BatchBuffers buf;           // single-graph update buffers
     // BFS state
     uint32_t bfs_cap = 0;
-    uint32_t *bfs_visited = nullptr;   // row_num/32 + 2 words
-    uint32_t *bfs_front[2] = {nullptr, nullptr};  // frontier bitmaps, row_num/32 + 2 words
-    uint2 *bfs_chunks = nullptr;       // big-row chunk list
-    uint32_t bfs_chunk_cap = 0;        // its entries: size / 16 + 1024, more than one level can queue
-    uint32_t *bfs_levels = nullptr;
+    uint32_t *bfs_map = nullptr;       // BFS_MAPS bitmaps of row_num/32 + 2 words
+    uint2 *bfs_items = nullptr;        // work items of a level
+    uint32_t bfs_item_cap = 0;         // its entries, as many as one level can queue
+    uint32_t *bfs_levels = nullptr;    // levels on their way to host memory
+    uint32_t bfs_levels_cap = 0;
     uint32_t *bfs_ctl = nullptr;       // counters + status
-    uint32_t *h_bfs_ctl = nullptr;     // pinned
+    uint32_t *h_bfs_ctl = nullptr;     // pinned; the kernel writes its control words here at its end
+    bool bfs_dirty = true;             // bfs_ctl must be cleared before the next launch
     int bfs_grid = 0;                  // resident BFS-kernel CTAs per SM (0: not yet known)
     gpma_batch *own_batch = nullptr;   // multi-source BFS context of this graph
     uint32_t *an_buf = nullptr;        // analytics: 4 x row_num words + control words, kept between calls
@@ -440,30 +442,20 @@ size_t update_status_bytes(uint32_t k);
 gpma_status update_finish(gpma_graph *const *graphs, uint32_t k, BatchBuffers &buf, const unsigned char *stat,
                           cudaStream_t s, gpma_profile *prof, double kernel_ms);
 bool update_needs_host(const unsigned char *stat, uint32_t k);
-gpma_status bfs_run(gpma_graph *g, uint32_t src, cudaStream_t s, uint64_t *reached);
-// The host parts of bfs_run, for callers that enqueue it themselves: the
-// buffers to zero, the one-thread init kernel (its five arguments) and the
-// cooperative BFS kernel; ctl_bytes of g->bfs_ctl are read back into
-// g->h_bfs_ctl and checked by bfs_finish.
+gpma_status bfs_run(gpma_graph *g, uint32_t src, uint32_t *levels, cudaStream_t s, uint64_t *reached);
+// The host parts of bfs_run, for callers that enqueue it themselves: bfs_plan
+// sizes the buffers and records the cooperative launch (direct: the levels go
+// to `levels` itself, else to g->bfs_levels); bfs_begin readies the control
+// words on the stream before each launch (gate: the status slot of an update
+// enqueued before it, whose call for host work or error keeps the search from
+// running); bfs_finish, after the stream is
+// done, reads what the kernel reported into g->h_bfs_ctl.
 struct BfsPlan {
-    static constexpr int CLEARS = 5;
-    void *clear_ptr[CLEARS];
-    size_t clear_bytes[CLEARS];
-    const void *init_func;
-    uint32_t *init_levels, *init_visited, *init_front0, *init_ctl;
-    uint32_t init_src;
-    void *init_params[5];  // point at the init_* fields when handed to CUDA
     KernelLaunch main;
-    size_t ctl_bytes;
-    void bind_init() {
-        init_params[0] = &init_levels;
-        init_params[1] = &init_visited;
-        init_params[2] = &init_front0;
-        init_params[3] = &init_ctl;
-        init_params[4] = &init_src;
-    }
+    bool direct;
 };
-gpma_status bfs_plan(gpma_graph *g, uint32_t src, BfsPlan *P);
+gpma_status bfs_plan(gpma_graph *g, uint32_t src, uint32_t *levels, BfsPlan *P, const unsigned char *gate = nullptr);
+gpma_status bfs_begin(gpma_graph *g, cudaStream_t s);
 gpma_status bfs_finish(gpma_graph *g, uint64_t *reached);
 gpma_status bfs_noalloc_run(gpma_graph *g, uint32_t src, uint32_t *levels, uint64_t *reached, cudaStream_t s);
 gpma_status batch_bfs_run(gpma_batch *b, gpma_graph *const *graphs, const uint32_t *const *srcs, const uint32_t *nsrc,

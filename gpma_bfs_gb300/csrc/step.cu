@@ -5,20 +5,22 @@
 // and then gpma_bfs for every slide step; each call is a chain of launches,
 // copies and host synchronisations. Here the device work of a whole step is
 // one graph launch:
-//   table upload -> update kernel (cooperative) -> 5 BFS clears -> BFS init ->
-//   BFS kernel (cooperative) -> status and BFS control read-back
-// with a single host synchronisation. The batch upload and the optional copy
+//   table upload -> update kernel (cooperative) -> BFS kernel (cooperative) ->
+//   status read-back
+// with a single host synchronisation (the BFS kernel writes its own result to
+// page-locked memory, and the levels to the caller's array if that is on the
+// device). The batch upload and the optional copy
 // of the levels go on the same stream outside the graph, so the caller's
 // buffers may be pageable, pinned or device memory.
 //
 // The graph is rebuilt only when something baked into its nodes changes
 // (buffers reallocated, the kernel variant or grid, the array geometry
 // enlarging the BFS buffers); the per-step arguments (batch size, status
-// slot, source) are updated in place with cudaGraphExecKernelNodeSetParams.
+// slot, source, levels array) are updated in place with cudaGraphExecKernelNodeSetParams.
 // When the update kernel asks for host work (root resize, the bulk rebuild
 // of a large batch) or fails, the step finishes on the host exactly as
-// update_gpma does and the BFS is run again on the final array, so results
-// are always those of update_gpma followed by gpma_bfs.
+// update_gpma does and the BFS, which returned at once, runs on the final
+// array, so results are always those of update_gpma followed by gpma_bfs.
 #include "gpma_internal.cuh"
 
 #include <new>
@@ -28,19 +30,15 @@ struct gpma_step {
     gpma_graph *g = nullptr;
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
-    cudaGraphNode_t n_update = nullptr, n_init = nullptr, n_bfs = nullptr;
+    cudaGraphNode_t n_update = nullptr, n_bfs = nullptr;
     // what the nodes were built with
     gpma::KernelLaunch upd, bfs;
-    uint32_t *init_args[4] = {};
-    uint32_t init_src = 0;
     struct Baked {
-        const void *h_tab, *d_tab, *d_stat, *bfs_ctl, *h_bfs_ctl;
-        size_t tab_bytes, stat_slot, ctl_bytes;
+        const void *h_tab, *d_tab, *d_stat;
+        size_t tab_bytes, stat_slot;
         const void *upd_func, *bfs_func;
         unsigned upd_grid, bfs_grid;
         size_t upd_smem;
-        void *clear_ptr[gpma::BfsPlan::CLEARS];
-        size_t clear_bytes[gpma::BfsPlan::CLEARS];
     } baked{};
     unsigned char *h_stat = nullptr;  // pinned copy of both status slots
     size_t h_stat_bytes = 0;
@@ -58,7 +56,7 @@ void drop_graph(gpma_step *st) {
         cudaGraphDestroy(st->graph);
     st->exec = nullptr;
     st->graph = nullptr;
-    st->n_update = st->n_init = st->n_bfs = nullptr;
+    st->n_update = st->n_bfs = nullptr;
 }
 
 gpma_step::Baked bake(const gpma_graph *g, size_t tab_bytes, const KernelLaunch &upd, const BfsPlan &bp) {
@@ -67,20 +65,13 @@ gpma_step::Baked bake(const gpma_graph *g, size_t tab_bytes, const KernelLaunch 
     b.h_tab = g->buf.h_tab;
     b.d_tab = g->buf.d_tab;
     b.d_stat = g->buf.d_stat;
-    b.bfs_ctl = g->bfs_ctl;
-    b.h_bfs_ctl = g->h_bfs_ctl;
     b.tab_bytes = tab_bytes;
     b.stat_slot = g->buf.stat_slot;
-    b.ctl_bytes = bp.ctl_bytes;
     b.upd_func = upd.func;
     b.bfs_func = bp.main.func;
     b.upd_grid = upd.grid.x;
     b.bfs_grid = bp.main.grid.x;
     b.upd_smem = upd.smem;
-    for (int i = 0; i < BfsPlan::CLEARS; ++i) {
-        b.clear_ptr[i] = bp.clear_ptr[i];
-        b.clear_bytes[i] = bp.clear_bytes[i];
-    }
     return b;
 }
 
@@ -162,43 +153,15 @@ gpma_status build_graph(gpma_step *st, size_t tab_bytes, KernelLaunch &upd, BfsP
     GPMA_CUDA(cudaGraphAddKernelNode(&st->n_update, st->graph, deps(), ndeps(), &kp));
     GPMA_TRY(set_cooperative(st->n_update));
     prev = st->n_update;
-    for (int i = 0; i < BfsPlan::CLEARS; ++i) {
-        cudaMemsetParams mp{};
-        mp.dst = bp.clear_ptr[i];
-        mp.value = 0;
-        mp.elementSize = 4;  // every cleared buffer is 32-bit words
-        mp.width = bp.clear_bytes[i] / 4;
-        mp.height = 1;
-        mp.pitch = 0;
-        GPMA_CUDA(cudaGraphAddMemsetNode(&node, st->graph, deps(), ndeps(), &mp));
-        prev = node;
-    }
-    bp.bind_init();
-    cudaKernelNodeParams ip{};
-    ip.func = const_cast<void *>(bp.init_func);
-    ip.gridDim = dim3(1, 1, 1);
-    ip.blockDim = dim3(1, 1, 1);
-    ip.sharedMemBytes = 0;
-    ip.kernelParams = bp.init_params;
-    GPMA_CUDA(cudaGraphAddKernelNode(&st->n_init, st->graph, deps(), ndeps(), &ip));
-    prev = st->n_init;
     kp = bp.main.node();
     GPMA_CUDA(cudaGraphAddKernelNode(&st->n_bfs, st->graph, deps(), ndeps(), &kp));
     GPMA_TRY(set_cooperative(st->n_bfs));
     prev = st->n_bfs;
     GPMA_CUDA(cudaGraphAddMemcpyNode1D(&node, st->graph, deps(), ndeps(), st->h_stat, g->buf.d_stat, stat_bytes,
                                        cudaMemcpyDeviceToHost));
-    prev = node;
-    GPMA_CUDA(cudaGraphAddMemcpyNode1D(&node, st->graph, deps(), ndeps(), g->h_bfs_ctl, g->bfs_ctl, bp.ctl_bytes,
-                                       cudaMemcpyDeviceToHost));
     GPMA_CUDA(cudaGraphInstantiate(&st->exec, st->graph, 0));
     st->upd = upd;
     st->bfs = bp.main;
-    st->init_args[0] = bp.init_levels;
-    st->init_args[1] = bp.init_visited;
-    st->init_args[2] = bp.init_front0;
-    st->init_args[3] = bp.init_ctl;
-    st->init_src = bp.init_src;
     st->baked = bake(g, tab_bytes, upd, bp);
     st->stats.builds++;
     return GPMA_OK;
@@ -210,25 +173,6 @@ gpma_status refresh_params(gpma_step *st, KernelLaunch &upd, BfsPlan &bp) {
         cudaKernelNodeParams kp = upd.node();
         GPMA_CUDA(cudaGraphExecKernelNodeSetParams(st->exec, st->n_update, &kp));
         st->upd = upd;
-        st->stats.param_updates++;
-    }
-    const uint32_t *ia[4] = {bp.init_levels, bp.init_visited, bp.init_front0, bp.init_ctl};
-    bool init_same = bp.init_src == st->init_src;
-    for (int i = 0; i < 4; ++i)
-        init_same = init_same && ia[i] == st->init_args[i];
-    if (!init_same) {
-        bp.bind_init();
-        cudaKernelNodeParams ip{};
-        ip.func = const_cast<void *>(bp.init_func);
-        ip.gridDim = dim3(1, 1, 1);
-        ip.blockDim = dim3(1, 1, 1);
-        ip.kernelParams = bp.init_params;
-        GPMA_CUDA(cudaGraphExecKernelNodeSetParams(st->exec, st->n_init, &ip));
-        st->init_args[0] = bp.init_levels;
-        st->init_args[1] = bp.init_visited;
-        st->init_args[2] = bp.init_front0;
-        st->init_args[3] = bp.init_ctl;
-        st->init_src = bp.init_src;
         st->stats.param_updates++;
     }
     if (!bp.main.same(st->bfs)) {
@@ -251,7 +195,8 @@ gpma_status step_run(gpma_step *st, const uint64_t *keys, const uint8_t *values,
     if (n == 0) {
         // nothing to update: the step is the BFS alone
         st->stats.host_runs++;
-        GPMA_TRY(bfs_run(g, src, s, reached));
+        GPMA_TRY(bfs_run(g, src, levels, s, reached));
+        levels = nullptr;  // written
     } else {
         GPMA_TRY(ensure_buffers(g->buf, n, 1));
         GPMA_TRY(copy_any(g->buf.bkeys[0], keys, n * sizeof(uint64_t), s));
@@ -264,7 +209,7 @@ gpma_status step_run(gpma_step *st, const uint64_t *keys, const uint8_t *values,
         BfsPlan bp;
         const bool profiling = g->profiling;
         g->profiling = false;  // no per-level stamps inside a recorded step
-        const gpma_status ps = bfs_plan(g, src, &bp);
+        const gpma_status ps = bfs_plan(g, src, levels, &bp, g->buf.d_stat + g->buf.parity * g->buf.stat_slot);
         g->profiling = profiling;
         GPMA_TRY(ps);
         if (!st->exec || !same_baked(bake(g, tab_bytes, upd, bp), st->baked))
@@ -272,6 +217,7 @@ gpma_status step_run(gpma_step *st, const uint64_t *keys, const uint8_t *values,
         else
             GPMA_TRY(refresh_params(st, upd, bp));
         GPMA_TRY(update_clear(g->buf, s));
+        GPMA_TRY(bfs_begin(g, s));
         const unsigned char *stat = st->h_stat + g->buf.parity * g->buf.stat_slot;
         GPMA_CUDA(cudaEventRecord(st->ev[0], s));
         g->buf.tab_shadow_valid = false;  // the graph uploads its own table
@@ -286,16 +232,19 @@ gpma_status step_run(gpma_step *st, const uint64_t *keys, const uint8_t *values,
         st->stats.last_ms = ms;
         st->stats.total_ms += ms;
         st->stats.graph_launches++;
-        g->prof.kernel_launches += 3;  // update, BFS init, BFS
+        g->prof.kernel_launches += 2;  // update, BFS
         const bool host_work = update_needs_host(stat, 1);
         GPMA_TRY(update_finish(gl, 1, g->buf, stat, s, nullptr, 0.0));
         if (host_work) {
-            // the array changed on the host after the recorded BFS ran: redo it
+            // the array changed on the host: the recorded BFS, which did not run, runs now
             st->stats.host_runs++;
-            GPMA_TRY(bfs_run(g, src, s, reached));
+            GPMA_TRY(bfs_run(g, src, levels, s, reached));
+            levels = nullptr;
         } else {
             GPMA_TRY(bfs_finish(g, reached));
         }
+        if (bp.direct)
+            levels = nullptr;
     }
     if (levels) {
         GPMA_TRY(copy_any(levels, g->bfs_levels, sizeof(uint32_t) * g->row_num, s));
