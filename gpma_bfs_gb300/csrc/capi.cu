@@ -390,9 +390,10 @@ gpma_status gpma_update(gpma_graph *g, const uint64_t *keys, const uint8_t *valu
         return update_device(g, n, s, keys, values);  // the kernel reads the caller's batch in place
     {
         // page-locked host batches: the kernel reads them over the host link
-        // itself (the keys twice: ranks, then the scatter), no staging copy
+        // itself (the keys twice: ranks, then the scatter), no staging copy;
+        // small ones are copied, since there every CTA reads the whole batch
         const void *dk = mapped_host_pointer(keys), *dv = mapped_host_pointer(values);
-        if (dk && dv)
+        if (dk && dv && n > update_small_keys())
             return update_device(g, n, s, static_cast<const uint64_t *>(dk), static_cast<const uint8_t *>(dv));
     }
     GPMA_TRY(copy_in(g, g->buf.bkeys[0], keys, n * sizeof(uint64_t), s));

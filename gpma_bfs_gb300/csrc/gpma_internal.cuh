@@ -501,7 +501,8 @@ gpma_status batch_bfs_enqueue_readback(gpma_batch *b, const BatchBfsPlan &P, cud
 gpma_status batch_bfs_finish(gpma_batch *b, const uint32_t *nsrc, uint32_t k, uint64_t *reached);
 void free_bfs(gpma_graph *g);
 void free_batch_bfs(gpma_batch *b);
-int update_grid_size(int sms, uint64_t n);
+int update_grid_size(int sms, uint64_t n, uint32_t k);
+uint64_t update_small_keys();  // keys up to which every CTA of a single-graph update reads the whole batch
 
 // Launch shapes and switch points: they change speed, never results
 // (process-wide, set through gpma_set_tuning; defaults from measurement).

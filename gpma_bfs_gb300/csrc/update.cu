@@ -13,6 +13,8 @@
 //   P3 group them by (graph, leaf) into level-0 windows
 //      (group_insertion_by_node, :846-873). A window is (graph, node, [a, b))
 //      into the current insertion buffer;
+// A batch of a few thousand keys of one graph goes through S to P3 with one
+// barrier (small_front).
 //   level loop (:1012-1029): each window of width W = seg << level counts its
 //      live slots, is accepted iff lower <= live + pending <= upper (the
 //      graph's thresholds), and an accepted window is rewritten as the stable
@@ -973,12 +975,162 @@ __device__ __forceinline__ void level_prefix(const UpdateArgs &A, const Windows 
     total_i = s.w;
 }
 
+// ---- small batches of one graph: sort, locate and group with one barrier -----
+// A batch of at most SMALL_KEYS keys. Every CTA keeps the whole batch in shared
+// memory, so a warp finds its key's place in the stable order by counting, with
+// no exchange between CTAs, and goes on to locate the key: five levels of the
+// descent per round of loads (lane l reads the head that node l of the next
+// five levels' heap compares; the comparisons taken are the reference's,
+// gpma.cuh:209-216), then the leaf's slots, a lane each. After one grid barrier
+// every CTA compacts and groups the sorted insertions for itself and writes
+// only the windows and insertions of its own part, which it dispatches next.
+// The general phases need seven barriers to get there, each with its own chain
+// of loads: 43 us of kernel for 1,000 keys into the social graph (2^25 slots),
+// 17 here. The counting grows with the square of the batch, which draws the
+// line: a call takes 42 / 51 / 52 / 64 us with 2 / 512 / 2,048 / 4,096 keys,
+// against 67 / 78 / 78 / 78 by the general phases.
+constexpr uint32_t SMALL_KEYS = 4096;
+static_assert(SMALL_KEYS * 9 <= UPDATE_SMEM && SMALL_KEYS * 12 + 4 <= UPDATE_SMEM, "small batch staging");
+
+// The leaf of `key` (its first slot), by all lanes of a warp.
+__device__ __forceinline__ uint32_t warp_descend(const GraphDesc &D, uint64_t key, uint32_t lane) {
+    const uint32_t depth = lane ? 31 - __clz(lane) : 0, path = lane - (1u << depth);
+    uint32_t prefix = 0;  // heads index so far
+    for (uint32_t rem = D.height; rem > 0;) {
+        const uint32_t t = min(5u, rem);
+        bool right = false;
+        if (lane && depth < t)
+            right = D.heads[prefix | (path << (rem - depth)) | (1u << (rem - depth - 1))] <= key;
+        const uint32_t taken = __ballot_sync(0xFFFFFFFFu, right);
+        uint32_t node = 1;
+        for (uint32_t d = 0; d < t; ++d)
+            node = 2 * node + ((taken >> node) & 1u);
+        rem -= t;
+        prefix |= (node - (1u << t)) << rem;
+    }
+    return prefix << D.log2seg;
+}
+
+// Leaves the level-0 windows and their insertions in wnode/wgraph/wa/wb[0] and
+// ikeys/ivals[0] (each CTA those of its cta_range), the insertion and window
+// counts in m and nw. False: the launch ends (invalid keys or an error).
+__device__ bool small_front(const UpdateArgs &A, unsigned char *smem, uint32_t *tmp, uint32_t &m, uint32_t &nw) {
+    DeviceStatus *st = A.st;
+    const GraphDesc &D = A.gd[0];
+    const uint32_t n = A.n, lane = threadIdx.x & 31;
+    const bool stamper = blockIdx.x == 0 && threadIdx.x == 0;
+    {
+        uint64_t *s_key = reinterpret_cast<uint64_t *>(smem);
+        uint8_t *s_val = smem + (size_t)SMALL_KEYS * 8;
+        bool bad = false;
+        for (uint32_t i = threadIdx.x; i < n; i += BLOCK) {
+            const uint64_t k = A.in_k[i];
+            s_key[i] = k;
+            s_val[i] = A.in_v[i];
+            bad |= (k & COL_NONE) == COL_NONE;
+        }
+        if (__syncthreads_or(bad)) {
+            if (stamper)
+                st->invalid_keys = 1;
+            return false;  // every CTA: rejected before any change
+        }
+        // test hook: a barrier that never completes, before any change as in
+        // the general phases
+        if (A.stall && !grid_barrier(A.bar, &st->err, A.stall, A.stall_limit_ns))
+            return false;
+        if (stamper)
+            st->stamp[1] = globaltimer_ns();
+        const uint32_t nwarps = gridDim.x * (BLOCK / 32);
+        for (uint32_t i = blockIdx.x * (BLOCK / 32) + (threadIdx.x >> 5); i < n; i += nwarps) {
+            const uint64_t key = s_key[i];
+            const uint8_t value = s_val[i];
+            uint32_t before = 0;
+            for (uint32_t j = lane; j < n; j += 32) {
+                const uint64_t o = s_key[j];
+                before += (uint32_t)(o < key) | ((uint32_t)(o == key) & (uint32_t)(j < i));
+            }
+            const uint32_t rank = __reduce_add_sync(0xFFFFFFFFu, before);
+            uint32_t leaf = warp_descend(D, key, lane);
+            const bool ok = in_bounds(&st->err, (uint64_t)leaf + D.seg <= D.size, BS_LEAF);
+            const uint32_t hits =
+                __ballot_sync(0xFFFFFFFFu, ok && lane < D.seg && D.keys[leaf + lane] == key);
+            if (lane == 0) {
+                if (hits)
+                    D.vals[leaf + __ffs(hits) - 1] = value;  // delete / modify / revive in place
+                if (hits || !ok || value == 0)
+                    leaf = SIZE_NONE;
+                // not bk[0] / bv[0]: the batch itself may be there
+                A.bk[1][rank] = key;
+                A.bv[1][rank] = value;
+                A.leaf[rank] = leaf;
+            }
+        }
+    }
+    if (!grid_barrier(A.bar, &st->err))
+        return false;
+    for (uint32_t i = blockIdx.x * BLOCK + threadIdx.x; i < A.next_slot_words; i += gridDim.x * BLOCK)
+        A.next_slot[i] = 0;
+    if (stamper)
+        st->stamp[2] = globaltimer_ns();
+    uint32_t *s_leaf = reinterpret_cast<uint32_t *>(smem);  // per sorted key
+    uint32_t *s_ins = s_leaf + SMALL_KEYS;                  // sorted position of every insertion
+    uint32_t *s_win = s_ins + SMALL_KEYS;                   // first insertion of every window
+    for (uint32_t i = threadIdx.x; i < n; i += BLOCK)
+        s_leaf[i] = A.leaf[i];
+    __syncthreads();
+    {
+        const uint32_t per = (n + BLOCK - 1) / BLOCK, i0 = threadIdx.x * per, i1 = min(n, i0 + per);
+        uint32_t c = 0;
+        for (uint32_t i = i0; i < i1; ++i)
+            c += s_leaf[i] != SIZE_NONE;
+        uint32_t o = block_excl_scan(c, &m, tmp);
+        for (uint32_t i = i0; i < i1; ++i)
+            if (s_leaf[i] != SIZE_NONE)
+                s_ins[o++] = i;
+    }
+    __syncthreads();
+    {
+        const uint32_t per = (m + BLOCK - 1) / BLOCK, j0 = threadIdx.x * per, j1 = min(m, j0 + per);
+        auto head = [&](uint32_t j) { return j == 0 || s_leaf[s_ins[j]] != s_leaf[s_ins[j - 1]]; };
+        uint32_t c = 0;
+        for (uint32_t j = j0; j < j1; ++j)
+            c += head(j);
+        uint32_t e = block_excl_scan(c, &nw, tmp);
+        for (uint32_t j = j0; j < j1; ++j)
+            if (head(j))
+                s_win[e++] = j;
+    }
+    __syncthreads();
+    uint32_t lo, hi;
+    cta_range(nw, lo, hi);
+    const uint32_t a0 = lo < nw ? s_win[lo] : m, a1 = hi < nw ? s_win[hi] : m;
+    for (uint32_t e = lo + threadIdx.x; e < hi; e += BLOCK) {
+        const uint32_t a = s_win[e];
+        A.wnode[0][e] = s_leaf[s_ins[a]];
+        A.wgraph[0][e] = 0;
+        A.wa[0][e] = a;
+        A.wb[0][e] = e + 1 < nw ? s_win[e + 1] : m;
+    }
+    for (uint32_t j = a0 + threadIdx.x; j < a1; j += BLOCK) {
+        A.ikeys[0][j] = A.bk[1][s_ins[j]];
+        A.ivals[0][j] = A.bv[1][s_ins[j]];
+    }
+    if (stamper) {
+        A.gs[0].ins_base = 0;
+        A.gs[0].inserts = m;  // end; the first is insertion 0
+    }
+    __syncthreads();  // the CTA's part is visible to all its threads, and the staging is free
+    return true;
+}
+
 // Two register budgets of the same kernel: MINB resident CTAs per SM. Two
 // (128 registers, almost no spills) suits single large graphs, whose phases
 // are short and barrier-bound; three (80 registers, some spills to local
 // memory) suits many graphs per launch, whose phases are longer and gain from
 // the extra warps. gpma_tuning.update_blocks_per_sm selects one.
-template <int MINB>
+// SMALL: the build for small batches of one graph (small_front); apart, so that
+// it costs the others no registers.
+template <int MINB, bool SMALL>
 __global__ void __launch_bounds__(BLOCK, MINB) update_kernel(UpdateArgs A) {
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ uint32_t tmp[BLOCK / 32 + 1];
@@ -988,152 +1140,114 @@ __global__ void __launch_bounds__(BLOCK, MINB) update_kernel(UpdateArgs A) {
     const bool stamper = blockIdx.x == 0 && threadIdx.x == 0;
     if (stamper)
         st->stamp[0] = globaltimer_ns();
-    // One graph: the heads at every stride-th segment, which every CTA copies
-    // into shared memory for the top of the descent, are gathered once into a
-    // contiguous array here (before the sort's first barrier), so each CTA's
-    // copy is a coalesced read instead of LOCATE_CACHE scattered ones.
-    if (A.G == 1 && blockIdx.x < LOCATE_CACHE / BLOCK) {
-        const GraphDesc &D = A.gd[0];
-        const uint32_t segs = D.size >> D.log2seg;
-        const uint32_t cached = segs < LOCATE_CACHE ? segs : LOCATE_CACHE;
-        const uint32_t hstep = (31 - __clz(D.size / cached)) - D.log2seg;
-        for (uint32_t j = blockIdx.x * BLOCK + threadIdx.x; j < cached; j += gridDim.x * BLOCK)
-            A.top[j] = D.heads[(size_t)j << hstep];
-    }
-
-    // S: stable sort of each graph's batch (gpma.cuh:977): the bucket sort,
-    // or digit passes separated by grid barriers (digits constant over all
-    // batches skipped) when it is off or a bucket is crowded.
-    const uint64_t *bk = A.bk[0];
-    const uint8_t *bv = A.bv[1];
-    bool digits = A.q.nq == 0;
-    if (!digits) {
-        bsort_rank(A.in_k, A.boff, A.G, A.gd, A.q, st);
-        if (!grid_barrier(A.bar, &st->err, A.stall, A.stall_limit_ns))
-            return;
-        if (ld_volatile(&st->invalid_keys) != 0)
-            return;  // reserved-column keys: reject the batch before any change
-        bsort_scan(A.q, A.cta_cnt, st, tmp);
-        if (!grid_barrier(A.bar, &st->err))
-            return;
-        digits = cta_broadcast_read(&st->sort_fallback) != 0;
-        if (!digits) {
-            // records of the batch scattered into buckets, then items sorted into bk[0] / bv[1]
-            uint32_t *cpre = reinterpret_cast<uint32_t *>(smem + BSORT_SMEM_ITEM);
-            bsort_chunk_prefix(A.cta_cnt, cpre, tmp);
-            bsort_scatter(A.in_k, A.in_v, A.boff, A.G, A.q, cpre);
-            if (!grid_barrier(A.bar, &st->err))
-                return;
-            bsort_items(A.bk[0], A.bv[1], A.boff, A.G, A.q, cpre, smem);
-            if (!grid_barrier(A.bar, &st->err))
-                return;
-        }
-    }
-    if (digits) {
-        sort_histogram(A.in_k, A.boff, A.G, A.sort_hist, st, reinterpret_cast<uint32_t *>(smem));
-        if (!grid_barrier(A.bar, &st->err, A.q.nq == 0 ? A.stall : 0u, A.stall_limit_ns))
-            return;
-        if (ld_volatile(&st->invalid_keys) != 0)
-            return;  // reserved-column keys: reject the batch before any change
-        uint32_t sel = 0;
-        bool first = true;  // the first pass reads the batch as submitted
-        {
-            const uint32_t trivial = sort_trivial_mask(A.sort_hist + (size_t)(A.G == 1 ? 0 : A.G) * 2048, A.n);
-            const uint32_t tiles = A.toff[A.G];
-            for (int p = 0; p < 8; ++p) {
-                if (trivial & (1u << p))
-                    continue;
-                const uint64_t *ink = first ? A.in_k : (sel ? A.bk[1] : A.bk[0]);
-                const uint8_t *inv = first ? A.in_v : (sel ? A.bv[1] : A.bv[0]);
-                uint64_t *outk = sel ? A.bk[0] : A.bk[1];
-                uint8_t *outv = sel ? A.bv[0] : A.bv[1];
-                first = false;
-                // CTA b takes tiles b, b + G, b + 2G, ... in order: every look-back
-                // waits on lower tiles only, and the lowest unfinished tile never
-                // waits on anything unfinished, so the pass always progresses
-                for (uint32_t tile = blockIdx.x; tile < tiles; tile += gridDim.x)
-                    sort_tile(p, tile, ink, inv, outk, outv, A.boff, A.toff, A.G, A.sort_hist, A.sort_status, st, smem,
-                              tmp);
-                sel ^= 1u;
-                if (!grid_barrier(A.bar, &st->err))
-                    return;
-            }
-        }
-        bk = first ? A.in_k : (sel ? A.bk[1] : A.bk[0]);  // no pass: every digit constant
-        bv = first ? A.in_v : (sel ? A.bv[1] : A.bv[0]);
-    }
     const uint32_t G = gridDim.x;
-
     uint32_t scan_id = 0;
 #define CNT(id) ((id) ? A.cta_cnt + G : A.cta_cnt)
 #define CNTI(id) ((id) ? A.cta_cnt + 3 * G : A.cta_cnt + 2 * G)
 #define SLICES(p) (A.cta_cnt + 4 * G + 2 * (p) * G)  // per CTA (lo, hi) of its windows, by level parity
     unsigned long long acc = 0, acc_slots = 0;
-    if (stamper)
-        st->stamp[1] = globaltimer_ns();
-
-    // P1: locate every update, applying deletes / modifies in place. The top
-    // of the descent comes from a shared-memory copy of the first keys at
-    // every `stride`-th slot (of the one graph, or of each graph in turn).
-    {
-        const uint64_t *fk = nullptr;
-        uint32_t log2stride = 0;
-        if (A.G == 1) {
+    uint32_t lo = 0, hi = 0, base = 0;
+    uint32_t m = 0, nw = 0;  // insertions; windows of the current level
+    if constexpr (SMALL) {
+        if (!small_front(A, smem, tmp, m, nw))
+            return;
+    } else {
+        // One graph: the heads at every stride-th segment, which every CTA copies
+        // into shared memory for the top of the descent, are gathered once into a
+        // contiguous array here (before the sort's first barrier), so each CTA's
+        // copy is a coalesced read instead of LOCATE_CACHE scattered ones.
+        if (A.G == 1 && blockIdx.x < LOCATE_CACHE / BLOCK) {
             const GraphDesc &D = A.gd[0];
             const uint32_t segs = D.size >> D.log2seg;
             const uint32_t cached = segs < LOCATE_CACHE ? segs : LOCATE_CACHE;
-            log2stride = 31 - __clz(D.size / cached);
-            uint64_t *f = reinterpret_cast<uint64_t *>(smem);
-            // the contiguous copy gathered at the start of the launch; all of
-            // a thread's loads issued together
-            uint64_t hv[LOCATE_CACHE / BLOCK];
-#pragma unroll
-            for (uint32_t r = 0; r < LOCATE_CACHE / BLOCK; ++r) {
-                const uint32_t j = threadIdx.x + r * BLOCK;
-                hv[r] = j < cached ? A.top[j] : 0ull;
-            }
-#pragma unroll
-            for (uint32_t r = 0; r < LOCATE_CACHE / BLOCK; ++r) {
-                const uint32_t j = threadIdx.x + r * BLOCK;
-                if (j < cached)
-                    f[j] = hv[r];
-            }
-            __syncthreads();
-            fk = f;
+            const uint32_t hstep = (31 - __clz(D.size / cached)) - D.log2seg;
+            for (uint32_t j = blockIdx.x * BLOCK + threadIdx.x; j < cached; j += gridDim.x * BLOCK)
+                A.top[j] = D.heads[(size_t)j << hstep];
         }
-        if (A.G == 1) {
-            // one graph: each CTA takes a contiguous range (neighbouring keys
-            // share descent paths in L1) and counts its insertions for the
-            // compaction after the barrier
-            uint32_t lo, hi, mine = 0;
-            cta_range(A.n, lo, hi);
-            for (uint32_t i0 = lo + threadIdx.x; i0 < hi; i0 += LOC_ILP * BLOCK)
-                mine += locate_keys<true>(A, bk, bv, i0, BLOCK, hi, fk, log2stride);
-            const uint32_t t = block_sum(mine, tmp);
-            if (threadIdx.x == 0)
-                CNT(scan_id)[blockIdx.x] = t;
-        } else {
-            // many graphs: each CTA takes a contiguous range of the sorted
-            // batches (a graph or two) and, graph by graph, copies the graph's
-            // top-of-tree heads into shared memory, so its keys walk the upper
-            // levels there as with one graph
-            uint64_t *f = reinterpret_cast<uint64_t *>(smem);
-            uint32_t lo, hi;
-            cta_range(A.n, lo, hi);
-            uint32_t pos = lo;
-            while (__syncthreads_or(pos < hi)) {
-                const uint32_t g = segment_of(A.boff, A.G, pos);
-                const uint32_t end = min(hi, A.boff[g + 1]);
-                const GraphDesc &D = A.gd[g];
+
+        // S: stable sort of each graph's batch (gpma.cuh:977): the bucket sort,
+        // or digit passes separated by grid barriers (digits constant over all
+        // batches skipped) when it is off or a bucket is crowded.
+        const uint64_t *bk = A.bk[0];
+        const uint8_t *bv = A.bv[1];
+        bool digits = A.q.nq == 0;
+        if (!digits) {
+            bsort_rank(A.in_k, A.boff, A.G, A.gd, A.q, st);
+            if (!grid_barrier(A.bar, &st->err, A.stall, A.stall_limit_ns))
+                return;
+            if (ld_volatile(&st->invalid_keys) != 0)
+                return;  // reserved-column keys: reject the batch before any change
+            bsort_scan(A.q, A.cta_cnt, st, tmp);
+            if (!grid_barrier(A.bar, &st->err))
+                return;
+            digits = cta_broadcast_read(&st->sort_fallback) != 0;
+            if (!digits) {
+                // records of the batch scattered into buckets, then items sorted into bk[0] / bv[1]
+                uint32_t *cpre = reinterpret_cast<uint32_t *>(smem + BSORT_SMEM_ITEM);
+                bsort_chunk_prefix(A.cta_cnt, cpre, tmp);
+                bsort_scatter(A.in_k, A.in_v, A.boff, A.G, A.q, cpre);
+                if (!grid_barrier(A.bar, &st->err))
+                    return;
+                bsort_items(A.bk[0], A.bv[1], A.boff, A.G, A.q, cpre, smem);
+                if (!grid_barrier(A.bar, &st->err))
+                    return;
+            }
+        }
+        if (digits) {
+            sort_histogram(A.in_k, A.boff, A.G, A.sort_hist, st, reinterpret_cast<uint32_t *>(smem));
+            if (!grid_barrier(A.bar, &st->err, A.q.nq == 0 ? A.stall : 0u, A.stall_limit_ns))
+                return;
+            if (ld_volatile(&st->invalid_keys) != 0)
+                return;  // reserved-column keys: reject the batch before any change
+            uint32_t sel = 0;
+            bool first = true;  // the first pass reads the batch as submitted
+            {
+                const uint32_t trivial = sort_trivial_mask(A.sort_hist + (size_t)(A.G == 1 ? 0 : A.G) * 2048, A.n);
+                const uint32_t tiles = A.toff[A.G];
+                for (int p = 0; p < 8; ++p) {
+                    if (trivial & (1u << p))
+                        continue;
+                    const uint64_t *ink = first ? A.in_k : (sel ? A.bk[1] : A.bk[0]);
+                    const uint8_t *inv = first ? A.in_v : (sel ? A.bv[1] : A.bv[0]);
+                    uint64_t *outk = sel ? A.bk[0] : A.bk[1];
+                    uint8_t *outv = sel ? A.bv[0] : A.bv[1];
+                    first = false;
+                    // CTA b takes tiles b, b + G, b + 2G, ... in order: every look-back
+                    // waits on lower tiles only, and the lowest unfinished tile never
+                    // waits on anything unfinished, so the pass always progresses
+                    for (uint32_t tile = blockIdx.x; tile < tiles; tile += gridDim.x)
+                        sort_tile(p, tile, ink, inv, outk, outv, A.boff, A.toff, A.G, A.sort_hist, A.sort_status, st, smem,
+                                  tmp);
+                    sel ^= 1u;
+                    if (!grid_barrier(A.bar, &st->err))
+                        return;
+                }
+            }
+            bk = first ? A.in_k : (sel ? A.bk[1] : A.bk[0]);  // no pass: every digit constant
+            bv = first ? A.in_v : (sel ? A.bv[1] : A.bv[0]);
+        }
+        if (stamper)
+            st->stamp[1] = globaltimer_ns();
+
+        // P1: locate every update, applying deletes / modifies in place. The top
+        // of the descent comes from a shared-memory copy of the first keys at
+        // every `stride`-th slot (of the one graph, or of each graph in turn).
+        {
+            const uint64_t *fk = nullptr;
+            uint32_t log2stride = 0;
+            if (A.G == 1) {
+                const GraphDesc &D = A.gd[0];
                 const uint32_t segs = D.size >> D.log2seg;
                 const uint32_t cached = segs < LOCATE_CACHE ? segs : LOCATE_CACHE;
-                const uint32_t l2s = 31 - __clz(D.size / cached);
-                const uint32_t hstep = l2s - D.log2seg;
+                log2stride = 31 - __clz(D.size / cached);
+                uint64_t *f = reinterpret_cast<uint64_t *>(smem);
+                // the contiguous copy gathered at the start of the launch; all of
+                // a thread's loads issued together
                 uint64_t hv[LOCATE_CACHE / BLOCK];
 #pragma unroll
                 for (uint32_t r = 0; r < LOCATE_CACHE / BLOCK; ++r) {
                     const uint32_t j = threadIdx.x + r * BLOCK;
-                    hv[r] = j < cached ? D.heads[(size_t)j << hstep] : 0ull;
+                    hv[r] = j < cached ? A.top[j] : 0ull;
                 }
 #pragma unroll
                 for (uint32_t r = 0; r < LOCATE_CACHE / BLOCK; ++r) {
@@ -1142,200 +1256,242 @@ __global__ void __launch_bounds__(BLOCK, MINB) update_kernel(UpdateArgs A) {
                         f[j] = hv[r];
                 }
                 __syncthreads();
-                for (uint32_t i0 = pos + threadIdx.x; i0 < end; i0 += LOC_ILP * BLOCK)
-                    locate_keys<false>(A, bk, bv, i0, BLOCK, end, f, l2s);
-                __syncthreads();  // the copy is replaced for the next graph
-                pos = end;
+                fk = f;
+            }
+            if (A.G == 1) {
+                // one graph: each CTA takes a contiguous range (neighbouring keys
+                // share descent paths in L1) and counts its insertions for the
+                // compaction after the barrier
+                uint32_t lo, hi, mine = 0;
+                cta_range(A.n, lo, hi);
+                for (uint32_t i0 = lo + threadIdx.x; i0 < hi; i0 += LOC_ILP * BLOCK)
+                    mine += locate_keys<true>(A, bk, bv, i0, BLOCK, hi, fk, log2stride);
+                const uint32_t t = block_sum(mine, tmp);
+                if (threadIdx.x == 0)
+                    CNT(scan_id)[blockIdx.x] = t;
+            } else {
+                // many graphs: each CTA takes a contiguous range of the sorted
+                // batches (a graph or two) and, graph by graph, copies the graph's
+                // top-of-tree heads into shared memory, so its keys walk the upper
+                // levels there as with one graph
+                uint64_t *f = reinterpret_cast<uint64_t *>(smem);
+                uint32_t lo, hi;
+                cta_range(A.n, lo, hi);
+                uint32_t pos = lo;
+                while (__syncthreads_or(pos < hi)) {
+                    const uint32_t g = segment_of(A.boff, A.G, pos);
+                    const uint32_t end = min(hi, A.boff[g + 1]);
+                    const GraphDesc &D = A.gd[g];
+                    const uint32_t segs = D.size >> D.log2seg;
+                    const uint32_t cached = segs < LOCATE_CACHE ? segs : LOCATE_CACHE;
+                    const uint32_t l2s = 31 - __clz(D.size / cached);
+                    const uint32_t hstep = l2s - D.log2seg;
+                    uint64_t hv[LOCATE_CACHE / BLOCK];
+#pragma unroll
+                    for (uint32_t r = 0; r < LOCATE_CACHE / BLOCK; ++r) {
+                        const uint32_t j = threadIdx.x + r * BLOCK;
+                        hv[r] = j < cached ? D.heads[(size_t)j << hstep] : 0ull;
+                    }
+#pragma unroll
+                    for (uint32_t r = 0; r < LOCATE_CACHE / BLOCK; ++r) {
+                        const uint32_t j = threadIdx.x + r * BLOCK;
+                        if (j < cached)
+                            f[j] = hv[r];
+                    }
+                    __syncthreads();
+                    for (uint32_t i0 = pos + threadIdx.x; i0 < end; i0 += LOC_ILP * BLOCK)
+                        locate_keys<false>(A, bk, bv, i0, BLOCK, end, f, l2s);
+                    __syncthreads();  // the copy is replaced for the next graph
+                    pos = end;
+                }
             }
         }
-    }
-    if (!grid_barrier(A.bar, &st->err))
-        return;
-    {
-        // every CTA is past the sort (trivial-digit mask, passes): zero its
-        // state and the next launch's status slot
-        const uint32_t gt = blockIdx.x * BLOCK + threadIdx.x, nt = G * BLOCK;
-        for (uint32_t i = gt; i < A.hist_words; i += nt)
-            A.sort_hist[i] = 0;
-        for (uint32_t i = gt; i < A.status_words; i += nt)
-            A.sort_status[i] = 0;
-        for (uint32_t i = gt; i < A.q.nq; i += nt)
-            A.q.qcnt[i] = 0;
-        if (gt < 8)
-            A.sort_tiles[gt] = 0;
-        for (uint32_t i = gt; i < A.next_slot_words; i += nt)
-            A.next_slot[i] = 0;
-    }
-    if (stamper)
-        st->stamp[2] = globaltimer_ns();
+        if (!grid_barrier(A.bar, &st->err))
+            return;
+        {
+            // every CTA is past the sort (trivial-digit mask, passes): zero its
+            // state and the next launch's status slot
+            const uint32_t gt = blockIdx.x * BLOCK + threadIdx.x, nt = G * BLOCK;
+            for (uint32_t i = gt; i < A.hist_words; i += nt)
+                A.sort_hist[i] = 0;
+            for (uint32_t i = gt; i < A.status_words; i += nt)
+                A.sort_status[i] = 0;
+            for (uint32_t i = gt; i < A.q.nq; i += nt)
+                A.q.qcnt[i] = 0;
+            if (gt < 8)
+                A.sort_tiles[gt] = 0;
+            for (uint32_t i = gt; i < A.next_slot_words; i += nt)
+                A.next_slot[i] = 0;
+        }
+        if (stamper)
+            st->stamp[2] = globaltimer_ns();
 
-    // P2: stable compaction of the insertions (with their graph), each CTA
-    // writing the insertions of its locate range; then it counts the
-    // run-length heads of its own output (its first insertion counted as one).
-    uint32_t lo, hi;
-    cta_range(A.n, lo, hi);
-    if (A.G > 1) {
-        uint32_t cl = 0;
-        for (uint32_t i = lo + threadIdx.x; i < hi; i += BLOCK)
-            cl += A.leaf[i] != SIZE_NONE;
-        const uint32_t t = block_sum(cl, tmp);
-        if (threadIdx.x == 0)
-            CNT(scan_id)[blockIdx.x] = t;
+        // P2: stable compaction of the insertions (with their graph), each CTA
+        // writing the insertions of its locate range; then it counts the
+        // run-length heads of its own output (its first insertion counted as one).
+        cta_range(A.n, lo, hi);
+        if (A.G > 1) {
+            uint32_t cl = 0;
+            for (uint32_t i = lo + threadIdx.x; i < hi; i += BLOCK)
+                cl += A.leaf[i] != SIZE_NONE;
+            const uint32_t t = block_sum(cl, tmp);
+            if (threadIdx.x == 0)
+                CNT(scan_id)[blockIdx.x] = t;
+            if (!grid_barrier(A.bar, &st->err))
+                return;
+        }
+        uint32_t unused_b, unused_t;
+        cta_prefix2(CNT(scan_id), nullptr, base, m, unused_b, unused_t);
+        const uint32_t out_lo = base;
+        // GROUP_ITEMS consecutive items per thread and one scan per round
+        for (uint32_t r0 = lo; r0 < hi; r0 += GROUP_ITEMS * BLOCK) {
+            const uint32_t i0 = r0 + GROUP_ITEMS * threadIdx.x;
+            uint32_t lf[GROUP_ITEMS], cnt = 0;
+#pragma unroll
+            for (uint32_t j = 0; j < GROUP_ITEMS; ++j) {
+                lf[j] = i0 + j < hi ? A.leaf[i0 + j] : SIZE_NONE;
+                cnt += lf[j] != SIZE_NONE;
+            }
+            uint32_t tot;
+            uint32_t o = base + block_excl_scan(cnt, &tot, tmp);
+#pragma unroll
+            for (uint32_t j = 0; j < GROUP_ITEMS; ++j) {
+                if (lf[j] == SIZE_NONE)
+                    continue;
+                const uint32_t i = i0 + j;
+                A.ikeys[0][o] = bk[i];
+                A.ivals[0][o] = bv[i];
+                A.ileaf[o] = lf[j];
+                A.igraph[o] = graph_of(A, i);
+                ++o;
+            }
+            base += tot;
+        }
+        const uint32_t out_hi = base;
+        __syncthreads();  // this CTA's output is visible to all its threads
+        {
+            uint32_t h = 0;
+            for (uint32_t j = out_lo + threadIdx.x; j < out_hi; j += BLOCK)
+                h += (j == out_lo || A.ileaf[j] != A.ileaf[j - 1] || A.igraph[j] != A.igraph[j - 1]);
+            const uint32_t t = block_sum(h, tmp);
+            if (threadIdx.x == 0)
+                CNT(scan_id ^ 1)[blockIdx.x] = t;
+        }
+        if (!grid_barrier(A.bar, &st->err))
+            return;
+        if (A.G == 1 && m >= SIGNIFICANT_INSERTS) {
+            if (stamper) {
+                st->significant = 1;
+                st->inserts = m;
+                A.gs[0].inserts = m;
+                A.gs[0].ins_base = 0;
+            }
+            return;
+        }
+
+        // P3: run-length grouping of the insertions by (graph, leaf) -> level-0
+        // windows; also each graph's first insertion and its count. A CTA whose
+        // first insertion continues the run of the previous output counted one
+        // head too many: the window offsets subtract those.
+        {
+            const uint32_t *ins_cnt = CNT(scan_id);
+            const uint32_t *head_cnt = CNT(scan_id ^ 1);
+            uint32_t carry = 0, before = 0, all = 0;
+            // two CTAs' counts per thread per step, each kind of load issued for
+            // both before the first is used
+            for (uint32_t c0 = 0; c0 < G; c0 += 2 * BLOCK) {
+                uint32_t n_c[2], h_c[2], b_c[2];
+#pragma unroll
+                for (int u = 0; u < 2; ++u) {
+                    const uint32_t c = c0 + u * BLOCK + threadIdx.x;
+                    n_c[u] = c < G ? __ldcg(ins_cnt + c) : 0u;
+                    h_c[u] = c < G ? __ldcg(head_cnt + c) : 0u;
+                }
+#pragma unroll
+                for (int u = 0; u < 2; ++u) {
+                    uint32_t tot;
+                    b_c[u] = carry + block_excl_scan(n_c[u], &tot, tmp);  // first output of CTA c
+                    carry += tot;
+                }
+                uint32_t l0[2], l1[2], g0[2], g1[2];
+#pragma unroll
+                for (int u = 0; u < 2; ++u) {
+                    const bool chk = n_c[u] && b_c[u] > 0;
+                    l0[u] = chk ? A.ileaf[b_c[u]] : 0u;
+                    l1[u] = chk ? A.ileaf[b_c[u] - 1] : 1u;
+                    g0[u] = chk ? A.igraph[b_c[u]] : 0u;
+                    g1[u] = chk ? A.igraph[b_c[u] - 1] : 0u;
+                }
+#pragma unroll
+                for (int u = 0; u < 2; ++u) {
+                    const uint32_t c = c0 + u * BLOCK + threadIdx.x;
+                    uint32_t h = 0;
+                    if (c < G && n_c[u]) {
+                        h = h_c[u];
+                        if (l0[u] == l1[u] && g0[u] == g1[u])  // continues the previous CTA's last run
+                            --h;
+                    }
+                    all += h;
+                    if (c < blockIdx.x)
+                        before += h;
+                }
+            }
+            const uint4 t = block_sum4(make_uint4(all, before, 0, 0));
+            nw = t.x;
+            base = t.y;
+        }
+        for (uint32_t r0 = out_lo; r0 < out_hi; r0 += GROUP_ITEMS * BLOCK) {
+            const uint32_t j0 = r0 + GROUP_ITEMS * threadIdx.x;
+            // items j0 - 1 .. j0 + GROUP_ITEMS: each item's run test needs its
+            // neighbours on both sides
+            uint32_t lf[GROUP_ITEMS + 2], gr[GROUP_ITEMS + 2];
+#pragma unroll
+            for (uint32_t q = 0; q < GROUP_ITEMS + 2; ++q) {
+                const uint32_t j = j0 + q - 1;  // wraps to UINT32_MAX for j0 == 0, q == 0
+                const bool ok = j0 + q >= 1 && j < m;
+                lf[q] = ok ? A.ileaf[j] : SIZE_NONE;
+                gr[q] = ok ? A.igraph[j] : SIZE_NONE;
+            }
+            uint32_t heads = 0;
+            uint32_t hd[GROUP_ITEMS];
+#pragma unroll
+            for (uint32_t q = 0; q < GROUP_ITEMS; ++q) {
+                const uint32_t j = j0 + q;
+                hd[q] = 0;
+                if (j < out_hi) {
+                    const bool new_graph = j == 0 || gr[q] != gr[q + 1];
+                    hd[q] = (new_graph || lf[q + 1] != lf[q]) ? 1u : 0u;
+                    if (new_graph)
+                        A.gs[gr[q + 1]].ins_base = j;
+                    if (j + 1 == m || gr[q + 2] != gr[q + 1])
+                        A.gs[gr[q + 1]].inserts = j + 1;  // end for now; made a count by the host
+                }
+                heads += hd[q];
+            }
+            uint32_t tot;
+            // a run continued from the previous CTA's output extends window base - 1
+            uint32_t e = base + block_excl_scan(heads, &tot, tmp);
+#pragma unroll
+            for (uint32_t q = 0; q < GROUP_ITEMS; ++q) {
+                const uint32_t j = j0 + q;
+                if (j >= out_hi)
+                    continue;
+                if (hd[q]) {
+                    A.wnode[0][e] = lf[q + 1];
+                    A.wgraph[0][e] = gr[q + 1];
+                    A.wa[0][e] = j;
+                    ++e;
+                }
+                const bool last = j + 1 == m || lf[q + 2] != lf[q + 1] || gr[q + 2] != gr[q + 1];
+                if (last)
+                    A.wb[0][e - 1] = j + 1;
+            }
+            base += tot;
+        }
+        scan_id ^= 1;
         if (!grid_barrier(A.bar, &st->err))
             return;
     }
-    uint32_t base, m, unused_b, unused_t;
-    cta_prefix2(CNT(scan_id), nullptr, base, m, unused_b, unused_t);
-    const uint32_t out_lo = base;
-    // GROUP_ITEMS consecutive items per thread and one scan per round
-    for (uint32_t r0 = lo; r0 < hi; r0 += GROUP_ITEMS * BLOCK) {
-        const uint32_t i0 = r0 + GROUP_ITEMS * threadIdx.x;
-        uint32_t lf[GROUP_ITEMS], cnt = 0;
-#pragma unroll
-        for (uint32_t j = 0; j < GROUP_ITEMS; ++j) {
-            lf[j] = i0 + j < hi ? A.leaf[i0 + j] : SIZE_NONE;
-            cnt += lf[j] != SIZE_NONE;
-        }
-        uint32_t tot;
-        uint32_t o = base + block_excl_scan(cnt, &tot, tmp);
-#pragma unroll
-        for (uint32_t j = 0; j < GROUP_ITEMS; ++j) {
-            if (lf[j] == SIZE_NONE)
-                continue;
-            const uint32_t i = i0 + j;
-            A.ikeys[0][o] = bk[i];
-            A.ivals[0][o] = bv[i];
-            A.ileaf[o] = lf[j];
-            A.igraph[o] = graph_of(A, i);
-            ++o;
-        }
-        base += tot;
-    }
-    const uint32_t out_hi = base;
-    __syncthreads();  // this CTA's output is visible to all its threads
-    {
-        uint32_t h = 0;
-        for (uint32_t j = out_lo + threadIdx.x; j < out_hi; j += BLOCK)
-            h += (j == out_lo || A.ileaf[j] != A.ileaf[j - 1] || A.igraph[j] != A.igraph[j - 1]);
-        const uint32_t t = block_sum(h, tmp);
-        if (threadIdx.x == 0)
-            CNT(scan_id ^ 1)[blockIdx.x] = t;
-    }
-    if (!grid_barrier(A.bar, &st->err))
-        return;
-    if (A.G == 1 && m >= SIGNIFICANT_INSERTS) {
-        if (stamper) {
-            st->significant = 1;
-            st->inserts = m;
-            A.gs[0].inserts = m;
-            A.gs[0].ins_base = 0;
-        }
-        return;
-    }
-
-    // P3: run-length grouping of the insertions by (graph, leaf) -> level-0
-    // windows; also each graph's first insertion and its count. A CTA whose
-    // first insertion continues the run of the previous output counted one
-    // head too many: the window offsets subtract those.
-    uint32_t nw = 0;
-    {
-        const uint32_t *ins_cnt = CNT(scan_id);
-        const uint32_t *head_cnt = CNT(scan_id ^ 1);
-        uint32_t carry = 0, before = 0, all = 0;
-        // two CTAs' counts per thread per step, each kind of load issued for
-        // both before the first is used
-        for (uint32_t c0 = 0; c0 < G; c0 += 2 * BLOCK) {
-            uint32_t n_c[2], h_c[2], b_c[2];
-#pragma unroll
-            for (int u = 0; u < 2; ++u) {
-                const uint32_t c = c0 + u * BLOCK + threadIdx.x;
-                n_c[u] = c < G ? __ldcg(ins_cnt + c) : 0u;
-                h_c[u] = c < G ? __ldcg(head_cnt + c) : 0u;
-            }
-#pragma unroll
-            for (int u = 0; u < 2; ++u) {
-                uint32_t tot;
-                b_c[u] = carry + block_excl_scan(n_c[u], &tot, tmp);  // first output of CTA c
-                carry += tot;
-            }
-            uint32_t l0[2], l1[2], g0[2], g1[2];
-#pragma unroll
-            for (int u = 0; u < 2; ++u) {
-                const bool chk = n_c[u] && b_c[u] > 0;
-                l0[u] = chk ? A.ileaf[b_c[u]] : 0u;
-                l1[u] = chk ? A.ileaf[b_c[u] - 1] : 1u;
-                g0[u] = chk ? A.igraph[b_c[u]] : 0u;
-                g1[u] = chk ? A.igraph[b_c[u] - 1] : 0u;
-            }
-#pragma unroll
-            for (int u = 0; u < 2; ++u) {
-                const uint32_t c = c0 + u * BLOCK + threadIdx.x;
-                uint32_t h = 0;
-                if (c < G && n_c[u]) {
-                    h = h_c[u];
-                    if (l0[u] == l1[u] && g0[u] == g1[u])  // continues the previous CTA's last run
-                        --h;
-                }
-                all += h;
-                if (c < blockIdx.x)
-                    before += h;
-            }
-        }
-        const uint4 t = block_sum4(make_uint4(all, before, 0, 0));
-        nw = t.x;
-        base = t.y;
-    }
-    for (uint32_t r0 = out_lo; r0 < out_hi; r0 += GROUP_ITEMS * BLOCK) {
-        const uint32_t j0 = r0 + GROUP_ITEMS * threadIdx.x;
-        // items j0 - 1 .. j0 + GROUP_ITEMS: each item's run test needs its
-        // neighbours on both sides
-        uint32_t lf[GROUP_ITEMS + 2], gr[GROUP_ITEMS + 2];
-#pragma unroll
-        for (uint32_t q = 0; q < GROUP_ITEMS + 2; ++q) {
-            const uint32_t j = j0 + q - 1;  // wraps to UINT32_MAX for j0 == 0, q == 0
-            const bool ok = j0 + q >= 1 && j < m;
-            lf[q] = ok ? A.ileaf[j] : SIZE_NONE;
-            gr[q] = ok ? A.igraph[j] : SIZE_NONE;
-        }
-        uint32_t heads = 0;
-        uint32_t hd[GROUP_ITEMS];
-#pragma unroll
-        for (uint32_t q = 0; q < GROUP_ITEMS; ++q) {
-            const uint32_t j = j0 + q;
-            hd[q] = 0;
-            if (j < out_hi) {
-                const bool new_graph = j == 0 || gr[q] != gr[q + 1];
-                hd[q] = (new_graph || lf[q + 1] != lf[q]) ? 1u : 0u;
-                if (new_graph)
-                    A.gs[gr[q + 1]].ins_base = j;
-                if (j + 1 == m || gr[q + 2] != gr[q + 1])
-                    A.gs[gr[q + 1]].inserts = j + 1;  // end for now; made a count by the host
-            }
-            heads += hd[q];
-        }
-        uint32_t tot;
-        // a run continued from the previous CTA's output extends window base - 1
-        uint32_t e = base + block_excl_scan(heads, &tot, tmp);
-#pragma unroll
-        for (uint32_t q = 0; q < GROUP_ITEMS; ++q) {
-            const uint32_t j = j0 + q;
-            if (j >= out_hi)
-                continue;
-            if (hd[q]) {
-                A.wnode[0][e] = lf[q + 1];
-                A.wgraph[0][e] = gr[q + 1];
-                A.wa[0][e] = j;
-                ++e;
-            }
-            const bool last = j + 1 == m || lf[q + 2] != lf[q + 1] || gr[q + 2] != gr[q + 1];
-            if (last)
-                A.wb[0][e - 1] = j + 1;
-        }
-        base += tot;
-    }
-    scan_id ^= 1;
-    if (!grid_barrier(A.bar, &st->err))
-        return;
     if (stamper)
         st->stamp[3] = globaltimer_ns();
 
@@ -2456,19 +2612,26 @@ GraphDesc describe(const gpma_graph *g) {
     return d;
 }
 
-int g_update_fit[64][2] = {};  // resident CTAs per SM of the two variants, per device
+// Builds of the update kernel.
+enum UpdateVariant { UPDATE_NARROW, UPDATE_WIDE, UPDATE_SMALL, UPDATE_VARIANTS };
+int g_update_fit[64][UPDATE_VARIANTS] = {};  // resident CTAs per SM of each, per device
 
-// The variant for a launch of n keys: the tuned CTAs per SM (3 or more
-// selects the 3-CTA build), or when left to the library (0) the 3-CTA build
-// for launches of at least AUTO_WIDE_KEYS keys.
+// The build for a launch of n keys over k graphs: small batches of one graph
+// have their own (unless the digit passes are asked for); else the tuned CTAs
+// per SM (3 or more selects the 3-CTA build), or when left to the library (0)
+// the 3-CTA build for launches of at least AUTO_WIDE_KEYS keys.
 constexpr uint64_t AUTO_WIDE_KEYS = 1u << 20;
-int update_variant(uint64_t n) {
+UpdateVariant update_variant(uint64_t n, uint32_t k) {
+    if (k == 1 && n <= SMALL_KEYS && g_tuning.update_sort == 0)
+        return UPDATE_SMALL;
     const uint32_t t = g_tuning.update_blocks_per_sm;
-    return t >= 3 || (t == 0 && n >= AUTO_WIDE_KEYS) ? 1 : 0;
+    return t >= 3 || (t == 0 && n >= AUTO_WIDE_KEYS) ? UPDATE_WIDE : UPDATE_NARROW;
 }
 
-const void *update_kernel_ptr(int variant) {
-    return variant ? (const void *)update_kernel<3> : (const void *)update_kernel<2>;
+const void *update_kernel_ptr(UpdateVariant v) {
+    return v == UPDATE_SMALL  ? (const void *)update_kernel<2, true>
+           : v == UPDATE_WIDE ? (const void *)update_kernel<3, false>
+                              : (const void *)update_kernel<2, false>;
 }
 
 }  // namespace
@@ -2541,12 +2704,14 @@ gpma_status count_bad_heads(gpma_graph *g, cudaStream_t s, uint64_t *bad) {
 Tuning g_tuning;
 TestHooks g_test_hooks;
 
-int update_grid_size(int sms, uint64_t n) {
+uint64_t update_small_keys() { return SMALL_KEYS; }
+
+int update_grid_size(int sms, uint64_t n, uint32_t k) {
     int dev = 0;
     cudaGetDevice(&dev);
     if (dev < 0 || dev >= 64)
         dev = 0;
-    const int v = update_variant(n);
+    const UpdateVariant v = update_variant(n, k);
     if (g_update_fit[dev][v] == 0) {
         const void *k = update_kernel_ptr(v);
         if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)UPDATE_SMEM) != cudaSuccess)
@@ -2740,7 +2905,7 @@ gpma_status update_plan(gpma_graph *const *graphs, const uint64_t *off, uint32_t
         set_error("update launch of %llu keys: at most 2^31 - 1 keys per launch", (unsigned long long)n);
         return GPMA_ERR_CAPACITY;
     }
-    const int grid = update_grid_size(sms, n);
+    const int grid = update_grid_size(sms, n, k);
     if (grid == 0) {
         set_error("update kernel cannot be resident");
         return GPMA_ERR_CUDA;
@@ -2896,7 +3061,7 @@ gpma_status update_plan(gpma_graph *const *graphs, const uint64_t *off, uint32_t
     A.abort = abort;
     A.stall = g_test_hooks.update_stall;
     A.stall_limit_ns = g_test_hooks.update_stall ? g_test_hooks.wait_limit_ns : WAIT_LIMIT_NS;
-    L->set(update_kernel_ptr(update_variant(n)), grid, UPDATE_SMEM, &A, sizeof(A));
+    L->set(update_kernel_ptr(update_variant(n, k)), grid, UPDATE_SMEM, &A, sizeof(A));
     return GPMA_OK;
 }
 
