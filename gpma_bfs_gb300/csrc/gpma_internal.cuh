@@ -130,7 +130,7 @@ struct GraphStatus {
     uint32_t inserts;    // insertions of this graph after delete/modify
     uint32_t remaining;  // insertions the root rebalance still has to place
     uint32_t ins_base;   // first insertion of this graph in the compacted order
-    uint32_t pad;
+    uint32_t from;       // first remaining insertion in the insertion buffer | the buffer << 31
 };
 
 struct Geometry {

@@ -1495,10 +1495,11 @@ __global__ void __launch_bounds__(BLOCK, MINB) update_kernel(UpdateArgs A) {
     if (stamper)
         st->stamp[3] = globaltimer_ns();
 
-    // Level loop. Windows and their pending insertions live in ping-pong
-    // buffers selected by `cur`; each window's insertions are the contiguous
-    // range [wa, wb) of the current insertion buffer.
-    uint32_t cur = 0, level = 0;
+    // Level loop. Windows live in ping-pong buffers selected by `cur`, their
+    // pending insertions (m_cur of them) in ones selected by `icur`; each
+    // window's insertions are the contiguous range [wa, wb) of the current
+    // insertion buffer, and the ranges follow one another from 0.
+    uint32_t cur = 0, icur = 0, m_cur = m, level = 0;
     // own: this level's windows [olo, ohi) of this CTA are the ones it wrote
     // in the last level's carry pass, which ended without a grid barrier
     bool own = false;
@@ -1514,8 +1515,8 @@ __global__ void __launch_bounds__(BLOCK, MINB) update_kernel(UpdateArgs A) {
         L.a = cur ? A.wa[1] : A.wa[0];
         L.b = cur ? A.wb[1] : A.wb[0];
         L.flag = A.wflag[level & 1];
-        const uint64_t *pk = cur ? A.ikeys[1] : A.ikeys[0];
-        const uint8_t *pv = cur ? A.ivals[1] : A.ivals[0];
+        const uint64_t *pk = icur ? A.ikeys[1] : A.ikeys[0];
+        const uint8_t *pv = icur ? A.ivals[1] : A.ivals[0];
         // one run of windows per segment length (a single run for one graph)
         for (uint32_t s = 2; s <= 32; s <<= 1) {
             uint32_t r0 = 0, r1 = nw;
@@ -1588,8 +1589,8 @@ __global__ void __launch_bounds__(BLOCK, MINB) update_kernel(UpdateArgs A) {
         uint32_t *nwg = nxt ? A.wgraph[1] : A.wgraph[0];
         uint32_t *nwa = nxt ? A.wa[1] : A.wa[0];
         uint32_t *nwb = nxt ? A.wb[1] : A.wb[0];
-        uint64_t *nk = nxt ? A.ikeys[1] : A.ikeys[0];
-        uint8_t *nv = nxt ? A.ivals[1] : A.ivals[0];
+        uint64_t *nk = icur ? A.ikeys[0] : A.ikeys[1];
+        uint8_t *nv = icur ? A.ivals[0] : A.ivals[1];
         if (!fused) {
             count_rejected(A, L, level, lo, hi, false, CNT(scan_id), CNTI(scan_id));
             if (!grid_barrier(A.bar, &st->err))
@@ -1606,6 +1607,14 @@ __global__ void __launch_bounds__(BLOCK, MINB) update_kernel(UpdateArgs A) {
             ++level;
             break;
         }
+        // A level that accepted nothing leaves every insertion where it is: the
+        // compaction would copy the buffer onto itself, and where few windows
+        // hold most insertions (a load of a skewed graph, whose windows are all
+        // too full up to the root), through the few CTAs that own them: 0.75M
+        // edges into 100,000 rows spent 8.0 ms in 14 levels, LOADFIG. One
+        // graph's root window likewise hands its range to the host in place.
+        const bool keep = total_i == m_cur;
+        const bool in_place = keep || (A.G == 1 && level >= A.gd[0].height);
         // GROUP_ITEMS consecutive windows per thread per round; the rejected
         // windows' copy plan goes to a compact list in shared memory (free
         // again once the level's windows are written): source, destination
@@ -1687,6 +1696,7 @@ __global__ void __launch_bounds__(BLOCK, MINB) update_kernel(UpdateArgs A) {
                     // the root rebalance takes these: the graph's area of the
                     // remaining-insertion buffer, at its first insertion
                     A.gs[g].remaining = c;
+                    A.gs[g].from = wa[q + 1] | (icur << 31);  // where they are, for one graph
                     l_to[li] = A.gs[g].ins_base | 0x80000000u;
                     ++li;
                     continue;
@@ -1706,28 +1716,46 @@ __global__ void __launch_bounds__(BLOCK, MINB) update_kernel(UpdateArgs A) {
             __syncthreads();
             // copy the kept insertions: position p of the round's
             // concatenation (p < tot_a) is element p - l_pre[t] of entry t,
-            // the last entry with l_pre <= p
-            for (uint32_t p = threadIdx.x; p < tot_a; p += BLOCK) {
-                uint32_t lo2 = 0, hi2 = tot_r;  // answer in [0, tot_r)
-                while (hi2 - lo2 > 1) {
-                    const uint32_t mid = (lo2 + hi2) >> 1;
-                    if (l_pre[mid] <= p)
-                        lo2 = mid;
-                    else
-                        hi2 = mid;
+            // the last entry with l_pre <= p. COPY_ILP positions per thread
+            // together: a CTA may own a window of 100,000 insertions.
+            constexpr int COPY_ILP = 4;
+            for (uint32_t p0 = threadIdx.x; p0 < tot_a && !in_place; p0 += COPY_ILP * BLOCK) {
+                uint32_t e[COPY_ILP];
+#pragma unroll
+                for (int u = 0; u < COPY_ILP; ++u)
+                    e[u] = 0;
+                for (uint32_t step = 1u << (31 - __clz(tot_r)); step > 0; step >>= 1) {
+#pragma unroll
+                    for (int u = 0; u < COPY_ILP; ++u)
+                        if (e[u] + step < tot_r && l_pre[e[u] + step] <= p0 + u * BLOCK)
+                            e[u] += step;
                 }
-                const uint32_t k = p - l_pre[lo2], to = l_to[lo2];
-                const uint32_t from = l_src[lo2] + k;
-                uint64_t *dk = (to >> 31) ? A.rkeys : nk;
-                uint8_t *dv = (to >> 31) ? A.rvals : nv;
-                dk[(to & 0x7FFFFFFFu) + k] = pk[from];
-                dv[(to & 0x7FFFFFFFu) + k] = pv[from];
+                uint64_t k[COPY_ILP];
+                uint8_t v[COPY_ILP];
+#pragma unroll
+                for (int u = 0; u < COPY_ILP; ++u) {
+                    const uint32_t p = p0 + u * BLOCK;
+                    if (p < tot_a) {
+                        k[u] = pk[l_src[e[u]] + (p - l_pre[e[u]])];
+                        v[u] = pv[l_src[e[u]] + (p - l_pre[e[u]])];
+                    }
+                }
+#pragma unroll
+                for (int u = 0; u < COPY_ILP; ++u) {
+                    const uint32_t p = p0 + u * BLOCK;
+                    if (p < tot_a) {
+                        const uint32_t to = l_to[e[u]];
+                        const uint32_t at = (to & 0x7FFFFFFFu) + (p - l_pre[e[u]]);
+                        ((to >> 31) ? A.rkeys : nk)[at] = k[u];
+                        ((to >> 31) ? A.rvals : nv)[at] = v[u];
+                    }
+                }
             }
             __syncthreads();
             base += tot_h;
             base_i += tot_i;
         }
-        if (hi > lo && hi < nw) {
+        if (hi > lo && hi < nw && !in_place) {
             // the last window's right sibling, rejected, begins the next
             // CTA's range: its insertions follow this CTA's
             const uint32_t j = hi - 1;
@@ -1764,6 +1792,10 @@ __global__ void __launch_bounds__(BLOCK, MINB) update_kernel(UpdateArgs A) {
         }
         nw = nw_next;
         cur = nxt;
+        if (!keep) {
+            icur ^= 1;
+            m_cur = total_i;
+        }
     }
     if (stamper)
         st->stamp[4] = globaltimer_ns();
@@ -3123,9 +3155,13 @@ gpma_status update_finish(gpma_graph *const *graphs, uint32_t k, BatchBuffers &b
         return root_rebuild(graphs[0], true, buf.ikeys[0], buf.ivals[0], h.inserts, s);
     for (uint32_t i = 0; i < k; ++i) {
         const GraphStatus &gs = h_gs[i];
-        if (gs.remaining > 0)
-            GPMA_TRY(root_rebuild(graphs[i], false, buf.rkeys + gs.ins_base, buf.rvals + gs.ins_base, gs.remaining,
-                                  s));
+        if (gs.remaining == 0)
+            continue;
+        // one graph: its root window's insertions are still in the insertion buffer
+        const uint32_t at = k == 1 ? gs.from & 0x7FFFFFFFu : gs.ins_base;
+        const uint64_t *pk = (k > 1 ? buf.rkeys : buf.ikeys[gs.from >> 31]) + at;
+        const uint8_t *pv = (k > 1 ? buf.rvals : buf.ivals[gs.from >> 31]) + at;
+        GPMA_TRY(root_rebuild(graphs[i], false, pk, pv, gs.remaining, s));
     }
     return GPMA_OK;
 }
