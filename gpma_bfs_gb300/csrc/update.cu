@@ -1123,6 +1123,49 @@ __device__ bool small_front(const UpdateArgs &A, unsigned char *smem, uint32_t *
     return true;
 }
 
+// Copies a round's kept insertions: position p < tot_a of their concatenation is
+// element p - l_pre[t] of entry t of tot_r, the last entry with l_pre <= p, and
+// goes to l_to[t] onwards of nk/nv, or of rk/rv with bit 31 set. COPY_ILP
+// positions per thread together: a CTA may own a window of 100,000 insertions.
+// Not inlined: the level loop around it has no registers to spare.
+__device__ __noinline__ void copy_kept(const uint32_t *l_src, const uint32_t *l_pre, const uint32_t *l_to,
+                                       uint32_t tot_r, uint32_t tot_a, const uint64_t *pk, const uint8_t *pv,
+                                       uint64_t *nk, uint8_t *nv, uint64_t *rk, uint8_t *rv) {
+    constexpr int COPY_ILP = 4;
+    for (uint32_t p0 = threadIdx.x; p0 < tot_a; p0 += COPY_ILP * BLOCK) {
+        uint32_t e[COPY_ILP];
+#pragma unroll
+        for (int u = 0; u < COPY_ILP; ++u)
+            e[u] = 0;
+        for (uint32_t step = 1u << (31 - __clz(tot_r)); step > 0; step >>= 1) {
+#pragma unroll
+            for (int u = 0; u < COPY_ILP; ++u)
+                if (e[u] + step < tot_r && l_pre[e[u] + step] <= p0 + u * BLOCK)
+                    e[u] += step;
+        }
+        uint64_t k[COPY_ILP];
+        uint8_t v[COPY_ILP];
+#pragma unroll
+        for (int u = 0; u < COPY_ILP; ++u) {
+            const uint32_t p = p0 + u * BLOCK;
+            if (p < tot_a) {
+                k[u] = pk[l_src[e[u]] + (p - l_pre[e[u]])];
+                v[u] = pv[l_src[e[u]] + (p - l_pre[e[u]])];
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < COPY_ILP; ++u) {
+            const uint32_t p = p0 + u * BLOCK;
+            if (p < tot_a) {
+                const uint32_t to = l_to[e[u]];
+                const uint32_t at = (to & 0x7FFFFFFFu) + (p - l_pre[e[u]]);
+                ((to >> 31) ? rk : nk)[at] = k[u];
+                ((to >> 31) ? rv : nv)[at] = v[u];
+            }
+        }
+    }
+}
+
 // Two register budgets of the same kernel: MINB resident CTAs per SM. Two
 // (128 registers, almost no spills) suits single large graphs, whose phases
 // are short and barrier-bound; three (80 registers, some spills to local
@@ -1495,11 +1538,13 @@ __global__ void __launch_bounds__(BLOCK, MINB) update_kernel(UpdateArgs A) {
     if (stamper)
         st->stamp[3] = globaltimer_ns();
 
-    // Level loop. Windows live in ping-pong buffers selected by `cur`, their
-    // pending insertions (m_cur of them) in ones selected by `icur`; each
-    // window's insertions are the contiguous range [wa, wb) of the current
+    // Level loop. Windows and their pending insertions (s_pending of them) live
+    // in two pairs of ping-pong buffers; each window's insertions are the contiguous range [wa, wb) of the current
     // insertion buffer, and the ranges follow one another from 0.
-    uint32_t cur = 0, icur = 0, m_cur = m, level = 0;
+    uint32_t cur = 0, level = 0;  // cur: bit 0 the windows' buffers, bit 1 the insertions'
+    __shared__ uint32_t s_pending;
+    if (threadIdx.x == 0)
+        s_pending = m;  // read after the level's barriers
     // own: this level's windows [olo, ohi) of this CTA are the ones it wrote
     // in the last level's carry pass, which ended without a grid barrier
     bool own = false;
@@ -1510,13 +1555,13 @@ __global__ void __launch_bounds__(BLOCK, MINB) update_kernel(UpdateArgs A) {
         // ones right away, so the level needs one grid barrier fewer
         const bool fused = A.G == 1 && (A.gd[0].seg << level) <= CTA_WINDOW_MAX;
         Windows L;
-        L.node = cur ? A.wnode[1] : A.wnode[0];
-        L.graph = cur ? A.wgraph[1] : A.wgraph[0];
-        L.a = cur ? A.wa[1] : A.wa[0];
-        L.b = cur ? A.wb[1] : A.wb[0];
+        L.node = (cur & 1) ? A.wnode[1] : A.wnode[0];
+        L.graph = (cur & 1) ? A.wgraph[1] : A.wgraph[0];
+        L.a = (cur & 1) ? A.wa[1] : A.wa[0];
+        L.b = (cur & 1) ? A.wb[1] : A.wb[0];
         L.flag = A.wflag[level & 1];
-        const uint64_t *pk = icur ? A.ikeys[1] : A.ikeys[0];
-        const uint8_t *pv = icur ? A.ivals[1] : A.ivals[0];
+        const uint64_t *pk = (cur & 2) ? A.ikeys[1] : A.ikeys[0];
+        const uint8_t *pv = (cur & 2) ? A.ivals[1] : A.ivals[0];
         // one run of windows per segment length (a single run for one graph)
         for (uint32_t s = 2; s <= 32; s <<= 1) {
             uint32_t r0 = 0, r1 = nw;
@@ -1584,13 +1629,13 @@ __global__ void __launch_bounds__(BLOCK, MINB) update_kernel(UpdateArgs A) {
         // parent window (up_level, gpma.cuh:881-889 + regrouping). A rejected
         // root window leaves its insertions to the root rebalance: they go to
         // the graph's area of the remaining-insertion buffer.
-        const uint32_t nxt = cur ^ 1;
+        const bool nxt = !(cur & 1);
         uint32_t *nwn = nxt ? A.wnode[1] : A.wnode[0];
         uint32_t *nwg = nxt ? A.wgraph[1] : A.wgraph[0];
         uint32_t *nwa = nxt ? A.wa[1] : A.wa[0];
         uint32_t *nwb = nxt ? A.wb[1] : A.wb[0];
-        uint64_t *nk = icur ? A.ikeys[0] : A.ikeys[1];
-        uint8_t *nv = icur ? A.ivals[0] : A.ivals[1];
+        uint64_t *nk = (cur & 2) ? A.ikeys[0] : A.ikeys[1];
+        uint8_t *nv = (cur & 2) ? A.ivals[0] : A.ivals[1];
         if (!fused) {
             count_rejected(A, L, level, lo, hi, false, CNT(scan_id), CNTI(scan_id));
             if (!grid_barrier(A.bar, &st->err))
@@ -1611,9 +1656,9 @@ __global__ void __launch_bounds__(BLOCK, MINB) update_kernel(UpdateArgs A) {
         // compaction would copy the buffer onto itself, and where few windows
         // hold most insertions (a load of a skewed graph, whose windows are all
         // too full up to the root), through the few CTAs that own them: 0.75M
-        // edges into 100,000 rows spent 8.0 ms in 14 levels, LOADFIG. One
+        // edges into 100,000 rows spent 8.0 ms in 14 levels, 0.16 now. One
         // graph's root window likewise hands its range to the host in place.
-        const bool keep = total_i == m_cur;
+        const bool keep = total_i == s_pending;
         const bool in_place = keep || (A.G == 1 && level >= A.gd[0].height);
         // GROUP_ITEMS consecutive windows per thread per round; the rejected
         // windows' copy plan goes to a compact list in shared memory (free
@@ -1696,7 +1741,7 @@ __global__ void __launch_bounds__(BLOCK, MINB) update_kernel(UpdateArgs A) {
                     // the root rebalance takes these: the graph's area of the
                     // remaining-insertion buffer, at its first insertion
                     A.gs[g].remaining = c;
-                    A.gs[g].from = wa[q + 1] | (icur << 31);  // where they are, for one graph
+                    A.gs[g].from = wa[q + 1] | ((cur >> 1) << 31);  // where they are, for one graph
                     l_to[li] = A.gs[g].ins_base | 0x80000000u;
                     ++li;
                     continue;
@@ -1714,43 +1759,8 @@ __global__ void __launch_bounds__(BLOCK, MINB) update_kernel(UpdateArgs A) {
                 nb += c;
             }
             __syncthreads();
-            // copy the kept insertions: position p of the round's
-            // concatenation (p < tot_a) is element p - l_pre[t] of entry t,
-            // the last entry with l_pre <= p. COPY_ILP positions per thread
-            // together: a CTA may own a window of 100,000 insertions.
-            constexpr int COPY_ILP = 4;
-            for (uint32_t p0 = threadIdx.x; p0 < tot_a && !in_place; p0 += COPY_ILP * BLOCK) {
-                uint32_t e[COPY_ILP];
-#pragma unroll
-                for (int u = 0; u < COPY_ILP; ++u)
-                    e[u] = 0;
-                for (uint32_t step = 1u << (31 - __clz(tot_r)); step > 0; step >>= 1) {
-#pragma unroll
-                    for (int u = 0; u < COPY_ILP; ++u)
-                        if (e[u] + step < tot_r && l_pre[e[u] + step] <= p0 + u * BLOCK)
-                            e[u] += step;
-                }
-                uint64_t k[COPY_ILP];
-                uint8_t v[COPY_ILP];
-#pragma unroll
-                for (int u = 0; u < COPY_ILP; ++u) {
-                    const uint32_t p = p0 + u * BLOCK;
-                    if (p < tot_a) {
-                        k[u] = pk[l_src[e[u]] + (p - l_pre[e[u]])];
-                        v[u] = pv[l_src[e[u]] + (p - l_pre[e[u]])];
-                    }
-                }
-#pragma unroll
-                for (int u = 0; u < COPY_ILP; ++u) {
-                    const uint32_t p = p0 + u * BLOCK;
-                    if (p < tot_a) {
-                        const uint32_t to = l_to[e[u]];
-                        const uint32_t at = (to & 0x7FFFFFFFu) + (p - l_pre[e[u]]);
-                        ((to >> 31) ? A.rkeys : nk)[at] = k[u];
-                        ((to >> 31) ? A.rvals : nv)[at] = v[u];
-                    }
-                }
-            }
+            if (!in_place)
+                copy_kept(l_src, l_pre, l_to, tot_r, tot_a, pk, pv, nk, nv, A.rkeys, A.rvals);
             __syncthreads();
             base += tot_h;
             base_i += tot_i;
@@ -1791,11 +1801,10 @@ __global__ void __launch_bounds__(BLOCK, MINB) update_kernel(UpdateArgs A) {
             return;
         }
         nw = nw_next;
-        cur = nxt;
-        if (!keep) {
-            icur ^= 1;
-            m_cur = total_i;
-        }
+        cur ^= keep ? 1u : 3u;
+        __syncthreads();  // every thread has compared s_pending
+        if (threadIdx.x == 0)
+            s_pending = total_i;
     }
     if (stamper)
         st->stamp[4] = globaltimer_ns();
