@@ -162,6 +162,46 @@ __device__ __forceinline__ uint32_t leaf_find(const GraphDesc &D, uint32_t leaf,
     return hit;
 }
 
+// The same for each lane's leaf and key, by all lanes of the warp together (a
+// lane without work passes leaf SIZE_NONE): seg/2 lanes read a leaf, a slot pair
+// each, so that a load instruction touches 64/seg leaves as whole runs of slots
+// instead of 32 leaves 16 bytes at a time. SEG_PAIRS is seg/2 (1, 2, 4, 8, 16).
+// Its shuffles pay where many keys per thread keep the load path busy: 10.5M
+// keys, R-MAT 21, locate 627 -> 519 us; the social slide, four keys per thread,
+// 20 us with a leaf per lane, 33 this way, so the builds for smaller launches
+// scan a leaf per lane.
+template <uint32_t SEG_PAIRS>
+__device__ __forceinline__ uint32_t warp_leaf_find(const uint64_t *keys, uint32_t leaf, uint64_t key) {
+    const uint32_t lane = threadIdx.x & 31;
+    const uint32_t part = lane % SEG_PAIRS, grp = lane / SEG_PAIRS;
+    constexpr uint32_t PER = 32 / SEG_PAIRS;  // leaves per load
+    ulonglong2 q[SEG_PAIRS];
+#pragma unroll
+    for (uint32_t r = 0; r < SEG_PAIRS; ++r) {
+        const uint32_t lf = __shfl_sync(0xFFFFFFFFu, leaf, r * PER + grp);
+        q[r] = make_ulonglong2(0, 0);
+        if (lf != SIZE_NONE)
+            q[r] = *reinterpret_cast<const ulonglong2 *>(keys + lf + 2 * part);
+    }
+    uint32_t hit = SIZE_NONE;
+#pragma unroll
+    for (uint32_t r = 0; r < SEG_PAIRS; ++r) {
+        const uint64_t k = __shfl_sync(0xFFFFFFFFu, key, r * PER + grp);
+        const uint32_t first = __ballot_sync(0xFFFFFFFFu, q[r].x == k), second = __ballot_sync(0xFFFFFFFFu, q[r].y == k);
+        // this lane's own leaf was read in round lane / PER by group lane % PER
+        if (lane / PER == r) {
+            const uint32_t sh = (lane % PER) * SEG_PAIRS;
+            const uint32_t mask = SEG_PAIRS == 32 ? 0xFFFFFFFFu : (1u << SEG_PAIRS) - 1;
+            const uint32_t a = (first >> sh) & mask, b = (second >> sh) & mask;
+            if (a | b) {
+                const uint32_t p = __ffs(a | b) - 1;
+                hit = 2 * p + (((a >> p) & 1u) ? 0u : 1u);
+            }
+        }
+    }
+    return leaf == SIZE_NONE ? SIZE_NONE : hit;
+}
+
 // Locates LOC_ILP updates per thread together: at each level of the descent
 // every key's probe is issued before any comparison, so a thread keeps
 // LOC_ILP dependent chains in flight instead of one.
@@ -169,114 +209,90 @@ constexpr int LOC_ILP = 4;
 // Consecutive items per thread in the grouping passes.
 constexpr uint32_t GROUP_ITEMS = 4;
 
-// Keys i0 + j * stride (j < LOC_ILP) below `end`; returns how many of them
-// are insertions (leaf set).
-template <bool SCANS_FIRST>
-__device__ __forceinline__ uint32_t locate_keys(const UpdateArgs &A, const uint64_t *bk, const uint8_t *bv,
+template <uint32_t SEG_PAIRS>
+__device__ __forceinline__ void find_all(const uint64_t *keys, const uint32_t (&leaf)[LOC_ILP],
+                                         const uint64_t (&key)[LOC_ILP], uint32_t (&hit)[LOC_ILP]) {
+#pragma unroll
+    for (int j = 0; j < LOC_ILP; ++j)
+        hit[j] = warp_leaf_find<SEG_PAIRS>(keys, leaf[j], key[j]);
+}
+
+// Keys i0 + j * stride (j < LOC_ILP) below `end`, all of graph g; returns how
+// many of them are insertions (leaf set). fk: the heads at every 2^log2stride
+// slots, in shared memory. Whole warps only (a lane may be past `end`). COOP:
+// warps scan their leaves together.
+template <bool COOP>
+__device__ __forceinline__ uint32_t locate_keys(const UpdateArgs &A, uint32_t g, const uint64_t *bk, const uint8_t *bv,
                                                 uint32_t i0, uint32_t stride, uint32_t end, const uint64_t *fk,
                                                 uint32_t log2stride) {
-    uint32_t idx[LOC_ILP], prefix[LOC_ILP], bit[LOC_ILP], g[LOC_ILP];
+    const GraphDesc &D = A.gd[g];
+    uint32_t prefix[LOC_ILP];
     uint64_t key[LOC_ILP];
+    uint8_t value[LOC_ILP];
 #pragma unroll
     for (int j = 0; j < LOC_ILP; ++j) {
-        idx[j] = i0 + j * stride;
+        const uint32_t i = i0 + j * stride;
         prefix[j] = 0;
-        bit[j] = 0;
-        g[j] = 0;
-        key[j] = 0;
-        if (idx[j] < end) {
-            g[j] = graph_of(A, idx[j]);
-            const GraphDesc &D = A.gd[g[j]];
-            key[j] = bk[idx[j]];
-            bit[j] = (D.seg << D.height) >> 1;
-            if (fk) {  // one graph: the top levels from shared memory
-                const uint32_t sstride = 1u << log2stride;
-                while (sstride <= bit[j]) {
-                    if (fk[(prefix[j] | bit[j]) >> log2stride] <= key[j])
-                        prefix[j] |= bit[j];
-                    bit[j] >>= 1;
-                }
-            }
-        }
+        key[j] = i < end ? bk[i] : 0ull;
+        value[j] = i < end ? bv[i] : 0;
     }
-    // the remaining levels of the reference's descent (gpma.cuh:209-216),
-    // interleaved. Every probed slot starts a segment (prefix and bit are
-    // multiples of seg), so its key is read from the dense heads array.
-    for (;;) {
+    // the reference's descent (gpma.cuh:209-216), the keys level by level
+    // together, the level the same for all (a level per key, looked up with
+    // its graph, took 25 us on the social slide, this 20). Every probed slot starts a segment (prefix and bit are
+    // multiples of seg), so below the cached levels its key is read from the
+    // dense heads array.
+    const uint32_t seg = D.seg, log2seg = D.log2seg;
+    const uint64_t *heads = D.heads;
+    uint32_t bit = (seg << D.height) >> 1;
+    for (; bit >= 1u << log2stride; bit >>= 1) {
+#pragma unroll
+        for (int j = 0; j < LOC_ILP; ++j)
+            if (fk[(prefix[j] | bit) >> log2stride] <= key[j])
+                prefix[j] |= bit;
+    }
+    for (; bit >= seg; bit >>= 1) {
         uint64_t probe[LOC_ILP];
-        bool any = false;
 #pragma unroll
-        for (int j = 0; j < LOC_ILP; ++j) {
-            const GraphDesc &D = A.gd[g[j]];
-            const bool live = idx[j] < end && D.seg <= bit[j];
-            probe[j] = live ? D.heads[(prefix[j] | bit[j]) >> D.log2seg] : 0;
-            any |= live;
-        }
-        if (!any)
-            break;
+        for (int j = 0; j < LOC_ILP; ++j)
+            probe[j] = heads[(prefix[j] | bit) >> log2seg];
 #pragma unroll
-        for (int j = 0; j < LOC_ILP; ++j) {
-            if (idx[j] < end && A.gd[g[j]].seg <= bit[j]) {
-                if (probe[j] <= key[j])
-                    prefix[j] |= bit[j];
-                bit[j] >>= 1;
-            }
-        }
+        for (int j = 0; j < LOC_ILP; ++j)
+            if (probe[j] <= key[j])
+                prefix[j] |= bit;
     }
-    uint32_t inserts = 0;
-    if constexpr (SCANS_FIRST) {
-        // every leaf scan before any store: a value store (a byte) may alias
-        // the next scan's loads, which would otherwise wait for it (one graph:
-        // measured 30 -> 25 us on the social step; the many-graph build, with
-        // fewer registers, keeps the interleaved order)
-        uint32_t hit[LOC_ILP];
-        uint8_t value[LOC_ILP];
 #pragma unroll
-        for (int j = 0; j < LOC_ILP; ++j) {
-            hit[j] = SIZE_NONE;
-            value[j] = 0;
-            if (idx[j] >= end)
-                continue;
-            const GraphDesc &D = A.gd[g[j]];
-            value[j] = bv[idx[j]];
-            if (!in_bounds(&A.st->err, (uint64_t)prefix[j] + D.seg <= D.size, BS_LEAF)) {
-                prefix[j] = SIZE_NONE;  // the key is skipped
-                continue;
-            }
-            hit[j] = leaf_find(D, prefix[j], key[j]);
-        }
-#pragma unroll
-        for (int j = 0; j < LOC_ILP; ++j) {
-            if (idx[j] >= end)
-                continue;
-            uint32_t leaf = value[j] == 0 || prefix[j] == SIZE_NONE ? SIZE_NONE : prefix[j];
-            if (hit[j] != SIZE_NONE) {
-                A.gd[g[j]].vals[prefix[j] + hit[j]] = value[j];  // delete / modify / revive in place
-                leaf = SIZE_NONE;
-            }
-            A.leaf[idx[j]] = leaf;
-            inserts += leaf != SIZE_NONE;
+    for (int j = 0; j < LOC_ILP; ++j)
+        if (i0 + j * stride >= end || !in_bounds(&A.st->err, (uint64_t)prefix[j] + seg <= D.size, BS_LEAF))
+            prefix[j] = SIZE_NONE;  // no key, or skipped
+    // every leaf scan before any store: a value store (a byte) may alias the
+    // next scan's loads, which would otherwise wait for it
+    uint32_t hit[LOC_ILP];
+    if constexpr (COOP) {
+        switch (seg) {
+        case 2: find_all<1>(D.keys, prefix, key, hit); break;
+        case 4: find_all<2>(D.keys, prefix, key, hit); break;
+        case 8: find_all<4>(D.keys, prefix, key, hit); break;
+        case 16: find_all<8>(D.keys, prefix, key, hit); break;
+        default: find_all<16>(D.keys, prefix, key, hit); break;
         }
     } else {
 #pragma unroll
-        for (int j = 0; j < LOC_ILP; ++j) {
-            if (idx[j] >= end)
-                continue;
-            const GraphDesc &D = A.gd[g[j]];
-            const uint8_t value = bv[idx[j]];
-            uint32_t leaf = value == 0 ? SIZE_NONE : prefix[j];
-            if (!in_bounds(&A.st->err, (uint64_t)prefix[j] + D.seg <= D.size, BS_LEAF)) {
-                A.leaf[idx[j]] = SIZE_NONE;
-                continue;
-            }
-            const uint32_t hit = leaf_find(D, prefix[j], key[j]);
-            if (hit != SIZE_NONE) {
-                D.vals[prefix[j] + hit] = value;  // delete / modify / revive in place
-                leaf = SIZE_NONE;
-            }
-            A.leaf[idx[j]] = leaf;
-            inserts += leaf != SIZE_NONE;
+        for (int j = 0; j < LOC_ILP; ++j)
+            hit[j] = prefix[j] != SIZE_NONE ? leaf_find(D, prefix[j], key[j]) : SIZE_NONE;
+    }
+    uint32_t inserts = 0;
+#pragma unroll
+    for (int j = 0; j < LOC_ILP; ++j) {
+        const uint32_t i = i0 + j * stride;
+        if (i >= end)
+            continue;
+        uint32_t leaf = value[j] == 0 ? SIZE_NONE : prefix[j];
+        if (hit[j] != SIZE_NONE) {
+            D.vals[prefix[j] + hit[j]] = value[j];  // delete / modify / revive in place
+            leaf = SIZE_NONE;
         }
+        A.leaf[i] = leaf;
+        inserts += leaf != SIZE_NONE;
     }
     return inserts;
 }
@@ -1307,8 +1323,8 @@ __global__ void __launch_bounds__(BLOCK, MINB) update_kernel(UpdateArgs A) {
                 // compaction after the barrier
                 uint32_t lo, hi, mine = 0;
                 cta_range(A.n, lo, hi);
-                for (uint32_t i0 = lo + threadIdx.x; i0 < hi; i0 += LOC_ILP * BLOCK)
-                    mine += locate_keys<true>(A, bk, bv, i0, BLOCK, hi, fk, log2stride);
+                for (uint32_t r0 = lo; r0 < hi; r0 += LOC_ILP * BLOCK)
+                    mine += locate_keys<MINB == 3>(A, 0, bk, bv, r0 + threadIdx.x, BLOCK, hi, fk, log2stride);
                 const uint32_t t = block_sum(mine, tmp);
                 if (threadIdx.x == 0)
                     CNT(scan_id)[blockIdx.x] = t;
@@ -1342,8 +1358,8 @@ __global__ void __launch_bounds__(BLOCK, MINB) update_kernel(UpdateArgs A) {
                             f[j] = hv[r];
                     }
                     __syncthreads();
-                    for (uint32_t i0 = pos + threadIdx.x; i0 < end; i0 += LOC_ILP * BLOCK)
-                        locate_keys<false>(A, bk, bv, i0, BLOCK, end, f, l2s);
+                    for (uint32_t r0 = pos; r0 < end; r0 += LOC_ILP * BLOCK)
+                        locate_keys<MINB == 3>(A, g, bk, bv, r0 + threadIdx.x, BLOCK, end, f, l2s);
                     __syncthreads();  // the copy is replaced for the next graph
                     pos = end;
                 }
