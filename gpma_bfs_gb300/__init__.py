@@ -685,6 +685,16 @@ def read_edges_text(path: str):
     return n.value, src, dst
 
 
+def _source_lists(sources):
+    """(all sources in one uint32 array, the address of each list in it, their lengths)."""
+    srcs = [np.asarray(s, np.uint32) for s in sources]
+    srcs = [s if s.ndim == 1 else s.reshape(-1)[:len(s)] for s in srcs]
+    ns = np.array([len(s) for s in srcs], np.uint32)
+    flat = np.concatenate(srcs) if srcs else np.zeros(0, np.uint32)
+    starts = np.cumsum(ns, dtype=np.uint64) - ns
+    return flat, np.uint64(flat.ctypes.data) + np.uint64(4) * starts, ns
+
+
 class Batch:
     """Many graphs per launch (no reference counterpart).
 
@@ -751,19 +761,18 @@ class Batch:
     def bfs_multi(self, graphs, sources, levels: bool = False, stream=None):
         """(levels per graph or None, reached per graph) for up to 64 sources per graph."""
         k = len(graphs)
-        srcs = [np.ascontiguousarray(np.asarray(s, np.uint32)) for s in sources]
+        flat, sp, ns = _source_lists(sources)
         hs = (ctypes.c_void_p * k)(*[g.handle.value for g in graphs])
-        sp = (ctypes.c_void_p * k)(*[s.ctypes.data for s in srcs])
-        ns = (ctypes.c_uint32 * k)(*[len(s) for s in srcs])
-        outs = [np.zeros((len(s), g.row_num), np.uint32) for s, g in zip(srcs, graphs)] if levels else None
+        counts = ns.tolist()
+        outs = [np.zeros((n, g.row_num), np.uint32) for n, g in zip(counts, graphs)] if levels else None
         lp = (ctypes.c_void_p * k)(*[o.ctypes.data for o in outs]) if levels else None
-        reached = np.zeros(sum(len(s) for s in srcs), np.uint64)
-        _check(lib().gpma_batch_bfs_multi(self._h, hs, sp, ns, k, lp, reached.ctypes.data, _stream_ptr(stream)),
-               "gpma_batch_bfs_multi")
+        reached = np.zeros(len(flat), np.uint64)
+        _check(lib().gpma_batch_bfs_multi(self._h, hs, sp.ctypes.data, ns.ctypes.data, k, lp, reached.ctypes.data,
+                                          _stream_ptr(stream)), "gpma_batch_bfs_multi")
         parts, o = [], 0
-        for s in srcs:
-            parts.append(reached[o:o + len(s)])
-            o += len(s)
+        for n in counts:
+            parts.append(reached[o:o + n])
+            o += n
         return outs, parts
 
     def set_profiling(self, enabled: bool = True) -> None:
