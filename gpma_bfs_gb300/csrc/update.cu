@@ -25,10 +25,10 @@
 //      Windows are ordered by graph and graphs by segment length, so the list
 //      splits into one contiguous run per segment length and each run has one
 //      window width: up to 256 slots per warp group, up to 2048 per CTA in
-//      shared memory, wider ones chunk by chunk over the whole grid. For one
-//      graph, a level of windows up to 2048 slots costs one grid barrier:
-//      each CTA dispatches, counts and carries a contiguous range of the
-//      windows and goes on with the next-level windows it wrote itself.
+//      shared memory, wider ones chunk by chunk over the whole grid. A level
+//      whose windows all have up to 2048 slots costs one grid barrier: each
+//      CTA dispatches, counts and carries a contiguous range of the windows
+//      and goes on with the next-level windows it wrote itself.
 // The host reads the status blocks once. Only the root resize (:1034-1044)
 // and the >= 5M-insertion rebuild (:936-966) run host-driven, per graph.
 #include "gpma_internal.cuh"
@@ -78,6 +78,7 @@ struct UpdateArgs {
     uint32_t G;
     uint32_t max_height;
     uint32_t min_height;    // below it no graph has a root window
+    uint32_t seg_graph[5];  // first graph whose segments have 2 << i slots or more
     const uint32_t *boff;   // batch offsets, G + 1
     const uint32_t *toff;   // sort tile offsets, G + 1
     uint32_t n;
@@ -869,17 +870,17 @@ __device__ __forceinline__ void small_dispatch(const UpdateArgs &A, Windows L, u
         cta_windows<W>(A, L, r0, r1, level, pk, pv, smem, tmp, acc, part, parts);
 }
 
-// First window in [0, nw) whose graph has segment length >= s (windows are
-// ordered by graph, graphs by segment length).
-__device__ __forceinline__ uint32_t first_window_of_seg(const UpdateArgs &A, const uint32_t *wg, uint32_t nw,
-                                                        uint32_t s) {
-    uint32_t lo = 0, hi = nw;
+// First window in [0, nw) whose graph is `graph` or later (windows are ordered by
+// graph), by all lanes of a warp: 33 parts per round.
+__device__ __forceinline__ uint32_t warp_first_window(const uint32_t *wg, uint32_t nw, uint32_t graph, uint32_t lane) {
+    uint32_t lo = 0, hi = nw;  // the answer is in [lo, hi]
     while (lo < hi) {
-        uint32_t mid = (lo + hi) >> 1;
-        if (A.gd[wg[mid]].seg < s)
-            lo = mid + 1;
-        else
-            hi = mid;
+        const uint32_t step = (hi - lo + 32) / 33;
+        const uint32_t p = lo + (lane + 1) * step - 1;
+        const uint32_t before = __popc(__ballot_sync(0xFFFFFFFFu, p < hi && wg[p] < graph));
+        if (before < 32)  // else the answer lies past the last probe
+            hi = min(hi, lo + (before + 1) * step - 1);
+        lo += before * step;
     }
     return lo;
 }
@@ -934,7 +935,7 @@ __device__ __forceinline__ void count_rejected(const UpdateArgs &A, const Window
 
 // The level's prefix sums over the per-CTA counts of count_rejected (written
 // before the last grid barrier): this CTA's first next-level window (base_h)
-// and insertion (base_i), and the totals. fused: one graph, counts taken with
+// and insertion (base_i), and the totals. fused: counts taken with
 // first_is_head; a CTA c >= 1 whose first window was counted as a start but
 // joins its left neighbour (both rejected, one parent, not root windows) has
 // that start taken off here, its fields read in the same round as the counts.
@@ -944,9 +945,7 @@ __device__ __forceinline__ void level_prefix(const UpdateArgs &A, const Windows 
                                              const uint32_t *cnt_i, uint32_t &base_h, uint32_t &total_h,
                                              uint32_t &base_i, uint32_t &total_i) {
     const uint32_t per = (nw + gridDim.x - 1) / gridDim.x;
-    const GraphDesc &D = A.gd[0];
-    const uint32_t W = D.seg << level;
-    const bool starts = fused && level < D.height;  // else no correction
+    const bool starts = fused && (A.G > 1 || level < A.gd[0].height);  // else no correction
     constexpr int CU = 2;  // CTAs per thread per step
     uint4 s = make_uint4(0, 0, 0, 0);
     for (uint32_t j0 = 0; j0 < gridDim.x; j0 += CU * BLOCK) {
@@ -964,7 +963,7 @@ __device__ __forceinline__ void level_prefix(const UpdateArgs &A, const Windows 
                 w_end[u] = slices ? __ldcg(slices + 2 * c + 1) : min(nw, c * per + per);
             }
         }
-        uint32_t f0[CU], fl[CU], nd[CU], ndl[CU];
+        uint32_t f0[CU], fl[CU], nd[CU], ndl[CU], g[CU], gl[CU];
 #pragma unroll
         for (int u = 0; u < CU; ++u) {
             const bool chk = w[u] < w_end[u] && w[u] > 0;  // a non-empty range with a window to its left
@@ -972,11 +971,18 @@ __device__ __forceinline__ void level_prefix(const UpdateArgs &A, const Windows 
             fl[u] = chk ? L.flag[w[u] - 1] : 1u;
             nd[u] = chk ? L.node[w[u]] : 0u;
             ndl[u] = chk ? L.node[w[u] - 1] : 0u;
+            g[u] = chk && A.G > 1 ? L.graph[w[u]] : 0u;
+            gl[u] = chk && A.G > 1 ? L.graph[w[u] - 1] : 0u;
         }
 #pragma unroll
         for (int u = 0; u < CU; ++u) {
             const uint32_t c = j0 + u * BLOCK + threadIdx.x;
-            const uint32_t h = vh[u] - ((!f0[u] && !fl[u] && (nd[u] & ~W) == (ndl[u] & ~W)) ? 1u : 0u);
+            uint32_t h = vh[u];
+            if (!f0[u] && !fl[u] && g[u] == gl[u]) {
+                const GraphDesc &D = A.gd[g[u]];
+                const uint32_t W = D.seg << level;
+                h -= level < D.height && (nd[u] & ~W) == (ndl[u] & ~W) ? 1u : 0u;
+            }
             const bool before = c < blockIdx.x;
             s.x += before ? h : 0u;
             s.y += h;
@@ -1558,7 +1564,7 @@ __global__ void __launch_bounds__(BLOCK, MINB) update_kernel(UpdateArgs A) {
     // in two pairs of ping-pong buffers; each window's insertions are the contiguous range [wa, wb) of the current
     // insertion buffer, and the ranges follow one another from 0.
     uint32_t cur = 0, level = 0;  // cur: bit 0 the windows' buffers, bit 1 the insertions'
-    __shared__ uint32_t s_pending;
+    __shared__ uint32_t s_pending, s_run[6];
     if (threadIdx.x == 0)
         s_pending = m;  // read after the level's barriers
     // own: this level's windows [olo, ohi) of this CTA are the ones it wrote
@@ -1566,10 +1572,13 @@ __global__ void __launch_bounds__(BLOCK, MINB) update_kernel(UpdateArgs A) {
     bool own = false;
     uint32_t olo = 0, ohi = 0;
     for (; level <= A.max_height && nw > 0; ++level) {
-        // one graph, windows of at most CTA_WINDOW_MAX slots: each CTA
+        // windows of at most CTA_WINDOW_MAX slots in every graph: each CTA
         // dispatches a contiguous range of the windows and counts its rejected
-        // ones right away, so the level needs one grid barrier fewer
-        const bool fused = A.G == 1 && (A.gd[0].seg << level) <= CTA_WINDOW_MAX;
+        // ones right away, so the level needs one grid barrier fewer (two, where
+        // the next one is such a level too). 20 graphs, 0.35M keys: levels
+        // 169 -> 82 us with this and the runs' bounds found by warps.
+        const uint32_t max_seg = A.gd[A.G - 1].seg;  // graphs are ordered by segment length
+        const bool fused = (max_seg << level) <= CTA_WINDOW_MAX;
         Windows L;
         L.node = (cur & 1) ? A.wnode[1] : A.wnode[0];
         L.graph = (cur & 1) ? A.wgraph[1] : A.wgraph[0];
@@ -1578,36 +1587,40 @@ __global__ void __launch_bounds__(BLOCK, MINB) update_kernel(UpdateArgs A) {
         L.flag = A.wflag[level & 1];
         const uint64_t *pk = (cur & 2) ? A.ikeys[1] : A.ikeys[0];
         const uint8_t *pv = (cur & 2) ? A.ivals[1] : A.ivals[0];
-        // one run of windows per segment length (a single run for one graph)
-        for (uint32_t s = 2; s <= 32; s <<= 1) {
-            uint32_t r0 = 0, r1 = nw;
-            if (A.G > 1) {
-                r0 = first_window_of_seg(A, L.graph, nw, s);
-                r1 = first_window_of_seg(A, L.graph, nw, 2 * s);
-            } else if (A.gd[0].seg != s) {
-                continue;
+        if (own) {
+            lo = olo;
+            hi = ohi;
+        } else {
+            cta_range(nw, lo, hi);
+        }
+        // one run of windows per segment length (a single run for one graph);
+        // run i, of length 2 << i, is [s_run[i], s_run[i + 1]). A fused level
+        // looks at the CTA's own windows only: others may not be written yet.
+        const uint32_t w_lo = fused ? lo : 0u, w_hi = fused ? hi : nw;
+        if (A.G > 1) {
+            const uint32_t w = threadIdx.x >> 5;
+            if (w <= 5) {
+                const uint32_t at = w == 0   ? w_lo
+                                    : w == 5 ? w_hi
+                                             : w_lo + warp_first_window(L.graph + w_lo, w_hi - w_lo, A.seg_graph[w],
+                                                                        threadIdx.x & 31);
+                s_run[w] = at;
             }
-            if (r0 >= r1)
+            __syncthreads();
+        }
+        for (uint32_t i = 0; i < 5; ++i) {
+            const uint32_t s = 2u << i;
+            if (A.G == 1 && A.gd[0].seg != s)
                 continue;
-            uint32_t W = s << level;
+            const uint32_t d0 = A.G == 1 ? w_lo : s_run[i], d1 = A.G == 1 ? w_hi : s_run[i + 1];
+            if (d0 >= d1)
+                continue;
+            const uint32_t W = s << level;
             const unsigned long long before = acc;
             // windows over the grid; with the count fused into this phase,
             // each CTA takes the contiguous range it counts (and copies) next
-            uint32_t d0 = r0, d1 = r1, part = blockIdx.x, parts = gridDim.x;
-            if (fused) {
-                if (own) {
-                    d0 = olo;
-                    d1 = ohi;
-                } else {
-                    cta_range(nw, d0, d1);
-                }
-                part = 0;
-                parts = 1;
-                if (d0 >= d1)
-                    W = 0;  // nothing for this CTA: no dispatch
-            }
+            const uint32_t part = fused ? 0u : blockIdx.x, parts = fused ? 1u : gridDim.x;
             switch (W) {
-            case 0: break;
             case 2: small_dispatch<2>(A, L, d0, d1, level, pk, pv, smem, tmp, acc, part, parts); break;
             case 4: small_dispatch<4>(A, L, d0, d1, level, pk, pv, smem, tmp, acc, part, parts); break;
             case 8: small_dispatch<8>(A, L, d0, d1, level, pk, pv, smem, tmp, acc, part, parts); break;
@@ -1620,19 +1633,13 @@ __global__ void __launch_bounds__(BLOCK, MINB) update_kernel(UpdateArgs A) {
             case 1024: small_dispatch<1024>(A, L, d0, d1, level, pk, pv, smem, tmp, acc, part, parts); break;
             case 2048: small_dispatch<2048>(A, L, d0, d1, level, pk, pv, smem, tmp, acc, part, parts); break;
             default:
-                if (!grid_windows(A, L, r0, r1, W, level, pk, pv, smem, tmp, acc))
+                if (!grid_windows(A, L, d0, d1, W, level, pk, pv, smem, tmp, acc))
                     return;
             }
             acc_slots += (acc - before) * (unsigned long long)W;
             // the next run lays out shared memory differently: every warp of
             // the CTA must be done with this run's staging first
             __syncthreads();
-        }
-        if (own) {
-            lo = olo;
-            hi = ohi;
-        } else {
-            cta_range(nw, lo, hi);
         }
         if (fused)  // the CTA's own range was dispatched (and flagged) by its own warps
             count_rejected(A, L, level, lo, hi, true, CNT(scan_id), CNTI(scan_id));
@@ -1805,7 +1812,7 @@ __global__ void __launch_bounds__(BLOCK, MINB) update_kernel(UpdateArgs A) {
         // this level's barrier. The window flags alternate by level, so a CTA
         // flagging the next level's windows does not overwrite ones a slower
         // CTA still reads here.
-        own = fused && nw_next > 0 && level + 1 <= A.max_height && (A.gd[0].seg << (level + 1)) <= CTA_WINDOW_MAX;
+        own = fused && nw_next > 0 && level + 1 <= A.max_height && (max_seg << (level + 1)) <= CTA_WINDOW_MAX;
         if (own) {
             olo = next_lo;
             ohi = base;
@@ -3069,6 +3076,9 @@ gpma_status update_plan(gpma_graph *const *graphs, const uint64_t *off, uint32_t
     A.G = k;
     A.max_height = max_height;
     A.min_height = min_height;
+    for (uint32_t i = 0; i < 5; ++i)
+        while (A.seg_graph[i] < k && graphs[A.seg_graph[i]]->geo.seg < 2u << i)
+            ++A.seg_graph[i];
     A.boff = buf.boff;
     A.toff = buf.toff;
     A.n = (uint32_t)n;
