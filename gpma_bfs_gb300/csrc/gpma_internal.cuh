@@ -148,6 +148,9 @@ uint32_t fls32(uint32_t x);
 // lists, sort state, per-graph tables).
 struct BatchBuffers {
     uint64_t cap = 0;  // keys
+    // one allocation for the arrays of `cap` entries up to wlive and qrec (a
+    // first large batch spent 1 ms in 20 allocations); several share a place
+    unsigned char *slab = nullptr;
     uint64_t *bkeys[2] = {nullptr, nullptr};
     uint8_t *bvals[2] = {nullptr, nullptr};
     uint32_t *leaf = nullptr;
@@ -161,7 +164,7 @@ struct BatchBuffers {
     uint32_t *wgraph[2] = {nullptr, nullptr};
     uint32_t *wa[2] = {nullptr, nullptr};
     uint32_t *wb[2] = {nullptr, nullptr};
-    uint32_t *wflag = nullptr;  // 2 * cap: one array per level parity
+    uint32_t *wflag[2] = {nullptr, nullptr};  // one array per level parity
     uint32_t *wlive = nullptr;
     uint64_t *top = nullptr;    // one graph: its top-of-tree heads, gathered per launch for the locate cache
     // sort state
@@ -174,7 +177,6 @@ struct BatchBuffers {
     uint64_t *qinfo = nullptr;         // bucket sort: offset within the scan chunk | count << 32
     uint64_t q_cap = 0;                // buckets
     uint64_t *qrec = nullptr;          // bucket sort: 16-byte records (two words per key)
-    uint64_t qrec_cap = 0;             // keys
     uint32_t *qbound = nullptr;        // bucket sort: first position of every item
     uint64_t qbound_cap = 0;           // items
     // per-graph tables, one upload per launch from pinned memory:
@@ -209,6 +211,8 @@ struct BatchBuffers {
     // persistent-kernel scratch
     uint32_t *cta_cnt = nullptr;       // 8 * grid: four count arrays, two window-range arrays
 };
+// two batch buffers, two window lists, leaf, insertions, their leaves and graphs
+constexpr uint64_t SLAB_BYTES_PER_KEY = 2 * (8 + 1) + 2 * 16 + 4 + (8 + 1) + 2 * 4;
 constexpr uint32_t BFS_MAPS = 4;  // node bitmaps of a single-source BFS
 constexpr size_t STAT_GS_OFFSET = 128;
 static_assert(sizeof(DeviceStatus) <= STAT_GS_OFFSET, "status slot layout");

@@ -37,6 +37,7 @@
 #include <algorithm>
 #include <cmath>
 #include <numeric>
+#include <type_traits>
 
 namespace gpma {
 
@@ -2807,30 +2808,13 @@ gpma_status ensure_scratch(gpma_graph *g, uint32_t slots) {
 }
 
 void free_buffers(BatchBuffers &b) {
-    for (int i = 0; i < 2; ++i) {
-        dev_free(b.bkeys[i]);
-        dev_free(b.bvals[i]);
-        dev_free(b.ikeys[i]);
-        dev_free(b.ivals[i]);
-        dev_free(b.wnode[i]);
-        dev_free(b.wgraph[i]);
-        dev_free(b.wa[i]);
-        dev_free(b.wb[i]);
-    }
-    dev_free(b.leaf);
-    dev_free(b.rkeys);
-    dev_free(b.rvals);
-    dev_free(b.ileaf);
-    dev_free(b.igraph);
-    dev_free(b.wflag);
-    dev_free(b.wlive);
+    dev_free(b.slab);
     dev_free(b.sort_tiles);
     dev_free(b.top);
     dev_free(b.sort_status);
     dev_free(b.sort_hist);
     dev_free(b.qcnt);
     dev_free(b.qinfo);
-    dev_free(b.qrec);
     dev_free(b.qbound);
     dev_free(b.d_tab);
     dev_free(b.d_stat);
@@ -2852,7 +2836,6 @@ void free_buffers(BatchBuffers &b) {
     b.chunk_cap = 0;
     b.sort_status_cap = 0;
     b.q_cap = 0;
-    b.qrec_cap = 0;
     b.qbound_cap = 0;
     b.tab_shadow_valid = false;
 }
@@ -2864,57 +2847,54 @@ gpma_status ensure_buffers(BatchBuffers &b, uint64_t n, uint32_t graphs) {
     }
     if (!b.top)
         GPMA_TRY(dev_alloc(&b.top, LOCATE_CACHE));
-    if (n > b.cap || !b.bkeys[0]) {
-        // a multiple of 16 entries: every buffer is a whole number of 16-byte
-        // units, so a bulk copy of a range widened to 16-byte bounds stays inside
-        uint64_t cap = (std::max<uint64_t>(n, 1024) + 15) & ~uint64_t(15);
-        for (int i = 0; i < 2; ++i) {
-            dev_free(b.bkeys[i]);
-            dev_free(b.bvals[i]);
-            dev_free(b.ikeys[i]);
-            dev_free(b.ivals[i]);
-            dev_free(b.wnode[i]);
-            dev_free(b.wgraph[i]);
-            dev_free(b.wa[i]);
-            dev_free(b.wb[i]);
-        }
-        dev_free(b.leaf);
-        dev_free(b.rkeys);
-        dev_free(b.rvals);
-        dev_free(b.ileaf);
-        dev_free(b.igraph);
-        dev_free(b.wflag);
-        dev_free(b.wlive);
+    if (n > b.cap || !b.slab) {
+        // a multiple of 256 entries: every array starts on a 256-byte line and is
+        // a whole number of 16-byte units, so a bulk copy of a range widened to
+        // 16-byte bounds stays inside
+        const uint64_t cap = (std::max<uint64_t>(n, 1024) + 255) & ~uint64_t(255);
+        dev_free(b.slab);
         b.cap = 0;
+        GPMA_TRY(dev_alloc(&b.slab, cap * SLAB_BYTES_PER_KEY));
+        unsigned char *at = b.slab;
+        auto take = [&](auto **p) {
+            *p = reinterpret_cast<std::remove_reference_t<decltype(*p)>>(at);
+            at += cap * sizeof(**p);
+        };
         for (int i = 0; i < 2; ++i) {
-            GPMA_TRY(dev_alloc(&b.bkeys[i], cap));
-            GPMA_TRY(dev_alloc(&b.bvals[i], cap));
-            GPMA_TRY(dev_alloc(&b.ikeys[i], cap));
-            GPMA_TRY(dev_alloc(&b.ivals[i], cap));
-            GPMA_TRY(dev_alloc(&b.wnode[i], cap));
-            GPMA_TRY(dev_alloc(&b.wgraph[i], cap));
-            GPMA_TRY(dev_alloc(&b.wa[i], cap));
-            GPMA_TRY(dev_alloc(&b.wb[i], cap));
+            take(&b.bkeys[i]);
+            take(&b.bvals[i]);
+            take(&b.wnode[i]);
+            take(&b.wgraph[i]);
+            take(&b.wa[i]);
+            take(&b.wb[i]);
         }
-        GPMA_TRY(dev_alloc(&b.leaf, cap));
-        GPMA_TRY(dev_alloc(&b.rkeys, cap));
-        GPMA_TRY(dev_alloc(&b.rvals, cap));
-        GPMA_TRY(dev_alloc(&b.ileaf, cap));
-        GPMA_TRY(dev_alloc(&b.igraph, cap));
-        GPMA_TRY(dev_alloc(&b.wflag, 2 * cap));  // one array per level parity
-        GPMA_TRY(dev_alloc(&b.wlive, cap));
+        take(&b.leaf);
+        take(&b.ikeys[0]);
+        take(&b.ivals[0]);
+        take(&b.ileaf);
+        take(&b.igraph);
+        // arrays whose life begins after another's has ended, always with a
+        // grid barrier between: the sorted batch is read last when the
+        // insertions are gathered, before the level loop; the sort's 16-byte
+        // records are read before the first windows are written; ranks, leaves
+        // and their graphs are read last when the insertions are grouped
+        b.ikeys[1] = b.bkeys[1];
+        b.ivals[1] = b.bvals[1];
+        b.rkeys = b.bkeys[0];
+        b.rvals = b.bvals[0];
+        b.qrec = reinterpret_cast<uint64_t *>(b.wnode[0]);
+        b.wflag[0] = b.ileaf;
+        b.wflag[1] = b.igraph;
+        b.wlive = b.leaf;
         b.cap = cap;
         // the bucket sort's buffers grow with the batch buffers, so a served
         // round does not meet a first allocation later (a launch of n keys over
         // k graphs uses at most n/16 + k buckets and n/1024 + k items)
         const uint64_t gq = std::max<uint32_t>(graphs, std::max<uint32_t>(b.gcap, 1));
-        dev_free(b.qrec);
         dev_free(b.qcnt);
         dev_free(b.qinfo);
         dev_free(b.qbound);
-        b.qrec_cap = b.q_cap = b.qbound_cap = 0;
-        GPMA_TRY(dev_alloc(&b.qrec, 2 * cap));
-        b.qrec_cap = cap;
+        b.q_cap = b.qbound_cap = 0;
         GPMA_TRY(dev_alloc(&b.qcnt, cap / 16 + 2 * gq + 64));
         GPMA_TRY(dev_alloc(&b.qinfo, cap / 16 + 2 * gq + 64));
         b.q_cap = cap / 16 + 2 * gq + 64;
@@ -3033,12 +3013,6 @@ gpma_status update_plan(gpma_graph *const *graphs, const uint64_t *off, uint32_t
         buf.q_cap = nq;
         buf.dirty = true;
     }
-    if (use_buckets && n > buf.qrec_cap) {
-        dev_free(buf.qrec);
-        buf.qrec_cap = 0;
-        GPMA_TRY(dev_alloc(&buf.qrec, 2 * buf.cap));  // 16 bytes per key
-        buf.qrec_cap = buf.cap;
-    }
     if (use_buckets && h_qtoff[k] > buf.qbound_cap) {
         dev_free(buf.qbound);
         buf.qbound_cap = 0;
@@ -3113,8 +3087,8 @@ gpma_status update_plan(gpma_graph *const *graphs, const uint64_t *off, uint32_t
     A.rvals = buf.rvals;
     A.ileaf = buf.ileaf;
     A.igraph = buf.igraph;
-    A.wflag[0] = buf.wflag;
-    A.wflag[1] = buf.wflag + buf.cap;
+    A.wflag[0] = buf.wflag[0];
+    A.wflag[1] = buf.wflag[1];
     A.wlive = buf.wlive;
     A.chunk_cnt = buf.chunk_cnt;
     A.cta_cnt = buf.cta_cnt;
