@@ -78,7 +78,7 @@ def build(verbose: bool = False, ptxas_info: bool = False, checked: bool = False
     build_dir.mkdir(exist_ok=True)
     sort_items = os.environ.get("GPMA_SORT_ITEMS", "8")
     lane_slots = os.environ.get("GPMA_BFS_LANE_SLOTS", "4")
-    lookback = os.environ.get("GPMA_SORT_LOOKBACK", "8")
+    lookback = os.environ.get("GPMA_SORT_LOOKBACK", "4")
     defines = [f"-DGPMA_SORT_ITEMS={sort_items}", f"-DGPMA_BFS_LANE_SLOTS={lane_slots}",
                f"-DGPMA_SORT_LOOKBACK={lookback}", f"-DGPMA_BOUNDS_CHECK={int(checked)}"]
     stamp = build_dir / "options.txt"

@@ -515,7 +515,7 @@ struct Tuning {
     uint32_t bfs_blocks_per_sm = 8;
     uint32_t ms_dense_div = 8;
     uint32_t ms_blocks_per_sm = 8;
-    uint32_t update_blocks_per_sm = 0;  // 0: chosen per launch (3-CTA build from 1M keys)
+    uint32_t update_blocks_per_sm = 0;  // 0: as many as fit
     uint32_t update_sort = 0;           // 0: bucket sort (digit passes for crowded buckets), 1: digit passes
 };
 extern Tuning g_tuning;

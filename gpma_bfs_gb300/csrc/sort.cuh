@@ -26,18 +26,26 @@
 
 namespace gpma {
 
-// Keys per thread of a tile (build option; a tile of 2048 keys by default).
+// Keys per thread of a tile (build option; a tile of 2048 keys by default), and
+// of a tile of a large launch (as many as fit in shared memory): a tile costs a
+// look-back and about twenty CTA barriers, whatever it holds (15.3M keys, six
+// passes: 1.40 ms with the small tiles, 0.94 with the large). Launches that would not give every CTA a large tile, or
+// whose graphs would leave them part empty, keep the small ones.
 #ifndef GPMA_SORT_ITEMS
 #define GPMA_SORT_ITEMS 8
 #endif
 constexpr int SORT_ITEMS = GPMA_SORT_ITEMS;
-// Predecessor tiles a look-back step reads at once (build option).
+constexpr int SORT_ITEMS_LARGE = SORT_ITEMS > 18 ? SORT_ITEMS : 18;
+// Predecessor tiles a look-back step reads at once (build option; 15.3M keys:
+// 0.94 ms with 2 to 4, 0.96 with 8, 1.13 with 16).
 #ifndef GPMA_SORT_LOOKBACK
-#define GPMA_SORT_LOOKBACK 8
+#define GPMA_SORT_LOOKBACK 4
 #endif
 constexpr uint32_t SORT_LOOKBACK = GPMA_SORT_LOOKBACK;
 constexpr uint32_t SORT_TILE = BLOCK * SORT_ITEMS;
-static_assert(SORT_TILE * 9 + (BLOCK / 32 + 2) * 256 * 4 <= UPDATE_SMEM, "sort tile exceeds the update kernel's smem");
+constexpr uint32_t SORT_TILE_LARGE = BLOCK * SORT_ITEMS_LARGE;
+static_assert(SORT_TILE_LARGE * 9 + (BLOCK / 32 + 2) * 256 * 4 <= UPDATE_SMEM,
+              "sort tile exceeds the update kernel's smem");
 constexpr uint32_t SORT_FLAG_AGG = 1u << 30;
 constexpr uint32_t SORT_FLAG_INC = 2u << 30;
 constexpr uint32_t SORT_VALUE_MASK = (1u << 30) - 1;
@@ -97,11 +105,15 @@ __device__ __forceinline__ uint32_t sort_trivial_mask(const uint32_t *total, uin
     return mask;
 }
 
-// One tile of digit pass `pass`: keys in_k/in_v -> out_k/out_v.
+// One tile (ITEMS keys per thread) of digit pass `pass`: keys in_k/in_v ->
+// out_k/out_v. A digit's peers in the warp come from eight ballots (six passes
+// over 15.3M keys, large tiles: 0.96 ms, 1.19 with a match instruction).
+template <int ITEMS>
 __device__ void sort_tile(int pass, uint32_t tile, const uint64_t *__restrict__ in_k, const uint8_t *__restrict__ in_v,
                           uint64_t *__restrict__ out_k, uint8_t *__restrict__ out_v, const uint32_t *boff,
                           const uint32_t *toff, uint32_t G, const uint32_t *hist, uint32_t *status_all,
                           DeviceStatus *st, unsigned char *smem, uint32_t *tmp) {
+    constexpr uint32_t TILE = BLOCK * ITEMS;
     const int shift = 8 * pass;
     const uint32_t tiles = toff[G];
     const uint32_t g = G == 1 ? 0 : segment_of(toff, G, tile);
@@ -109,35 +121,40 @@ __device__ void sort_tile(int pass, uint32_t tile, const uint64_t *__restrict__ 
     const uint32_t seg_lo = boff[g], seg_hi = boff[g + 1];
     uint32_t *status = status_all + (size_t)pass * tiles * 256;
     uint64_t *s_keys = reinterpret_cast<uint64_t *>(smem);
-    uint8_t *s_vals = smem + SORT_TILE * 8;
-    uint32_t *whist = reinterpret_cast<uint32_t *>(smem + SORT_TILE * 9);  // [BLOCK/32][256]
+    uint8_t *s_vals = smem + TILE * 8;
+    uint32_t *whist = reinterpret_cast<uint32_t *>(smem + TILE * 9);  // [BLOCK/32][256]
     uint32_t *s_start = whist + (BLOCK / 32) * 256;
     uint32_t *s_global = s_start + 256;
 
     for (int i = threadIdx.x; i < (BLOCK / 32) * 256; i += BLOCK)
         whist[i] = 0;
     __syncthreads();
-    const uint32_t tile_lo = seg_lo + (tile - first_tile) * SORT_TILE;
+    const uint32_t tile_lo = seg_lo + (tile - first_tile) * TILE;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const uint32_t warp_lo = tile_lo + warp * 32 * SORT_ITEMS;
+    const uint32_t warp_lo = tile_lo + warp * 32 * ITEMS;
     uint32_t *wh = whist + warp * 256;
 
-    uint64_t k[SORT_ITEMS];
-    uint8_t v[SORT_ITEMS];
-    uint32_t rank[SORT_ITEMS];
+    uint64_t k[ITEMS];
+    uint8_t v[ITEMS];
+    uint32_t rank[ITEMS];
 #pragma unroll
-    for (int j = 0; j < SORT_ITEMS; ++j) {
+    for (int j = 0; j < ITEMS; ++j) {
         uint32_t idx = warp_lo + j * 32 + lane;
         bool ok = idx < seg_hi;
         k[j] = ok ? in_k[idx] : 0;
         v[j] = ok ? in_v[idx] : 0;
     }
 #pragma unroll
-    for (int j = 0; j < SORT_ITEMS; ++j) {
+    for (int j = 0; j < ITEMS; ++j) {
         uint32_t idx = warp_lo + j * 32 + lane;
         bool ok = idx < seg_hi;
         uint32_t d = ok ? (uint32_t)((k[j] >> shift) & 255) : 256u + lane;
-        uint32_t peers = __match_any_sync(0xFFFFFFFFu, d);
+        uint32_t peers = __ballot_sync(0xFFFFFFFFu, ok);
+#pragma unroll
+        for (int b = 0; b < 8; ++b) {
+            const uint32_t set = __ballot_sync(0xFFFFFFFFu, (d >> b) & 1u);
+            peers &= (d >> b) & 1u ? set : ~set;
+        }
         uint32_t prior = ok ? wh[d] : 0;
         __syncwarp();
         if (ok) {
@@ -216,7 +233,7 @@ __device__ void sort_tile(int pass, uint32_t tile, const uint64_t *__restrict__ 
 
     // Stage the tile in digit order, then write each digit run contiguously.
 #pragma unroll
-    for (int j = 0; j < SORT_ITEMS; ++j) {
+    for (int j = 0; j < ITEMS; ++j) {
         uint32_t idx = warp_lo + j * 32 + lane;
         if (idx < seg_hi) {
             uint32_t dd = (uint32_t)((k[j] >> shift) & 255);
@@ -226,7 +243,7 @@ __device__ void sort_tile(int pass, uint32_t tile, const uint64_t *__restrict__ 
         }
     }
     __syncthreads();
-    const uint32_t tile_n = min(SORT_TILE, seg_hi - tile_lo);
+    const uint32_t tile_n = min(TILE, seg_hi - tile_lo);
     for (uint32_t i = threadIdx.x; i < tile_n; i += BLOCK) {
         uint64_t kk = s_keys[i];
         uint32_t dd = (uint32_t)((kk >> shift) & 255);

@@ -82,6 +82,7 @@ struct UpdateArgs {
     uint32_t seg_graph[5];  // first graph whose segments have 2 << i slots or more
     const uint32_t *boff;   // batch offsets, G + 1
     const uint32_t *toff;   // sort tile offsets, G + 1
+    uint32_t large_tiles;   // tiles of SORT_TILE_LARGE keys, else SORT_TILE
     uint32_t n;
     const uint64_t *in_k;   // the batch as submitted (bk[0] or the caller's device buffer; only read)
     const uint8_t *in_v;
@@ -164,46 +165,6 @@ __device__ __forceinline__ uint32_t leaf_find(const GraphDesc &D, uint32_t leaf,
     return hit;
 }
 
-// The same for each lane's leaf and key, by all lanes of the warp together (a
-// lane without work passes leaf SIZE_NONE): seg/2 lanes read a leaf, a slot pair
-// each, so that a load instruction touches 64/seg leaves as whole runs of slots
-// instead of 32 leaves 16 bytes at a time. SEG_PAIRS is seg/2 (1, 2, 4, 8, 16).
-// Its shuffles pay where many keys per thread keep the load path busy: 10.5M
-// keys, R-MAT 21, locate 627 -> 519 us; the social slide, four keys per thread,
-// 20 us with a leaf per lane, 33 this way, so the builds for smaller launches
-// scan a leaf per lane.
-template <uint32_t SEG_PAIRS>
-__device__ __forceinline__ uint32_t warp_leaf_find(const uint64_t *keys, uint32_t leaf, uint64_t key) {
-    const uint32_t lane = threadIdx.x & 31;
-    const uint32_t part = lane % SEG_PAIRS, grp = lane / SEG_PAIRS;
-    constexpr uint32_t PER = 32 / SEG_PAIRS;  // leaves per load
-    ulonglong2 q[SEG_PAIRS];
-#pragma unroll
-    for (uint32_t r = 0; r < SEG_PAIRS; ++r) {
-        const uint32_t lf = __shfl_sync(0xFFFFFFFFu, leaf, r * PER + grp);
-        q[r] = make_ulonglong2(0, 0);
-        if (lf != SIZE_NONE)
-            q[r] = *reinterpret_cast<const ulonglong2 *>(keys + lf + 2 * part);
-    }
-    uint32_t hit = SIZE_NONE;
-#pragma unroll
-    for (uint32_t r = 0; r < SEG_PAIRS; ++r) {
-        const uint64_t k = __shfl_sync(0xFFFFFFFFu, key, r * PER + grp);
-        const uint32_t first = __ballot_sync(0xFFFFFFFFu, q[r].x == k), second = __ballot_sync(0xFFFFFFFFu, q[r].y == k);
-        // this lane's own leaf was read in round lane / PER by group lane % PER
-        if (lane / PER == r) {
-            const uint32_t sh = (lane % PER) * SEG_PAIRS;
-            const uint32_t mask = SEG_PAIRS == 32 ? 0xFFFFFFFFu : (1u << SEG_PAIRS) - 1;
-            const uint32_t a = (first >> sh) & mask, b = (second >> sh) & mask;
-            if (a | b) {
-                const uint32_t p = __ffs(a | b) - 1;
-                hit = 2 * p + (((a >> p) & 1u) ? 0u : 1u);
-            }
-        }
-    }
-    return leaf == SIZE_NONE ? SIZE_NONE : hit;
-}
-
 // Locates LOC_ILP updates per thread together: at each level of the descent
 // every key's probe is issued before any comparison, so a thread keeps
 // LOC_ILP dependent chains in flight instead of one.
@@ -211,19 +172,9 @@ constexpr int LOC_ILP = 4;
 // Consecutive items per thread in the grouping passes.
 constexpr uint32_t GROUP_ITEMS = 4;
 
-template <uint32_t SEG_PAIRS>
-__device__ __forceinline__ void find_all(const uint64_t *keys, const uint32_t (&leaf)[LOC_ILP],
-                                         const uint64_t (&key)[LOC_ILP], uint32_t (&hit)[LOC_ILP]) {
-#pragma unroll
-    for (int j = 0; j < LOC_ILP; ++j)
-        hit[j] = warp_leaf_find<SEG_PAIRS>(keys, leaf[j], key[j]);
-}
-
 // Keys i0 + j * stride (j < LOC_ILP) below `end`, all of graph g; returns how
 // many of them are insertions (leaf set). fk: the heads at every 2^log2stride
-// slots, in shared memory. Whole warps only (a lane may be past `end`). COOP:
-// warps scan their leaves together.
-template <bool COOP>
+// slots, in shared memory.
 __device__ __forceinline__ uint32_t locate_keys(const UpdateArgs &A, uint32_t g, const uint64_t *bk, const uint8_t *bv,
                                                 uint32_t i0, uint32_t stride, uint32_t end, const uint64_t *fk,
                                                 uint32_t log2stride) {
@@ -269,19 +220,9 @@ __device__ __forceinline__ uint32_t locate_keys(const UpdateArgs &A, uint32_t g,
     // every leaf scan before any store: a value store (a byte) may alias the
     // next scan's loads, which would otherwise wait for it
     uint32_t hit[LOC_ILP];
-    if constexpr (COOP) {
-        switch (seg) {
-        case 2: find_all<1>(D.keys, prefix, key, hit); break;
-        case 4: find_all<2>(D.keys, prefix, key, hit); break;
-        case 8: find_all<4>(D.keys, prefix, key, hit); break;
-        case 16: find_all<8>(D.keys, prefix, key, hit); break;
-        default: find_all<16>(D.keys, prefix, key, hit); break;
-        }
-    } else {
 #pragma unroll
-        for (int j = 0; j < LOC_ILP; ++j)
-            hit[j] = prefix[j] != SIZE_NONE ? leaf_find(D, prefix[j], key[j]) : SIZE_NONE;
-    }
+    for (int j = 0; j < LOC_ILP; ++j)
+        hit[j] = prefix[j] != SIZE_NONE ? leaf_find(D, prefix[j], key[j]) : SIZE_NONE;
     uint32_t inserts = 0;
 #pragma unroll
     for (int j = 0; j < LOC_ILP; ++j) {
@@ -1189,15 +1130,13 @@ __device__ __noinline__ void copy_kept(const uint32_t *l_src, const uint32_t *l_
     }
 }
 
-// Two register budgets of the same kernel: MINB resident CTAs per SM. Two
-// (128 registers, almost no spills) suits single large graphs, whose phases
-// are short and barrier-bound; three (80 registers, some spills to local
-// memory) suits many graphs per launch, whose phases are longer and gain from
-// the extra warps. gpma_tuning.update_blocks_per_sm selects one.
+// Two resident CTAs per SM (128 registers, almost no spills): a build for three
+// (80 registers) has more warps, but its spilled locate is the slower one (10.5M
+// keys, R-MAT 21: locate 519 us, the call 1852; with two 320 and 1700).
 // SMALL: the build for small batches of one graph (small_front); apart, so that
-// it costs the others no registers.
-template <int MINB, bool SMALL>
-__global__ void __launch_bounds__(BLOCK, MINB) update_kernel(UpdateArgs A) {
+// it costs the other no registers.
+template <bool SMALL>
+__global__ void __launch_bounds__(BLOCK, 2) update_kernel(UpdateArgs A) {
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ uint32_t tmp[BLOCK / 32 + 1];
     if (A.abort && ld_volatile(A.abort))
@@ -1281,9 +1220,14 @@ __global__ void __launch_bounds__(BLOCK, MINB) update_kernel(UpdateArgs A) {
                     // CTA b takes tiles b, b + G, b + 2G, ... in order: every look-back
                     // waits on lower tiles only, and the lowest unfinished tile never
                     // waits on anything unfinished, so the pass always progresses
-                    for (uint32_t tile = blockIdx.x; tile < tiles; tile += gridDim.x)
-                        sort_tile(p, tile, ink, inv, outk, outv, A.boff, A.toff, A.G, A.sort_hist, A.sort_status, st, smem,
-                                  tmp);
+                    for (uint32_t tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+                        if (A.large_tiles)
+                            sort_tile<SORT_ITEMS_LARGE>(p, tile, ink, inv, outk, outv, A.boff, A.toff, A.G, A.sort_hist,
+                                                        A.sort_status, st, smem, tmp);
+                        else
+                            sort_tile<SORT_ITEMS>(p, tile, ink, inv, outk, outv, A.boff, A.toff, A.G, A.sort_hist,
+                                                  A.sort_status, st, smem, tmp);
+                    }
                     sel ^= 1u;
                     if (!grid_barrier(A.bar, &st->err))
                         return;
@@ -1331,7 +1275,7 @@ __global__ void __launch_bounds__(BLOCK, MINB) update_kernel(UpdateArgs A) {
                 uint32_t lo, hi, mine = 0;
                 cta_range(A.n, lo, hi);
                 for (uint32_t r0 = lo; r0 < hi; r0 += LOC_ILP * BLOCK)
-                    mine += locate_keys<MINB == 3>(A, 0, bk, bv, r0 + threadIdx.x, BLOCK, hi, fk, log2stride);
+                    mine += locate_keys(A, 0, bk, bv, r0 + threadIdx.x, BLOCK, hi, fk, log2stride);
                 const uint32_t t = block_sum(mine, tmp);
                 if (threadIdx.x == 0)
                     CNT(scan_id)[blockIdx.x] = t;
@@ -1366,7 +1310,7 @@ __global__ void __launch_bounds__(BLOCK, MINB) update_kernel(UpdateArgs A) {
                     }
                     __syncthreads();
                     for (uint32_t r0 = pos; r0 < end; r0 += LOC_ILP * BLOCK)
-                        locate_keys<MINB == 3>(A, g, bk, bv, r0 + threadIdx.x, BLOCK, end, f, l2s);
+                        locate_keys(A, g, bk, bv, r0 + threadIdx.x, BLOCK, end, f, l2s);
                     __syncthreads();  // the copy is replaced for the next graph
                     pos = end;
                 }
@@ -2678,25 +2622,17 @@ GraphDesc describe(const gpma_graph *g) {
 }
 
 // Builds of the update kernel.
-enum UpdateVariant { UPDATE_NARROW, UPDATE_WIDE, UPDATE_SMALL, UPDATE_VARIANTS };
+enum UpdateVariant { UPDATE_LARGE, UPDATE_SMALL, UPDATE_VARIANTS };
 int g_update_fit[64][UPDATE_VARIANTS] = {};  // resident CTAs per SM of each, per device
 
 // The build for a launch of n keys over k graphs: small batches of one graph
-// have their own (unless the digit passes are asked for); else the tuned CTAs
-// per SM (3 or more selects the 3-CTA build), or when left to the library (0)
-// the 3-CTA build for launches of at least AUTO_WIDE_KEYS keys.
-constexpr uint64_t AUTO_WIDE_KEYS = 1u << 20;
+// have their own (unless the digit passes are asked for).
 UpdateVariant update_variant(uint64_t n, uint32_t k) {
-    if (k == 1 && n <= SMALL_KEYS && g_tuning.update_sort == 0)
-        return UPDATE_SMALL;
-    const uint32_t t = g_tuning.update_blocks_per_sm;
-    return t >= 3 || (t == 0 && n >= AUTO_WIDE_KEYS) ? UPDATE_WIDE : UPDATE_NARROW;
+    return k == 1 && n <= SMALL_KEYS && g_tuning.update_sort == 0 ? UPDATE_SMALL : UPDATE_LARGE;
 }
 
 const void *update_kernel_ptr(UpdateVariant v) {
-    return v == UPDATE_SMALL  ? (const void *)update_kernel<2, true>
-           : v == UPDATE_WIDE ? (const void *)update_kernel<3, false>
-                              : (const void *)update_kernel<2, false>;
+    return v == UPDATE_SMALL ? (const void *)update_kernel<true> : (const void *)update_kernel<false>;
 }
 
 }  // namespace
@@ -2974,12 +2910,14 @@ gpma_status update_plan(gpma_graph *const *graphs, const uint64_t *off, uint32_t
             return GPMA_ERR_INVALID;
         }
     }
+    const bool large_tiles = n >= (uint64_t)SORT_TILE_LARGE * std::max<uint32_t>(grid, k);
+    const uint32_t tile = large_tiles ? SORT_TILE_LARGE : SORT_TILE;
     h_toff[0] = 0;
     for (uint32_t i = 0; i <= k; ++i) {
         h_boff[i] = (uint32_t)off[i];
         if (i > 0) {
             const uint64_t ni = off[i] - off[i - 1];
-            h_toff[i] = h_toff[i - 1] + (uint32_t)((ni + SORT_TILE - 1) / SORT_TILE);
+            h_toff[i] = h_toff[i - 1] + (uint32_t)((ni + tile - 1) / tile);
         }
     }
     // bucket sort: per graph, 2^qlog equal slot ranges (about BSORT_AVG keys
@@ -3063,6 +3001,7 @@ gpma_status update_plan(gpma_graph *const *graphs, const uint64_t *off, uint32_t
             ++A.seg_graph[i];
     A.boff = buf.boff;
     A.toff = buf.toff;
+    A.large_tiles = large_tiles;
     A.n = (uint32_t)n;
     A.in_k = in_k ? in_k : buf.bkeys[0];
     A.in_v = in_v ? in_v : buf.bvals[0];
