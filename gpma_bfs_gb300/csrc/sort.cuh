@@ -18,8 +18,8 @@
 // waits only on tiles that are already being processed.
 //
 // The default is a bucket sort with no look-back and four grid barriers
-// (bsort_* below); the digit passes above remain for batches that crowd one
-// bucket (a burst into a few rows, a bulk load with hub rows).
+// (bsort_* below); the digit passes above are for loads and very large batches,
+// and for batches that crowd one bucket (a burst into a few rows).
 #pragma once
 
 #include "gpma_internal.cuh"
@@ -176,15 +176,14 @@ __device__ void sort_tile(int pass, uint32_t tile, const uint64_t *__restrict__ 
     }
     const uint32_t local = run;
     uint32_t total;
+    // Decoupled look-back for digit d over this graph's earlier tiles. The count
+    // is out before anything else is worked out, so that later tiles seldom
+    // find it missing (15.3M keys: 0.94 -> 0.91 ms).
+    uint32_t prefix = 0;
+    atomicExch(&status[(size_t)tile * 256 + d], (tile == first_tile ? SORT_FLAG_INC : SORT_FLAG_AGG) | local);
     s_start[d] = block_excl_scan(local, &total, tmp);
     const uint32_t base = seg_lo + block_excl_scan(hist[(size_t)g * 2048 + pass * 256 + d], &total, tmp);
-
-    // Decoupled look-back for digit d over this graph's earlier tiles.
-    uint32_t prefix = 0;
-    if (tile == first_tile) {
-        atomicExch(&status[(size_t)tile * 256 + d], SORT_FLAG_INC | local);
-    } else {
-        atomicExch(&status[(size_t)tile * 256 + d], SORT_FLAG_AGG | local);
+    if (tile != first_tile) {
         // windows of LOOKBACK predecessors are read at once and summed
         // nearest first, up to the first inclusive value or unpublished word
         int64_t t = (int64_t)tile - 1;
