@@ -2621,6 +2621,9 @@ GraphDesc describe(const gpma_graph *g) {
     return d;
 }
 
+// One graph's batches of this many keys are sorted by digit passes.
+constexpr uint64_t DIGIT_KEYS = 1u << 22;
+
 // Builds of the update kernel.
 enum UpdateVariant { UPDATE_LARGE, UPDATE_SMALL, UPDATE_VARIANTS };
 int g_update_fit[64][UPDATE_VARIANTS] = {};  // resident CTAs per SM of each, per device
@@ -2932,7 +2935,12 @@ gpma_status update_plan(gpma_graph *const *graphs, const uint64_t *off, uint32_t
     // serialise on one counter before the digit passes run after all (15.3M
     // edges into an array of guards: 0.55 of 1.70 ms of sort). Without hubs the
     // passes take about as long as the buckets would.
-    const bool buckets = g_tuning.update_sort == 0 && (uint32_t)grid <= BSORT_MAX_GRID && n <= slots;
+    // So do they from about DIGIT_KEYS keys, whose records no longer stay in L2,
+    // where rows and columns have at most three digits each (one graph, R-MAT 21,
+    // buckets against six passes: 2M keys 133 and 166 us, 4M 267 and 269, 7M 479
+    // and 437, 10.5M 716 and 631). Many graphs: not measured, buckets.
+    const bool digits = n > slots || (k == 1 && n >= DIGIT_KEYS && graphs[0]->row_num <= 1u << 24);
+    const bool buckets = g_tuning.update_sort == 0 && (uint32_t)grid <= BSORT_MAX_GRID && !digits;
     uint64_t nq = 0;
     h_qoff[0] = h_qtoff[0] = 0;
     for (uint32_t i = 0; i < k; ++i) {

@@ -75,3 +75,20 @@ def test_many_graphs(one_cta_per_sm, parts, more):
     b.close()
     for g in gs:
         g.close()
+
+
+@pytest.mark.parametrize("more", [-1, 0])
+def test_large_batches_of_one_graph(built_lib, more):
+    """The batch size where digit passes replace the buckets."""
+    import gpma_bfs_gb300 as G
+    rng = np.random.default_rng(9)
+    rows, n = 300000, (1 << 22) + more
+    g, orc = G.GPMA(rows), OracleGPMA(rows, threads=8)
+    k = np.unique(_keys(rng, rows, 5_000_000))
+    for step, (keys, value) in enumerate(((k, 1), (rng.permutation(k)[:n], 2), (rng.permutation(k)[:n], 0),
+                                          (rng.permutation(np.unique(_keys(rng, rows, n + 9000)))[:n], 3))):
+        v = np.full(len(keys), value, np.uint8)
+        G.update_gpma(g, keys, v)
+        orc.update(keys, v)
+        _same(g, orc, f"step {step}")
+    g.close()
