@@ -8,14 +8,14 @@
 //   1. one pass histograms all eight 8-bit digits of every graph's batch at
 //      once (and flags keys whose column is the reserved 0xFFFFFFFF);
 //   2. digits constant over every batch are skipped;
-//   3. per remaining digit, CTAs take tiles in the order of a global counter
-//      (graph g owns tiles [toff[g], toff[g+1])), rank the tile's keys with
-//      warp match/ballot (stable: input order), publish per-digit counts and
-//      resolve their offsets by decoupled look-back over the earlier tiles of
-//      the same graph (bounded waits), then write through shared memory so
-//      each digit run leaves as a contiguous burst.
-// Tiles are claimed in counter order by co-resident CTAs, so every look-back
-// waits only on tiles that are already being processed.
+//   3. per remaining digit, CTAs take tiles in turn (graph g owns tiles
+//      [toff[g], toff[g+1])), rank the tile's keys with warp ballots (stable:
+//      input order), publish per-digit counts and resolve their offsets by
+//      decoupled look-back over the earlier tiles of the same graph (bounded
+//      waits), then write through shared memory so each digit run leaves as a
+//      contiguous burst.
+// All CTAs are resident and each takes its tiles in order, so every look-back
+// waits only on tiles that are done or being processed.
 //
 // The default is a bucket sort with no look-back and four grid barriers
 // (bsort_* below); the digit passes above are for loads and very large batches,
