@@ -16,7 +16,8 @@
 //   the scan takes each warp's words of seen: what is not in done is the
 //     frontier; its nodes get their level (a warp's stores are one line) and
 //     the rows of a word's up to 32 nodes, taken as one concatenated slot
-//     range, are queued in pieces of ITEM_SLOTS slots;
+//     range, are queued in pieces of ITEM_SLOTS slots (LARGE_ITEM_SLOTS in
+//     large arrays);
 //   the walk, after a barrier, spreads the pieces over every warp (warp-level
 //     load balancing, LANE_SLOTS slots per lane per step, all loads issued
 //     before any claim). A target is claimed with one atomicOr on seen (a plain
@@ -73,9 +74,18 @@ constexpr uint32_t STEP_SLOTS = 32 * LANE_SLOTS;
 // the warp that owns the word (its long rows apart), warps spent 40 % of their
 // time waiting at the level's barrier. Social graph, kernel: 344 us with items
 // of one step, 360 with two (a warp reads its next item's rows one item ahead).
+// Arrays of LARGE_SLOTS slots and more have work for every warp at four steps an
+// item, and each item costs the offsets of its word's 32 rows again (R-MAT,
+// edge factor 32, items of 1 / 2 / 4 / 8 steps: scale 21, 2^27 slots, 511 / 481 /
+// 481 / 500 us; scale 24, 2^30 slots, 3651 / 3316 / 3180 / 3091; at 2^26 slots 302
+// / 287 / 287). A build of its own, so that the smaller one keeps its single step.
 constexpr uint32_t ITEM_SLOTS = STEP_SLOTS;
+constexpr uint32_t LARGE_ITEM_SLOTS = 4 * STEP_SLOTS;
+constexpr uint32_t LARGE_SLOTS = 1u << 27;
 // Items of one level at most: the last piece of every word and whole pieces.
-inline uint64_t bfs_item_need(uint32_t n, uint32_t size) { return n / 32 + 1 + size / ITEM_SLOTS; }
+inline uint64_t bfs_item_need(uint32_t n, uint32_t size) {
+    return n / 32 + 1 + size / (size >= LARGE_SLOTS ? LARGE_ITEM_SLOTS : ITEM_SLOTS);
+}
 // Items that a CTA collects in shared memory and adds to the grid's list under
 // one atomic; a warp that finds no room adds its own. (An atomic per frontier
 // word, all on one counter, serialises at 4.4 ns apiece.)
@@ -209,7 +219,7 @@ __device__ __forceinline__ void walk_word(const BfsArgs &A, const WordRows &W, u
     const uint32_t incl = warp_incl_scan(len);
     const uint32_t excl = incl - len;
     const uint32_t total = min(p1, __shfl_sync(0xFFFFFFFFu, incl, 31));
-    for (; p0 < total; p0 += STEP_SLOTS) {  // once, but for a word that no list took
+    for (; p0 < total; p0 += STEP_SLOTS) {  // once for an item of ITEM_SLOTS
         uint32_t sl[LANE_SLOTS];
 #pragma unroll
         for (uint32_t j = 0; j < LANE_SLOTS; ++j)
@@ -226,6 +236,7 @@ __device__ __forceinline__ void walk_word(const BfsArgs &A, const WordRows &W, u
 // two grid barriers per level. More slots per lane, fewer registers for more
 // warps, slots read an item ahead and runs of 2 or 4 slots per lane all
 // measured within 4 % of this or slower.
+template <uint32_t ITEM>
 __global__ void __launch_bounds__(BLOCK, 5) bfs_kernel(BfsArgs A) {
     __shared__ uint2 s_items[CTA_ITEMS];
     __shared__ uint32_t s_nit, s_end, s_at;  // items claimed and filled; place in the grid's list
@@ -299,7 +310,7 @@ __global__ void __launch_bounds__(BLOCK, 5) bfs_kernel(BfsArgs A) {
                     A.levels[(word << 5) + lane] = i + 1;
                 const uint32_t total = __reduce_add_sync(0xFFFFFFFFu, row_slots(A, bits, lane, b, e));
                 slots += lane == 0 ? total : 0u;
-                const uint32_t pieces = (total + ITEM_SLOTS - 1) / ITEM_SLOTS;
+                const uint32_t pieces = (total + ITEM - 1) / ITEM;
                 uint32_t base = 0;
                 if (lane == 0)
                     base = atomicAdd(&s_nit, pieces);
@@ -406,7 +417,7 @@ __global__ void __launch_bounds__(BLOCK, 5) bfs_kernel(BfsArgs A) {
                 WordRows N;
                 N.load(A, nxt.x, lane);
                 if (cur.y != SIZE_NONE)
-                    walk_word(A, W, cur.y * ITEM_SLOTS, (cur.y + 1) * ITEM_SLOTS, lane);
+                    walk_word(A, W, cur.y * ITEM, (cur.y + 1) * ITEM, lane);
                 W = N;
                 cur = nxt;
                 nxt = after;
@@ -415,7 +426,7 @@ __global__ void __launch_bounds__(BLOCK, 5) bfs_kernel(BfsArgs A) {
             for (uint32_t c = threadIdx.x >> 5; c < kept; c += BLOCK / 32) {
                 const uint2 own = s_items[c];
                 W.load(A, own.x, lane);
-                walk_word(A, W, own.y * ITEM_SLOTS, (own.y + 1) * ITEM_SLOTS, lane);
+                walk_word(A, W, own.y * ITEM, (own.y + 1) * ITEM, lane);
             }
             if (cta_broadcast_read(A.ctl + CTL_OVERFLOW)) {
                 for (uint32_t w = gwarp; w < words; w += nwarps) {
@@ -458,6 +469,20 @@ __global__ void __launch_bounds__(BLOCK, 5) bfs_kernel(BfsArgs A) {
     bar->count = 0;
 }
 
+const void *bfs_kernel_ptr(uint32_t size) {
+    return size >= LARGE_SLOTS ? (const void *)bfs_kernel<LARGE_ITEM_SLOTS> : (const void *)bfs_kernel<ITEM_SLOTS>;
+}
+
+// Resident CTAs per SM of either build.
+cudaError_t bfs_fit(int *per_sm) {
+    int large = 0;
+    cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(per_sm, bfs_kernel<ITEM_SLOTS>, BLOCK, 0);
+    if (e == cudaSuccess)
+        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&large, bfs_kernel<LARGE_ITEM_SLOTS>, BLOCK, 0);
+    *per_sm = std::min(*per_sm, large);
+    return e;
+}
+
 gpma_status ensure_bfs(gpma_graph *g) {
     if (g->bfs_cap >= g->row_num && g->bfs_map)
         return GPMA_OK;
@@ -474,7 +499,7 @@ gpma_status ensure_bfs(gpma_graph *g) {
     g->bfs_cap = n;
     if (g->bfs_grid == 0) {
         int per_sm = 0;
-        GPMA_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, bfs_kernel, BLOCK, 0));
+        GPMA_CUDA(bfs_fit(&per_sm));
         if (per_sm < 1) {
             set_error("BFS kernel cannot be resident (occupancy 0)");
             return GPMA_ERR_CUDA;
@@ -548,7 +573,7 @@ gpma_status bfs_plan(gpma_graph *g, uint32_t src, uint32_t *levels, BfsPlan *P, 
     A.stamps = g->profiling ? reinterpret_cast<unsigned long long *>(g->bfs_ctl + CTL_ALL) : nullptr;
     A.stall = g_test_hooks.bfs_stall;
     A.stall_limit_ns = g_test_hooks.bfs_stall ? g_test_hooks.wait_limit_ns : WAIT_LIMIT_NS;
-    P->main.set((const void *)bfs_kernel,
+    P->main.set(bfs_kernel_ptr(A.size),
                 bfs_ctas(g->geo.size, g->sms * blocks_per_sm(g->bfs_grid, g_tuning.bfs_blocks_per_sm)), 0, &A,
                 sizeof(A));
     return GPMA_OK;
@@ -639,7 +664,7 @@ gpma_status noalloc_scratch(uint32_t **out, int *grid, int sms) {
         if (e != cudaSuccess)
             return cuda_fail(e, "cudaGetSymbolAddress(g_noalloc_scratch)");
         int per_sm = 0;
-        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, bfs_kernel, BLOCK, 0);
+        e = bfs_fit(&per_sm);
         if (e != cudaSuccess)
             return cuda_fail(e, "cudaOccupancyMaxActiveBlocksPerMultiprocessor(bfs_kernel)");
         if (per_sm < 1) {
@@ -688,7 +713,7 @@ gpma_status bfs_noalloc_run(gpma_graph *g, uint32_t src, uint32_t *levels, uint6
     A.stall = g_test_hooks.bfs_stall;
     A.stall_limit_ns = g_test_hooks.bfs_stall ? g_test_hooks.wait_limit_ns : WAIT_LIMIT_NS;
     void *params[] = {&A};
-    GPMA_CUDA(cudaLaunchCooperativeKernel((const void *)bfs_kernel, dim3(bfs_ctas(A.size, grid)), dim3(BLOCK), params, 0, s));
+    GPMA_CUDA(cudaLaunchCooperativeKernel(bfs_kernel_ptr(A.size), dim3(bfs_ctas(A.size, grid)), dim3(BLOCK), params, 0, s));
     uint32_t h_ctl[CTL_WORDS];
     GPMA_CUDA(cudaMemcpyAsync(h_ctl, ctl, sizeof(h_ctl), cudaMemcpyDeviceToHost, s));
     GPMA_CUDA(cudaStreamSynchronize(s));
