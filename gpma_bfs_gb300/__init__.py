@@ -762,6 +762,8 @@ class Batch:
         """(levels per graph or None, reached per graph) for up to 64 sources per graph."""
         k = len(graphs)
         flat, sp, ns = _source_lists(sources)
+        if len(ns) != k:  # the C call reads one address and one count per graph
+            raise ValueError("one source list per graph")
         hs = (ctypes.c_void_p * k)(*[g.handle.value for g in graphs])
         counts = ns.tolist()
         outs = [np.zeros((n, g.row_num), np.uint32) for n, g in zip(counts, graphs)] if levels else None
