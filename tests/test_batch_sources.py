@@ -44,6 +44,8 @@ def test_list_count_must_match(monkeypatch, graphs, lists):
 
 @pytest.mark.parametrize("form, want", [
     ([[1], [2, 3]], [[1], [2, 3]]),
+    ([4, [5]], [[4], [5]]),  # a single node in place of a list
+    ([np.uint32(7), np.array(8)], [[7], [8]]),
     (np.array([[1, 2], [3, 4]]), [[1, 2], [3, 4]]),
     ((np.arange(6, dtype=np.int64)[::2], (5,)), [[0, 2, 4], [5]]),
 ])
