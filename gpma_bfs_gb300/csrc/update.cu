@@ -142,6 +142,13 @@ __device__ __forceinline__ uint32_t graph_of(const UpdateArgs &A, uint32_t i) {
 // their order are the reference's bit-by-bit descent (gpma.cuh:209-216).
 constexpr uint32_t LOCATE_CACHE = 4096;
 
+// Key 0 (the edge 0 -> 0) is also the key of the bulk rebuild's gaps, which lie
+// behind the elements of their leaf. The edge is the smallest key, so where the
+// leaf found for it holds it, the leaf begins with it; key 0 first met behind
+// the leaf's first slot is a gap, and a value written there would bring it to
+// life behind greater keys.
+__device__ __forceinline__ bool is_gap_hit(uint64_t key, uint32_t slot_in_leaf) { return key == 0 && slot_in_leaf != 0; }
+
 // The leaf's first slot equal to `key` (handle_del_mod scans all seg slots),
 // or SIZE_NONE. All seg/2 16-byte loads are issued before any comparison.
 __device__ __forceinline__ uint32_t leaf_find(const GraphDesc &D, uint32_t leaf, uint64_t key) {
@@ -162,7 +169,7 @@ __device__ __forceinline__ uint32_t leaf_find(const GraphDesc &D, uint32_t leaf,
                 hit = 2 * j;
         }
     }
-    return hit;
+    return is_gap_hit(key, hit) ? SIZE_NONE : hit;
 }
 
 // Locates LOC_ILP updates per thread together: at each level of the descent
@@ -1017,7 +1024,8 @@ __device__ bool small_front(const UpdateArgs &A, unsigned char *smem, uint32_t *
             uint32_t leaf = warp_descend(D, key, lane);
             const bool ok = in_bounds(&st->err, (uint64_t)leaf + D.seg <= D.size, BS_LEAF);
             const uint32_t hits =
-                __ballot_sync(0xFFFFFFFFu, ok && lane < D.seg && D.keys[leaf + lane] == key);
+                __ballot_sync(0xFFFFFFFFu, ok && lane < D.seg && D.keys[leaf + lane] == key &&
+                                               !is_gap_hit(key, lane));
             if (lane == 0) {
                 if (hits)
                     D.vals[leaf + __ffs(hits) - 1] = value;  // delete / modify / revive in place
