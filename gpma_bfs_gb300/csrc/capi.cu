@@ -21,7 +21,7 @@ void set_error(const char *fmt, ...) {
 
 gpma_status device_error(const char *where, uint32_t code) {
     if ((code & 0xFFu) == DERR_BOUNDS) {
-        set_error("out-of-range index in %s (bounds-checked build, site %u)", where, code >> 8);
+        set_error("out-of-range index in %s (site %u)", where, code >> 8);
         return GPMA_ERR_DEVICE;
     }
     set_error("device-side wait gave up in %s (code %u)", where, code);

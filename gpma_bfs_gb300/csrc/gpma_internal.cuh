@@ -55,7 +55,7 @@ enum : uint32_t {
 // checked against its buffer before the access. A failing check skips the
 // access and records DERR_BOUNDS | site << 8 in the launch's error word, and
 // the launch stops at its next grid barrier. The product build compiles the
-// checks away.
+// checks away, except those of the rebuild's merge splits (one per chunk).
 #ifndef GPMA_BOUNDS_CHECK
 #define GPMA_BOUNDS_CHECK 0
 #endif
@@ -64,7 +64,7 @@ enum BoundsSite : uint32_t {
     BS_WINDOW = 2,    // level loop: a warp/CTA window's slots
     BS_PENDING = 3,   // level loop: a window's pending insertions
     BS_CHUNK = 4,     // level loop: a grid-wide window's chunk
-    BS_REBUILD = 5,   // bulk rebuild / compacted layout: a slot
+    BS_REBUILD = 5,   // whole-array rebuild: a chunk's merge split
     BS_ROW = 6,       // BFS / multi-source BFS / analytics: a row's slot range
 };
 
@@ -541,15 +541,18 @@ __device__ __forceinline__ uint64_t globaltimer_ns() {
 
 __device__ __forceinline__ uint32_t ld_volatile(const uint32_t *p) { return *(const volatile uint32_t *)p; }
 
-// True when `ok`; in the bounds-checked build a false `ok` records the site
-// in *err (first error wins) and the caller skips the access.
+// `ok`; a false one records the site in *err (first error wins) and the caller
+// skips the access.
+__device__ __forceinline__ bool check_range(uint32_t *err, bool ok, uint32_t site) {
+    if (!ok)
+        atomicCAS(err, 0u, DERR_BOUNDS | (site << 8));
+    return ok;
+}
+
+// check_range in the bounds-checked build, true in the product build.
 __device__ __forceinline__ bool in_bounds(uint32_t *err, bool ok, uint32_t site) {
-    if constexpr (GPMA_BOUNDS_CHECK != 0) {
-        if (!ok) {
-            atomicCAS(err, 0u, DERR_BOUNDS | (site << 8));
-            return false;
-        }
-    }
+    if constexpr (GPMA_BOUNDS_CHECK != 0)
+        return check_range(err, ok, site);
     return true;
 }
 

@@ -1828,6 +1828,16 @@ __device__ __forceinline__ uint32_t merge_split(const uint64_t *lk, uint32_t L, 
     return lo;
 }
 
+// Whether merged elements [i_lo, i_hi) are live[x0 .. x1) and pending elements of
+// a staged chunk's size. The searches for x0 and x1 know nothing of each other:
+// over an array that is not sorted (written by another program, say) they may run
+// backwards, and the copies' lengths with them. One test per chunk, in every build.
+__device__ __forceinline__ bool split_ok(uint32_t i_lo, uint32_t i_hi, uint32_t x0, uint32_t x1, uint32_t L,
+                                         uint32_t P) {
+    return x0 <= x1 && x1 <= L && x0 <= i_lo && x1 <= i_hi && i_lo - x0 <= i_hi - x1 && i_hi - x1 <= P &&
+           i_hi - i_lo <= CHUNK;
+}
+
 // First merged element of each CHUNK-slot chunk of the redispatched array
 // (and of its end), split into live and pending parts: split[c] = live
 // elements before chunk c. One search per chunk boundary, all in parallel.
@@ -1867,10 +1877,7 @@ __global__ void __launch_bounds__(BLOCK) rebuild_kernel(uint64_t *keys, uint8_t 
         const uint32_t i_lo = (uint32_t)(f_lo < M ? f_lo : M), i_hi = (uint32_t)(f_hi < M ? f_hi : M);
         const uint32_t x0 = split[c], x1 = split[c + 1];
         // the same condition in every thread: the whole CTA skips the chunk
-        if (!in_bounds(err,
-                       x0 <= x1 && x1 <= L && x0 <= i_lo && x1 <= i_hi && i_lo - x0 <= i_hi - x1 &&
-                           i_hi - x1 <= P && i_hi - i_lo <= CHUNK,
-                       BS_REBUILD))
+        if (!check_range(err, split_ok(i_lo, i_hi, x0, x1, L, P), BS_REBUILD))
             continue;
         const uint32_t y0 = i_lo - x0, y1 = i_hi - x1;
         const uint32_t nl = x1 - x0, np = y1 - y0;  // nl + np = i_hi - i_lo <= len
@@ -2195,10 +2202,7 @@ __device__ __forceinline__ void rb_issue(uint32_t c, unsigned char *stage, RbDes
     const uint64_t f_lo = seg_first(t0 >> log2seg, M, log2F), f_hi = seg_first((t0 + CHUNK) >> log2seg, M, log2F);
     const uint32_t i_lo = (uint32_t)(f_lo < M ? f_lo : M), i_hi = (uint32_t)(f_hi < M ? f_hi : M);
     const uint32_t x0 = split[c], x1 = split[c + 1];
-    const bool ok = in_bounds(err,
-                              x0 <= x1 && x1 <= L && x0 <= i_lo && x1 <= i_hi && i_lo - x0 <= i_hi - x1 &&
-                                  i_hi - x1 <= P && i_hi - i_lo <= CHUNK,
-                              BS_REBUILD);
+    const bool ok = check_range(err, split_ok(i_lo, i_hi, x0, x1, L, P), BS_REBUILD);
     uint32_t bytes = 0;
     RbDesc r{};
     r.ok = ok ? 1u : 0u;
@@ -2291,7 +2295,7 @@ __global__ void __launch_bounds__(BLOCK, 4) rebuild_bulk_kernel(uint64_t *keys, 
         pending &= ~(1u << s);
         const RbDesc d = desc[s];
         if (!d.ok) {
-            // bounds-checked build: the chunk is skipped (the error is recorded)
+            // the chunk is skipped (the error is recorded)
             __syncthreads();
             continue;
         }
