@@ -687,8 +687,8 @@ def read_edges_text(path: str):
 
 def _source_lists(sources):
     """(all sources in one uint32 array, the address of each list in it, their lengths)."""
-    srcs = [np.atleast_1d(np.asarray(s, np.uint32)) for s in sources]
-    srcs = [s if s.ndim == 1 else s.reshape(-1)[:len(s)] for s in srcs]
+    srcs = [np.asarray(s, np.uint32) for s in sources]
+    srcs = [s if s.ndim == 1 else s.reshape(-1)[:len(s) if s.ndim else 1] for s in srcs]
     ns = np.array([len(s) for s in srcs], np.uint32)
     flat = np.concatenate(srcs) if srcs else np.zeros(0, np.uint32)
     starts = np.cumsum(ns, dtype=np.uint64) - ns
