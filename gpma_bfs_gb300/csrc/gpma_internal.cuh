@@ -87,7 +87,7 @@ extern TestHooks g_test_hooks;
 // the start of a launch, on a 128-byte line of its own, apart from the words
 // that kernels count in.
 struct alignas(128) GridBarrier {
-    unsigned int count;  // tickets taken
+    unsigned int count;  // tickets taken, modulo BARRIER_ROUNDS rounds
 };
 constexpr uint32_t BAR_WORDS = sizeof(GridBarrier) / sizeof(uint32_t);
 constexpr uint32_t BAR_ALIGN_WORDS = 32;
@@ -560,6 +560,10 @@ __device__ __forceinline__ bool in_bounds(uint32_t *err, bool ok, uint32_t site)
 // ticket from one counter (it must start each launch at zero) and waits until
 // the counter reaches the end of its ticket's round of gridDim.x; there is no
 // separate release write, so a barrier costs one atomic per CTA and polling.
+// The counter goes back to zero after BARRIER_ROUNDS rounds: 2^32 tickets are a
+// search of a few million levels, and would end a round of most grids early.
+// (A round's end kept per CTA in place of the ticket's: the social BFS 345 -> 368
+// us, as the CTAs poll sooner, and 353 with the arrival's count as the first poll.)
 // The polls are relaxed loads back to back, with one acquire at the end (an
 // acquire per poll drops the L1 lines of the CTAs still at work on the SM); the
 // error word and the clock are looked at in every 8th poll only. Alone, per
@@ -569,6 +573,19 @@ __device__ __forceinline__ bool in_bounds(uint32_t *err, bool ok, uint32_t site)
 // round trips); a fence in place of the acquire +0.4 us. Every wait is bounded:
 // after WAIT_LIMIT_NS the CTA records DERR_BARRIER_TIMEOUT and returns false;
 // CTAs that see an error stop waiting.
+constexpr uint32_t BARRIER_ROUNDS = 1u << 16;
+static_assert((uint64_t)BARRIER_ROUNDS * 0xFFFF <= 0xFFFFFFFFull, "tickets of any grid fit 32 bits");
+struct BarrierRound {
+    // limit of atomicInc: the last ticket before the counter is zero again
+    static __host__ __device__ __forceinline__ uint32_t last_ticket(uint32_t ctas) { return ctas * BARRIER_ROUNDS - 1; }
+    uint32_t ticket, end;
+    __host__ __device__ __forceinline__ BarrierRound(uint32_t ticket_, uint32_t ctas, uint32_t extra = 0)
+        : ticket(ticket_), end((ticket_ / ctas + 1) * ctas + extra) {}
+    // The count of this launch has passed the ticket: where it has not, it has
+    // started over, with the end of this round or since.
+    __host__ __device__ __forceinline__ bool over(uint32_t count) const { return count >= end || count <= ticket; }
+};
+
 // `extra` (test hooks only, 0 otherwise) adds arrivals that never come, so the
 // wait runs out after `limit_ns`.
 __device__ __forceinline__ bool grid_barrier(GridBarrier *bar, uint32_t *err, uint32_t extra = 0,
@@ -577,13 +594,12 @@ __device__ __forceinline__ bool grid_barrier(GridBarrier *bar, uint32_t *err, ui
     __shared__ uint32_t s_ok;
     if (threadIdx.x == 0) {
         __threadfence();
-        const uint32_t ticket = atomicAdd(&bar->count, 1u);
-        const uint32_t target = (ticket / gridDim.x + 1) * gridDim.x + extra;
+        const BarrierRound round(atomicInc(&bar->count, BarrierRound::last_ticket(gridDim.x)), gridDim.x, extra);
         uint64_t t0 = 0;
         uint32_t polls = 0, c;
         for (;;) {
             asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(c) : "l"(&bar->count) : "memory");
-            if ((int)(c - target) >= 0)
+            if (round.over(c))
                 break;
             if ((++polls & 7u) == 0) {
                 if (ld_volatile(err) != 0)
