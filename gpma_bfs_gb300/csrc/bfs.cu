@@ -546,8 +546,8 @@ gpma_status bfs_plan(gpma_graph *g, uint32_t src, uint32_t *levels, BfsPlan *P, 
         g->bfs_item_cap = (uint32_t)items;
     }
     const uint32_t n = g->row_num;
-    // levels go straight to the caller's array where that is device memory
-    P->direct = levels && is_device_pointer(levels) && reinterpret_cast<uintptr_t>(levels) % sizeof(uint32_t) == 0;
+    // levels go straight to the caller's array where that is this device's memory
+    P->direct = levels && levels_in_place(levels, g->device);
     if (!P->direct && n > g->bfs_levels_cap) {
         dev_free(g->bfs_levels);
         g->bfs_levels_cap = 0;

@@ -34,8 +34,6 @@ gpma_status cuda_fail(cudaError_t e, const char *what) {
     return e == cudaErrorMemoryAllocation ? GPMA_ERR_NOMEM : GPMA_ERR_CUDA;
 }
 
-namespace {
-// What CUDA knows about a pointer (type unregistered for plain host memory).
 cudaPointerAttributes pointer_attributes(const void *p) {
     cudaPointerAttributes attr{};
     if (cudaPointerGetAttributes(&attr, p) != cudaSuccess) {
@@ -44,10 +42,8 @@ cudaPointerAttributes pointer_attributes(const void *p) {
     }
     return attr;
 }
-bool is_device(const cudaPointerAttributes &a) {
-    return a.type == cudaMemoryTypeDevice || a.type == cudaMemoryTypeManaged;
-}
 
+namespace {
 // The first `count` words at src (host or device) into dst (host); sets *pending
 // when a copy was enqueued on s and has to be waited for. Plain host memory is
 // read here (a copy call per graph took 0.4 ms for 128 graphs); page-locked and
@@ -62,8 +58,6 @@ gpma_status fetch_words(uint32_t *dst, const uint32_t *src, uint32_t count, cuda
     return GPMA_OK;
 }
 }  // namespace
-
-bool is_device_pointer(const void *p) { return is_device(pointer_attributes(p)); }
 
 gpma_status copy_any(void *dst, const void *src, size_t bytes, cudaStream_t s) {
     if (bytes == 0)
@@ -242,7 +236,8 @@ gpma_status packed_plan(gpma_batch *b, gpma_graph *const *graphs, const uint64_t
     std::stable_sort(order.begin(), order.end(),
                      [&](uint32_t x, uint32_t y) { return graphs[x]->geo.seg < graphs[y]->geo.seg; });
     GPMA_TRY(ensure_buffers(b->buf, std::max<uint64_t>(total, all), P->m));
-    P->upload = !(is_device_pointer(keys) && is_device_pointer(values));
+    P->upload = !(read_in_place(pointer_attributes(keys), b->device) &&
+                  read_in_place(pointer_attributes(values), b->device));
     P->all_keys = all;
     const uint64_t src_base = P->upload ? offsets[0] : 0;
     const uint32_t m = P->m;
@@ -399,7 +394,7 @@ gpma_status gpma_update(gpma_graph *g, const uint64_t *keys, const uint8_t *valu
     cudaStream_t s = (cudaStream_t)stream;
     GPMA_TRY(ensure_buffers(g->buf, n, 1));
     const cudaPointerAttributes ka = pointer_attributes(keys), va = pointer_attributes(values);
-    if (is_device(ka) && is_device(va))
+    if (read_in_place(ka, g->device) && read_in_place(va, g->device))
         return update_device(g, n, s, keys, values);  // the kernel reads the caller's batch in place
     // page-locked host batches: the kernel reads them over the host link
     // itself (the keys twice: ranks, then the scatter), no staging copy; small
@@ -445,8 +440,9 @@ gpma_status gpma_bfs_noalloc(gpma_graph *g, uint32_t src, uint32_t *levels, uint
         set_error("gpma_bfs_noalloc: start node %u out of range (row_num %u)", src, g->row_num);
         return GPMA_ERR_INVALID;
     }
-    if (!is_device_pointer(levels)) {
-        set_error("gpma_bfs_noalloc: levels must be device memory (no staging buffer can be allocated)");
+    if (!read_in_place(pointer_attributes(levels), g->device)) {
+        set_error("gpma_bfs_noalloc: levels must be device memory of the graph's GPU (no staging buffer "
+                  "can be allocated)");
         return GPMA_ERR_INVALID;
     }
     return bfs_noalloc_run(g, src, levels, reached, (cudaStream_t)stream);

@@ -318,8 +318,22 @@ struct CallRange {
             return _s;                                                                                                 \
     } while (0)
 
-// true if p is device-accessible memory of the current device
-bool is_device_pointer(const void *p);
+// What CUDA knows about a pointer (type unregistered for plain host memory).
+cudaPointerAttributes pointer_attributes(const void *p);
+// Whether kernels on `device` write the caller's memory themselves: its own
+// memory. Another GPU's needs peer access, which a copy does not.
+inline bool written_in_place(const cudaPointerAttributes &a, int device) {
+    return a.type == cudaMemoryTypeDevice && a.device == device;
+}
+// ... or read it: managed memory too.
+inline bool read_in_place(const cudaPointerAttributes &a, int device) {
+    return written_in_place(a, device) || a.type == cudaMemoryTypeManaged;
+}
+// Whether a search writes its levels there (else they are copied there).
+inline bool levels_in_place(const uint32_t *levels, int device) {
+    return reinterpret_cast<uintptr_t>(levels) % sizeof(uint32_t) == 0 &&
+           written_in_place(pointer_attributes(levels), device);
+}
 // copies between host or device pointers on a stream (kind inferred)
 gpma_status copy_any(void *dst, const void *src, size_t bytes, cudaStream_t s);
 template <typename T>

@@ -790,8 +790,8 @@ gpma_status batch_bfs_finish(gpma_batch *b, const uint32_t *nsrc, uint32_t k, ui
 // those are host memory; reached receives sum(nsrc) counts.
 gpma_status batch_bfs_run(gpma_batch *b, gpma_graph *const *graphs, const uint32_t *const *srcs, const uint32_t *nsrc,
                           uint32_t k, uint32_t *const *levels, uint64_t *reached, cudaStream_t s) {
-    // where the kernel writes each graph's levels: the caller's own device
-    // array, or staging memory copied out afterwards (every entry is written,
+    // where the kernel writes each graph's levels: the caller's array on this
+    // device, or staging memory copied out afterwards (every entry is written,
     // so neither needs clearing)
     std::vector<uint32_t *> stage(k, nullptr), staged(k, nullptr);
     auto cleanup = [&]() {
@@ -804,7 +804,7 @@ gpma_status batch_bfs_run(gpma_batch *b, gpma_graph *const *graphs, const uint32
             for (uint32_t i = 0; i < k; ++i) {
                 if (!levels[i])
                     continue;
-                if (is_device_pointer(levels[i]) && reinterpret_cast<uintptr_t>(levels[i]) % sizeof(uint32_t) == 0) {
+                if (levels_in_place(levels[i], b->device)) {
                     stage[i] = levels[i];
                     continue;
                 }

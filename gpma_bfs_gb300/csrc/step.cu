@@ -507,7 +507,8 @@ gpma_status batch_step_run_many(gpma_batch_step *st, uint32_t S, const uint64_t 
     };
     bool eligible = S > 1;
     for (uint32_t t = 0; t < S && eligible; ++t) {
-        eligible = is_device_pointer(keys[t]) && is_device_pointer(values[t]);
+        eligible = read_in_place(pointer_attributes(keys[t]), st->b->device) &&
+                   read_in_place(pointer_attributes(values[t]), st->b->device);
         const uint64_t *o = off_of(t);
         for (uint32_t i = 0; i < k && eligible; ++i) {
             const uint64_t c = o[i + 1] - o[i];
