@@ -44,12 +44,13 @@ cudaPointerAttributes pointer_attributes(const void *p) {
 }
 
 namespace {
-// The first `count` words at src (host or device) into dst (host); sets *pending
-// when a copy was enqueued on s and has to be waited for. Plain host memory is
-// read here (a copy call per graph took 0.4 ms for 128 graphs); page-locked and
-// device memory in stream order, as work before it on s may still write it.
+// The first `count` words at src (host or device) into dst (host), on a stream
+// that has been waited for; sets *pending when a copy was enqueued on s and has
+// to be waited for. Host memory is read here (a copy call per graph took 0.4 ms
+// for 128 graphs).
 gpma_status fetch_words(uint32_t *dst, const uint32_t *src, uint32_t count, cudaStream_t s, bool *pending) {
-    if (pointer_attributes(src).type == cudaMemoryTypeUnregistered) {
+    const cudaMemoryType type = pointer_attributes(src).type;
+    if (type == cudaMemoryTypeUnregistered || type == cudaMemoryTypeHost) {
         memcpy(dst, src, sizeof(uint32_t) * count);
         return GPMA_OK;
     }
@@ -458,6 +459,7 @@ gpma_status gpma_bfs_multi(gpma_graph *g, const uint32_t *srcs, uint32_t k, uint
     cudaStream_t s = (cudaStream_t)stream;
     uint32_t hs[64];
     bool pending = false;
+    GPMA_CUDA(cudaStreamSynchronize(s));  // work before the search may still write the sources
     GPMA_TRY(fetch_words(hs, srcs, k, s, &pending));
     if (pending)
         GPMA_CUDA(cudaStreamSynchronize(s));
@@ -651,12 +653,14 @@ gpma_status gpma_batch_bfs_multi(gpma_batch *b, gpma_graph *const *graphs, const
     std::vector<std::vector<uint32_t>> hs(k);
     std::vector<const uint32_t *> hp(k);
     uint64_t nodes = 0;
-    bool pending = false;
-    for (uint32_t i = 0; i < k; ++i) {
+    for (uint32_t i = 0; i < k; ++i)
         if (!graphs[i] || !srcs[i] || nsrc[i] == 0 || nsrc[i] > 64) {
             set_error("gpma_batch_bfs_multi: graph %u: null pointer or source count not in 1..64", i);
             return GPMA_ERR_INVALID;
         }
+    bool pending = false;
+    GPMA_CUDA(cudaStreamSynchronize(s));  // work before the search may still write the sources
+    for (uint32_t i = 0; i < k; ++i) {
         hs[i].resize(nsrc[i]);
         GPMA_TRY(fetch_words(hs[i].data(), srcs[i], nsrc[i], s, &pending));
         nodes += graphs[i]->row_num;
