@@ -46,9 +46,17 @@ constexpr uint32_t SORT_TILE = BLOCK * SORT_ITEMS;
 constexpr uint32_t SORT_TILE_LARGE = BLOCK * SORT_ITEMS_LARGE;
 static_assert(SORT_TILE_LARGE * 9 + (BLOCK / 32 + 2) * 256 * 4 <= UPDATE_SMEM,
               "sort tile exceeds the update kernel's smem");
-constexpr uint32_t SORT_FLAG_AGG = 1u << 30;
-constexpr uint32_t SORT_FLAG_INC = 2u << 30;
-constexpr uint32_t SORT_VALUE_MASK = (1u << 30) - 1;
+// A look-back word: 0 not published yet, a tile's own count of a digit (01 in the
+// top bits), or the count up to and with the tile (1 in the top bit: up to 2^31 - 1
+// keys of a launch, which may all have one digit).
+struct SortWord {
+    uint32_t w;
+    static __host__ __device__ __forceinline__ SortWord own(uint32_t count) { return {1u << 30 | count}; }
+    static __host__ __device__ __forceinline__ SortWord upto(uint32_t count) { return {1u << 31 | count}; }
+    __host__ __device__ __forceinline__ bool published() const { return w != 0; }
+    __host__ __device__ __forceinline__ bool is_upto() const { return w >> 31; }
+    __host__ __device__ __forceinline__ uint32_t count() const { return w & (is_upto() ? 0x7FFFFFFFu : 0x3FFFFFFFu); }
+};
 
 // Histograms of all 8 digits into hist[g][8][256] for each graph g < G and
 // the totals into hist[G][8][256] (zeroed by the caller); sets
@@ -180,7 +188,7 @@ __device__ void sort_tile(int pass, uint32_t tile, const uint64_t *__restrict__ 
     // is out before anything else is worked out, so that later tiles seldom
     // find it missing (15.3M keys: 0.94 -> 0.91 ms).
     uint32_t prefix = 0;
-    atomicExch(&status[(size_t)tile * 256 + d], (tile == first_tile ? SORT_FLAG_INC : SORT_FLAG_AGG) | local);
+    atomicExch(&status[(size_t)tile * 256 + d], (tile == first_tile ? SortWord::upto(local) : SortWord::own(local)).w);
     s_start[d] = block_excl_scan(local, &total, tmp);
     const uint32_t base = seg_lo + block_excl_scan(hist[(size_t)g * 2048 + pass * 256 + d], &total, tmp);
     if (tile != first_tile) {
@@ -190,25 +198,25 @@ __device__ void sort_tile(int pass, uint32_t tile, const uint64_t *__restrict__ 
         uint64_t t0 = 0;
         unsigned ns = 32;
         while (t >= (int64_t)first_tile) {
-            uint32_t w[SORT_LOOKBACK];
+            SortWord w[SORT_LOOKBACK];
 #pragma unroll
             for (uint32_t i = 0; i < SORT_LOOKBACK; ++i)
-                w[i] = t - (int64_t)i >= (int64_t)first_tile ? ld_volatile(&status[(size_t)(t - i) * 256 + d])
-                                                              : SORT_FLAG_INC;  // never read: the first tile is inclusive
+                w[i].w = t - (int64_t)i >= (int64_t)first_tile
+                             ? ld_volatile(&status[(size_t)(t - i) * 256 + d])
+                             : SortWord::upto(0).w;  // never looked at: the first tile's count ends the look-back
             uint32_t take = 0;
             bool inc = false, blocked = false;
 #pragma unroll
             for (uint32_t i = 0; i < SORT_LOOKBACK; ++i) {
                 if (inc || blocked)
                     continue;
-                const uint32_t flag = w[i] & ~SORT_VALUE_MASK;
-                if (flag == 0) {
+                if (!w[i].published()) {
                     blocked = true;
                     continue;
                 }
-                prefix += w[i] & SORT_VALUE_MASK;
+                prefix += w[i].count();
                 ++take;
-                inc = flag == SORT_FLAG_INC;
+                inc = w[i].is_upto();
             }
             if (inc)
                 break;
@@ -225,7 +233,7 @@ __device__ void sort_tile(int pass, uint32_t tile, const uint64_t *__restrict__ 
                 }
             }
         }
-        atomicExch(&status[(size_t)tile * 256 + d], SORT_FLAG_INC | (prefix + local));
+        atomicExch(&status[(size_t)tile * 256 + d], SortWord::upto(prefix + local).w);
     }
     s_global[d] = base + prefix;
     __syncthreads();
