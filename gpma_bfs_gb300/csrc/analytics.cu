@@ -111,6 +111,16 @@ __device__ __forceinline__ double block_sum_f64(double x, double *tmp) {
     return t;  // valid in thread 0
 }
 
+// PageRank calls of up to SHORT_CALL iterations (three barriers each) take fewer than
+// 2^32 tickets and so the plain barrier, in builds of their own (20 iterations on
+// the social graph, by gathering: 1,995 us, 2,040 with the other).
+constexpr uint32_t SHORT_CALL = 1u << 18;
+template <bool LONG>
+__device__ __forceinline__ bool an_barrier(GridBarrier *bar, uint32_t *err) {
+    return LONG ? grid_barrier_long(bar, err) : grid_barrier(bar, err);
+}
+
+template <bool LONG>
 __global__ void __launch_bounds__(BLOCK) pagerank_kernel(AnArgs A) {
     GridBarrier *bar = reinterpret_cast<GridBarrier *>(A.ctl + AN_BAR);
     uint32_t *err = A.ctl + AN_ERR;
@@ -126,7 +136,7 @@ __global__ void __launch_bounds__(BLOCK) pagerank_kernel(AnArgs A) {
         A.rank[v] = 1.0f / (float)A.n;
         A.acc[v] = 0.0f;
     }
-    if (!grid_barrier(bar, err))
+    if (!an_barrier<LONG>(bar, err))
         return;
     for (uint32_t o = gtid; o < groups || (A.size < 8 && o == 0); o += nthreads) {
         uint32_t u[8], v[8];
@@ -153,7 +163,7 @@ __global__ void __launch_bounds__(BLOCK) pagerank_kernel(AnArgs A) {
         if (A.size < 8)
             break;
     }
-    if (!grid_barrier(bar, err))
+    if (!an_barrier<LONG>(bar, err))
         return;
     uint32_t it = 0;
     for (; it < A.max_iter; ++it) {
@@ -172,7 +182,7 @@ __global__ void __launch_bounds__(BLOCK) pagerank_kernel(AnArgs A) {
         dang = block_sum_f64(dang, tmp);
         if (threadIdx.x == 0 && dang != 0.0)
             atomicAdd(an_dbl(A, 0, it), dang);
-        if (!grid_barrier(bar, err))
+        if (!an_barrier<LONG>(bar, err))
             return;
         for (uint32_t o = gtid; o < groups || (A.size < 8 && o == 0); o += nthreads) {
             uint32_t u[8], v[8];
@@ -192,7 +202,7 @@ __global__ void __launch_bounds__(BLOCK) pagerank_kernel(AnArgs A) {
             if (A.size < 8)
                 break;
         }
-        if (!grid_barrier(bar, err))
+        if (!an_barrier<LONG>(bar, err))
             return;
         if (threadIdx.x == 0)
             s_val = *reinterpret_cast<volatile double *>(an_dbl(A, 0, it));
@@ -208,7 +218,7 @@ __global__ void __launch_bounds__(BLOCK) pagerank_kernel(AnArgs A) {
         delta = block_sum_f64(delta, tmp);
         if (threadIdx.x == 0)
             atomicAdd(an_dbl(A, 1, it), delta);
-        if (!grid_barrier(bar, err))
+        if (!an_barrier<LONG>(bar, err))
             return;
         if (threadIdx.x == 0)
             s_val = *reinterpret_cast<volatile double *>(an_dbl(A, 1, it));
@@ -256,6 +266,7 @@ struct PrNode {
 // float atomic per edge (198 us per iteration). Bound by the 4-byte gathers of
 // the contributions (L2). 20 iterations on the social graph: 4.37 ms -> 1.99 ms
 // per call, 0.44 of it the layout.
+template <bool LONG>
 __global__ void __launch_bounds__(BLOCK) pagerank_gather_kernel(AnArgs A) {
     GridBarrier *bar = reinterpret_cast<GridBarrier *>(A.ctl + AN_BAR);
     uint32_t *err = A.ctl + AN_ERR;
@@ -271,7 +282,7 @@ __global__ void __launch_bounds__(BLOCK) pagerank_gather_kernel(AnArgs A) {
         A.deg[v] = 0;
         A.end[v] = 0;
     }
-    if (!grid_barrier(bar, err))
+    if (!an_barrier<LONG>(bar, err))
         return;
     // out-degrees (one atomic per run of a source) and in-degrees
     for (uint32_t o = gtid; o < groups; o += nthreads) {
@@ -295,7 +306,7 @@ __global__ void __launch_bounds__(BLOCK) pagerank_gather_kernel(AnArgs A) {
         if (run)
             atomicAdd(&A.deg[run_u], run);
     }
-    if (!grid_barrier(bar, err))
+    if (!an_barrier<LONG>(bar, err))
         return;
     // each CTA's nodes: in-edge total, initial ranks' contributions
     const uint32_t per = (A.n + gridDim.x - 1) / gridDim.x;
@@ -320,7 +331,7 @@ __global__ void __launch_bounds__(BLOCK) pagerank_gather_kernel(AnArgs A) {
                 atomicAdd(an_dbl(A, 0, 0), dang);
         }
     }
-    if (!grid_barrier(bar, err))
+    if (!an_barrier<LONG>(bar, err))
         return;
     {
         // first in-edge of every row (the cursor of the scatter, which leaves
@@ -350,7 +361,7 @@ __global__ void __launch_bounds__(BLOCK) pagerank_gather_kernel(AnArgs A) {
             run += tot;
         }
     }
-    if (!grid_barrier(bar, err))
+    if (!an_barrier<LONG>(bar, err))
         return;
     for (uint32_t o = gtid; o < groups; o += nthreads) {
         uint32_t u[8], v[8], at[8];
@@ -364,7 +375,7 @@ __global__ void __launch_bounds__(BLOCK) pagerank_gather_kernel(AnArgs A) {
             if (e[j])
                 A.csc[at[j]] = u[j];
     }
-    if (!grid_barrier(bar, err))
+    if (!an_barrier<LONG>(bar, err))
         return;
     const uint32_t nch = cta_broadcast_read(A.ctl + AN_CHUNKS), nmulti = cta_broadcast_read(A.ctl + AN_MULTI);
     uint32_t it = 0;
@@ -461,7 +472,7 @@ __global__ void __launch_bounds__(BLOCK) pagerank_gather_kernel(AnArgs A) {
         }
         if (nmulti) {
             // rows of several chunks, once every chunk has been added
-            if (!grid_barrier(bar, err))
+            if (!an_barrier<LONG>(bar, err))
                 return;
             for (uint32_t m = gtid; m < nmulti; m += nthreads) {
                 const uint2 r = A.multi[m];
@@ -477,7 +488,7 @@ __global__ void __launch_bounds__(BLOCK) pagerank_gather_kernel(AnArgs A) {
             if (threadIdx.x == 0)
                 atomicAdd(an_dbl(A, 1, it), delta);
         }
-        if (!grid_barrier(bar, err))
+        if (!an_barrier<LONG>(bar, err))
             return;
         if (P.want_delta) {
             if (threadIdx.x == 0)
@@ -624,12 +635,16 @@ __global__ void __launch_bounds__(BLOCK) components_kernel(AnArgs A) {
 }
 
 // Rows of the fit table: the kernels of this file.
-enum AnKernel { AN_PAGERANK, AN_PAGERANK_GATHER, AN_COMPONENTS, AN_KERNELS };
+enum AnKernel { AN_PAGERANK, AN_PAGERANK_GATHER, AN_PAGERANK_LONG, AN_PAGERANK_GATHER_LONG, AN_COMPONENTS, AN_KERNELS };
 int an_fit[64][AN_KERNELS] = {};  // resident CTAs per SM, per device
 
 gpma_status launch(AnKernel which, AnArgs &A, int sms, cudaStream_t s, uint32_t *h_ctl) {
-    const void *const kernels[AN_KERNELS] = {(const void *)pagerank_kernel, (const void *)pagerank_gather_kernel,
-                                             (const void *)components_kernel};
+    const void *const kernels[AN_KERNELS] = {
+        (const void *)pagerank_kernel<false>, (const void *)pagerank_gather_kernel<false>,
+        (const void *)pagerank_kernel<true>, (const void *)pagerank_gather_kernel<true>,
+        (const void *)components_kernel};
+    if (A.max_iter > SHORT_CALL && which != AN_COMPONENTS)
+        which = which == AN_PAGERANK ? AN_PAGERANK_LONG : AN_PAGERANK_GATHER_LONG;
     const void *kernel = kernels[which];
     int dev = 0;
     GPMA_CUDA(cudaGetDevice(&dev));

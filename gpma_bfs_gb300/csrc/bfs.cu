@@ -91,6 +91,14 @@ inline uint64_t bfs_item_need(uint32_t n, uint32_t size) {
 // word, all on one counter, serialises at 4.4 ns apiece.)
 constexpr uint32_t CTA_ITEMS = 1024;
 
+// bfs_long_kernel takes over after so many levels; a level of it is short when the
+// one before had at most SHORT_NODES nodes per CTA, and a CTA then walks its first
+// SHORT_ITEMS items before the barrier.
+constexpr uint32_t LONG_LEVELS = 64;
+constexpr uint32_t SHORT_NODES = 4;
+constexpr uint32_t SHORT_ITEMS = 2 * (BLOCK / 32);
+constexpr int LONG_CTAS_PER_SM = 3;
+
 struct BfsArgs {
     const uint64_t *keys;
     const uint8_t *vals;
@@ -101,6 +109,7 @@ struct BfsArgs {
     uint32_t *levels;
     // bitmaps of n/32+2 words each; over: non-zero for words whose items no list took
     uint32_t *seen, *done, *front, *over;
+    uint32_t *claimed[2];  // bfs_long_kernel: bitmaps of what short levels claim
     uint2 *items;      // {word, piece}
     uint32_t item_cap;
     uint32_t *ctl;
@@ -119,18 +128,19 @@ struct BfsArgs {
 // flight. A target that was not seen when its word was read is claimed without
 // waiting for a result (an old word costs an atomic that changes nothing).
 template <uint32_t N>
-__device__ __forceinline__ void visit_slots(const BfsArgs &A, const uint32_t (&sl)[N]) {
+__device__ __forceinline__ void visit_slots(const BfsArgs &A, const uint32_t (&sl)[N], uint32_t *claims) {
     uint32_t w[N], seen[N];
 #pragma unroll
     for (uint32_t j = 0; j < N; ++j) {
-        uint64_t k = KEY_NONE;
+        // only the target, the low word of the key
+        uint32_t k = 0xFFFFFFFFu;
         uint8_t v = 0;
         if (sl[j] != SIZE_NONE) {
-            k = A.keys[sl[j]];
+            k = reinterpret_cast<const uint32_t *>(A.keys)[2 * (size_t)sl[j]];
             v = A.vals[sl[j]];
         }
-        w[j] = (uint32_t)k;
-        seen[j] = (w[j] != 0xFFFFFFFFu && v != 0 && w[j] < A.n) ? 0u : 0xFFFFFFFFu;
+        w[j] = k;
+        seen[j] = (v != 0 && k < A.n) ? 0u : 0xFFFFFFFFu;
     }
 #pragma unroll
     for (uint32_t j = 0; j < N; ++j)
@@ -140,7 +150,7 @@ __device__ __forceinline__ void visit_slots(const BfsArgs &A, const uint32_t (&s
     for (uint32_t j = 0; j < N; ++j) {
         const uint32_t bit = 1u << (w[j] & 31);
         if (!(seen[j] & bit))
-            atomicOr(&A.seen[w[j] >> 5], bit);
+            atomicOr(&claims[w[j] >> 5], bit);
     }
 }
 
@@ -174,10 +184,10 @@ __device__ __forceinline__ void dense_visit8(const BfsArgs &A, const uint64_t (&
     }
 }
 
-// Slot of concatenated-range position p (< total) of a warp's rows: lane r
-// holds its row start b and exclusive prefix excl; finds the last r with
-// excl[r] <= p. All lanes must call it together.
-__device__ __forceinline__ uint32_t lb_slot(uint32_t p, uint32_t total, uint32_t b, uint32_t excl) {
+// Slot of concatenated-range position p (< total) of a warp's rows: lane r holds
+// its exclusive prefix excl and how far its row's start lies from it; finds the last
+// r with excl[r] <= p. All lanes must call it together.
+__device__ __forceinline__ uint32_t lb_slot(uint32_t p, uint32_t total, uint32_t start, uint32_t excl) {
     uint32_t r = 0;
 #pragma unroll
     for (uint32_t step = 16; step >= 1; step >>= 1) {
@@ -186,9 +196,8 @@ __device__ __forceinline__ uint32_t lb_slot(uint32_t p, uint32_t total, uint32_t
         if (cand < 32 && ex_c <= p)
             r = cand;
     }
-    const uint32_t rb = __shfl_sync(0xFFFFFFFFu, b, r);
-    const uint32_t rex = __shfl_sync(0xFFFFFFFFu, excl, r);
-    return p < total ? rb + (p - rex) : SIZE_NONE;
+    const uint32_t from = __shfl_sync(0xFFFFFFFFu, start, r);
+    return p < total ? p + from : SIZE_NONE;
 }
 
 // One frontier word as a warp walks it: lane l's row of node 32 * word + l.
@@ -214,7 +223,7 @@ __device__ __forceinline__ uint32_t row_slots(const BfsArgs &A, uint32_t bits, u
 
 // Walks slots [p0, p1) of a word's concatenated rows (p1: or their end).
 __device__ __forceinline__ void walk_word(const BfsArgs &A, const WordRows &W, uint32_t p0, uint32_t p1,
-                                          uint32_t lane) {
+                                          uint32_t lane, uint32_t *claims) {
     const uint32_t len = row_slots(A, W.f, lane, W.b, W.e);
     const uint32_t incl = warp_incl_scan(len);
     const uint32_t excl = incl - len;
@@ -223,9 +232,29 @@ __device__ __forceinline__ void walk_word(const BfsArgs &A, const WordRows &W, u
         uint32_t sl[LANE_SLOTS];
 #pragma unroll
         for (uint32_t j = 0; j < LANE_SLOTS; ++j)
-            sl[j] = lb_slot(p0 + 32 * j + lane, total, W.b, excl);
-        visit_slots<LANE_SLOTS>(A, sl);
+            sl[j] = lb_slot(p0 + 32 * j + lane, total, W.b - excl, excl);
+        visit_slots<LANE_SLOTS>(A, sl, claims);
     }
+}
+
+// The end of a search: the CTA's reached nodes (reached, in thread 0) are added, and
+// the last CTA to come here hands the control words to the host.
+__device__ __forceinline__ void report(const BfsArgs &A, uint32_t levels, uint32_t reached) {
+    if (threadIdx.x != 0)
+        return;
+    if (reached)
+        atomicAdd(A.ctl + CTL_REACHED, reached);
+    if (blockIdx.x == 0)
+        A.ctl[CTL_LEVELS] = levels;
+    __threadfence();
+    if (!A.host || atomicAdd(A.ctl + CTL_DONE, 1u) != gridDim.x - 1)
+        return;
+    __threadfence();
+    for (uint32_t c = 0; c < CTL_WORDS; ++c) {
+        A.host[c] = ld_volatile(A.ctl + c);
+        A.ctl[c] = 0;
+    }
+    reinterpret_cast<GridBarrier *>(A.ctl + CTL_BAR)->count = 0;
 }
 
 // Social graph (1.6M nodes, 15.3M edges, 33.5M slots), 13 levels: 344 us, 374
@@ -264,7 +293,7 @@ __global__ void __launch_bounds__(BLOCK, 5) bfs_kernel(BfsArgs A) {
         return;
     uint32_t reached = 0;
     uint32_t i = 0;
-    for (;; ++i) {
+    for (; i < LONG_LEVELS; ++i) {
         const bool stamper = A.stamps && gtid == 0 && i < CTL_PROFILE_LEVELS;
         if (stamper)
             A.stamps[i] = globaltimer_ns();
@@ -417,7 +446,7 @@ __global__ void __launch_bounds__(BLOCK, 5) bfs_kernel(BfsArgs A) {
                 WordRows N;
                 N.load(A, nxt.x, lane);
                 if (cur.y != SIZE_NONE)
-                    walk_word(A, W, cur.y * ITEM, (cur.y + 1) * ITEM, lane);
+                    walk_word(A, W, cur.y * ITEM, (cur.y + 1) * ITEM, lane, A.seen);
                 W = N;
                 cur = nxt;
                 nxt = after;
@@ -426,14 +455,14 @@ __global__ void __launch_bounds__(BLOCK, 5) bfs_kernel(BfsArgs A) {
             for (uint32_t c = threadIdx.x >> 5; c < kept; c += BLOCK / 32) {
                 const uint2 own = s_items[c];
                 W.load(A, own.x, lane);
-                walk_word(A, W, own.y * ITEM, (own.y + 1) * ITEM, lane);
+                walk_word(A, W, own.y * ITEM, (own.y + 1) * ITEM, lane, A.seen);
             }
             if (cta_broadcast_read(A.ctl + CTL_OVERFLOW)) {
                 for (uint32_t w = gwarp; w < words; w += nwarps) {
                     if (!A.over[w])
                         continue;
                     W.load(A, w, lane);
-                    walk_word(A, W, 0, SIZE_NONE, lane);
+                    walk_word(A, W, 0, SIZE_NONE, lane, A.seen);
                     __syncwarp();
                     if (lane == 0)
                         A.over[w] = 0;
@@ -452,33 +481,204 @@ __global__ void __launch_bounds__(BLOCK, 5) bfs_kernel(BfsArgs A) {
     if (lane == 0 && reached)
         atomicAdd(&s_at, reached);
     __syncthreads();
-    if (threadIdx.x != 0)
-        return;
-    if (s_at)
-        atomicAdd(A.ctl + CTL_REACHED, s_at);
-    if (blockIdx.x == 0)
-        A.ctl[CTL_LEVELS] = i;
-    __threadfence();
-    if (!A.host || atomicAdd(A.ctl + CTL_DONE, 1u) != gridDim.x - 1)
-        return;
-    __threadfence();
-    for (uint32_t c = 0; c < CTL_WORDS; ++c) {
-        A.host[c] = ld_volatile(A.ctl + c);
-        A.ctl[c] = 0;
-    }
-    bar->count = 0;
+    report(A, i, s_at);
 }
 
-const void *bfs_kernel_ptr(uint32_t size) {
+// A search from level LONG_LEVELS on, over the maps that bfs_kernel left: levels of
+// few nodes end with one grid barrier instead of two (a 300 x 300 grid, 599 levels:
+// 8.4 us per level with two, 5.8 with one). A short level claims nodes in a bitmap of
+// the level's parity, which the next level's scan adds to seen, so that a CTA can
+// walk its items while others still scan; items beyond SHORT_ITEMS go to the grid's
+// list for a walk behind the barrier, and where no CTA has any the level is done.
+// A kernel of its own, since bfs_kernel is 3 to 15 % slower on the social graph with
+// any of this inside. (No dense levels here: they would be the same.)
+template <uint32_t ITEM>
+__global__ void __launch_bounds__(BLOCK, LONG_CTAS_PER_SM) bfs_long_kernel(BfsArgs A) {
+    __shared__ uint2 s_items[CTA_ITEMS];
+    __shared__ uint32_t s_nit, s_end, s_at;  // as in bfs_kernel
+    __shared__ uint32_t s_cnt[BLOCK / 32];
+    GridBarrier *bar = reinterpret_cast<GridBarrier *>(A.ctl + CTL_BAR);
+    uint32_t *err = A.ctl + CTL_ERR;
+    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const uint32_t gwarp = blockIdx.x * (BLOCK / 32) + warp;
+    const uint32_t nwarps = gridDim.x * (BLOCK / 32);
+    const uint32_t gtid = blockIdx.x * BLOCK + threadIdx.x, nthreads = gridDim.x * BLOCK;
+    const uint32_t words = (A.n + 31) >> 5;
+    for (uint32_t w = gtid; w < words; w += nthreads) {
+        A.claimed[0][w] = 0;
+        A.claimed[1][w] = 0;
+    }
+    if (!grid_barrier_long(bar, err))
+        return;
+    uint32_t reached = 0, frontier = SIZE_NONE;  // nodes of all levels, of the last one
+    bool brief = false;                          // the last level was a short one
+    uint32_t i = LONG_LEVELS;
+    for (;; ++i) {
+        if (threadIdx.x == 0) {
+            s_nit = 0;
+            s_end = CTA_ITEMS;
+        }
+        __syncthreads();
+        // scan, as in bfs_kernel
+        uint32_t *item_cnt = A.ctl + CTL_ITEMS + i % 3;
+        uint32_t count = 0;
+        for (uint32_t it = 0; gwarp + it * nwarps < words; it += 32) {
+            const uint32_t w0 = gwarp + it * nwarps, wl = w0 + lane * nwarps;
+            uint32_t mine = 0;
+            if (wl < words) {
+                uint32_t s = A.seen[wl];
+                if (brief) {
+                    // what the short level before claimed; only this lane has the word
+                    uint32_t *p = A.claimed[(i + 1) & 1] + wl;
+                    const uint32_t c = *p;
+                    if (c) {
+                        *p = 0;
+                        s |= c;
+                        A.seen[wl] = s;
+                    }
+                }
+                mine = s & ~A.done[wl];
+                A.front[wl] = mine;
+                if (mine)
+                    A.done[wl] = s;
+            }
+            count += __popc(mine);
+            uint32_t pending = __ballot_sync(0xFFFFFFFFu, mine != 0u);
+            uint32_t nb = 0, ne = 0;
+            auto offsets = [&]() {
+                const uint32_t u = ((w0 + (__ffs(pending) - 1) * nwarps) << 5) + lane;
+                nb = u < A.n ? A.ro[u] : 0u;
+                ne = u < A.n ? A.ro[u + 1] : 0u;
+            };
+            if (pending)
+                offsets();
+            while (pending) {
+                const uint32_t at = __ffs(pending) - 1;
+                pending &= pending - 1;
+                const uint32_t word = w0 + at * nwarps;
+                const uint32_t bits = __shfl_sync(0xFFFFFFFFu, mine, at);
+                const uint32_t b = nb, e = ne;
+                if (pending)
+                    offsets();
+                if ((bits >> lane) & 1u)
+                    A.levels[(word << 5) + lane] = i + 1;
+                const uint32_t total = __reduce_add_sync(0xFFFFFFFFu, row_slots(A, bits, lane, b, e));
+                const uint32_t pieces = (total + ITEM - 1) / ITEM;
+                uint32_t base = 0;
+                if (lane == 0)
+                    base = atomicAdd(&s_nit, pieces);
+                base = __shfl_sync(0xFFFFFFFFu, base, 0);
+                uint2 *list = s_items;
+                if (base + pieces > CTA_ITEMS) {
+                    // no room: to the grid's list, or, that being full too, left
+                    // to this warp's walk
+                    if (lane == 0) {
+                        atomicMin(&s_end, base);  // every later warp finds no room either
+                        base = atomicAdd(item_cnt, pieces);
+                    }
+                    base = __shfl_sync(0xFFFFFFFFu, base, 0);
+                    list = A.items;
+                    if (base + pieces > A.item_cap) {
+                        for (uint32_t c = base + lane; c < min(base + pieces, A.item_cap); c += 32)
+                            A.items[c] = make_uint2(0, SIZE_NONE);
+                        if (lane == 0) {
+                            A.over[word] = 1;
+                            atomicAdd(A.ctl + CTL_OVERFLOW, 1u);
+                        }
+                        continue;
+                    }
+                }
+                for (uint32_t c = lane; c < pieces; c += 32)
+                    list[base + c] = make_uint2(word, c);
+            }
+        }
+        brief = frontier <= SHORT_NODES * gridDim.x;
+        uint32_t *claims = brief ? A.claimed[i & 1] : A.seen;
+        count = __reduce_add_sync(0xFFFFFFFFu, count);
+        if (lane == 0)
+            s_cnt[warp] = count;
+        __syncthreads();
+        const uint32_t filled = min(s_nit, s_end), own = brief ? min(filled, SHORT_ITEMS) : 0u;
+        uint32_t kept = filled - own;  // for the grid's list, or, where that is full, for this CTA
+        if (threadIdx.x == 0) {
+            for (int w = 1; w < BLOCK / 32; ++w)
+                count += s_cnt[w];
+            if (count)
+                atomicAdd(A.ctl + CTL_CNT + i % 3, count);
+            s_at = kept ? atomicAdd(item_cnt, kept) : 0u;
+        }
+        __syncthreads();
+        if (s_at + kept <= A.item_cap) {
+            for (uint32_t c = threadIdx.x; c < kept; c += BLOCK)
+                A.items[s_at + c] = s_items[own + c];
+            kept = 0;
+        } else {
+            for (uint32_t c = s_at + threadIdx.x; c < min(s_at + kept, A.item_cap); c += BLOCK)
+                A.items[c] = make_uint2(0, SIZE_NONE);
+            if (threadIdx.x == 0)
+                atomicAdd(A.ctl + CTL_OVERFLOW, 1u);
+        }
+        // items c0, c0 + step, ... below c1
+        auto walk = [&](const uint2 *items, uint32_t c0, uint32_t step, uint32_t c1) {
+            for (uint32_t c = c0; c < c1; c += step) {
+                const uint2 it = items[c];
+                if (it.y == SIZE_NONE)
+                    continue;  // neutral
+                WordRows W;
+                W.load(A, it.x, lane);
+                walk_word(A, W, it.y * ITEM, (it.y + 1) * ITEM, lane, claims);
+            }
+        };
+        walk(s_items, warp, BLOCK / 32, own);
+        if (!grid_barrier_long(bar, err))
+            return;
+        frontier = cta_broadcast_read(A.ctl + CTL_CNT + i % 3);
+        if (frontier == 0)
+            break;
+        reached += frontier;
+        if (gtid == 0) {
+            // read last before this barrier, added to after the next one
+            A.ctl[CTL_CNT + (i + 2) % 3] = 0;
+            A.ctl[CTL_ITEMS + (i + 2) % 3] = 0;
+        }
+        const uint32_t nit = min(cta_broadcast_read(item_cnt), A.item_cap);
+        const bool overflow = cta_broadcast_read(A.ctl + CTL_OVERFLOW) != 0;
+        if (brief && nit == 0 && !overflow)
+            continue;
+        walk(A.items, gwarp, nwarps, nit);
+        walk(s_items, own + warp, BLOCK / 32, own + kept);
+        if (overflow) {
+            for (uint32_t w = gwarp; w < words; w += nwarps) {
+                if (!A.over[w])
+                    continue;
+                WordRows W;
+                W.load(A, w, lane);
+                walk_word(A, W, 0, SIZE_NONE, lane, claims);
+                __syncwarp();
+                if (lane == 0)
+                    A.over[w] = 0;
+            }
+        }
+        if (!grid_barrier_long(bar, err))
+            return;
+    }
+    report(A, i, blockIdx.x == 0 ? reached : 0u);
+}
+
+const void *bfs_kernel_ptr(uint32_t size, bool long_search = false) {
+    if (long_search)
+        return size >= LARGE_SLOTS ? (const void *)bfs_long_kernel<LARGE_ITEM_SLOTS>
+                                   : (const void *)bfs_long_kernel<ITEM_SLOTS>;
     return size >= LARGE_SLOTS ? (const void *)bfs_kernel<LARGE_ITEM_SLOTS> : (const void *)bfs_kernel<ITEM_SLOTS>;
 }
 
-// Resident CTAs per SM of either build.
+// Resident CTAs per SM of either build (of those for long searches,
+// LONG_CTAS_PER_SM by their launch bounds).
 cudaError_t bfs_fit(int *per_sm) {
     int large = 0;
-    cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(per_sm, bfs_kernel<ITEM_SLOTS>, BLOCK, 0);
+    cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(per_sm, bfs_kernel_ptr(0), BLOCK, 0);
     if (e == cudaSuccess)
-        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&large, bfs_kernel<LARGE_ITEM_SLOTS>, BLOCK, 0);
+        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&large, bfs_kernel_ptr(LARGE_SLOTS), BLOCK, 0);
     *per_sm = std::min(*per_sm, large);
     return e;
 }
@@ -523,12 +723,28 @@ void fill_maps(BfsArgs &A, uint32_t *maps, size_t words) {
     A.over = maps + 3 * words;
 }
 
+// The launch that goes on with a search after LONG_LEVELS levels, from its
+// arguments and two more maps; the control words are zero.
+cudaError_t launch_long(BfsArgs A, uint32_t *maps, size_t words, int sms, int per_sm, cudaStream_t s) {
+    A.claimed[0] = maps;
+    A.claimed[1] = maps + words;
+    A.gate = nullptr;
+    A.stamps = nullptr;
+    A.stall = 0;
+    A.stall_limit_ns = WAIT_LIMIT_NS;
+    void *params[] = {&A};
+    return cudaLaunchCooperativeKernel(bfs_kernel_ptr(A.size, true),
+                                       dim3(bfs_ctas(A.size, sms * std::min(per_sm, LONG_CTAS_PER_SM))), dim3(BLOCK),
+                                       params, 0, s);
+}
+
 }  // namespace
 
 void free_bfs(gpma_graph *g) {
     dev_free(g->bfs_levels);
     g->bfs_levels_cap = 0;
     dev_free(g->bfs_map);
+    dev_free(g->bfs_claimed);
     dev_free(g->bfs_items);
     g->bfs_item_cap = 0;
     dev_free(g->bfs_ctl);
@@ -587,7 +803,21 @@ gpma_status bfs_begin(gpma_graph *g, cudaStream_t s) {
     return GPMA_OK;
 }
 
-gpma_status bfs_finish(gpma_graph *g, uint64_t *reached) {
+gpma_status bfs_finish(gpma_graph *g, const BfsPlan &P, cudaStream_t s, uint64_t *reached) {
+    uint32_t before = 0;  // nodes reached by the first launch of a long search
+    if (g->h_bfs_ctl[CTL_ERR] == 0 && g->h_bfs_ctl[CTL_LEVELS] == LONG_LEVELS) {
+        before = g->h_bfs_ctl[CTL_REACHED];
+        BfsArgs A;
+        memcpy(&A, P.main.args, sizeof(A));
+        const size_t words = g->bfs_cap / 32 + 2;
+        if (!g->bfs_claimed)
+            GPMA_TRY(dev_alloc(&g->bfs_claimed, 2 * words));
+        g->h_bfs_ctl[CTL_ERR] = HOST_PENDING;
+        GPMA_CUDA(launch_long(A, g->bfs_claimed, words, g->sms, blocks_per_sm(g->bfs_grid, g_tuning.bfs_blocks_per_sm), s));
+        prof_mark(g, 1, s);
+        GPMA_CUDA(cudaStreamSynchronize(s));
+        g->prof.kernel_launches += 1;
+    }
     if (g->h_bfs_ctl[CTL_ERR] == HOST_PENDING) {
         // the kernel stopped before its end: its error word is on the device
         GPMA_CUDA(cudaMemcpy(g->h_bfs_ctl, g->bfs_ctl, sizeof(uint32_t) * CTL_WORDS, cudaMemcpyDeviceToHost));
@@ -597,7 +827,7 @@ gpma_status bfs_finish(gpma_graph *g, uint64_t *reached) {
     if (g->h_bfs_ctl[CTL_ERR])
         return device_error("the BFS kernel", g->h_bfs_ctl[CTL_ERR]);
     if (reached)
-        *reached = g->h_bfs_ctl[CTL_REACHED];
+        *reached = (uint64_t)before + g->h_bfs_ctl[CTL_REACHED];
     return GPMA_OK;
 }
 
@@ -616,8 +846,8 @@ gpma_status bfs_run(gpma_graph *g, uint32_t src, uint32_t *levels, cudaStream_t 
     GPMA_CUDA(cudaStreamSynchronize(s));
     g->prof.kernel_launches += 1;
     g->prof.bfs_kernels++;
+    GPMA_TRY(bfs_finish(g, P, s, reached));
     g->prof.bfs_ms += prof_elapsed(g, 0, 1);
-    GPMA_TRY(bfs_finish(g, reached));
     if (levels && !P.direct) {
         GPMA_TRY(copy_any(levels, g->bfs_levels, sizeof(uint32_t) * g->row_num, s));
         GPMA_CUDA(cudaStreamSynchronize(s));
@@ -629,16 +859,16 @@ gpma_status bfs_run(gpma_graph *g, uint32_t src, uint32_t *levels, cudaStream_t 
 // Some callers cannot allocate device memory on the fly: code that runs under
 // a host-side memory arena or a fixed device-memory budget, plug-ins whose
 // host process owns every cudaMalloc, or hosts whose pool forbids growth once
-// serving starts. For them gpma_bfs_noalloc keeps the BFS working set (four
+// serving starts. For them gpma_bfs_noalloc keeps the BFS working set (six
 // bitmaps, item list, control words) in one file-scope device array
 // of a fixed size instead of buffers allocated per graph. Every GPU that loads
-// this library holds the array (about 1.6 MB) until the process exits.
+// this library holds the array (about 2.1 MB) until the process exits.
 namespace {
 
 constexpr uint32_t NOALLOC_MAX_ROWS = 1u << 21;  // 2,097,152 nodes
 constexpr uint32_t NOALLOC_BITMAP_WORDS = NOALLOC_MAX_ROWS / 32 + 2;
 constexpr uint32_t NOALLOC_ITEM_CAP = 1u << 16;  // further items stay with the CTA that found them
-constexpr size_t NOALLOC_WORDS = CTL_ALL + (size_t)BFS_MAPS * NOALLOC_BITMAP_WORDS + 2ull * NOALLOC_ITEM_CAP;
+constexpr size_t NOALLOC_WORDS = CTL_ALL + (size_t)(BFS_MAPS + 2) * NOALLOC_BITMAP_WORDS + 2ull * NOALLOC_ITEM_CAP;
 constexpr int NOALLOC_MAX_DEVICES = 64;
 
 static __device__ __align__(256) uint32_t g_noalloc_scratch[NOALLOC_WORDS];
@@ -704,7 +934,7 @@ gpma_status bfs_noalloc_run(gpma_graph *g, uint32_t src, uint32_t *levels, uint6
     A.levels = levels;
     A.src = src;
     fill_maps(A, maps, NOALLOC_BITMAP_WORDS);
-    A.items = reinterpret_cast<uint2 *>(maps + (size_t)BFS_MAPS * NOALLOC_BITMAP_WORDS);
+    A.items = reinterpret_cast<uint2 *>(maps + (size_t)(BFS_MAPS + 2) * NOALLOC_BITMAP_WORDS);
     A.item_cap = g_test_hooks.noalloc_chunk_cap ? std::min(g_test_hooks.noalloc_chunk_cap, NOALLOC_ITEM_CAP)
                                                 : NOALLOC_ITEM_CAP;
     A.ctl = ctl;
@@ -714,14 +944,23 @@ gpma_status bfs_noalloc_run(gpma_graph *g, uint32_t src, uint32_t *levels, uint6
     A.stall_limit_ns = g_test_hooks.bfs_stall ? g_test_hooks.wait_limit_ns : WAIT_LIMIT_NS;
     void *params[] = {&A};
     GPMA_CUDA(cudaLaunchCooperativeKernel(bfs_kernel_ptr(A.size), dim3(bfs_ctas(A.size, grid)), dim3(BLOCK), params, 0, s));
-    uint32_t h_ctl[CTL_WORDS];
+    uint32_t h_ctl[CTL_WORDS], before = 0;
     GPMA_CUDA(cudaMemcpyAsync(h_ctl, ctl, sizeof(h_ctl), cudaMemcpyDeviceToHost, s));
     GPMA_CUDA(cudaStreamSynchronize(s));
+    if (!h_ctl[CTL_ERR] && h_ctl[CTL_LEVELS] == LONG_LEVELS) {
+        before = h_ctl[CTL_REACHED];
+        const uint32_t overflows = h_ctl[CTL_OVERFLOW];
+        GPMA_CUDA(cudaMemsetAsync(ctl, 0, sizeof(uint32_t) * CTL_ALL, s));
+        GPMA_CUDA(launch_long(A, maps + (size_t)BFS_MAPS * NOALLOC_BITMAP_WORDS, NOALLOC_BITMAP_WORDS, g->sms, grid / g->sms, s));
+        GPMA_CUDA(cudaMemcpyAsync(h_ctl, ctl, sizeof(h_ctl), cudaMemcpyDeviceToHost, s));
+        GPMA_CUDA(cudaStreamSynchronize(s));
+        h_ctl[CTL_OVERFLOW] += overflows;
+    }
     g_test_hooks.noalloc_overflows = h_ctl[CTL_OVERFLOW];
     if (h_ctl[CTL_ERR])
         return device_error("the BFS kernel", h_ctl[CTL_ERR]);
     if (reached)
-        *reached = h_ctl[CTL_REACHED];
+        *reached = (uint64_t)before + h_ctl[CTL_REACHED];
     return GPMA_OK;
 }
 

@@ -87,7 +87,7 @@ extern TestHooks g_test_hooks;
 // the start of a launch, on a 128-byte line of its own, apart from the words
 // that kernels count in.
 struct alignas(128) GridBarrier {
-    unsigned int count;  // tickets taken, modulo BARRIER_ROUNDS rounds
+    unsigned int count;  // tickets taken
 };
 constexpr uint32_t BAR_WORDS = sizeof(GridBarrier) / sizeof(uint32_t);
 constexpr uint32_t BAR_ALIGN_WORDS = 32;
@@ -240,6 +240,7 @@ struct gpma_graph {
     // BFS state
     uint32_t bfs_cap = 0;
     uint32_t *bfs_map = nullptr;       // BFS_MAPS bitmaps of row_num/32 + 2 words
+    uint32_t *bfs_claimed = nullptr;   // two more of them, for searches of many levels
     uint2 *bfs_items = nullptr;        // work items of a level
     uint32_t bfs_item_cap = 0;         // its entries, as many as one level can queue
     uint32_t *bfs_levels = nullptr;    // levels on their way to host memory
@@ -474,7 +475,7 @@ struct BfsPlan {
 };
 gpma_status bfs_plan(gpma_graph *g, uint32_t src, uint32_t *levels, BfsPlan *P, const unsigned char *gate = nullptr);
 gpma_status bfs_begin(gpma_graph *g, cudaStream_t s);
-gpma_status bfs_finish(gpma_graph *g, uint64_t *reached);
+gpma_status bfs_finish(gpma_graph *g, const BfsPlan &P, cudaStream_t s, uint64_t *reached);
 gpma_status bfs_noalloc_run(gpma_graph *g, uint32_t src, uint32_t *levels, uint64_t *reached, cudaStream_t s);
 gpma_status batch_bfs_run(gpma_batch *b, gpma_graph *const *graphs, const uint32_t *const *srcs, const uint32_t *nsrc,
                           uint32_t k, uint32_t *const *levels, uint64_t *reached, cudaStream_t s);
@@ -574,10 +575,6 @@ __device__ __forceinline__ bool in_bounds(uint32_t *err, bool ok, uint32_t site)
 // ticket from one counter (it must start each launch at zero) and waits until
 // the counter reaches the end of its ticket's round of gridDim.x; there is no
 // separate release write, so a barrier costs one atomic per CTA and polling.
-// The counter goes back to zero after BARRIER_ROUNDS rounds: 2^32 tickets are a
-// search of a few million levels, and would end a round of most grids early.
-// (A round's end kept per CTA in place of the ticket's: the social BFS 345 -> 368
-// us, as the CTAs poll sooner, and 353 with the arrival's count as the first poll.)
 // The polls are relaxed loads back to back, with one acquire at the end (an
 // acquire per poll drops the L1 lines of the CTAs still at work on the SM); the
 // error word and the clock are looked at in every 8th poll only. Alone, per
@@ -587,6 +584,11 @@ __device__ __forceinline__ bool in_bounds(uint32_t *err, bool ok, uint32_t site)
 // round trips); a fence in place of the acquire +0.4 us. Every wait is bounded:
 // after WAIT_LIMIT_NS the CTA records DERR_BARRIER_TIMEOUT and returns false;
 // CTAs that see an error stop waiting.
+// Searches and iterations without a bound use grid_barrier_long, whose counter goes
+// back to zero after BARRIER_ROUNDS rounds: 2^32 tickets are a few million levels,
+// and would end a round of most grids early. (With it everywhere the social BFS
+// took 357 us in place of 348; a round's end kept per CTA in place of the ticket's
+// 368, as the CTAs poll sooner, and 353 with the arrival's count as the first poll.)
 constexpr uint32_t BARRIER_ROUNDS = 1u << 16;
 static_assert((uint64_t)BARRIER_ROUNDS * 0xFFFF <= 0xFFFFFFFFull, "tickets of any grid fit 32 bits");
 struct BarrierRound {
@@ -595,25 +597,30 @@ struct BarrierRound {
     uint32_t ticket, end;
     __host__ __device__ __forceinline__ BarrierRound(uint32_t ticket_, uint32_t ctas, uint32_t extra = 0)
         : ticket(ticket_), end((ticket_ / ctas + 1) * ctas + extra) {}
+    __host__ __device__ __forceinline__ bool over(uint32_t count) const { return (int)(count - end) >= 0; }
     // The count of this launch has passed the ticket: where it has not, it has
     // started over, with the end of this round or since.
-    __host__ __device__ __forceinline__ bool over(uint32_t count) const { return count >= end || count <= ticket; }
+    __host__ __device__ __forceinline__ bool over_long(uint32_t count) const {
+        return count >= end || count <= ticket;
+    }
 };
 
 // `extra` (test hooks only, 0 otherwise) adds arrivals that never come, so the
 // wait runs out after `limit_ns`.
-__device__ __forceinline__ bool grid_barrier(GridBarrier *bar, uint32_t *err, uint32_t extra = 0,
-                                             uint64_t limit_ns = WAIT_LIMIT_NS) {
+template <bool LONG>
+__device__ __forceinline__ bool grid_barrier_any(GridBarrier *bar, uint32_t *err, uint32_t extra, uint64_t limit_ns) {
     __syncthreads();
     __shared__ uint32_t s_ok;
     if (threadIdx.x == 0) {
         __threadfence();
-        const BarrierRound round(atomicInc(&bar->count, BarrierRound::last_ticket(gridDim.x)), gridDim.x, extra);
+        const uint32_t ticket =
+            LONG ? atomicInc(&bar->count, BarrierRound::last_ticket(gridDim.x)) : atomicAdd(&bar->count, 1u);
+        const BarrierRound round(ticket, gridDim.x, extra);
         uint64_t t0 = 0;
         uint32_t polls = 0, c;
         for (;;) {
             asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(c) : "l"(&bar->count) : "memory");
-            if (round.over(c))
+            if (LONG ? round.over_long(c) : round.over(c))
                 break;
             if ((++polls & 7u) == 0) {
                 if (ld_volatile(err) != 0)
@@ -635,6 +642,14 @@ __device__ __forceinline__ bool grid_barrier(GridBarrier *bar, uint32_t *err, ui
     }
     __syncthreads();
     return s_ok != 0;
+}
+
+__device__ __forceinline__ bool grid_barrier(GridBarrier *bar, uint32_t *err, uint32_t extra = 0,
+                                             uint64_t limit_ns = WAIT_LIMIT_NS) {
+    return grid_barrier_any<false>(bar, err, extra, limit_ns);
+}
+__device__ __forceinline__ bool grid_barrier_long(GridBarrier *bar, uint32_t *err) {
+    return grid_barrier_any<true>(bar, err, 0, WAIT_LIMIT_NS);
 }
 
 // One volatile read per CTA, broadcast through shared memory: a word that

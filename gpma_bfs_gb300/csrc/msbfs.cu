@@ -350,17 +350,17 @@ __global__ void __launch_bounds__(BLOCK) msbfs_kernel(MsArgs A) {
     unsigned long long traversed = 0;
     for (uint32_t w = gtid; w < N; w += nthreads)
         seen[w] = 0;
-    if (!grid_barrier(bar, err))
+    if (!grid_barrier_long(bar, err))
         return;
     for (uint32_t t = gtid; t < A.G * 64; t += nthreads) {
         const uint32_t g = t >> 6, j = t & 63;
         if (j < A.gr[g].nsrc)
             mask_or(&seen[A.voff[g] + A.src[t]], M(1) << j);
     }
-    if (!grid_barrier(bar, err))
+    if (!grid_barrier_long(bar, err))
         return;
     ms_commit<M>(A, 1, N, gwarp, nwarps, lane);
-    if (!grid_barrier(bar, err))
+    if (!grid_barrier_long(bar, err))
         return;
     uint32_t level = 1;
     for (;; ++level) {
@@ -485,7 +485,7 @@ __global__ void __launch_bounds__(BLOCK) msbfs_kernel(MsArgs A) {
             for (uint32_t c = threadIdx.x; c < mine; c += BLOCK)
                 if (in_bounds(err, s_nch + c < A.chunk_cap, BS_ROW))  // the list holds every level's chunks
                     A.chunks[s_nch + c] = s_chunks[c];
-            if (!grid_barrier(bar, err))
+            if (!grid_barrier_long(bar, err))
                 return;
         }
         // expand, phase 2: long-row chunks
@@ -509,10 +509,10 @@ __global__ void __launch_bounds__(BLOCK) msbfs_kernel(MsArgs A) {
             }
             traversed += ms_visit<M, MS_LANE_SLOTS>(seen, gr, cvo, sl, fm);
         }
-        if (!grid_barrier(bar, err))
+        if (!grid_barrier_long(bar, err))
             return;
         ms_commit<M>(A, level + 1, N, gwarp, nwarps, lane);
-        if (!grid_barrier(bar, err))
+        if (!grid_barrier_long(bar, err))
             return;
         if (cta_broadcast_read(A.ctl + MS_CHANGE + level % 3) == 0)
             break;

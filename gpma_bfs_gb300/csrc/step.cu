@@ -241,7 +241,7 @@ gpma_status step_run(gpma_step *st, const uint64_t *keys, const uint8_t *values,
             GPMA_TRY(bfs_run(g, src, levels, s, reached));
             levels = nullptr;
         } else {
-            GPMA_TRY(bfs_finish(g, reached));
+            GPMA_TRY(bfs_finish(g, bp, s, reached));
         }
         if (bp.direct)
             levels = nullptr;

@@ -105,9 +105,9 @@ GPMA_API gpma_status gpma_bfs_multi(gpma_graph *g, const uint32_t *srcs, uint32_
 /* BFS for callers that cannot allocate device memory (a host-side arena or a
  * fixed device budget owns every allocation, or allocation is forbidden
  * while serving). No counterpart in the reference. Same result as gpma_bfs,
- * but it allocates nothing: its working set (four node bitmaps, the list
+ * but it allocates nothing: its working set (six node bitmaps, the list
  * of work items, control words) is one fixed device array inside the library,
- * about 1.6 MB. A device commits it when the library's kernels are
+ * about 2.1 MB. A device commits it when the library's kernels are
  * first used there (CUDA loads modules lazily by default) and holds it until
  * the process exits. Work items that find the list (65,536 entries) full are
  * walked by the CTA that found them: slower, same result.

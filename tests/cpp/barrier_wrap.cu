@@ -21,19 +21,19 @@ int main() {
                     waiting.emplace_back(ticket, ctas);
                     // the first, the last and one waiting CTA between them
                     for (const uint32_t w : {0u, c / 2, c})
-                        if (waiting[w].over(count) != (c == ctas - 1))
+                        if (waiting[w].over_long(count) != (c == ctas - 1))
                             return std::printf("%u CTAs, round %d: CTA %u after arrival %u\n", ctas, round, w, c), 1;
                 }
                 // a slow poll still sees the end while others take the next round's tickets
                 for (uint32_t ahead = 0; ahead < ctas; ++ahead)
-                    if (!waiting[0].over(count + ahead))
+                    if (!waiting[0].over_long(count + ahead))
                         return std::printf("%u CTAs, round %d: lost after %u\n", ctas, round, ahead), 1;
             }
         }
     }
     // arrivals that never come keep a round open
     const gpma::BarrierRound stalled(303, 304, 1);
-    if (stalled.over(304))
+    if (stalled.over(304) || stalled.over_long(304))
         return std::puts("a stalled round ended"), 1;
     std::puts("ok");
     return 0;
