@@ -11,8 +11,8 @@
 // PageRank (y = d * A^T (x / deg) + teleport): per iteration
 //   contrib[u] = rank[u] / outdeg[u] (dangling nodes pool their rank),
 //   acc[v]     = sum of contrib[u] over the edges u -> v (gathered from the
-//                in-edges laid out at the start of the call, or, in calls of
-//                few iterations, by float atomics),
+//                in-edges laid out once per call, or, for few iterations,
+//                by float atomics),
 //   rank'[v]   = (1 - d) / n + d * (acc[v] + dangling / n);
 // it stops after `iterations` or when sum |rank' - rank| < tol.
 // Weakly connected components: parents start as the node ids; an edge links
@@ -120,25 +120,20 @@ __device__ __forceinline__ bool an_barrier(GridBarrier *bar, uint32_t *err) {
     return LONG ? grid_barrier_long(bar, err) : grid_barrier(bar, err);
 }
 
+// Ranks, degrees and sums of a call's start, and the out-degrees: slots are sorted
+// by source, so a thread's 8 slots form a few runs of one source, with one atomic
+// each. False when a barrier gave up.
 template <bool LONG>
-__global__ void __launch_bounds__(BLOCK) pagerank_kernel(AnArgs A) {
-    GridBarrier *bar = reinterpret_cast<GridBarrier *>(A.ctl + AN_BAR);
+__device__ __forceinline__ bool pr_begin(const AnArgs &A, GridBarrier *bar, uint32_t gtid, uint32_t nthreads) {
     uint32_t *err = A.ctl + AN_ERR;
-    __shared__ double tmp[BLOCK / 32];
-    __shared__ double s_val;
-    const uint32_t gtid = blockIdx.x * BLOCK + threadIdx.x, nthreads = gridDim.x * BLOCK;
-    const uint32_t groups = A.size >> 3;
-    const float teleport = (1.0f - A.damping) / (float)A.n;
-    // out-degrees: slots are sorted by source, so a thread's 8 slots form a few
-    // runs of one source; one atomic per run
     for (uint32_t v = gtid; v < A.n; v += nthreads) {
         A.deg[v] = 0;
         A.rank[v] = 1.0f / (float)A.n;
         A.acc[v] = 0.0f;
     }
     if (!an_barrier<LONG>(bar, err))
-        return;
-    for (uint32_t o = gtid; o < groups || (A.size < 8 && o == 0); o += nthreads) {
+        return false;
+    for (uint32_t o = gtid; o < A.size >> 3 || (A.size < 8 && o == 0); o += nthreads) {
         uint32_t u[8], v[8];
         bool e[8];
         if (A.size < 8)
@@ -163,67 +158,91 @@ __global__ void __launch_bounds__(BLOCK) pagerank_kernel(AnArgs A) {
         if (A.size < 8)
             break;
     }
+    return an_barrier<LONG>(bar, err);
+}
+
+// Iteration `it` by adding every edge's contribution; the change of the ranks, the
+// same in every thread of the grid, or a negative number when a barrier gave up.
+template <bool LONG>
+__device__ __forceinline__ double pr_push(const AnArgs &A, GridBarrier *bar, uint32_t it, uint32_t gtid,
+                                          uint32_t nthreads, double *tmp, double &s_val) {
+    uint32_t *err = A.ctl + AN_ERR;
+    const float teleport = (1.0f - A.damping) / (float)A.n;
+    if (gtid == 0) {
+        *an_dbl(A, 0, it + 1) = 0.0;  // next iteration's sums start at zero
+        *an_dbl(A, 1, it + 1) = 0.0;
+    }
+    double dang = 0;
+    for (uint32_t v = gtid; v < A.n; v += nthreads) {
+        const uint32_t d = A.deg[v];
+        const float r = A.rank[v];
+        A.contrib[v] = d ? r / (float)d : 0.0f;
+        if (!d)
+            dang += r;
+    }
+    dang = block_sum_f64(dang, tmp);
+    if (threadIdx.x == 0 && dang != 0.0)
+        atomicAdd(an_dbl(A, 0, it), dang);
     if (!an_barrier<LONG>(bar, err))
+        return -1.0;
+    for (uint32_t o = gtid; o < A.size >> 3 || (A.size < 8 && o == 0); o += nthreads) {
+        uint32_t u[8], v[8];
+        bool e[8];
+        if (A.size < 8)
+            load_small(A, u, v, e);
+        else
+            load8(A, o, u, v, e);
+        float c[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j)
+            c[j] = e[j] ? A.contrib[u[j]] : 0.0f;
+#pragma unroll
+        for (int j = 0; j < 8; ++j)
+            if (e[j] && c[j] != 0.0f)
+                atomicAdd(&A.acc[v[j]], c[j]);
+        if (A.size < 8)
+            break;
+    }
+    if (!an_barrier<LONG>(bar, err))
+        return -1.0;
+    if (threadIdx.x == 0)
+        s_val = *reinterpret_cast<volatile double *>(an_dbl(A, 0, it));
+    __syncthreads();
+    const float base = teleport + A.damping * (float)(s_val / (double)A.n);
+    double delta = 0;
+    for (uint32_t v = gtid; v < A.n; v += nthreads) {
+        const float nr = base + A.damping * A.acc[v];
+        delta += fabs((double)nr - (double)A.rank[v]);
+        A.rank[v] = nr;
+        A.acc[v] = 0.0f;
+    }
+    delta = block_sum_f64(delta, tmp);
+    if (threadIdx.x == 0)
+        atomicAdd(an_dbl(A, 1, it), delta);
+    if (!an_barrier<LONG>(bar, err))
+        return -1.0;
+    if (threadIdx.x == 0)
+        s_val = *reinterpret_cast<volatile double *>(an_dbl(A, 1, it));
+    __syncthreads();
+    delta = s_val;
+    __syncthreads();  // s_val is written again
+    return delta;
+}
+
+template <bool LONG>
+__global__ void __launch_bounds__(BLOCK) pagerank_kernel(AnArgs A) {
+    GridBarrier *bar = reinterpret_cast<GridBarrier *>(A.ctl + AN_BAR);
+    __shared__ double tmp[BLOCK / 32];
+    __shared__ double s_val;
+    const uint32_t gtid = blockIdx.x * BLOCK + threadIdx.x, nthreads = gridDim.x * BLOCK;
+    if (!pr_begin<LONG>(A, bar, gtid, nthreads))
         return;
     uint32_t it = 0;
     for (; it < A.max_iter; ++it) {
-        if (blockIdx.x == 0 && threadIdx.x == 0) {
-            *an_dbl(A, 0, it + 1) = 0.0;  // next iteration's sums start at zero
-            *an_dbl(A, 1, it + 1) = 0.0;
-        }
-        double dang = 0;
-        for (uint32_t v = gtid; v < A.n; v += nthreads) {
-            const uint32_t d = A.deg[v];
-            const float r = A.rank[v];
-            A.contrib[v] = d ? r / (float)d : 0.0f;
-            if (!d)
-                dang += r;
-        }
-        dang = block_sum_f64(dang, tmp);
-        if (threadIdx.x == 0 && dang != 0.0)
-            atomicAdd(an_dbl(A, 0, it), dang);
-        if (!an_barrier<LONG>(bar, err))
+        const double delta = pr_push<LONG>(A, bar, it, gtid, nthreads, tmp, s_val);
+        if (delta < 0.0)
             return;
-        for (uint32_t o = gtid; o < groups || (A.size < 8 && o == 0); o += nthreads) {
-            uint32_t u[8], v[8];
-            bool e[8];
-            if (A.size < 8)
-                load_small(A, u, v, e);
-            else
-                load8(A, o, u, v, e);
-            float c[8];
-#pragma unroll
-            for (int j = 0; j < 8; ++j)
-                c[j] = e[j] ? A.contrib[u[j]] : 0.0f;
-#pragma unroll
-            for (int j = 0; j < 8; ++j)
-                if (e[j] && c[j] != 0.0f)
-                    atomicAdd(&A.acc[v[j]], c[j]);
-            if (A.size < 8)
-                break;
-        }
-        if (!an_barrier<LONG>(bar, err))
-            return;
-        if (threadIdx.x == 0)
-            s_val = *reinterpret_cast<volatile double *>(an_dbl(A, 0, it));
-        __syncthreads();
-        const float base = teleport + A.damping * (float)(s_val / (double)A.n);
-        double delta = 0;
-        for (uint32_t v = gtid; v < A.n; v += nthreads) {
-            const float nr = base + A.damping * A.acc[v];
-            delta += fabs((double)nr - (double)A.rank[v]);
-            A.rank[v] = nr;
-            A.acc[v] = 0.0f;
-        }
-        delta = block_sum_f64(delta, tmp);
-        if (threadIdx.x == 0)
-            atomicAdd(an_dbl(A, 1, it), delta);
-        if (!an_barrier<LONG>(bar, err))
-            return;
-        if (threadIdx.x == 0)
-            s_val = *reinterpret_cast<volatile double *>(an_dbl(A, 1, it));
-        __syncthreads();
-        if (s_val < A.tol) {
+        if (delta < A.tol) {
             ++it;
             break;
         }
@@ -242,6 +261,15 @@ __global__ void __launch_bounds__(BLOCK) pagerank_kernel(AnArgs A) {
 constexpr uint32_t PR_STEP = 8;
 constexpr uint32_t PR_SHORT = 64;
 constexpr uint32_t PR_CHUNK = 4096;
+// PageRank calls of at least PR_GATHER_ITERATIONS iterations lay out the
+// in-edges first (one count and one scatter sweep with an atomic per edge):
+// social graph, 3 / 4 / 5 iterations, adding per edge 734 / 930 / 1130 us,
+// gathering 738 / 812 / 883 us; R-MAT scale 14 123 / 150 / 178 against 118 /
+// 126 / 136 us.
+constexpr uint32_t PR_GATHER_ITERATIONS = 4;
+// How far the ranks' change falls from the first iteration to the second, about
+// (R-MAT graphs 0.35, the social graph 0.47, uniformly random ones 0.2).
+constexpr double PR_FALL = 0.4;
 
 // New rank, next contribution and this thread's share of the sums of node v.
 struct PrNode {
@@ -266,7 +294,12 @@ struct PrNode {
 // float atomic per edge (198 us per iteration). Bound by the 4-byte gathers of
 // the contributions (L2). 20 iterations on the social graph: 4.37 ms -> 1.99 ms
 // per call, 0.44 of it the layout.
-template <bool LONG>
+// TOL (a tolerance is given): the iterations are not known beforehand. The call begins
+// with iterations by atomics, and lays out the in-edges after the first one from which
+// PR_GATHER_ITERATIONS more are to be expected: R-MAT 18, tolerance 0.5 (2 iterations)
+// 402 us with the layout at once, 315 so, 313 by atomics alone; 1e-2 (6 iterations)
+// 597, 708 and 822.
+template <bool LONG, bool TOL>
 __global__ void __launch_bounds__(BLOCK) pagerank_gather_kernel(AnArgs A) {
     GridBarrier *bar = reinterpret_cast<GridBarrier *>(A.ctl + AN_BAR);
     uint32_t *err = A.ctl + AN_ERR;
@@ -278,33 +311,71 @@ __global__ void __launch_bounds__(BLOCK) pagerank_gather_kernel(AnArgs A) {
     const uint32_t gwarp = gtid >> 5, nwarps = nthreads >> 5;
     const uint32_t groups = A.size >> 3;
     const float teleport = (1.0f - A.damping) / (float)A.n;
-    for (uint32_t v = gtid; v < A.n; v += nthreads) {
-        A.deg[v] = 0;
-        A.end[v] = 0;
-    }
-    if (!an_barrier<LONG>(bar, err))
-        return;
-    // out-degrees (one atomic per run of a source) and in-degrees
-    for (uint32_t o = gtid; o < groups; o += nthreads) {
-        uint32_t u[8], v[8];
-        bool e[8];
-        load8(A, o, u, v, e);
-        uint32_t run_u = 0xFFFFFFFFu, run = 0;
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            if (!e[j])
-                continue;
-            if (u[j] != run_u) {
-                if (run)
-                    atomicAdd(&A.deg[run_u], run);
-                run_u = u[j];
-                run = 0;
+    uint32_t first = 0;  // iterations done before the layout
+    if constexpr (TOL) {
+        for (uint32_t v = gtid; v < A.n; v += nthreads)
+            A.end[v] = 0;
+        if (!pr_begin<LONG>(A, bar, gtid, nthreads))
+            return;
+        for (double last = 0.0;;) {
+            const double delta = pr_push<LONG>(A, bar, first, gtid, nthreads, tmp, s_val);
+            if (delta < 0.0)
+                return;
+            ++first;
+            if (delta < A.tol || first == A.max_iter) {
+                if (gtid == 0)
+                    A.ctl[AN_ITERS] = first;
+                return;
             }
-            ++run;
-            atomicAdd(&A.end[v[j]], 1u);
+            // iterations to come, if the change goes on falling as it did
+            const double fall = first == 1 ? PR_FALL : delta / last;
+            uint32_t more = 0;
+            for (double x = delta; x >= A.tol && more < PR_GATHER_ITERATIONS; x *= fall)
+                ++more;
+            if (more == PR_GATHER_ITERATIONS && A.max_iter - first >= PR_GATHER_ITERATIONS)
+                break;
+            last = delta;
         }
-        if (run)
-            atomicAdd(&A.deg[run_u], run);
+        if (gtid == 0)
+            *an_dbl(A, 0, first + 1) = 0.0;
+        for (uint32_t o = gtid; o < groups; o += nthreads) {
+            uint32_t u[8], v[8];
+            bool e[8];
+            load8(A, o, u, v, e);
+#pragma unroll
+            for (int j = 0; j < 8; ++j)
+                if (e[j])
+                    atomicAdd(&A.end[v[j]], 1u);
+        }
+    } else {
+        for (uint32_t v = gtid; v < A.n; v += nthreads) {
+            A.deg[v] = 0;
+            A.end[v] = 0;
+        }
+        if (!an_barrier<LONG>(bar, err))
+            return;
+        // out-degrees (one atomic per run of a source) and in-degrees
+        for (uint32_t o = gtid; o < groups; o += nthreads) {
+            uint32_t u[8], v[8];
+            bool e[8];
+            load8(A, o, u, v, e);
+            uint32_t run_u = 0xFFFFFFFFu, run = 0;
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                if (!e[j])
+                    continue;
+                if (u[j] != run_u) {
+                    if (run)
+                        atomicAdd(&A.deg[run_u], run);
+                    run_u = u[j];
+                    run = 0;
+                }
+                ++run;
+                atomicAdd(&A.end[v[j]], 1u);
+            }
+            if (run)
+                atomicAdd(&A.deg[run_u], run);
+        }
     }
     if (!an_barrier<LONG>(bar, err))
         return;
@@ -318,17 +389,19 @@ __global__ void __launch_bounds__(BLOCK) pagerank_gather_kernel(AnArgs A) {
         for (uint32_t v = lo + threadIdx.x; v < hi; v += BLOCK) {
             const uint32_t d = A.deg[v];
             in += A.end[v];
-            A.rank[v] = r0;
-            A.contrib[v] = d ? r0 / (float)d : 0.0f;
+            const float r = TOL ? A.rank[v] : r0;
+            if (!TOL)
+                A.rank[v] = r0;
+            A.contrib[v] = d ? r / (float)d : 0.0f;
             if (!d)
-                dang += r0;
+                dang += r;
         }
         in = block_sum(in, utmp);
         dang = block_sum_f64(dang, tmp);
         if (threadIdx.x == 0) {
             A.cta[blockIdx.x] = in;
             if (dang != 0.0)
-                atomicAdd(an_dbl(A, 0, 0), dang);
+                atomicAdd(an_dbl(A, 0, first), dang);
         }
     }
     if (!an_barrier<LONG>(bar, err))
@@ -378,7 +451,7 @@ __global__ void __launch_bounds__(BLOCK) pagerank_gather_kernel(AnArgs A) {
     if (!an_barrier<LONG>(bar, err))
         return;
     const uint32_t nch = cta_broadcast_read(A.ctl + AN_CHUNKS), nmulti = cta_broadcast_read(A.ctl + AN_MULTI);
-    uint32_t it = 0;
+    uint32_t it = first;
     for (; it < A.max_iter; ++it) {
         if (gtid == 0) {
             *an_dbl(A, 0, it + 2) = 0.0;  // the sums of the iteration after next / of the next start at zero
@@ -387,12 +460,12 @@ __global__ void __launch_bounds__(BLOCK) pagerank_gather_kernel(AnArgs A) {
         if (threadIdx.x == 0)
             s_val = *reinterpret_cast<volatile double *>(an_dbl(A, 0, it));
         __syncthreads();
-        const float *cur = it & 1 ? A.acc : A.contrib;
+        const float *cur = (it - first) & 1 ? A.acc : A.contrib;
         PrNode P;
         P.base = teleport + A.damping * (float)(s_val / (double)A.n);
         P.damping = A.damping;
-        P.next = it & 1 ? A.contrib : A.acc;
-        P.want_delta = A.tol > 0.0;
+        P.next = (it - first) & 1 ? A.contrib : A.acc;
+        P.want_delta = TOL;
         P.dang = P.delta = 0.0;
         for (uint32_t c = gwarp; c < nch; c += nwarps) {
             const uint4 ch = A.chunks[c];
@@ -635,15 +708,23 @@ __global__ void __launch_bounds__(BLOCK) components_kernel(AnArgs A) {
 }
 
 // Rows of the fit table: the kernels of this file.
-enum AnKernel { AN_PAGERANK, AN_PAGERANK_GATHER, AN_PAGERANK_LONG, AN_PAGERANK_GATHER_LONG, AN_COMPONENTS, AN_KERNELS };
+enum AnKernel {
+    AN_PAGERANK,
+    AN_PAGERANK_GATHER,
+    AN_PAGERANK_LONG,
+    AN_PAGERANK_GATHER_LONG,
+    AN_PAGERANK_TOL,
+    AN_COMPONENTS,
+    AN_KERNELS
+};
 int an_fit[64][AN_KERNELS] = {};  // resident CTAs per SM, per device
 
 gpma_status launch(AnKernel which, AnArgs &A, int sms, cudaStream_t s, uint32_t *h_ctl) {
     const void *const kernels[AN_KERNELS] = {
-        (const void *)pagerank_kernel<false>, (const void *)pagerank_gather_kernel<false>,
-        (const void *)pagerank_kernel<true>, (const void *)pagerank_gather_kernel<true>,
-        (const void *)components_kernel};
-    if (A.max_iter > SHORT_CALL && which != AN_COMPONENTS)
+        (const void *)pagerank_kernel<false>,      (const void *)pagerank_gather_kernel<false, false>,
+        (const void *)pagerank_kernel<true>,       (const void *)pagerank_gather_kernel<true, false>,
+        (const void *)pagerank_gather_kernel<true, true>, (const void *)components_kernel};
+    if (A.max_iter > SHORT_CALL && which <= AN_PAGERANK_GATHER)
         which = which == AN_PAGERANK ? AN_PAGERANK_LONG : AN_PAGERANK_GATHER_LONG;
     const void *kernel = kernels[which];
     int dev = 0;
@@ -686,13 +767,7 @@ gpma_status an_buffers(gpma_graph *g, uint32_t **base, uint32_t **ctl) {
     return GPMA_OK;
 }
 
-// PageRank calls of at least PR_GATHER_ITERATIONS iterations lay out the
-// in-edges first (one count and one scatter sweep with an atomic per edge):
-// social graph, 3 / 4 / 5 iterations, adding per edge 734 / 930 / 1130 us,
-// gathering 738 / 812 / 883 us; R-MAT scale 14 123 / 150 / 178 against 118 /
-// 126 / 136 us. Arrays of 8 slots or more are a whole number of the sweeps'
-// slot groups.
-constexpr uint32_t PR_GATHER_ITERATIONS = 4;
+// Arrays of 8 slots or more are a whole number of the sweeps' slot groups.
 constexpr uint32_t PR_GATHER_MIN_SLOTS = 1024;
 
 }  // namespace
@@ -745,7 +820,7 @@ gpma_status gpma_pagerank(gpma_graph *g, float damping, uint32_t iterations, dou
             A.multi = reinterpret_cast<uint2 *>(A.csc + g->geo.size + g->geo.size / 2);
         }
         prof_mark(g, 0, s);
-        GPMA_TRY(launch(gather ? AN_PAGERANK_GATHER : AN_PAGERANK, A, g->sms, s, h_ctl));
+        GPMA_TRY(launch(!gather ? AN_PAGERANK : tol > 0.0 ? AN_PAGERANK_TOL : AN_PAGERANK_GATHER, A, g->sms, s, h_ctl));
         prof_mark(g, 1, s);
         GPMA_TRY(copy_any(ranks, rank, sizeof(float) * n, s));
         GPMA_CUDA(cudaStreamSynchronize(s));
