@@ -2633,8 +2633,9 @@ GraphDesc describe(const gpma_graph *g) {
     return d;
 }
 
-// One graph's batches of this many keys are sorted by digit passes.
-constexpr uint64_t DIGIT_KEYS = 1u << 22;
+// One graph's batches of this many keys are sorted by digit passes, and loads of
+// this many.
+constexpr uint64_t DIGIT_KEYS = 1u << 22, DIGIT_LOAD_KEYS = 1u << 17;
 
 // Builds of the update kernel.
 enum UpdateVariant { UPDATE_LARGE, UPDATE_SMALL, UPDATE_VARIANTS };
@@ -2946,12 +2947,18 @@ gpma_status update_plan(gpma_graph *const *graphs, const uint64_t *off, uint32_t
     // not know its degrees yet, so hub rows crowd one bucket each, whose ranks
     // serialise on one counter before the digit passes run after all (15.3M
     // edges into an array of guards: 0.55 of 1.70 ms of sort). Without hubs the
-    // passes take about as long as the buckets would.
-    // So do they from about DIGIT_KEYS keys, whose records no longer stay in L2,
-    // where rows and columns have at most three digits each (one graph, R-MAT 21,
-    // buckets against six passes: 2M keys 133 and 166 us, 4M 267 and 269, 7M 479
-    // and 437, 10.5M 716 and 631). Many graphs: not measured, buckets.
-    const bool digits = n > slots || (k == 1 && n >= DIGIT_KEYS && graphs[0]->row_num <= 1u << 24);
+    // buckets are faster in smaller loads. Whole load, digit passes against
+    // buckets, uniform / a hub with 30 % of the keys: 20,000 keys 2,048 rows 531
+    // and 502 / 519 and 538 us; 150,000 keys 50,000 rows 757 and 752 / 763 and 816;
+    // 1.2M keys 994 and 985 / 977 and 1,230.
+    // From about DIGIT_KEYS keys, whose records no longer stay in L2, the passes
+    // take as long as the buckets where rows and columns have at most three digits
+    // each (sort, one graph, R-MAT 21, buckets against six passes: 2M keys 133 and
+    // 166 us, 4M 267 and 269, 7M 479 and 437, 10.5M 716 and 631). Many graphs keep
+    // the buckets, though the passes would not be slower either (16 graphs of 300,000
+    // keys 304 and 304, 64 of 100,000 408 and 291, 8 of 1.2M 639 and 604).
+    const bool digits = (n > slots && n >= DIGIT_LOAD_KEYS) ||
+                        (k == 1 && n >= DIGIT_KEYS && graphs[0]->row_num <= 1u << 24);
     const bool buckets = g_tuning.update_sort == 0 && (uint32_t)grid <= BSORT_MAX_GRID && !digits;
     uint64_t nq = 0;
     h_qoff[0] = h_qtoff[0] = 0;

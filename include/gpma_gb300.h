@@ -480,8 +480,9 @@ typedef struct gpma_tuning {
     uint32_t update_sort;          /* batch sort inside the update kernel: 0 buckets (equal slot ranges of the
                                       array, a key placed by its row's slots) ranked, scattered and sorted in
                                       shared memory, with the digit passes taken when one bucket holds more than
-                                      1024 keys, for loads (more keys than slots) and for one
-                                      graph's batches of 4M keys and more; 1 digit passes always */
+                                      1024 keys, for loads (more keys than slots) of 131,072
+                                      keys and more and for one graph's batches of 4M keys
+                                      and more; 1 digit passes always */
     uint32_t reserved[2];
 } gpma_tuning;
 GPMA_API gpma_status gpma_get_tuning(gpma_tuning *out);
