@@ -72,13 +72,14 @@ constexpr uint32_t STEP_SLOTS = 32 * LANE_SLOTS;
 // Slots of one work item: a step of a warp. A word's rows hold 20 slots per
 // frontier node on average, up to hundreds of thousands with a hub; walked by
 // the warp that owns the word (its long rows apart), warps spent 40 % of their
-// time waiting at the level's barrier. Social graph, kernel: 344 us with items
-// of one step, 360 with two (a warp reads its next item's rows one item ahead).
+// time waiting at the level's barrier. Social graph, 2^25 slots: 358 us with items
+// of one step, 445 with four (a warp reads its next item's rows one item ahead).
 // Arrays of LARGE_SLOTS slots and more have work for every warp at four steps an
-// item, and each item costs the offsets of its word's 32 rows again (R-MAT,
-// edge factor 32, items of 1 / 2 / 4 / 8 steps: scale 21, 2^27 slots, 511 / 481 /
-// 481 / 500 us; scale 24, 2^30 slots, 3651 / 3316 / 3180 / 3091; at 2^26 slots 302
-// / 287 / 287). A build of its own, so that the smaller one keeps its single step.
+// item, and each item costs the offsets of its word's 32 rows again (R-MAT, items of
+// 1 / 2 / 4 / 8 steps: scale 21, 2^27 slots, 511 / 481 / 481 / 500 us; scale 24, 2^30
+// slots, 3651 / 3316 / 3180 / 3091). Below, one step: scale 20, 2^26 slots, 308 and
+// 308 with four, 2^25 slots 228 and 243. A build of its own, so that the smaller one
+// keeps its single step.
 constexpr uint32_t ITEM_SLOTS = STEP_SLOTS;
 constexpr uint32_t LARGE_ITEM_SLOTS = 4 * STEP_SLOTS;
 constexpr uint32_t LARGE_SLOTS = 1u << 27;
