@@ -213,6 +213,10 @@ struct BatchBuffers {
 };
 // two batch buffers, two window lists, leaf, insertions, their leaves and graphs
 constexpr uint64_t SLAB_BYTES_PER_KEY = 2 * (8 + 1) + 2 * 16 + 4 + (8 + 1) + 2 * 4;
+// ... and what an update launch has beside them: bucket counts and places (12 bytes
+// per 16 keys) and item bounds (4 per 1,024), look-back words of the digit passes
+// (8 passes x 256 digits x 4 bytes per tile of 2,048 keys or more)
+constexpr uint64_t UPDATE_BYTES_PER_KEY = SLAB_BYTES_PER_KEY + 1 + 4;
 constexpr uint32_t BFS_MAPS = 4;  // node bitmaps of a single-source BFS
 constexpr size_t STAT_GS_OFFSET = 128;
 static_assert(sizeof(DeviceStatus) <= STAT_GS_OFFSET, "status slot layout");

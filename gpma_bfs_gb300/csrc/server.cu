@@ -300,8 +300,8 @@ gpma_status gpma_server_create(const gpma_server_config *cfg, void *stream, gpma
     s->cfg = *cfg;
     s->plan_only = (cfg->flags & GPMA_SERVER_PLAN_ONLY) != 0;
     s->stream = (cudaStream_t)stream;
-    // each lane's round update buffers (about 120 bytes per key) are charged up front
-    s->fixed_bytes = 120ull * cfg->max_round_keys * lanes;
+    // each lane's round update buffers are charged up front
+    s->fixed_bytes = UPDATE_BYTES_PER_KEY * cfg->max_round_keys * lanes;
     if (s->fixed_bytes > cfg->hbm_budget_bytes) {
         delete s;
         set_error("gpma_server_create: round buffers for %llu keys exceed the budget",

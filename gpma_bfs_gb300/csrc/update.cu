@@ -2633,6 +2633,9 @@ GraphDesc describe(const gpma_graph *g) {
     return d;
 }
 
+static_assert(SORT_TILE * UPDATE_BYTES_PER_KEY >= SORT_TILE * (SLAB_BYTES_PER_KEY + 1) + 8 * 256 * sizeof(uint32_t),
+              "look-back words of a tile exceed the charge for its keys");
+
 // One graph's batches of this many keys are sorted by digit passes, and loads of
 // this many.
 constexpr uint64_t DIGIT_KEYS = 1u << 22, DIGIT_LOAD_KEYS = 1u << 17;
