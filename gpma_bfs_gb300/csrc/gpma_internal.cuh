@@ -168,7 +168,6 @@ struct BatchBuffers {
     uint32_t *wlive = nullptr;
     uint64_t *top = nullptr;    // one graph: its top-of-tree heads, gathered per launch for the locate cache
     // sort state
-    uint32_t *sort_tiles = nullptr;    // 8 tile counters
     uint32_t *sort_status = nullptr;   // look-back words, 8 x tiles x 256
     uint64_t sort_status_cap = 0;
     uint32_t *sort_hist = nullptr;     // [graph][8][256] digit counts

@@ -89,7 +89,6 @@ struct UpdateArgs {
     uint64_t *bk[2];        // batches, ping-pong buffers of the sort
     uint8_t *bv[2];
     uint32_t *sort_hist;    // [G + 1][8][256] digit counts (zeroed per update)
-    uint32_t *sort_tiles;   // 8 tile counters (zeroed per update)
     uint32_t *sort_status;  // look-back words, 8 x tiles x 256 (zeroed per update)
     BucketSort q;           // bucket sort state (q.nq == 0: digit passes only)
     uint32_t *leaf;
@@ -1336,8 +1335,6 @@ __global__ void __launch_bounds__(BLOCK, 2) update_kernel(UpdateArgs A) {
                 A.sort_status[i] = 0;
             for (uint32_t i = gt; i < A.q.nq; i += nt)
                 A.q.qcnt[i] = 0;
-            if (gt < 8)
-                A.sort_tiles[gt] = 0;
             for (uint32_t i = gt; i < A.next_slot_words; i += nt)
                 A.next_slot[i] = 0;
         }
@@ -2764,7 +2761,6 @@ gpma_status ensure_scratch(gpma_graph *g, uint32_t slots) {
 
 void free_buffers(BatchBuffers &b) {
     dev_free(b.slab);
-    dev_free(b.sort_tiles);
     dev_free(b.top);
     dev_free(b.sort_status);
     dev_free(b.sort_hist);
@@ -2796,10 +2792,6 @@ void free_buffers(BatchBuffers &b) {
 }
 
 gpma_status ensure_buffers(BatchBuffers &b, uint64_t n, uint32_t graphs) {
-    if (!b.sort_tiles) {
-        GPMA_TRY(dev_alloc(&b.sort_tiles, 8));
-        b.dirty = true;
-    }
     if (!b.top)
         GPMA_TRY(dev_alloc(&b.top, LOCATE_CACHE));
     if (n > b.cap || !b.slab) {
@@ -3046,7 +3038,6 @@ gpma_status update_plan(gpma_graph *const *graphs, const uint64_t *off, uint32_t
         A.wb[i] = buf.wb[i];
     }
     A.sort_hist = buf.sort_hist;
-    A.sort_tiles = buf.sort_tiles;
     A.sort_status = buf.sort_status;
     if (use_buckets) {
         A.q.qoff = buf.qoff;
@@ -3090,7 +3081,6 @@ gpma_status update_clear(BatchBuffers &buf, cudaStream_t s) {
     // kernel otherwise leaves zeroed for its successor
     GPMA_CUDA(cudaMemsetAsync(buf.d_stat, 0, 2 * buf.stat_slot, s));
     GPMA_CUDA(cudaMemsetAsync(buf.sort_hist, 0, sizeof(uint32_t) * buf.hist_cap * 2048, s));
-    GPMA_CUDA(cudaMemsetAsync(buf.sort_tiles, 0, 8 * sizeof(uint32_t), s));
     GPMA_CUDA(cudaMemsetAsync(buf.sort_status, 0, buf.sort_status_cap * sizeof(uint32_t), s));
     if (buf.q_cap)
         GPMA_CUDA(cudaMemsetAsync(buf.qcnt, 0, buf.q_cap * sizeof(uint32_t), s));
