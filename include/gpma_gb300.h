@@ -92,7 +92,10 @@ GPMA_API gpma_status gpma_update(gpma_graph *g, const uint64_t *keys, const uint
  * results) (gpma_bfs.cuh:511-515). levels (host or device, row_num entries)
  * receives the BFS level of every node: 1 for src, L+1 for a neighbour of a
  * level-L node, 0 for unreached. reached (optional, host) receives the
- * number of non-zero levels. */
+ * number of non-zero levels. The kernels write levels in place where it is
+ * memory of the graph's GPU: a search that fails on the device (GPMA_ERR_TIMEOUT,
+ * GPMA_ERR_DEVICE) may leave such an array partly written, other memory as it
+ * was. The same holds for the levels of every other search below. */
 GPMA_API gpma_status gpma_bfs(gpma_graph *g, uint32_t src, uint32_t *levels, uint64_t *reached, void *stream);
 
 /* Multi-source BFS: k (1..64) independent searches in one traversal, one bit
@@ -124,8 +127,10 @@ GPMA_API gpma_status gpma_bfs_noalloc(gpma_graph *g, uint32_t src, uint32_t *lev
  * One slide step of the reference's demo loop (gpma_bfs_demo.cu: update_gpma
  * of the step's batch, then gpma_bfs from a source) whose device work is
  * recorded once as a CUDA graph and replayed for every later step: table
- * upload, update kernel, BFS clears and kernels, status read-back, one host
- * synchronisation. The graph is rebuilt only when a buffer or the launch
+ * upload, update kernel, BFS kernel, status read-back, one host
+ * synchronisation. (A step whose update needs the host, a root resize or a bulk
+ * rebuild, runs its BFS after that; a search of more than 64 levels ends in a
+ * launch of its own.) The graph is rebuilt only when a buffer or the launch
  * shape it holds changes; batch size and source may differ per step.
  * gpma_step_run gives exactly the results of gpma_update(keys, values, n)
  * followed by gpma_bfs(src, levels, reached) (levels may be NULL: the levels
