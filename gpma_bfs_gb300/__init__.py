@@ -580,7 +580,7 @@ TEST_HOOK_FIELDS = ("update_stall", "bfs_stall", "wait_limit_us", "noalloc_chunk
 
 def get_test_hooks() -> dict:
     """Error-path test hooks in effect, plus noalloc_overflows: how often the
-    last gpma_bfs_noalloc call found its long-row chunk list full."""
+    last gpma_bfs_noalloc call found its list of work items full."""
     h = _TestHooks()
     _check(lib().gpma_get_test_hooks(ctypes.byref(h)), "gpma_get_test_hooks")
     return {n: getattr(h, n) for n in TEST_HOOK_FIELDS + ("noalloc_overflows",)}
@@ -590,7 +590,7 @@ def set_test_hooks(**values) -> dict:
     """Changes some test-hook fields (update_stall / bfs_stall: the next
     launches' first grid barrier waits for an arrival that never comes and
     gives up after wait_limit_us; noalloc_chunk_cap: entries of the
-    no-allocation BFS's chunk list); returns the previous settings."""
+    no-allocation BFS's list of work items); returns the previous settings."""
     old = get_test_hooks()
     unknown = set(values) - set(TEST_HOOK_FIELDS)
     if unknown:

@@ -2,8 +2,8 @@
 //
 // No reference counterpart: the reference's only analytic is the BFS
 // (gpma_bfs.cuh); GPMA+'s setting also covers connected components and
-// PageRank. Both run as persistent cooperative kernels whose hot loop is one
-// coalesced sweep over every slot of the array (16-byte key loads, 8 slots
+// PageRank. Both run as persistent cooperative kernels that read the edges in
+// coalesced sweeps over every slot of the array (16-byte key loads, 8 slots
 // per thread): a slot is an edge u -> v when its value is non-zero and its
 // column is not 0xFFFFFFFF (the BFS's rule), with u = key >> 32 and
 // v = low word, both < row_num. No in-edge index is kept between calls.
@@ -18,9 +18,10 @@
 // Weakly connected components: parents start as the node ids; an edge links
 // its endpoints' trees by hooking the larger root under the smaller (a
 // compare-and-swap retried from the parents it found), so one sweep over the
-// edges finishes the components. A first pass links the edges in the first few
-// slots of every row and flattens the trees; the sweep then finds most
-// endpoints with equal parents and only reads. Parents only decrease and stay
+// edges finishes the components. Before it, passes over the first few slots of
+// every row link some edges and flatten the trees; the sweep then finds most
+// endpoints with equal parents and only reads (linking and sampling as in
+// Afforest: Sutton, Ben-Nun and Barak, 2018). Parents only decrease and stay
 // inside their component, so each node ends labelled with the smallest node id
 // of its component, whatever the order of the atomics.
 #include "gpma_internal.cuh"
@@ -290,10 +291,10 @@ struct PrNode {
 
 // PageRank with the in-edges of the array's current edges laid out once per
 // call (counts, a grid-wide scan, one scatter of source ids), so that an
-// iteration gathers contributions and writes each rank once instead of one
-// float atomic per edge (198 us per iteration). Bound by the 4-byte gathers of
-// the contributions (L2). 20 iterations on the social graph: 4.37 ms -> 1.99 ms
-// per call, 0.44 of it the layout.
+// iteration gathers contributions and writes each rank once (one float atomic
+// per edge takes 198 us per iteration). Bound by the 4-byte gathers of the
+// contributions (L2). 20 iterations on the social graph: 1.99 ms per call, 0.44 of
+// it the layout; 4.37 by atomics.
 // TOL (a tolerance is given): the iterations are not known beforehand. The call begins
 // with iterations by atomics, and lays out the in-edges after the first one from which
 // PR_GATHER_ITERATIONS more are to be expected: R-MAT 18, tolerance 0.5 (2 iterations)
@@ -653,11 +654,11 @@ __device__ __forceinline__ void cc_sample(const AnArgs &A, uint32_t which, uint3
 }
 
 // Bound by the 4-byte parent gathers of the edges' targets (L2) beside one
-// read of the array. Hooking parents found once per round took three sweeps
-// with an atomicMin per edge in the first: 2.11 ms on 15.3M edges, 1.6M nodes
-// (33.5M slots); linking to completion takes one sweep, and few of its edges
+// read of the array. Linking to completion takes one sweep, and few of its edges
 // link anything after the sampled passes, whose trees are flattened after each
-// so that the next pass finds roots with one read: 0.22 ms.
+// so that the next pass finds roots with one read: 0.22 ms on 15.3M edges, 1.6M
+// nodes (33.5M slots). Hooking parents found once per round takes three sweeps with
+// an atomicMin per edge in the first: 2.11 ms.
 __global__ void __launch_bounds__(BLOCK) components_kernel(AnArgs A) {
     GridBarrier *bar = reinterpret_cast<GridBarrier *>(A.ctl + AN_BAR);
     uint32_t *err = A.ctl + AN_ERR;

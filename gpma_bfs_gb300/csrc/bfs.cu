@@ -9,7 +9,8 @@
 // from level L gets L+1.
 //
 // Single source: one persistent cooperative kernel runs every level,
-// separated by bounded grid barriers. Node sets are bitmaps (no queue, no queue
+// separated by bounded grid barriers (a second one goes on after LONG_LEVELS
+// levels). Node sets are bitmaps (no queue, no queue
 // atomics): seen (every node reached, the only one that searching threads
 // write), done (those that have their level) and front (the level's frontier).
 // Per level,
@@ -258,14 +259,13 @@ __device__ __forceinline__ void report(const BfsArgs &A, uint32_t levels, uint32
     reinterpret_cast<GridBarrier *>(A.ctl + CTL_BAR)->count = 0;
 }
 
-// Social graph (1.6M nodes, 15.3M edges, 33.5M slots), 13 levels: 344 us, 374
-// before with claims of three L2 operations (two bitmaps and the level), counts
-// and chunk lists by one atomic per warp and a phase of its own for long rows.
-// The walks of the middle levels (a key, a value and a seen word per slot; the
-// largest moves about 230 MB in 52 us) are 185 us of it, the rest the scans and
-// two grid barriers per level. More slots per lane, fewer registers for more
-// warps, slots read an item ahead and runs of 2 or 4 slots per lane all
-// measured within 4 % of this or slower.
+// Social graph (1.6M nodes, 15.3M edges, 33.5M slots), a search of 18 levels: 358 us
+// (374 with claims of three L2 operations, two bitmaps and the level). The walks of
+// the middle levels (a key, a value and a seen word per slot; the largest moves about
+// 230 MB) are 190 us of it, the rest the scans and two grid barriers per level. More
+// slots per lane, fewer registers for more warps, slots read an item ahead and runs
+// of 2 or 4 slots per lane all measured within 4 % of this or slower, and so do
+// builds that differ in little but the compiler's schedule.
 template <uint32_t ITEM>
 __global__ void __launch_bounds__(BLOCK, 5) bfs_kernel(BfsArgs A) {
     __shared__ uint2 s_items[CTA_ITEMS];
@@ -487,12 +487,13 @@ __global__ void __launch_bounds__(BLOCK, 5) bfs_kernel(BfsArgs A) {
 
 // A search from level LONG_LEVELS on, over the maps that bfs_kernel left: levels of
 // few nodes end with one grid barrier instead of two (a 300 x 300 grid, 599 levels:
-// 8.4 us per level with two, 5.8 with one). A short level claims nodes in a bitmap of
+// 8.4 us per level with two, 5.5 with one). A short level claims nodes in a bitmap of
 // the level's parity, which the next level's scan adds to seen, so that a CTA can
 // walk its items while others still scan; items beyond SHORT_ITEMS go to the grid's
 // list for a walk behind the barrier, and where no CTA has any the level is done.
-// A kernel of its own, since bfs_kernel is 3 to 15 % slower on the social graph with
-// any of this inside. (No dense levels here: they would be the same.)
+// A kernel of its own, since bfs_kernel is up to 15 % slower on the social graph with
+// any of this inside. (No dense levels here: they would be the same.) Three CTAs per
+// SM: 72 registers without spills, and a cheaper barrier.
 template <uint32_t ITEM>
 __global__ void __launch_bounds__(BLOCK, LONG_CTAS_PER_SM) bfs_long_kernel(BfsArgs A) {
     __shared__ uint2 s_items[CTA_ITEMS];

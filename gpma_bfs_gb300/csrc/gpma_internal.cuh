@@ -73,12 +73,12 @@ constexpr uint64_t WAIT_LIMIT_NS = 2000000000ull;
 
 // Test hooks (process-wide, gpma_set_test_hooks): make one bounded wait run
 // out on purpose so its error path runs on a GPU without hanging it, and
-// shrink the no-allocation BFS's chunk list so its full-list branch runs.
+// shrink the no-allocation BFS's item list so its full-list branch runs.
 struct TestHooks {
     uint32_t update_stall = 0;         // 1: the update kernel's first grid barrier waits for one arrival too many
     uint32_t bfs_stall = 0;            // 1: the BFS kernel's first grid barrier does the same
     uint64_t wait_limit_ns = WAIT_LIMIT_NS;  // limit of those two waits
-    uint32_t noalloc_chunk_cap = 0;    // gpma_bfs_noalloc chunk-list entries (0: all it has)
+    uint32_t noalloc_chunk_cap = 0;    // gpma_bfs_noalloc item-list entries (0: all it has)
     uint32_t noalloc_overflows = 0;    // full-list events of the last gpma_bfs_noalloc call (written by it)
 };
 extern TestHooks g_test_hooks;
@@ -253,7 +253,7 @@ struct gpma_graph {
     bool bfs_dirty = true;             // bfs_ctl must be cleared before the next launch
     int bfs_grid = 0;                  // resident BFS-kernel CTAs per SM (0: not yet known)
     gpma_batch *own_batch = nullptr;   // multi-source BFS context of this graph
-    uint32_t *an_buf = nullptr;        // analytics: 4 x row_num words + control words, kept between calls
+    uint32_t *an_buf = nullptr;        // analytics: 5 x row_num words, CTA and control words, kept between calls
     uint32_t an_cap = 0;               // row_num it was sized for
     gpma_stats stats{};
     // profiling: events on the caller's stream around each phase

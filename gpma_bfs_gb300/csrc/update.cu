@@ -196,10 +196,10 @@ __device__ __forceinline__ uint32_t locate_keys(const UpdateArgs &A, uint32_t g,
         value[j] = i < end ? bv[i] : 0;
     }
     // the reference's descent (gpma.cuh:209-216), the keys level by level
-    // together, the level the same for all (a level per key, looked up with
-    // its graph, took 25 us on the social slide, this 20). Every probed slot starts a segment (prefix and bit are
-    // multiples of seg), so below the cached levels its key is read from the
-    // dense heads array.
+    // together, the level the same for all (social slide 20 us; 25 with a level
+    // per key, looked up with its graph). Every probed slot starts a segment
+    // (prefix and bit are multiples of seg), so below the cached levels its key
+    // is read from the dense heads array.
     const uint32_t seg = D.seg, log2seg = D.log2seg;
     const uint64_t *heads = D.heads;
     uint32_t bit = (seg << D.height) >> 1;
@@ -1628,9 +1628,10 @@ __global__ void __launch_bounds__(BLOCK, 2) update_kernel(UpdateArgs A) {
         // A level that accepted nothing leaves every insertion where it is: the
         // compaction would copy the buffer onto itself, and where few windows
         // hold most insertions (a load of a skewed graph, whose windows are all
-        // too full up to the root), through the few CTAs that own them: 0.75M
-        // edges into 100,000 rows spent 8.0 ms in 14 levels, 0.16 now. One
-        // graph's root window likewise hands its range to the host in place.
+        // too full up to the root), through the few CTAs that own them: 14
+        // levels of 0.75M edges into 100,000 rows take 0.16 ms in place, 8.0
+        // copied. One graph's root window likewise hands its range to the host
+        // in place.
         const bool keep = total_i == s_pending;
         const bool in_place = keep || (A.G == 1 && level >= A.gd[0].height);
         // GROUP_ITEMS consecutive windows per thread per round; the rejected
@@ -1639,7 +1640,6 @@ __global__ void __launch_bounds__(BLOCK, 2) update_kernel(UpdateArgs A) {
         // (the next level's buffer, or the remaining buffer for a root
         // window) and the exclusive prefix of the counts, so the whole CTA
         // copies the concatenated ranges (a window of a million insertions is
-        // not left to one warp)
         // not left to one warp). A window whose left sibling ends the previous
         // CTA's range has its insertions copied by that CTA, which writes the
         // parent window: every next-level window's insertions come from the
@@ -2388,9 +2388,8 @@ __global__ void compacted_layout_kernel(uint64_t *keys, uint8_t *vals, uint64_t 
 // gaps) or, where that many do not fit the root's density (dropped), the two
 // KEY_MAX entries alone at the front. The guards are in key order as they are
 // numbered, so every slot is written from its index: one pass of coalesced
-// 16-byte stores. Before, the guards went through the batch update, whose sort
-// finds them all in one bucket (1.6M atomics on one word, 7.1 ms for 1,632,803
-// rows); creating that graph and loading 15.3M edges went from 16.2 to 7.2 ms.
+// 16-byte stores. (As a batch update the sort finds all guards in one bucket, 1.6M
+// atomics on one word for 1,632,803 rows: 7.1 ms in place of 3 us.)
 __global__ void guard_layout_kernel(uint64_t *keys, uint8_t *vals, uint64_t *heads, uint32_t *row_offset,
                                     uint32_t row_num, uint32_t size, uint32_t log2seg, uint32_t log2F,
                                     uint64_t gap_key, bool dropped) {
