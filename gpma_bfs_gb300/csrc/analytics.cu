@@ -768,8 +768,9 @@ gpma_status an_buffers(gpma_graph *g, uint32_t **base, uint32_t **ctl) {
     return GPMA_OK;
 }
 
-// Arrays of 8 slots or more are a whole number of the sweeps' slot groups.
-constexpr uint32_t PR_GATHER_MIN_SLOTS = 1024;
+// The gathering's sweeps take whole groups of 8 slots. It pays in the smallest arrays
+// too (256 slots, 4 / 20 iterations: 90 / 250 us, by atomics 114 / 413).
+constexpr uint32_t PR_GATHER_MIN_SLOTS = 8;
 
 }  // namespace
 }  // namespace gpma

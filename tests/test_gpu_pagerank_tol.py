@@ -89,3 +89,17 @@ def test_a_tolerance_met_at_once_is_cheap(built_lib):
     # repeated edges are few, so the change is small, far below the tolerance
     assert best(iterations=100, tol=0.1) < 1.25 * best(iterations=1)
     g.close()
+
+
+@pytest.mark.parametrize("n", [1, 2, 3, 5, 9, 20, 40])
+def test_smallest_arrays(built_lib, n):
+    """Arrays of 4 to 128 slots, on both sides of the smallest that is gathered."""
+    rng = np.random.default_rng(n)
+    s, d = rng.integers(0, n, (2, 2 * n))
+    g, s, d = _graph(n, s, d)
+    ranks, _ = _power(n, s, d, 0.85, 12)
+    for its in (1, 3, 4, 12):
+        got, done = G.pagerank(g, 0.85, its)
+        assert done == its
+        np.testing.assert_allclose(got, ranks[its], rtol=2e-4, atol=1e-9)
+    g.close()
