@@ -178,6 +178,14 @@ constexpr int LOC_ILP = 4;
 // Consecutive items per thread in the grouping passes.
 constexpr uint32_t GROUP_ITEMS = 4;
 
+// Windows per CTA up to which a level of several graphs is fused. A CTA's range of
+// more windows of different graphs, and so widths, is uneven work; one by one round
+// the CTAs they are not. Levels of a launch, 256 graphs with 5.3M keys / 64 with
+// 1.3M / 64 with 0.46M: 923 / 320 / 177 us fused whatever their number, 512 / 212 /
+// 144 with 160 windows, 535 / 212 / 179 with 640, 496 / 206 / 143 with 30; with none
+// 498 / 232 / 178.
+constexpr uint32_t FUSED_WINDOWS = 160;
+
 // Keys i0 + j * stride (j < LOC_ILP) below `end`, all of graph g; returns how
 // many of them are insertions (leaf set). fk: the heads at every 2^log2stride
 // slots, in shared memory.
@@ -1525,10 +1533,12 @@ __global__ void __launch_bounds__(BLOCK, 2) update_kernel(UpdateArgs A) {
         // windows of at most CTA_WINDOW_MAX slots in every graph: each CTA
         // dispatches a contiguous range of the windows and counts its rejected
         // ones right away, so the level needs one grid barrier fewer (two, where
-        // the next one is such a level too). 20 graphs, 0.35M keys: levels
-        // 169 -> 82 us with this and the runs' bounds found by warps.
+        // the next one is such a level too).
         const uint32_t max_seg = A.gd[A.G - 1].seg;  // graphs are ordered by segment length
-        const bool fused = (max_seg << level) <= CTA_WINDOW_MAX;
+        auto can_fuse = [&](uint32_t lv, uint32_t windows) {
+            return (max_seg << lv) <= CTA_WINDOW_MAX && (A.G == 1 || windows <= FUSED_WINDOWS * gridDim.x);
+        };
+        const bool fused = can_fuse(level, nw);
         Windows L;
         L.node = (cur & 1) ? A.wnode[1] : A.wnode[0];
         L.graph = (cur & 1) ? A.wgraph[1] : A.wgraph[0];
@@ -1762,7 +1772,7 @@ __global__ void __launch_bounds__(BLOCK, 2) update_kernel(UpdateArgs A) {
         // this level's barrier. The window flags alternate by level, so a CTA
         // flagging the next level's windows does not overwrite ones a slower
         // CTA still reads here.
-        own = fused && nw_next > 0 && level + 1 <= A.max_height && (max_seg << (level + 1)) <= CTA_WINDOW_MAX;
+        own = fused && nw_next > 0 && level + 1 <= A.max_height && can_fuse(level + 1, nw_next);
         if (own) {
             olo = next_lo;
             ohi = base;
