@@ -521,7 +521,7 @@ def run_analytics(G, g, n, stream):
     per_iter = sweep + 16.0 * n  # + degree, rank, contribution, accumulator traffic per node
     return {"pagerank": {"iterations": iters, "ms": pr_ms, "ms_per_iteration": pr_ms / iters,
                          "hbm_frac": per_iter * iters / (pr_ms * 1e-3) / 1e9 / peak,
-                         "note": "call time (CUDA events) incl. the initial ranks upload and the result copy; bytes = 9 B/slot + 16 B/node per iteration"},
+                         "note": "call time (CUDA events) incl. the in-edge layout and the result copy; bytes = 9 B/slot + 16 B/node per iteration"},
             "components": {"components": comps, "rounds": rounds, "ms": cc_ms,
                            "hbm_frac": sweep * (rounds + 1) / (cc_ms * 1e-3) / 1e9 / peak}}
 

@@ -897,6 +897,11 @@ gpma_status noalloc_scratch(uint32_t **out, int *grid, int sms) {
             return cuda_fail(e, "cudaGetSymbolAddress(g_noalloc_scratch)");
         int per_sm = 0;
         e = bfs_fit(&per_sm);
+        // a kernel is loaded when it is first used, which takes device memory: not in the middle of a later search
+        cudaFuncAttributes attr;
+        for (uint32_t size : {0u, LARGE_SLOTS})
+            if (e == cudaSuccess)
+                e = cudaFuncGetAttributes(&attr, bfs_kernel_ptr(size, true));
         if (e != cudaSuccess)
             return cuda_fail(e, "cudaOccupancyMaxActiveBlocksPerMultiprocessor(bfs_kernel)");
         if (per_sm < 1) {

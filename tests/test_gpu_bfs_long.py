@@ -2,6 +2,9 @@
 sides of that line, long thin graphs whose levels end with one barrier, levels too
 large for that in between, through every call that searches one graph."""
 import ctypes
+import subprocess
+import sys
+from pathlib import Path
 
 import numpy as np
 import pytest
@@ -88,6 +91,32 @@ def test_without_allocation(built_lib, cap):
     assert np.array_equal(levels.cpu().numpy(), want) and reached.value == n
     assert (overflows > 0) == (cap > 0)
     g.close()
+
+
+def test_first_long_search_without_allocation_takes_no_memory():
+    """In a process of its own: the second kernel is loaded by the first call, not
+    by the first search that needs it."""
+    code = """
+import ctypes, numpy as np, torch
+import gpma_bfs_gb300 as G
+n = 300
+u = np.arange(n - 1, dtype=np.uint64)
+g = G.GPMA(n)
+G.update_gpma(g, (u << np.uint64(32)) | (u + np.uint64(1)), np.ones(n - 1, np.uint8))
+levels = torch.zeros(n, dtype=torch.int32, device="cuda")
+def search(s):
+    r = ctypes.c_uint64()
+    assert G.lib().gpma_bfs_noalloc(g.handle, s, ctypes.c_void_p(levels.data_ptr()), ctypes.byref(r), None) == 0
+    torch.cuda.synchronize()
+    return r.value
+assert search(n - 5) == 5
+free = torch.cuda.mem_get_info()[0]
+assert search(0) == n
+assert torch.cuda.mem_get_info()[0] == free, free - torch.cuda.mem_get_info()[0]
+"""
+    r = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, timeout=300,
+                       cwd=Path(__file__).resolve().parent.parent)
+    assert r.returncode == 0, r.stderr[-2000:]
 
 
 def test_recorded_step(built_lib):
