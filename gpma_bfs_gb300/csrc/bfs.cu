@@ -73,8 +73,8 @@ constexpr uint32_t STEP_SLOTS = 32 * LANE_SLOTS;
 // Slots of one work item: a step of a warp. A word's rows hold 20 slots per
 // frontier node on average, up to hundreds of thousands with a hub; walked by
 // the warp that owns the word (its long rows apart), warps spent 40 % of their
-// time waiting at the level's barrier. Social graph, 2^25 slots: 358 us with items
-// of one step, 445 with four (a warp reads its next item's rows one item ahead).
+// time waiting at the level's barrier. Social graph, 2^25 slots: 350 us with items
+// of one step, about 445 with four (a warp reads its next item's rows one item ahead).
 // Arrays of LARGE_SLOTS slots and more have work for every warp at four steps an
 // item, and each item costs the offsets of its word's 32 rows again (R-MAT, items of
 // 1 / 2 / 4 / 8 steps: scale 21, 2^27 slots, 511 / 481 / 481 / 500 us; scale 24, 2^30
@@ -93,7 +93,8 @@ inline uint64_t bfs_item_need(uint32_t n, uint32_t size) {
 // word, all on one counter, serialises at 4.4 ns apiece.)
 constexpr uint32_t CTA_ITEMS = 1024;
 
-// bfs_long_kernel takes over after so many levels; a level of it is short when the
+// bfs_long_kernel takes over at this level (counted from 0), which bfs_kernel has
+// scanned and not walked; a level of it is short when the
 // one before had at most SHORT_NODES nodes per CTA, and a CTA then walks its first
 // SHORT_ITEMS items before the barrier.
 constexpr uint32_t LONG_LEVELS = 64;
@@ -134,15 +135,14 @@ __device__ __forceinline__ void visit_slots(const BfsArgs &A, const uint32_t (&s
     uint32_t w[N], seen[N];
 #pragma unroll
     for (uint32_t j = 0; j < N; ++j) {
-        // only the target, the low word of the key
-        uint32_t k = 0xFFFFFFFFu;
+        uint64_t k = KEY_NONE;
         uint8_t v = 0;
         if (sl[j] != SIZE_NONE) {
-            k = reinterpret_cast<const uint32_t *>(A.keys)[2 * (size_t)sl[j]];
+            k = A.keys[sl[j]];
             v = A.vals[sl[j]];
         }
-        w[j] = k;
-        seen[j] = (v != 0 && k < A.n) ? 0u : 0xFFFFFFFFu;
+        w[j] = (uint32_t)k;
+        seen[j] = (w[j] != 0xFFFFFFFFu && v != 0 && w[j] < A.n) ? 0u : 0xFFFFFFFFu;
     }
 #pragma unroll
     for (uint32_t j = 0; j < N; ++j)
@@ -259,13 +259,14 @@ __device__ __forceinline__ void report(const BfsArgs &A, uint32_t levels, uint32
     reinterpret_cast<GridBarrier *>(A.ctl + CTL_BAR)->count = 0;
 }
 
-// Social graph (1.6M nodes, 15.3M edges, 33.5M slots), a search of 18 levels: 358 us
+// Social graph (1.6M nodes, 15.3M edges, 33.5M slots), a search of 18 levels: 350 us
 // (374 with claims of three L2 operations, two bitmaps and the level). The walks of
 // the middle levels (a key, a value and a seen word per slot; the largest moves about
 // 230 MB) are 190 us of it, the rest the scans and two grid barriers per level. More
 // slots per lane, fewer registers for more warps, slots read an item ahead and runs
-// of 2 or 4 slots per lane all measured within 4 % of this or slower, and so do
-// builds that differ in little but the compiler's schedule.
+// of 2 or 4 slots per lane all measured within 4 % of this or slower. The compiler's
+// schedule of the walk hangs on little: with the limit of levels in the loop's head
+// the same search takes 361 us, and one of 2^28 slots 909 in place of 823.
 template <uint32_t ITEM>
 __global__ void __launch_bounds__(BLOCK, 5) bfs_kernel(BfsArgs A) {
     __shared__ uint2 s_items[CTA_ITEMS];
@@ -294,7 +295,7 @@ __global__ void __launch_bounds__(BLOCK, 5) bfs_kernel(BfsArgs A) {
         return;
     uint32_t reached = 0;
     uint32_t i = 0;
-    for (; i < LONG_LEVELS; ++i) {
+    for (;; ++i) {
         const bool stamper = A.stamps && gtid == 0 && i < CTL_PROFILE_LEVELS;
         if (stamper)
             A.stamps[i] = globaltimer_ns();
@@ -408,7 +409,7 @@ __global__ void __launch_bounds__(BLOCK, 5) bfs_kernel(BfsArgs A) {
         if (!grid_barrier(bar, err))
             return;
         const uint32_t frontier = cta_broadcast_read(A.ctl + CTL_CNT + i % 3);
-        if (frontier == 0)
+        if (frontier == 0 || i == LONG_LEVELS)  // done, or bfs_long_kernel's, whose nodes are in front
             break;
         if (gtid == 0) {
             A.ctl[CTL_CNT + (i + 1) % 3] = 0;
@@ -485,7 +486,8 @@ __global__ void __launch_bounds__(BLOCK, 5) bfs_kernel(BfsArgs A) {
     report(A, i, s_at);
 }
 
-// A search from level LONG_LEVELS on, over the maps that bfs_kernel left: levels of
+// A search from the walk of level LONG_LEVELS on, over the maps that bfs_kernel left
+// (that level's frontier is in front, and has its levels and counts): levels of
 // few nodes end with one grid barrier instead of two (a 300 x 300 grid, 599 levels:
 // 8.4 us per level with two, 5.5 with one). A short level claims nodes in a bitmap of
 // the level's parity, which the next level's scan adds to seen, so that a CTA can
@@ -527,7 +529,9 @@ __global__ void __launch_bounds__(BLOCK, LONG_CTAS_PER_SM) bfs_long_kernel(BfsAr
         for (uint32_t it = 0; gwarp + it * nwarps < words; it += 32) {
             const uint32_t w0 = gwarp + it * nwarps, wl = w0 + lane * nwarps;
             uint32_t mine = 0;
-            if (wl < words) {
+            if (wl < words && i == LONG_LEVELS) {
+                mine = A.front[wl];  // scanned and counted by bfs_kernel
+            } else if (wl < words) {
                 uint32_t s = A.seen[wl];
                 if (brief) {
                     // what the short level before claimed; only this lane has the word
@@ -637,7 +641,7 @@ __global__ void __launch_bounds__(BLOCK, LONG_CTAS_PER_SM) bfs_long_kernel(BfsAr
         frontier = cta_broadcast_read(A.ctl + CTL_CNT + i % 3);
         if (frontier == 0)
             break;
-        reached += frontier;
+        reached += i == LONG_LEVELS ? 0u : frontier;
         if (gtid == 0) {
             // read last before this barrier, added to after the next one
             A.ctl[CTL_CNT + (i + 2) % 3] = 0;
@@ -725,6 +729,11 @@ void fill_maps(BfsArgs &A, uint32_t *maps, size_t words) {
     A.over = maps + 3 * words;
 }
 
+// Whether a launch ended at LONG_LEVELS with a frontier left to walk.
+bool long_search(const uint32_t *h_ctl) {
+    return h_ctl[CTL_LEVELS] == LONG_LEVELS && h_ctl[CTL_CNT + LONG_LEVELS % 3] != 0;
+}
+
 // The launch that goes on with a search after LONG_LEVELS levels, from its
 // arguments and two more maps; the control words are zero.
 cudaError_t launch_long(BfsArgs A, uint32_t *maps, size_t words, int sms, int per_sm, cudaStream_t s) {
@@ -807,7 +816,7 @@ gpma_status bfs_begin(gpma_graph *g, cudaStream_t s) {
 
 gpma_status bfs_finish(gpma_graph *g, const BfsPlan &P, cudaStream_t s, uint64_t *reached) {
     uint32_t before = 0;  // nodes reached by the first launch of a long search
-    if (g->h_bfs_ctl[CTL_ERR] == 0 && g->h_bfs_ctl[CTL_LEVELS] == LONG_LEVELS) {
+    if (g->h_bfs_ctl[CTL_ERR] == 0 && long_search(g->h_bfs_ctl)) {
         before = g->h_bfs_ctl[CTL_REACHED];
         BfsArgs A;
         memcpy(&A, P.main.args, sizeof(A));
@@ -954,7 +963,7 @@ gpma_status bfs_noalloc_run(gpma_graph *g, uint32_t src, uint32_t *levels, uint6
     uint32_t h_ctl[CTL_WORDS], before = 0;
     GPMA_CUDA(cudaMemcpyAsync(h_ctl, ctl, sizeof(h_ctl), cudaMemcpyDeviceToHost, s));
     GPMA_CUDA(cudaStreamSynchronize(s));
-    if (!h_ctl[CTL_ERR] && h_ctl[CTL_LEVELS] == LONG_LEVELS) {
+    if (!h_ctl[CTL_ERR] && long_search(h_ctl)) {
         before = h_ctl[CTL_REACHED];
         const uint32_t overflows = h_ctl[CTL_OVERFLOW];
         GPMA_CUDA(cudaMemsetAsync(ctl, 0, sizeof(uint32_t) * CTL_ALL, s));
